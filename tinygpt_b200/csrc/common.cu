@@ -89,6 +89,59 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, int64_t rows, int64_t 
   return B200_OK;
 }
 
+int make_tmap_sw128(CUtensorMap* out, int rank, const void* base, int64_t batch, int64_t rows, int64_t cols, int64_t batch_stride,
+                    int64_t row_stride, int box_rows) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc) {
+    set_error("cuTensorMapEncodeTiled is not available (no CUDA driver / device?)");
+    return B200_ERR_NO_DEVICE;
+  }
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
+  // one batch element: any stride that is a multiple of 16 bytes serves
+  cuuint64_t strides[2] = {(cuuint64_t)row_stride * 2, (cuuint64_t)(batch > 1 ? batch_stride : row_stride) * 2};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled(swizzle 128B) failed with CUresult %d (batch=%lld rows=%lld cols=%lld)", (int)r, (long long)batch,
+              (long long)rows, (long long)cols);
+    return B200_ERR_CUDA;
+  }
+  return B200_OK;
+}
+
+// One word of mapped host memory per process.  The allocation must not disturb a capture that may be running on this thread.
+int wait_word(unsigned** out) {
+  static unsigned* word = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+      word = static_cast<unsigned*>(p);
+      *word = 0;
+    } else {
+      (void)cudaGetLastError();
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  });
+  if (word == nullptr) {
+    set_error("no pinned host memory for the kernels' error word");
+    return B200_ERR_CUDA;
+  }
+  const unsigned code = *reinterpret_cast<volatile unsigned*>(word);
+  if (code != 0) {
+    *reinterpret_cast<volatile unsigned*>(word) = 0;
+    set_error("a kernel gave up waiting (code 0x%x): what it wrote is not valid", code);
+    return B200_ERR_CUDA;
+  }
+  *out = word;
+  return B200_OK;
+}
+
 const char* last_error();
 
 }  // namespace b200

@@ -24,7 +24,7 @@ void set_error(const char* fmt, ...);
 // cross-kernel L2 prefetch, whole-token persistent kernel) are not here any more: profiles/experiments/.
 struct Defaults {
   static constexpr bool kPrefillAttnMma = true;   // B200_PREFILL_ATTN   "mma" (tensor cores) | "cuda" (CUDA cores)
-  // B200_GEMM "persistent" | "tile": chosen per shape when unset (gemm.cu launch_gemm_bf16)
+  // B200_GEMM "persistent" | "tile": chosen per shape when unset (gemm.cu pick_gemm)
 };
 bool env_flag(const char* name, bool dflt);                       // unset → dflt; else first character == '1'
 bool env_choice(const char* name, char yes_initial, bool dflt);   // unset → dflt; else first character == yes_initial
@@ -126,6 +126,18 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&p);
 }
 
+// two bf16 at a time: the sum, and bf16(silu(g))·u, each rounded once per operation
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 r = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ float silu_f(float g) { return __fdividef(g, 1.f + expf(-g)); }
+__device__ __forceinline__ uint32_t silu_mul_bf16x2(uint32_t g, uint32_t u) {
+  const __nv_bfloat162 s = __floats2bfloat162_rn(silu_f(bf16_lo(g)), silu_f(bf16_hi(g)));
+  const __nv_bfloat162 r = __hmul2(s, *reinterpret_cast<const __nv_bfloat162*>(&u));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 // ---- programmatic dependent launch
@@ -202,6 +214,20 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
 }
 #endif  // __CUDACC__
 
+// every pointer lies on a 16-byte boundary (null does)
+template <typename... P>
+inline bool aligned16(P... p) {
+  return ((reinterpret_cast<uintptr_t>(static_cast<const void*>(p)) | ...) & 15) == 0;
+}
+
+// Word (mapped host memory) in which a kernel whose bounded wait gives up leaves a code; the next launch that asks for the word
+// reports it and fails.
+int wait_word(unsigned** out);
+
+// [batch, rows, cols] bf16 (rank 3, strides in elements) or [rows, cols] (rank 2: batch 1), with boxes of 64 columns × box_rows rows,
+// 128-byte swizzle; what lies outside is zero
+int make_tmap_sw128(CUtensorMap* out, int rank, const void* base, int64_t batch, int64_t rows, int64_t cols, int64_t batch_stride,
+                    int64_t row_stride, int box_rows);
 // 2-D bf16 row-major [rows, cols] tensor map with box {box_cols, box_rows}, no swizzle (host).
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, int64_t rows, int64_t cols, int box_rows, int box_cols);
 

@@ -4,151 +4,339 @@
 //
 // Replaces, for m > 1, op::matmul → cublasGemmStridedBatchedEx / cublasGemmEx
 //   [ref: third_party/TinyTorch/src/Operation/OpLinalg.cpp:244-277, OpLinalgCuda.cuh:193-216,276-293]
-// with the reference's numerics: bf16 × bf16 products, fp32 accumulation, ONE rounding to bf16 (bias / residual are
-// applied by separate kernels in the prefill path, exactly where the reference rounds).  Decode (m = 1) never comes
+// with the reference's numerics: bf16 × bf16 products, fp32 accumulation, ONE rounding to bf16; what the reference does in a kernel
+// of its own behind a Linear keeps its own rounding when it rides on the store.  Decode (m = 1) never comes
 // here — it is HBM-bound and runs on the CUDA-core GEMV (gemv.cu).
 //
-// Structure (one 128×128 output tile per CTA, 192 threads, warp-specialised):
-//   warp 0   TMA producer: per 64-column k-block one 128×64 box of A and one of B (128-byte swizzle) into a 4-stage
-//            shared-memory ring, completion on `full[s]` (expect_tx)
-//   warp 1   MMA issuer: one elected thread issues 4 × tcgen05.mma.cta_group::1.kind::f16 (M128 N128 K16) per k-block,
-//            accumulator in TMEM (128 lanes × 128 fp32 columns); tcgen05.commit releases the stage to the producer
-//            (`empty[s]`) and, after the last k-block, signals the epilogue (`tmem_full`)
-//   warps 2-5 epilogue: tcgen05.ld 32x32b.x16 (each warp owns the TMEM lane quarter warp_id % 4), fp32 → bf16,
-//            32-byte stores of 16 consecutive columns per thread
-// TMA zero-fills out-of-range rows/columns, so M, N, K need not be multiples of the tile.
-#include "common.cuh"
+// Two kernels, chosen per shape (pick_gemm): persistent CTA pairs on 256 × 256 tiles when the tiles fill the GPU, split-K clusters
+// when they do not.  In both (192 threads, warp-specialised):
+//   warp 0   TMA producer: 64-column k-blocks of A and B (128-byte swizzle) into a shared-memory ring, completion on `full[s]`
+//   warp 1   MMA issuer: one thread issues 4 × tcgen05.mma.kind::f16 (K16) per k-block, accumulator in TMEM; tcgen05.commit
+//            releases the stage to the producer (`empty[s]`) and signals the epilogue (`tmem_full`)
+//   warps 2-5 epilogue: tcgen05.ld 32x32b (each warp owns the TMEM lane quarter warp_id % 4)
+// TMA zero-fills out-of-range rows/columns, so M, N, K need not be multiples of the tile.  Every wait is bounded: one that gives up
+// leaves a code in the host-visible word of wait_word() and lets the kernel end.
 #include "ops.cuh"
+#include "tc.cuh"
 
 #include <algorithm>
-#include <cstdlib>
+#include <atomic>
 #include <mutex>
 
 namespace b200 {
 
 namespace {
 
-constexpr int kBM = 128, kBN = 128, kBK = 64;   // tile; kBK bf16 = 128 bytes = one swizzle row
-constexpr int kGemmStages = 4;
+constexpr int kBK = 64;                          // bf16 per k-block: 128 bytes = one swizzle row
 constexpr int kGemmThreads = 192;
-constexpr int kTileBytes = kBM * kBK * 2;        // 16 KB per operand per stage
-constexpr int kTmemCols = 128;
-constexpr int kGemmSmem = kGemmStages * 2 * kTileBytes + 1024 /*align*/ + 256 /*barriers*/;
+constexpr int kTileBytes = 128 * kBK * 2;        // 16 KB: 128 rows of an operand's k-block
+constexpr unsigned kGemmWaitCode = 0x6e000000u;
 
-// kind::f16 instruction descriptor: D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1), both K-major
-// (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-
-// shared-memory matrix descriptor, K-major, SWIZZLE_128B: start address >> 4 (bits 0-13), LBO = 0 (bits 16-29, unused
-// for swizzled K-major), SBO = 1024 B >> 4 (bits 32-45: 8 rows × 128 B between core-matrix groups), version 1
-// (bits 46-47), layout type 2 = SWIZZLE_128B (bits 61-63).
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
-  return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// sixteen consecutive columns of one output row (`left` of them exist): bf16(acc + bias) or fp32 acc + bias
+// what the epilogue does with the fp32 sums
+enum GemmEpi : int {
+  GEPI_STORE = 0,      // C = T(acc + bias) (fp32 bias, may be null)
+  GEPI_RESIDUAL = 1,   // C = bf16(add + bf16(acc)); add [M, N] may be C itself: a linear followed by the residual's add
+  GEPI_BIAS = 2,       // C = bf16(bf16(acc) + add), add [N]: a linear followed by its bias as the second rounding
+  GEPI_SILU = 3,       // B holds N gate rows, then N up rows: C = bf16(bf16(silu(bf16 gate)) · bf16 up)
+};
 template <typename OT>
-__device__ __forceinline__ void store16(OT* dst, uint32_t (&r)[16], int left, const float* bias);
-template <>
-__device__ __forceinline__ void store16<__nv_bfloat16>(__nv_bfloat16* dst, uint32_t (&r)[16], int left, const float* bias) {
-  if (bias != nullptr) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (j < left) r[j] = __float_as_uint(__uint_as_float(r[j]) + bias[j]);
-  }
-  if (left >= 16 && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
-    uint4 o0, o1;
-    o0.x = pack2(__uint_as_float(r[0]), __uint_as_float(r[1]));
-    o0.y = pack2(__uint_as_float(r[2]), __uint_as_float(r[3]));
-    o0.z = pack2(__uint_as_float(r[4]), __uint_as_float(r[5]));
-    o0.w = pack2(__uint_as_float(r[6]), __uint_as_float(r[7]));
-    o1.x = pack2(__uint_as_float(r[8]), __uint_as_float(r[9]));
-    o1.y = pack2(__uint_as_float(r[10]), __uint_as_float(r[11]));
-    o1.z = pack2(__uint_as_float(r[12]), __uint_as_float(r[13]));
-    o1.w = pack2(__uint_as_float(r[14]), __uint_as_float(r[15]));
-    reinterpret_cast<uint4*>(dst)[0] = o0;
-    reinterpret_cast<uint4*>(dst)[1] = o1;
-  } else {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (j < left) dst[j] = f_to_bf16(__uint_as_float(r[j]));
-  }
-}
-template <>
-__device__ __forceinline__ void store16<float>(float* dst, uint32_t (&r)[16], int left, const float* bias) {
-  float v[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + (bias != nullptr && j < left ? bias[j] : 0.f);
-  if (left >= 16 && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) reinterpret_cast<float4*>(dst)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-  } else {
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (j < left) dst[j] = v[j];
-  }
+struct GemmArgs {
+  OT* C;
+  const float* bias;
+  const __nv_bfloat16* add;
+  int M, N, K;
+  unsigned* err;
+};
+
+// bf16(silu(bf16 g))·bf16 u of two fp32 sums each
+__device__ __forceinline__ uint32_t silu_mul2(uint32_t g0, uint32_t g1, uint32_t u0, uint32_t u1) {
+  return silu_mul_bf16x2(pack2(__uint_as_float(g0), __uint_as_float(g1)), pack2(__uint_as_float(u0), __uint_as_float(u1)));
 }
 
-template <typename OT>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                    OT* __restrict__ C, const float* __restrict__ bias, int M, int N, int K) {
+// ------------------------------------------------------------------------------------------- persistent CTA pairs
+// One tcgen05.mma.cta_group::2 covers a 256 × 256 tile (M256 N256 K16): CTA r of the pair holds rows 128·r of A and half of B's
+// 256 rows, so per 64-wide k-block an SM loads 32 KB where two one-CTA 128 × 256 tiles take 48 KB each.  Persistent pairs (grid =
+// min(tiles, #SMs / 2) pairs) walk tiles m-fastest, so pairs that run side by side share weight rows in L2; the fp32
+// accumulator is double-buffered in TMEM (2 × 256 columns): the epilogue of tile i drains one buffer while the MMA warp
+// fills the other.  The epilogue turns rows of TMEM lanes into whole 128-byte row pieces through a swizzled 4 KB patch per
+// warp and stores 16 bytes per lane along the row.  Bound by the tensor pipe under the power cap: 2 048 × 12 288 × 2 048 in 74 µs
+// (1.39 PFLOP/s; one-CTA 128 × 256 tiles: 80 µs), 2 048 × 16 384 × 3 072 in 138 µs (1.49 PFLOP/s).
+constexpr int kPairBN = 256;
+constexpr int kPairStages = 6;
+constexpr int kPairStageBytes = 2 * kTileBytes;
+constexpr int kPairPatch = 4096;   // 32 rows × 128 bytes per epilogue warp
+constexpr int kPairSmem = kPairStages * kPairStageBytes + 4 * kPairPatch + 1024 /*align*/ + 256 /*barriers*/;
+
+template <typename OT, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmArgs<OT> p) {
+  constexpr int BN = kPairBN, ST = kPairStages, HB = BN / 2;
+  constexpr int OUT = EPI == GEPI_SILU ? HB : BN;   // output columns of a tile
+  constexpr uint32_t kIdesc = umma_idesc(256, BN);
+  constexpr int kCols = 2 * BN;                     // TMEM: two accumulators
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sA = smem;                                   // [stages][128 × 64 bf16], 1024-byte aligned (swizzle atom)
-  uint8_t* sB = smem + kGemmStages * kTileBytes;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + 2 * kGemmStages * kTileBytes);
-  uint64_t* empty = full + kGemmStages;
-  uint64_t* tmem_full = empty + kGemmStages;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
+  uint8_t* sA = smem;                               // [stages][128 × 64 bf16]
+  uint8_t* sB = smem + ST * kTileBytes;             // [stages][128 × 64 bf16]
+  uint8_t* patch = smem + ST * kPairStageBytes;     // [4 warps][32 rows × 128 bytes]
+  uint64_t* full = reinterpret_cast<uint64_t*>(patch + 4 * kPairPatch);   // CTA 0's count the pair's bytes
+  uint64_t* empty = full + ST;
+  uint64_t* tmem_full = empty + ST;                 // [2]
+  uint64_t* tmem_empty = tmem_full + 2;             // [2], CTA 0's: one arrival per epilogue warp of the pair
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * kBN, m0 = blockIdx.y * kBM;
-  const int kblocks = (K + kBK - 1) / kBK;
+  const int rank = (int)cluster_rank(), pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+  const int mt = (p.M + 255) / 256, nt = (p.N + OUT - 1) / OUT;
+  const int tiles = mt * nt;
+  const int kblocks = (p.K + kBK - 1) / kBK;
+  bool ok = true;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
-    for (int s = 0; s < kGemmStages; ++s) {
+    for (int s = 0; s < ST; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&tmem_full[a], 1);
+      mbar_init(&tmem_empty[a], 8);
+    }
+    fence_mbar_init();
+  }
+  if (warp == 2) tmem_alloc<2>(tmem_slot, kCols);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();   // the pair's barriers exist
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 1;
+      for (int t = pair; t < tiles && ok; t += pairs) {
+        const int m0 = (t % mt) * 256 + rank * 128;
+        const int n0 = (t / mt) * OUT + rank * (EPI == GEPI_SILU ? p.N : HB);
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!(ok = mbar_wait_limited(&empty[s], ph, p.err, kGemmWaitCode | 1))) break;
+          if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * kPairStageBytes);
+          const uint32_t bar = mapa_u32(smem_u32(&full[s]), 0);
+          tma_load_2d_pair(sA + s * kTileBytes, &tmap_a, kb * kBK, m0, bar);
+          tma_load_2d_pair(sB + s * kTileBytes, &tmap_b, kb * kBK, n0, bar);
+          if (++s == ST) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+      }
+      if (!ok) drain_loads();
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------------------------ MMA issuer (CTA 0)
+    if (lane == 0 && rank == 0) {
+      int s = 0;
+      uint32_t ph = 0;
+      int i = 0;
+      for (int t = pair; t < tiles && ok; t += pairs, ++i) {
+        const int acc = i & 1;
+        if (!(ok = mbar_wait_limited(&tmem_empty[acc], (uint32_t)(((i >> 1) & 1) ^ 1), p.err, kGemmWaitCode | 2))) break;
+        tc_fence_after();
+        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
+        for (int kb = 0; kb < kblocks; ++kb) {
+          if (!(ok = mbar_wait_limited(&full[s], ph, p.err, kGemmWaitCode | 3))) break;
+          tc_fence_after();
+          const uint32_t a_addr = smem_u32(sA + s * kTileBytes), b_addr = smem_u32(sB + s * kTileBytes);
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k)
+            umma_bf16_pair(tmem_d, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), kIdesc, (kb > 0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(&empty[s]);
+          if (++s == ST) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+        if (ok) umma_commit_pair(&tmem_full[acc]);
+      }
+    }
+  } else {
+    // ---------------------------------------------------------------------------------------------- epilogue
+    constexpr int CW = 128 / (int)sizeof(OT);       // columns of a patch row
+    constexpr int VW = 16 / (int)sizeof(OT);        // columns per lane when the patch is read back
+    const int q = warp & 3;
+    uint8_t* const pw = patch + q * kPairPatch;
+    const int rr = lane >> 3, cc = lane & 7;        // read-back: lane takes 16-byte piece cc of rows rr, rr + 4, …
+    const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
+    int i = 0;
+    for (int t = pair; t < tiles; t += pairs, ++i) {
+      const int acc = i & 1;
+      const int row0 = (t % mt) * 256 + rank * 128 + q * 32, n0 = (t / mt) * OUT;
+      ok = __all_sync(0xffffffffu, mbar_wait_limited(&tmem_full[acc], (uint32_t)((i >> 1) & 1), p.err, kGemmWaitCode | 4));
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; c < OUT; c += CW) {
+        if constexpr (EPI == GEPI_SILU) {           // 64 columns: gate at c, up at HB + c
+          uint32_t g[32], u[32];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            tmem_ld32(lane_base + (uint32_t)(acc * BN + c + 32 * h), g);
+            tmem_ld32(lane_base + (uint32_t)(acc * BN + HB + c + 32 * h), u);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint4 o;
+              o.x = silu_mul2(g[8 * j], g[8 * j + 1], u[8 * j], u[8 * j + 1]);
+              o.y = silu_mul2(g[8 * j + 2], g[8 * j + 3], u[8 * j + 2], u[8 * j + 3]);
+              o.z = silu_mul2(g[8 * j + 4], g[8 * j + 5], u[8 * j + 4], u[8 * j + 5]);
+              o.w = silu_mul2(g[8 * j + 6], g[8 * j + 7], u[8 * j + 6], u[8 * j + 7]);
+              *reinterpret_cast<uint4*>(pw + lane * 128 + (((4 * h + j) ^ (lane & 7)) << 4)) = o;
+            }
+          }
+        } else if constexpr (sizeof(OT) == 2) {
+          uint32_t a[32], b[32];
+          tmem_ld32(lane_base + (uint32_t)(acc * BN + c), a);
+          tmem_ld32(lane_base + (uint32_t)(acc * BN + c + 32), b);
+          tmem_wait_ld();
+          if (EPI == GEPI_STORE && p.bias != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              if (n0 + c + j < p.N) a[j] = __float_as_uint(__uint_as_float(a[j]) + p.bias[n0 + c + j]);
+              if (n0 + c + 32 + j < p.N) b[j] = __float_as_uint(__uint_as_float(b[j]) + p.bias[n0 + c + 32 + j]);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t* v = j < 4 ? a + 8 * j : b + 8 * (j - 4);
+            uint4 o;
+            o.x = pack2(__uint_as_float(v[0]), __uint_as_float(v[1]));
+            o.y = pack2(__uint_as_float(v[2]), __uint_as_float(v[3]));
+            o.z = pack2(__uint_as_float(v[4]), __uint_as_float(v[5]));
+            o.w = pack2(__uint_as_float(v[6]), __uint_as_float(v[7]));
+            *reinterpret_cast<uint4*>(pw + lane * 128 + ((j ^ (lane & 7)) << 4)) = o;
+          }
+        } else {
+          uint32_t a[32];
+          tmem_ld32(lane_base + (uint32_t)(acc * BN + c), a);
+          tmem_wait_ld();
+          if (p.bias != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (n0 + c + j < p.N) a[j] = __float_as_uint(__uint_as_float(a[j]) + p.bias[n0 + c + j]);
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(pw + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
+        }
+        if (c + CW >= OUT) {   // this warp holds the tile's last columns: the accumulator may be filled again
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty[acc]), 0));
+        }
+        __syncwarp();
+        const int col = n0 + c + cc * VW;
+        if (col < p.N) {       // N is a multiple of 8: a 16-byte piece lies inside the row or outside it
+          uint4 add[8];
+          if constexpr (EPI == GEPI_RESIDUAL) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              if (row0 + rr + 4 * k < p.M) add[k] = *reinterpret_cast<const uint4*>(p.add + (size_t)(row0 + rr + 4 * k) * p.N + col);
+          } else if constexpr (EPI == GEPI_BIAS) {
+            add[0] = *reinterpret_cast<const uint4*>(p.add + col);
+          }
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const int r = rr + 4 * k;
+            if (row0 + r >= p.M) continue;
+            uint4 v = *reinterpret_cast<const uint4*>(pw + r * 128 + ((cc ^ (r & 7)) << 4));
+            if constexpr (EPI == GEPI_RESIDUAL || EPI == GEPI_BIAS) {
+              const uint4 w = add[EPI == GEPI_BIAS ? 0 : k];
+              v = make_uint4(add_bf16x2(w.x, v.x), add_bf16x2(w.y, v.y), add_bf16x2(w.z, v.z), add_bf16x2(w.w, v.w));
+            }
+            *reinterpret_cast<uint4*>(p.C + (size_t)(row0 + r) * p.N + col) = v;
+          }
+        }
+        __syncwarp();          // the patch is free again
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncwarp();
+  __syncthreads();
+  cluster_sync_all();   // neither CTA still reads the pair's operands, barriers or accumulators
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_free<2>(tmem_base, kCols);
+  }
+  cluster_sync_all();
+}
+
+// ------------------------------------------------------------------------------------------------ split-K clusters
+// The kernel for shapes with fewer tiles than the persistent pairs need: short prompts, and the o_proj / down_proj of
+// middling ones, where whole-K tiles leave most SMs idle while the few busy ones stream all of W.  One tile per cluster, 128 × 128
+// on one CTA or 256 × 256 on a CTA pair (PAIR); the cluster's `splits` CTAs (pairs) take neighbouring ranges of K, leave
+// their fp32 partial tiles in their own shared memory (the drained operand ring), and after one cluster barrier each sums
+// its share of the rows over all partials through distributed shared memory, in rank order, and stores it.  No workspace, no
+// second launch, no atomics; splits = 1 is the plain tile.  A rows past M are neither loaded nor stored (box of ≤ 128
+// rows; what the MMA reads there only reaches rows that nobody reads).
+// The ring holds as many stages as 192 KB take: six of 128 rows of A, ten of 16 rows and fewer.
+constexpr int kSplitRing = 192 * 1024;
+constexpr int kSplitStagesMax = 10;
+constexpr int kSplitSmem = kSplitRing + 1024 /*align*/ + 256 /*barriers*/;
+static_assert(128 * (256 + 4) * 4 <= kSplitRing, "a partial tile fits in the drained ring");
+__host__ __device__ constexpr int split_stages(int box_rows) {   // the MMA reads 128 rows (16 KB) from the last stage's A on
+  return (kSplitRing - kTileBytes + box_rows * kBK * 2) / (box_rows * kBK * 2 + kTileBytes) < kSplitStagesMax
+             ? (kSplitRing - kTileBytes + box_rows * kBK * 2) / (box_rows * kBK * 2 + kTileBytes) : kSplitStagesMax;
+}
+constexpr int split_ring_end(int box_rows) { return split_stages(box_rows) * kTileBytes + (split_stages(box_rows) - 1) * box_rows * kBK * 2 + kTileBytes; }
+static_assert(split_ring_end(8) <= kSplitRing && split_ring_end(24) <= kSplitRing && split_ring_end(64) <= kSplitRing &&
+                  split_ring_end(96) <= kSplitRing && split_ring_end(128) <= kSplitRing,
+              "what the MMA reads stays inside the ring");
+
+template <typename OT, int EPI, bool PAIR>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmArgs<OT> p,
+                  const int splits, const int box_rows) {
+  constexpr int BN = PAIR ? 256 : 128, BMT = PAIR ? 256 : 128, LD = BN + 4, GROUP = PAIR ? 2 : 1;
+  constexpr int OUT = EPI == GEPI_SILU ? BN / 2 : BN;
+  constexpr uint32_t kIdesc = umma_idesc(BMT, BN);
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int stages = split_stages(box_rows), a_bytes = box_rows * kBK * 2;
+  uint8_t* sB = smem;                                       // [stages][128 × 64 bf16], two boxes of 64 rows
+  uint8_t* sA = smem + stages * kTileBytes;                 // [stages][box_rows × 64 bf16]
+  float* part = reinterpret_cast<float*>(smem);             // [128][LD] once the ring has drained
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kSplitRing);
+  uint64_t* empty = full + kSplitStagesMax;
+  uint64_t* tmem_full = empty + kSplitStagesMax;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int crank = (int)cluster_rank(), half = PAIR ? crank & 1 : 0, split = PAIR ? crank >> 1 : crank;
+  const int tile = (int)blockIdx.x / (splits * GROUP);
+  const int n0 = tile * OUT, m0 = (int)blockIdx.y * BMT + half * 128;
+  const int kblocks = (p.K + kBK - 1) / kBK;
+  const int kb0 = (int)((int64_t)kblocks * split / splits), kb1 = (int)((int64_t)kblocks * (split + 1) / splits);
+  const int valid = max(0, min(128, p.M - m0));             // rows of this CTA that exist
+  bool ok = true;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmap_a);
+    tma_prefetch_desc(&tmap_b);
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
     mbar_init(tmem_full, 1);
     fence_mbar_init();
   }
-  if (warp == 2) {  // TMEM allocation: one whole warp, the same warp frees it
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(kTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 2) tmem_alloc<GROUP>(tmem_slot, BN);
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();   // the pair's barriers exist
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -157,301 +345,322 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 1;
-      for (int kb = 0; kb < kblocks; ++kb) {
-        mbar_wait(&empty[s], ph);
-        mbar_arrive_expect_tx(&full[s], 2 * kTileBytes);
-        tma_load_2d(sA + s * kTileBytes, &tmap_a, kb * kBK, m0, &full[s]);
-        tma_load_2d(sB + s * kTileBytes, &tmap_b, kb * kBK, n0, &full[s]);
-        if (++s == kGemmStages) {
+      const uint32_t bytes = (uint32_t)(a_bytes + kTileBytes) * (uint32_t)GROUP;
+      // the two 64-row boxes of B: neighbouring rows, or (SiLU) gate rows and the up rows that belong to them
+      const int b0 = PAIR ? n0 + half * (EPI == GEPI_SILU ? p.N : 128) : n0;
+      const int b1 = !PAIR && EPI == GEPI_SILU ? n0 + p.N : b0 + 64;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait_limited(&empty[s], ph, p.err, kGemmWaitCode | 5))) break;
+        uint8_t *b_dst = sB + s * kTileBytes, *a_dst = sA + s * a_bytes;
+        if constexpr (PAIR) {
+          if (half == 0) mbar_arrive_expect_tx(&full[s], bytes);
+          const uint32_t bar = mapa_u32(smem_u32(&full[s]), (uint32_t)(crank & ~1));
+          tma_load_2d_pair(b_dst, &tmap_b, kb * kBK, b0, bar);
+          tma_load_2d_pair(b_dst + kTileBytes / 2, &tmap_b, kb * kBK, b1, bar);
+          tma_load_2d_pair(a_dst, &tmap_a, kb * kBK, m0, bar);
+        } else {
+          mbar_arrive_expect_tx(&full[s], bytes);
+          tma_load_2d(b_dst, &tmap_b, kb * kBK, b0, &full[s]);
+          tma_load_2d(b_dst + kTileBytes / 2, &tmap_b, kb * kBK, b1, &full[s]);
+          tma_load_2d(a_dst, &tmap_a, kb * kBK, m0, &full[s]);
+        }
+        if (++s == stages) {
           s = 0;
           ph ^= 1;
         }
       }
+      if (!ok) drain_loads();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (lane == 0 && half == 0) {
       int s = 0;
       uint32_t ph = 0;
-      for (int kb = 0; kb < kblocks; ++kb) {
-        mbar_wait(&full[s], ph);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait_limited(&full[s], ph, p.err, kGemmWaitCode | 6))) break;
         tc_fence_after();
-        const uint32_t a_addr = smem_u32(sA + s * kTileBytes), b_addr = smem_u32(sB + s * kTileBytes);
+        const uint32_t a_addr = smem_u32(sA + s * a_bytes), b_addr = smem_u32(sB + s * kTileBytes);
 #pragma unroll
-        for (int k = 0; k < kBK / 16; ++k) {
-          // 16 bf16 = 32 bytes further along K inside the 128-byte swizzle row
-          umma_bf16(tmem_base, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), kIdesc,
-                    (kb > 0 || k > 0) ? 1u : 0u);
+        for (int k = 0; k < kBK / 16; ++k) {   // 16 bf16 = 32 bytes further along K inside the 128-byte swizzle row
+          const uint32_t accumulate = (kb > kb0 || k > 0) ? 1u : 0u;
+          if constexpr (PAIR) umma_bf16_pair(tmem_base, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), kIdesc, accumulate);
+          else umma_bf16(tmem_base, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), kIdesc, accumulate);
         }
-        umma_commit(&empty[s]);  // frees the stage once these MMAs have read it
-        if (++s == kGemmStages) {
+        if constexpr (PAIR) umma_commit_pair(&empty[s], (uint16_t)(3u << crank));
+        else umma_commit(&empty[s]);
+        if (++s == stages) {
           s = 0;
           ph ^= 1;
         }
       }
-      umma_commit(tmem_full);  // accumulator complete
-    }
-  } else {
-    // ---------------------------------------------------------------------------------------------- epilogue
-    mbar_wait(tmem_full, 0);
-    tc_fence_after();
-    const int q = warp & 3;                 // TMEM lane quarter this warp may access
-    const int row = m0 + q * 32 + lane;
-#pragma unroll 1
-    for (int c = 0; c < kBN; c += 16) {
-      uint32_t r[16];
-      tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c, r);
-      if (row < M && n0 + c < N)
-        store16<OT>(C + (size_t)row * N + n0 + c, r, N - n0 - c, bias != nullptr ? bias + n0 + c : nullptr);
-    }
-  }
-
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 2) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
-  }
-}
-
-// ------------------------------------------------------------------------------------------------ persistent variant
-// The kernel for shapes whose tiles fill the GPU (launch_gemm_bf16 chooses; tests/test_prefill_gpu.py: bit-identical to
-// the 128 × 128 kernel on ≥ 99.9 % of the elements, ≤ 1 ulp against the oracle).  Same roles and the same descriptors /
-// TMEM access shapes as gemm_tcgen05_kernel, re-arranged for throughput:
-//   * 128 × 256 output tiles (one tcgen05.mma is M128 N256 K16): per 64-wide k-block the MMA pipe is busy 512 cycles
-//     and reads 48 KB of shared memory (96 B/clk; the 128 × 128 tile sits exactly on the 128 B/clk limit),
-//   * persistent CTAs (grid = min(tiles, #SMs)) walking tiles m-fastest, so concurrently running CTAs share weight rows
-//     in L2 and barrier init / TMEM allocation are paid once per CTA instead of once per tile,
-//   * the fp32 accumulator is double-buffered in TMEM (2 × 256 of the 512 columns): the epilogue of tile i drains
-//     buffer i & 1 while the MMA warp already accumulates tile i + 1 (tmem_full / tmem_empty barriers).
-constexpr int kPBN = 256;
-constexpr int kPStages = 4;
-constexpr int kPTileA = kBM * kBK * 2;    // 16 KB
-constexpr int kPTileB = kPBN * kBK * 2;   // 32 KB
-constexpr int kPTmemCols = 512;
-constexpr int kPGemmSmem = kPStages * (kPTileA + kPTileB) + 1024 /*align*/ + 256 /*barriers*/;
-constexpr uint32_t kPIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-
-// mbarrier wait that traps after ~2 s instead of spinning forever: a protocol bug in this not-yet-run kernel must fail
-// the launch, not hang the GPU
-__device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
-  unsigned int spins = 0;
-  unsigned long long t0 = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if ((++spins & 0xffffu) == 0) {
-      const unsigned long long now = global_timer_ns();
-      if (t0 == 0) t0 = now;
-      if (now - t0 > 2000000000ull) __trap();
-    }
-  }
-}
-
-template <typename OT>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                               OT* __restrict__ C, const float* __restrict__ bias, int M, int N, int K) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sA = smem;                                   // [stages][128 × 64 bf16]
-  uint8_t* sB = smem + kPStages * kPTileA;              // [stages][256 × 64 bf16]
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kPStages * (kPTileA + kPTileB));
-  uint64_t* empty = full + kPStages;
-  uint64_t* tmem_full = empty + kPStages;               // [2]
-  uint64_t* tmem_empty = tmem_full + 2;                 // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int mt = (M + kBM - 1) / kBM, nt = (N + kPBN - 1) / kPBN;
-  const int tiles = mt * nt;
-  const int kblocks = (K + kBK - 1) / kBK;
-
-  if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmap_a);
-    tma_prefetch_desc(&tmap_b);
-    for (int s = 0; s < kPStages; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
-    }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(&tmem_full[a], 1);
-      mbar_init(&tmem_empty[a], 128);   // every epilogue thread arrives once it holds its part of the tile in registers
-    }
-    fence_mbar_init();
-  }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(kPTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
-  if (warp == 0) {
-    // ------------------------------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 1;
-      for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const int m0 = (t % mt) * kBM, n0 = (t / mt) * kPBN;
-        for (int kb = 0; kb < kblocks; ++kb) {
-          mbar_wait_bounded(&empty[s], ph);
-          mbar_arrive_expect_tx(&full[s], kPTileA + kPTileB);
-          tma_load_2d(sA + s * kPTileA, &tmap_a, kb * kBK, m0, &full[s]);
-          tma_load_2d(sB + s * kPTileB, &tmap_b, kb * kBK, n0, &full[s]);
-          if (++s == kPStages) {
-            s = 0;
-            ph ^= 1;
-          }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 0;
-      int i = 0;
-      for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
-        const int acc = i & 1;
-        mbar_wait_bounded(&tmem_empty[acc], (uint32_t)(((i >> 1) & 1) ^ 1));   // the epilogue drained this buffer's last use
-        tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(acc * kPBN);
-        for (int kb = 0; kb < kblocks; ++kb) {
-          mbar_wait_bounded(&full[s], ph);
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + s * kPTileA), b_addr = smem_u32(sB + s * kPTileB);
-#pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)
-            umma_bf16(tmem_d, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), kPIdesc,
-                      (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit(&empty[s]);
-          if (++s == kPStages) {
-            s = 0;
-            ph ^= 1;
-          }
-        }
-        umma_commit(&tmem_full[acc]);
+      if (ok) {
+        if constexpr (PAIR) umma_commit_pair(tmem_full, (uint16_t)(3u << crank));
+        else umma_commit(tmem_full);
       }
     }
   } else {
-    // ---------------------------------------------------------------------------------------------- epilogue
-    const int q = warp & 3;
-    int i = 0;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
-      const int acc = i & 1;
-      const int m0 = (t % mt) * kBM, n0 = (t / mt) * kPBN;
-      mbar_wait_bounded(&tmem_full[acc], (uint32_t)((i >> 1) & 1));
+    // ------------------------------------------------------------------------- the partial tile, into shared memory
+    const int q = warp & 3, row = q * 32 + lane;
+    ok = __all_sync(0xffffffffu, mbar_wait_limited(tmem_full, 0, p.err, kGemmWaitCode | 7));
+    if (ok && q * 32 < valid) {
       tc_fence_after();
-      const int row = m0 + q * 32 + lane;
 #pragma unroll 1
-      for (int c = 0; c < kPBN; c += 16) {
-        uint32_t r[16];
-        tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kPBN + c), r);
-        if (row < M && n0 + c < N)
-          store16<OT>(C + (size_t)row * N + n0 + c, r, N - n0 - c, bias != nullptr ? bias + n0 + c : nullptr);
+      for (int c = 0; c < BN; c += 32) {
+        uint32_t r[32];
+        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c, r);
+        tmem_wait_ld();
+        if (row < valid) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(part + row * LD + c + 4 * j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+        }
       }
-      // all of this thread's tcgen05.ld have completed (tmem_ld16 waits): hand the buffer back to the MMA warp
-      tc_fence_before();
-      mbar_arrive(&tmem_empty[acc]);
     }
   }
-
   tc_fence_before();
+  __syncwarp();
   __syncthreads();
+  cluster_sync_all();   // every partial of the tile is in place
+
+  // ---------------------------------------------------------------------------------- sum, epilogue, store: 8 columns at a time
+  {
+    const int share = (valid + splits - 1) / splits, r_lo = split * share, r_hi = min(valid, r_lo + share);
+    const uint32_t part_u = smem_u32(part);
+    constexpr int G = OUT / 8;
+    for (int it = threadIdx.x; it < (r_hi - r_lo) * G; it += kGemmThreads) {
+      const int r = r_lo + it / G, c = (it % G) * 8, col = n0 + c;
+      if (col >= p.N) continue;              // N is a multiple of 8: a piece lies inside the row or outside it
+      const size_t o = (size_t)(m0 + r) * p.N + col;
+      uint4 add = make_uint4(0, 0, 0, 0);
+      if constexpr (EPI == GEPI_RESIDUAL) add = *reinterpret_cast<const uint4*>(p.add + o);
+      if constexpr (EPI == GEPI_BIAS) add = *reinterpret_cast<const uint4*>(p.add + col);
+      float v[8], u[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = u[j] = 0.f;
+#pragma unroll 4
+      for (int sp = 0; sp < splits; ++sp) {
+        const uint32_t base = mapa_u32(part_u + (uint32_t)(r * LD + c) * 4u, (uint32_t)(PAIR ? 2 * sp + half : sp));
+        const float4 x = ld_cluster_f4(base), y = ld_cluster_f4(base + 16);
+        v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+        v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+        if constexpr (EPI == GEPI_SILU) {
+          const float4 z = ld_cluster_f4(base + OUT * 4), w = ld_cluster_f4(base + OUT * 4 + 16);
+          u[0] += z.x; u[1] += z.y; u[2] += z.z; u[3] += z.w;
+          u[4] += w.x; u[5] += w.y; u[6] += w.z; u[7] += w.w;
+        }
+      }
+      if (EPI == GEPI_STORE && p.bias != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] += p.bias[col + j];
+      }
+      if constexpr (sizeof(OT) == 4) {
+        reinterpret_cast<float4*>(p.C + o)[0] = make_float4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<float4*>(p.C + o)[1] = make_float4(v[4], v[5], v[6], v[7]);
+      } else {
+        uint32_t w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if constexpr (EPI == GEPI_SILU) w[j] = silu_mul2(__float_as_uint(v[2 * j]), __float_as_uint(v[2 * j + 1]), __float_as_uint(u[2 * j]), __float_as_uint(u[2 * j + 1]));
+          else w[j] = pack2(v[2 * j], v[2 * j + 1]);
+        }
+        if constexpr (EPI == GEPI_RESIDUAL || EPI == GEPI_BIAS) {
+          w[0] = add_bf16x2(add.x, w[0]); w[1] = add_bf16x2(add.y, w[1]); w[2] = add_bf16x2(add.z, w[2]); w[3] = add_bf16x2(add.w, w[3]);
+        }
+        *reinterpret_cast<uint4*>(p.C + o) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+  }
+  __syncthreads();
+  cluster_sync_all();   // no CTA leaves while another still reads its partial
   if (warp == 2) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kPTmemCols) : "memory");
+    tc_fence_after();
+    tmem_free<GROUP>(tmem_base, BN);
   }
+  if constexpr (PAIR) cluster_sync_all();
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-int make_tmap_sw128(CUtensorMap* out, const void* base, int64_t rows, int64_t cols, int box_rows = kBM) {
-  void* p = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-      q != cudaDriverEntryPointSuccess) {
-    (void)cudaGetLastError();
-    set_error("cuTensorMapEncodeTiled is not available (no CUDA driver / device?)");
-    return B200_ERR_NO_DEVICE;
-  }
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-  cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = reinterpret_cast<EncodeTiledFn>(p)(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims,
-                                                  strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_error("cuTensorMapEncodeTiled(swizzle 128B) failed with CUresult %d (rows=%lld cols=%lld)", (int)r,
-              (long long)rows, (long long)cols);
-    return B200_ERR_CUDA;
-  }
-  return B200_OK;
+int make_tmap(CUtensorMap* out, const void* base, int64_t rows, int64_t cols, int box_rows) {
+  return make_tmap_sw128(out, 2, base, 1, rows, cols, rows * cols, cols, box_rows);
 }
 
-}  // namespace
-
-template <typename OT>
-static int launch_gemm_t(OT* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
-  B200_CHECK_ARG(C && A && B && M > 0 && N > 0 && K > 0, "gemm: bad arguments");
-  B200_CHECK_ARG(K % 8 == 0 && N % 8 == 0, "gemm: K=%lld and N=%lld must be multiples of 8 (16-byte rows)", (long long)K,
-                 (long long)N);
-  B200_CHECK_ARG(((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) == 0,
-                 "gemm: operands must be 16-byte aligned");
-  B200_CHECK_ARG(M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), "gemm: shape out of range");
-  static bool attr_set = false;
-  if (!attr_set) {
-    B200_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<OT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
-    attr_set = true;
+// SM pairs of the current device (0 on error)
+int sm_pairs() {
+  static std::atomic<int> known{0};
+  int n = known.load(std::memory_order_relaxed);
+  if (n == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    n /= 2;
+    known.store(n, std::memory_order_relaxed);
   }
-  CUtensorMap ta, tb;
+  return n;
+}
+
+template <typename OT, int EPI>
+int launch_pair(const GemmArgs<OT>& args, const void* A, const void* B, int64_t rows_b, cudaStream_t st) {
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] { attr_err = cudaFuncSetAttribute(gemm_pair_kernel<OT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem); });
+  B200_CUDA(attr_err);
+  GemmArgs<OT> p = args;
   int rc;
-  // Which kernel: the persistent 128×256 one when its tiles fill the GPU (measured on B200, tools/gemm_bench.py: 0.55–0.74
-  // of the cuBLAS bf16 peak at M = 2048 against 0.39–0.49 for one 128×128 tile per CTA; with fewer than ~100 tiles the
-  // small-tile kernel wins).  B200_GEMM = "persistent" | "tile" forces either.
-  const int64_t ptiles = ((M + kBM - 1) / kBM) * ((N + kPBN - 1) / kPBN);
-  if (env_choice("B200_GEMM", 'p', ptiles >= 100)) {
-    static std::once_flag p_once;
-    static cudaError_t p_err = cudaSuccess;
-    static int sms = 0;
-    std::call_once(p_once, [] {
-      p_err = cudaFuncSetAttribute(gemm_tcgen05_persistent_kernel<OT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPGemmSmem);
-      int dev = 0;
-      if (p_err == cudaSuccess) p_err = cudaGetDevice(&dev);
-      if (p_err == cudaSuccess) p_err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    });
-    B200_CUDA(p_err);
-    if ((rc = make_tmap_sw128(&ta, A, M, K, kBM)) != B200_OK) return rc;
-    if ((rc = make_tmap_sw128(&tb, B, N, K, kPBN)) != B200_OK) return rc;
-    const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + kPBN - 1) / kPBN);
-    g_launches.fetch_add(1);
-    gemm_tcgen05_persistent_kernel<OT><<<(unsigned)std::min<int64_t>(tiles, sms), kGemmThreads, kPGemmSmem, st>>>(
-        ta, tb, C, bias, (int)M, (int)N, (int)K);
-    B200_CUDA(cudaGetLastError());
-    return B200_OK;
-  }
-  if ((rc = make_tmap_sw128(&ta, A, M, K)) != B200_OK) return rc;
-  if ((rc = make_tmap_sw128(&tb, B, N, K)) != B200_OK) return rc;
-  dim3 grid((unsigned)((N + kBN - 1) / kBN), (unsigned)((M + kBM - 1) / kBM));
+  if ((rc = wait_word(&p.err)) != B200_OK) return rc;
+  CUtensorMap ta, tb;
+  if ((rc = make_tmap(&ta, A, p.M, p.K, 128)) != B200_OK) return rc;
+  if ((rc = make_tmap(&tb, B, rows_b, p.K, 128)) != B200_OK) return rc;
+  constexpr int OUT = EPI == GEPI_SILU ? kPairBN / 2 : kPairBN;
+  const int64_t tiles = (int64_t)((p.M + 255) / 256) * ((p.N + OUT - 1) / OUT);
+  const int pairs = sm_pairs();
+  B200_CHECK_ARG(pairs > 0 && tiles < (1ll << 30), "gemm: no device, or shape out of range");
   g_launches.fetch_add(1);
-  gemm_tcgen05_kernel<OT><<<grid, kGemmThreads, kGemmSmem, st>>>(ta, tb, C, bias, (int)M, (int)N, (int)K);
+  gemm_pair_kernel<OT, EPI><<<(unsigned)(2 * std::min<int64_t>(tiles, pairs)), kGemmThreads, kPairSmem, st>>>(ta, tb, p);
   B200_CUDA(cudaGetLastError());
   return B200_OK;
 }
 
+template <typename OT, int EPI, bool PAIR>
+int split_setup() {
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] { attr_err = cudaFuncSetAttribute(gemm_split_kernel<OT, EPI, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem); });
+  B200_CUDA(attr_err);
+  return B200_OK;
+}
+
+struct ClusterLaunch {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  ClusterLaunch(dim3 grid, unsigned cluster, cudaStream_t st) {
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = kSplitSmem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+};
+
+// CTAs of clusters of `n` ≤ 8 CTAs that the GPU holds at a time
+template <typename OT, int EPI, bool PAIR>
+int split_capacity(int n) {
+  static std::atomic<int> known[9];
+  const int c = known[n].load(std::memory_order_relaxed);
+  if (c != 0) return c;
+  ClusterLaunch l(dim3((unsigned)n, 64), (unsigned)n, nullptr);
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, gemm_split_kernel<OT, EPI, PAIR>, &l.cfg) != cudaSuccess || clusters < 1) {
+    (void)cudaGetLastError();
+    clusters = std::max(1, 2 * sm_pairs() / n);
+  }
+  known[n].store(clusters * n, std::memory_order_relaxed);
+  return clusters * n;
+}
+
+template <typename OT, int EPI, bool PAIR>
+int launch_split(const GemmArgs<OT>& args, const void* A, const void* B, int64_t rows_b, int splits, cudaStream_t st) {
+  GemmArgs<OT> p = args;
+  int rc;
+  if ((rc = wait_word(&p.err)) != B200_OK) return rc;
+  constexpr int W = PAIR ? 2 : 1, OUT = (PAIR ? 256 : 128) / (EPI == GEPI_SILU ? 2 : 1);
+  const int box_rows = (int)std::min<int64_t>(128, ((int64_t)p.M + 7) / 8 * 8);
+  CUtensorMap ta, tb;
+  if ((rc = make_tmap(&ta, A, p.M, p.K, box_rows)) != B200_OK) return rc;
+  if ((rc = make_tmap(&tb, B, rows_b, p.K, 64)) != B200_OK) return rc;
+  ClusterLaunch l(dim3((unsigned)((p.N + OUT - 1) / OUT * splits * W), (unsigned)((p.M + 128 * W - 1) / (128 * W))), (unsigned)(splits * W), st);
+  g_launches.fetch_add(1);
+  B200_CUDA(cudaLaunchKernelEx(&l.cfg, gemm_split_kernel<OT, EPI, PAIR>, ta, tb, (const GemmArgs<OT>)p, splits, box_rows));
+  return B200_OK;
+}
+
+constexpr int kSplitMinKb = 8;   // k-blocks that a split takes at least: shorter ones save less than their sum costs
+
+// Which kernel, by what each would take (µs): rounds of resident tiles × (k-blocks × the time of one + what a tile costs
+// besides).  The constants are fits to graph-timed launches over M = 16 … 2 048 and the (N, K) of the four model
+// configurations: a k-block is 0.29 µs for either tile, a pair's grows to 0.40 µs when
+// every SM runs several tiles (power); the rest is launch, pipeline fill and epilogue.  Measured, µs, M × N × K: 128 × 3 072 × 8 192
+// whole-K tiles 44, five splits 19; 16 × 896 × 4 864 27 → 9 (eight splits); 512 × 3 072 × 8 192 44 → 33 (pairs, two splits);
+// 2 048 × 12 288 × 2 048 persistent pairs 74, one-CTA tiles 174.  B200_GEMM = "persistent" | "tile" forces the
+// persistent pairs or one whole-K tile per CTA.
+struct GemmPick {
+  int kind;     // 0: split-K, one CTA per tile; 1: split-K, a pair per tile; 2: persistent pairs
+  int splits;
+};
+template <typename OT, int EPI>
+int pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
+  int rc;
+  if ((rc = split_setup<OT, EPI, false>()) != B200_OK || (rc = split_setup<OT, EPI, true>()) != B200_OK) return rc;
+  constexpr int D = EPI == GEPI_SILU ? 2 : 1;
+  const int64_t kb = (K + kBK - 1) / kBK;
+  const int pairs = std::max(1, sm_pairs());
+  auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+  double best = 1e30;
+  auto consider = [&](int kind, int splits, double cost) {
+    if (cost < best) {
+      best = cost;
+      *out = GemmPick{kind, splits};
+    }
+  };
+  const bool whole = env_choice("B200_GEMM", 't', false), any_split = !env_choice("B200_GEMM", 'p', false);
+  if (!whole) {
+    const int64_t rounds = up(up(M, 256) * up(N, 256 / D), pairs);
+    consider(2, 1, 5.5 + (double)(rounds * kb) * (0.30 + 0.02 * (double)std::min<int64_t>(rounds - 1, 5)));
+  }
+  if (any_split) {
+    const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
+    for (int s = 1; s <= (whole ? 1 : 8) && (s == 1 || s * kSplitMinKb <= kb); ++s) {
+      const int64_t t = up(M, 128) * up(N, 128 / D) * s;
+      consider(0, s, (double)up(t, split_capacity<OT, EPI, false>(s)) * (5.0 + 0.15 * s + rows * (2.0 + 0.25 * s) + 0.29 * (double)up(kb, s)));
+    }
+    for (int s = 1; s <= 4 && (s == 1 || s * kSplitMinKb <= kb) && M > 128 && !whole; ++s) {
+      const int64_t t = up(M, 256) * up(N, 256 / D) * 2 * s;
+      consider(1, s, (double)up(t, split_capacity<OT, EPI, true>(2 * s)) * (9.5 + 1.0 * s + 0.33 * (double)up(kb, s)));
+    }
+  }
+  return B200_OK;
+}
+
+template <typename OT, int EPI>
+int launch_gemm(const GemmArgs<OT>& p, const void* A, const void* B, int64_t rows_b, cudaStream_t st) {
+  GemmPick g{};
+  int rc = pick_gemm<OT, EPI>(p.M, p.N, p.K, &g);
+  if (rc != B200_OK) return rc;
+  if (g.kind == 0) return launch_split<OT, EPI, false>(p, A, B, rows_b, g.splits, st);
+  if (g.kind == 1) return launch_split<OT, EPI, true>(p, A, B, rows_b, g.splits, st);
+  return launch_pair<OT, EPI>(p, A, B, rows_b, st);
+}
+
+int check_gemm(const void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K) {
+  B200_CHECK_ARG(C && A && B && M > 0 && N > 0 && K > 0, "gemm: bad arguments");
+  B200_CHECK_ARG(K % 8 == 0 && N % 8 == 0, "gemm: K=%lld and N=%lld must be multiples of 8 (16-byte rows)", (long long)K,
+                 (long long)N);
+  B200_CHECK_ARG(aligned16(A, B, C), "gemm: operands must be 16-byte aligned");
+  B200_CHECK_ARG(M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), "gemm: shape out of range");
+  return B200_OK;
+}
+
+template <typename OT>
+int launch_gemm_store(OT* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
+  int rc = check_gemm(C, A, B, M, N, K);
+  if (rc != B200_OK) return rc;
+  return launch_gemm<OT, GEPI_STORE>(GemmArgs<OT>{C, bias, nullptr, (int)M, (int)N, (int)K, nullptr}, A, B, N, st);
+}
+
+}  // namespace
+
 int launch_gemm_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
-  return launch_gemm_t<__nv_bfloat16>((__nv_bfloat16*)C, A, B, nullptr, M, N, K, st);
+  return launch_gemm_store<__nv_bfloat16>((__nv_bfloat16*)C, A, B, nullptr, M, N, K, st);
 }
 int launch_gemm_bf16_bias(void* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
-  return launch_gemm_t<__nv_bfloat16>((__nv_bfloat16*)C, A, B, bias, M, N, K, st);
+  return launch_gemm_store<__nv_bfloat16>((__nv_bfloat16*)C, A, B, bias, M, N, K, st);
 }
 int launch_gemm_bf16_f32(float* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
-  return launch_gemm_t<float>(C, A, B, bias, M, N, K, st);
+  return launch_gemm_store<float>(C, A, B, bias, M, N, K, st);
 }
 
 }  // namespace b200
