@@ -131,7 +131,7 @@ __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
   const __nv_bfloat162 r = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
   return *reinterpret_cast<const uint32_t*>(&r);
 }
-__device__ __forceinline__ float silu_f(float g) { return __fdividef(g, 1.f + expf(-g)); }
+__device__ __forceinline__ float silu_f(float g) { return g / (1.f + expf(-g)); }
 __device__ __forceinline__ uint32_t silu_mul_bf16x2(uint32_t g, uint32_t u) {
   const __nv_bfloat162 s = __floats2bfloat162_rn(silu_f(bf16_lo(g)), silu_f(bf16_hi(g)));
   const __nv_bfloat162 r = __hmul2(s, *reinterpret_cast<const __nv_bfloat162*>(&u));

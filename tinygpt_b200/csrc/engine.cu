@@ -671,8 +671,8 @@ static int engine_build(const b200_model_desc* desc, const b200_weight_table* w,
 }
 
 // ------------------------------------------------------------------------------------------------ batched prefill
-// S prompt tokens at once (single GPU): activations [S, ·], every Linear on the tcgen05 GEMM, the reference's rounding
-// points kept by running bias / residual / SiLU·mul / norms as the separate ops they are in the reference
+// S prompt tokens at once (single GPU): activations [S, ·], every Linear on the tcgen05 GEMM with bias / residual / SiLU·mul on its
+// store, each rounded where the reference's separate op rounds
 // [ref: src/model/GPTModel.h:51-58; src/layer/Attention.h:71-112; src/layer/GatedMLP.h:37-41].  K/V rows of all S
 // tokens are written in place; the lm_head runs for the LAST position only (GPTEngine::genNextToken narrows to it).
 static constexpr int kPrefillChunk = 2048;
@@ -695,17 +695,14 @@ static int prefill_workspace(b200_engine* e, int chunk) {
   };
   const size_t o_x = take((size_t)chunk * d.hidden), o_h = take((size_t)chunk * d.hidden);
   const size_t o_qkv = take((size_t)chunk * nqkv), o_attn = take((size_t)chunk * e->qdim);
-  const size_t o_gu = take((size_t)chunk * 2 * e->I_l), o_act = take((size_t)chunk * e->I_l);
-  const size_t o_t = take((size_t)chunk * d.hidden);
+  const size_t o_act = take((size_t)chunk * e->I_l);
   B200_CUDA(cudaMalloc((void**)&e->pf_arena, off));
   e->pf_chunk = chunk;
   e->pf_x = (__nv_bfloat16*)(e->pf_arena + o_x);
   e->pf_h = (__nv_bfloat16*)(e->pf_arena + o_h);
   e->pf_qkv = (__nv_bfloat16*)(e->pf_arena + o_qkv);
   e->pf_attn = (__nv_bfloat16*)(e->pf_arena + o_attn);
-  e->pf_gu = (__nv_bfloat16*)(e->pf_arena + o_gu);
   e->pf_act = (__nv_bfloat16*)(e->pf_arena + o_act);
-  e->pf_t = (__nv_bfloat16*)(e->pf_arena + o_t);
   return B200_OK;
 }
 
@@ -719,8 +716,12 @@ static int prefill_chunk(b200_engine* e, const int64_t* ids, int S, int p0, bool
   for (int l = 0; l < d.layers; ++l) {
     const b200_layer_weights& lw = e->lw[l];
     if ((rc = launch_rmsnorm(e->pf_h, e->pf_x, lw.input_norm, S, H, d.rms_eps, st, false)) != B200_OK) return rc;
-    if ((rc = launch_gemm_bf16(e->pf_qkv, e->pf_h, lw.qkv_w, S, nqkv, H, st)) != B200_OK) return rc;
-    if (d.qkv_bias && (rc = launch_bias_add(e->pf_qkv, lw.qkv_b, S, nqkv, st)) != B200_OK) return rc;
+    // a bias that is not 16-byte aligned (a caller's own view) cannot ride on the store
+    const bool bias_tail = d.qkv_bias && aligned16(lw.qkv_b);
+    if ((rc = launch_linear_bf16(e->pf_qkv, e->pf_h, lw.qkv_w, S, nqkv, H, bias_tail ? LinearTail::bias : LinearTail::none,
+                                 bias_tail ? lw.qkv_b : nullptr, st)) != B200_OK)
+      return rc;
+    if (d.qkv_bias && !bias_tail && (rc = launch_bias_add(e->pf_qkv, lw.qkv_b, S, nqkv, st)) != B200_OK) return rc;
     __nv_bfloat16* kc = e->kcache + (size_t)l * kv_layer;
     __nv_bfloat16* vc = e->vcache + (size_t)l * kv_layer;
     if ((rc = launch_prefill_qk(e->pf_qkv, lw.q_norm, lw.k_norm, d.rms_eps, e->rope, kc, vc, S, e->Hq_l, e->Hkv_l,
@@ -728,13 +729,10 @@ static int prefill_chunk(b200_engine* e, const int64_t* ids, int S, int p0, bool
       return rc;
     if ((rc = launch_attn_prefill(e->pf_attn, e->pf_qkv, kc, vc, S, e->Hq_l, e->Hkv_l, d.head_dim, p0, st)) != B200_OK)
       return rc;
-    if ((rc = launch_gemm_bf16(e->pf_t, e->pf_attn, lw.o_w, S, H, e->qdim, st)) != B200_OK) return rc;
-    if ((rc = launch_add(e->pf_x, e->pf_x, e->pf_t, (int64_t)S * H, st, false)) != B200_OK) return rc;
+    if ((rc = launch_linear_bf16(e->pf_x, e->pf_attn, lw.o_w, S, H, e->qdim, LinearTail::residual, e->pf_x, st)) != B200_OK) return rc;
     if ((rc = launch_rmsnorm(e->pf_h, e->pf_x, lw.post_norm, S, H, d.rms_eps, st, false)) != B200_OK) return rc;
-    if ((rc = launch_gemm_bf16(e->pf_gu, e->pf_h, lw.gate_up_w, S, 2 * (int64_t)e->I_l, H, st)) != B200_OK) return rc;
-    if ((rc = launch_silu_mul(e->pf_act, e->pf_gu, S, e->I_l, st, false)) != B200_OK) return rc;
-    if ((rc = launch_gemm_bf16(e->pf_t, e->pf_act, lw.down_w, S, H, e->I_l, st)) != B200_OK) return rc;
-    if ((rc = launch_add(e->pf_x, e->pf_x, e->pf_t, (int64_t)S * H, st, false)) != B200_OK) return rc;
+    if ((rc = launch_linear_bf16(e->pf_act, e->pf_h, lw.gate_up_w, S, e->I_l, H, LinearTail::silu_mul, nullptr, st)) != B200_OK) return rc;
+    if ((rc = launch_linear_bf16(e->pf_x, e->pf_act, lw.down_w, S, H, e->I_l, LinearTail::residual, e->pf_x, st)) != B200_OK) return rc;
   }
   if (last)
     B200_CUDA(cudaMemcpyAsync(e->x, e->pf_x + (size_t)(S - 1) * H, (size_t)H * 2, cudaMemcpyDeviceToDevice, st));

@@ -49,8 +49,7 @@ struct b200_engine {
   // batched prefill (tcgen05 GEMM path), workspace allocated on first use
   uint8_t* pf_arena = nullptr;
   int pf_chunk = 0;  // tokens the workspace holds
-  __nv_bfloat16 *pf_x = nullptr, *pf_h = nullptr, *pf_qkv = nullptr, *pf_attn = nullptr, *pf_gu = nullptr,
-                *pf_act = nullptr, *pf_t = nullptr;
+  __nv_bfloat16 *pf_x = nullptr, *pf_h = nullptr, *pf_qkv = nullptr, *pf_attn = nullptr, *pf_act = nullptr;
   bool use_prefill_gemm = true;
   const void* final_norm_w = nullptr;
   // tensor parallel

@@ -591,8 +591,10 @@ struct GemmPick {
   int kind;     // 0: split-K, one CTA per tile; 1: split-K, a pair per tile; 2: persistent pairs
   int splits;
 };
+// whole_k: no splits — the order in which a row's products are summed is then the same whatever M is, so a prompt's rows have the same
+// bits in one pass, in portions and in a batch.
 template <typename OT, int EPI>
-int pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
+int pick_gemm(int64_t M, int64_t N, int64_t K, bool whole_k, GemmPick* out) {
   int rc;
   if ((rc = split_setup<OT, EPI, false>()) != B200_OK || (rc = split_setup<OT, EPI, true>()) != B200_OK) return rc;
   constexpr int D = EPI == GEPI_SILU ? 2 : 1;
@@ -606,18 +608,18 @@ int pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
       *out = GemmPick{kind, splits};
     }
   };
-  const bool whole = env_choice("B200_GEMM", 't', false), any_split = !env_choice("B200_GEMM", 'p', false);
-  if (!whole) {
+  const bool tile = env_choice("B200_GEMM", 't', false), any_split = !env_choice("B200_GEMM", 'p', false);
+  if (!tile) {
     const int64_t rounds = up(up(M, 256) * up(N, 256 / D), pairs);
     consider(2, 1, 5.5 + (double)(rounds * kb) * (0.30 + 0.02 * (double)std::min<int64_t>(rounds - 1, 5)));
   }
   if (any_split) {
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
-    for (int s = 1; s <= (whole ? 1 : 8) && (s == 1 || s * kSplitMinKb <= kb); ++s) {
+    for (int s = 1; s <= (tile || whole_k ? 1 : 8) && (s == 1 || s * kSplitMinKb <= kb); ++s) {
       const int64_t t = up(M, 128) * up(N, 128 / D) * s;
       consider(0, s, (double)up(t, split_capacity<OT, EPI, false>(s)) * (5.0 + 0.15 * s + rows * (2.0 + 0.25 * s) + 0.29 * (double)up(kb, s)));
     }
-    for (int s = 1; s <= 4 && (s == 1 || s * kSplitMinKb <= kb) && M > 128 && !whole; ++s) {
+    for (int s = 1; s <= (whole_k ? 1 : 4) && (s == 1 || s * kSplitMinKb <= kb) && M > 128 && !tile; ++s) {
       const int64_t t = up(M, 256) * up(N, 256 / D) * 2 * s;
       consider(1, s, (double)up(t, split_capacity<OT, EPI, true>(2 * s)) * (9.5 + 1.0 * s + 0.33 * (double)up(kb, s)));
     }
@@ -626,9 +628,9 @@ int pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
 }
 
 template <typename OT, int EPI>
-int launch_gemm(const GemmArgs<OT>& p, const void* A, const void* B, int64_t rows_b, cudaStream_t st) {
+int launch_gemm(const GemmArgs<OT>& p, const void* A, const void* B, int64_t rows_b, bool whole_k, cudaStream_t st) {
   GemmPick g{};
-  int rc = pick_gemm<OT, EPI>(p.M, p.N, p.K, &g);
+  int rc = pick_gemm<OT, EPI>(p.M, p.N, p.K, whole_k, &g);
   if (rc != B200_OK) return rc;
   if (g.kind == 0) return launch_split<OT, EPI, false>(p, A, B, rows_b, g.splits, st);
   if (g.kind == 1) return launch_split<OT, EPI, true>(p, A, B, rows_b, g.splits, st);
@@ -648,7 +650,7 @@ template <typename OT>
 int launch_gemm_store(OT* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   int rc = check_gemm(C, A, B, M, N, K);
   if (rc != B200_OK) return rc;
-  return launch_gemm<OT, GEPI_STORE>(GemmArgs<OT>{C, bias, nullptr, (int)M, (int)N, (int)K, nullptr}, A, B, N, st);
+  return launch_gemm<OT, GEPI_STORE>(GemmArgs<OT>{C, bias, nullptr, (int)M, (int)N, (int)K, nullptr}, A, B, N, false, st);
 }
 
 }  // namespace
@@ -658,6 +660,19 @@ int launch_gemm_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N
 }
 int launch_gemm_bf16_bias(void* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   return launch_gemm_store<__nv_bfloat16>((__nv_bfloat16*)C, A, B, bias, M, N, K, st);
+}
+int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, LinearTail tail, const void* add, cudaStream_t st) {
+  int rc = check_gemm(C, A, B, M, N, K);
+  if (rc != B200_OK) return rc;
+  B200_CHECK_ARG((tail == LinearTail::bias || tail == LinearTail::residual) == (add != nullptr) && aligned16(add), "linear: bad operand of the tail");
+  const GemmArgs<__nv_bfloat16> p{(__nv_bfloat16*)C, nullptr, (const __nv_bfloat16*)add, (int)M, (int)N, (int)K, nullptr};
+  switch (tail) {
+    case LinearTail::bias: return launch_gemm<__nv_bfloat16, GEPI_BIAS>(p, A, B, N, true, st);
+    case LinearTail::residual: return launch_gemm<__nv_bfloat16, GEPI_RESIDUAL>(p, A, B, N, true, st);
+    case LinearTail::silu_mul: return launch_gemm<__nv_bfloat16, GEPI_SILU>(p, A, B, 2 * N, true, st);
+    case LinearTail::none: break;
+  }
+  return launch_gemm<__nv_bfloat16, GEPI_STORE>(p, A, B, N, true, st);
 }
 int launch_gemm_bf16_f32(float* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   return launch_gemm_store<float>(C, A, B, bias, M, N, K, st);

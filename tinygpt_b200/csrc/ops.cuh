@@ -52,6 +52,12 @@ int launch_gemm_bf16_bias(void* C, const void* A, const void* B, const float* bi
 // the same products handed out as fp32 sums: C = A·Bᵀ + bias (bias may be null)
 int launch_gemm_bf16_f32(float* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st);
 
+// A Linear of the prompt pass with what follows it on its store, each with its own rounding: C = bf16(A·Bᵀ), then bf16(C + bias [N]),
+// bf16(add [M, N] + C) (C may be add), or — B holding N gate rows and N up rows — bf16(bf16(silu(gate))·up).  A row's result does
+// not depend on M.
+enum class LinearTail { none, bias, residual, silu_mul };
+int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, LinearTail tail, const void* add, cudaStream_t st);
+
 // ---- prefill helpers (prefill.cu)
 int launch_bias_add(void* y, const void* b, int64_t rows, int64_t n, cudaStream_t st);
 int launch_prefill_qk(void* qkv, const void* q_norm, const void* k_norm, float eps, const float* rope, void* kcache,

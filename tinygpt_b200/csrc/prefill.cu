@@ -1,10 +1,10 @@
 // prefill.cu — the small kernels around the tcgen05 GEMM in the batched PREFILL path (S prompt tokens at once):
-//   bias add (second rounding, like the reference's separate add kernel), q/k per-head RMSNorm + RoPE + in-place KV-cache
-//   write for all S tokens, and causal attention of the chunk against the cache.
+//   q/k per-head RMSNorm + RoPE + in-place KV-cache write for all S tokens, and causal attention of the chunk against the cache on
+//   the CUDA cores (one CTA per query row and head, online softmax over 128-key chunks; B200_PREFILL_ATTN=cuda — the
+//   tensor-core kernel is prefill_attn.cu).
 //   [ref: src/layer/Attention.h:71-112,156-163; TT/Operation/OpLinalg.cpp:273-275;
 //    TT/Operation/OpNNLayerCuda.cuh:252-299,412-440; TFA/mma/kernel.cuh:18-203 (causal prefill)]
-// Decode never comes here.  The attention kernel is a straightforward CUDA-core one (one CTA per query row and head,
-// online softmax over 128-key chunks); a tensor-core flash-attention prefill is the next step.
+// Decode never comes here.
 #include "common.cuh"
 #include "ops.cuh"
 
@@ -12,7 +12,7 @@ namespace b200 {
 
 namespace {
 
-// y[r, j] = bf16(y[r, j] + b[j])
+// y[r, j] = bf16(y[r, j] + b[j]): a bias that cannot ride on the GEMM's store (not 16-byte aligned)
 __global__ void __launch_bounds__(256) bias_add_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ b,
                                                        int64_t rows, int64_t n) {
   const int64_t total = rows * n;
@@ -20,59 +20,93 @@ __global__ void __launch_bounds__(256) bias_add_kernel(__nv_bfloat16* __restrict
     y[i] = __hadd(y[i], b[i % n]);
 }
 
-// One warp per (token, head) over the q heads and the k heads of the merged qkv rows [S, qdim + 2 kvdim]:
-// optional per-head RMSNorm, RoPE at position p0 + t, q written back in place, k and v written to the cache row.
+// q and k heads of the merged qkv rows [S, qdim + 2 kvdim]: optional per-head RMSNorm, RoPE at position p0 + t, q written back in
+// place, k and v written to the cache row.  HD / 16 lanes per (token, head): a lane holds 8 neighbouring elements of the
+// head's lower half and their 8 rotation partners of the upper half, so every access is a 16-byte vector and the norm's sum
+// goes over the head's lanes; a v head is a copy.  Bound by HBM; 2 048 tokens, 16 + 2·8 heads of 128: 16.1 µs with one
+// warp per head and 2-byte accesses, 12.4 µs like this (same bits).
 template <int HD>
 __global__ void __launch_bounds__(256) prefill_qk_kernel(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ q_norm,
                                                          const __nv_bfloat16* __restrict__ k_norm, float eps,
                                                          const float* __restrict__ rope, __nv_bfloat16* __restrict__ kcache,
                                                          __nv_bfloat16* __restrict__ vcache, int S, int Hq, int Hkv, int p0) {
-  constexpr int EPL = HD / 32;
-  const int lane = threadIdx.x & 31;
-  const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int heads = Hq + Hkv;
-  if (wid >= (int64_t)S * heads) return;
-  const int t = (int)(wid / heads), h = (int)(wid % heads);
-  const bool is_k = h >= Hq;
-  const int qdim = Hq * HD, kvdim = Hkv * HD;
-  const int64_t rowoff = (int64_t)t * (qdim + 2 * kvdim);
-  __nv_bfloat16* src = qkv + rowoff + (is_k ? qdim + (h - Hq) * HD : h * HD);
-  const __nv_bfloat16* nw = is_k ? k_norm : q_norm;
-  float x[EPL];
+  constexpr int L = HD / 16;   // lanes per head
+  const int heads = Hq + 2 * Hkv;
+  const unsigned item = (blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const int part = threadIdx.x % L;
+  const bool live = item < (unsigned)S * (unsigned)heads;
+  const int t = live ? (int)(item / (unsigned)heads) : 0, h = live ? (int)(item % (unsigned)heads) : 0;
+  uint4* src = reinterpret_cast<uint4*>(qkv + ((int64_t)t * heads + h) * HD);
+  uint4 lo = src[part], hi = src[part + L];
+  if (h < Hq + Hkv) {   // uniform among the lanes of a head
+    const __nv_bfloat16* nw = h < Hq ? q_norm : k_norm;
+    float a[8], b[8];
+    unpack8(lo, a);
+    unpack8(hi, b);
+    if (nw != nullptr) {
+      // The sum's order is that of one warp per head, where lane l adds elements l, l + 32, … before a butterfly over the lanes: a lane of
+      // the head's lower half gathers what belongs to its eight such lanes from its partner, the butterfly's first steps go
+      // over lanes, its last three over the eight sums.
+      const unsigned mask = ((1u << L) - 1u) << (threadIdx.x & 31 & ~(L - 1));
+      float s8[8];
 #pragma unroll
-  for (int j = 0; j < EPL; ++j) x[j] = bf16_to_f(src[lane + 32 * j]);
-  if (nw != nullptr) {
-    float ss = 0.f;
+      for (int e = 0; e < 8; ++e) {
+        if constexpr (HD == 128) {   // elements i, i + 32, i + 64, i + 96 with i = 8·(part & 3) + e
+          const float oa = __shfl_xor_sync(mask, a[e], 4), ob = __shfl_xor_sync(mask, b[e], 4);
+          const bool low = part < 4;
+          const float x0 = low ? a[e] : oa, x1 = low ? oa : a[e], x2 = low ? b[e] : ob, x3 = low ? ob : b[e];
+          s8[e] = __fmaf_rn(x3, x3, __fmaf_rn(x2, x2, __fmaf_rn(x1, x1, __fmul_rn(x0, x0))));
+        } else {                     // elements i, i + 32 with i = 8·part + e
+          s8[e] = __fmaf_rn(b[e], b[e], __fmul_rn(a[e], a[e]));
+        }
+      }
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) ss += x[j] * x[j];
-    ss = warp_sum(ss);
-    const float inv = rsqrtf(ss / (float)HD + eps);
+      for (int e = 0; e < 8; ++e) s8[e] += __shfl_xor_sync(mask, s8[e], 2);
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) x[j] = round_bf16(x[j] * inv * bf16_to_f(nw[lane + 32 * j]));
-  }
-  const float* row = rope + (size_t)(p0 + t) * HD * 2;
+      for (int e = 0; e < 8; ++e) s8[e] += __shfl_xor_sync(mask, s8[e], 1);
+      const float ss = ((s8[0] + s8[4]) + (s8[2] + s8[6])) + ((s8[1] + s8[5]) + (s8[3] + s8[7]));
+      const float inv = rsqrtf(ss / (float)HD + eps);
+      float wa[8], wb[8];
+      if ((reinterpret_cast<uintptr_t>(nw) & 15) == 0) {
+        unpack8(reinterpret_cast<const uint4*>(nw)[part], wa);
+        unpack8(reinterpret_cast<const uint4*>(nw)[part + L], wb);
+      } else {
 #pragma unroll
-  for (int j = 0; j < EPL / 2; ++j) {
-    const int i = lane + 32 * j;
-    const float c = row[i * 2], s = row[i * 2 + 1];
-    const float x1 = x[j], x2 = x[j + EPL / 2];
-    x[j] = round_bf16(x1 * c - x2 * s);
-    x[j + EPL / 2] = round_bf16(x2 * c + x1 * s);
-  }
-  if (is_k) {
-    const int kh = h - Hq;
-    __nv_bfloat16* kd = kcache + ((size_t)(p0 + t) * Hkv + kh) * HD;
-    __nv_bfloat16* vd = vcache + ((size_t)(p0 + t) * Hkv + kh) * HD;
-    const __nv_bfloat16* vs = qkv + rowoff + qdim + kvdim + kh * HD;
+        for (int e = 0; e < 8; ++e) {
+          wa[e] = bf16_to_f(nw[part * 8 + e]);
+          wb[e] = bf16_to_f(nw[(part + L) * 8 + e]);
+        }
+      }
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) {
-      kd[lane + 32 * j] = f_to_bf16(x[j]);
-      vd[lane + 32 * j] = vs[lane + 32 * j];
+      for (int e = 0; e < 8; ++e) {
+        a[e] = round_bf16(a[e] * inv * wa[e]);
+        b[e] = round_bf16(b[e] * inv * wb[e]);
+      }
     }
-  } else {
+    const float* row = rope + (size_t)(p0 + t) * HD * 2 + part * 16;
+    float cs[16];
+    if ((reinterpret_cast<uintptr_t>(rope) & 15) == 0) {
 #pragma unroll
-    for (int j = 0; j < EPL; ++j) src[lane + 32 * j] = f_to_bf16(x[j]);
+      for (int e = 0; e < 4; ++e) reinterpret_cast<float4*>(cs)[e] = reinterpret_cast<const float4*>(row)[e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) cs[e] = row[e];
+    }
+    float x[8], y[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float c = cs[2 * e], sn = cs[2 * e + 1];   // the roundings of each product are part of the result: spelled out
+      x[e] = __fmaf_rn(a[e], c, -__fmul_rn(b[e], sn));
+      y[e] = __fmaf_rn(a[e], sn, __fmul_rn(b[e], c));
+    }
+    lo = make_uint4(pack2(x[0], x[1]), pack2(x[2], x[3]), pack2(x[4], x[5]), pack2(x[6], x[7]));
+    hi = make_uint4(pack2(y[0], y[1]), pack2(y[2], y[3]), pack2(y[4], y[5]), pack2(y[6], y[7]));
   }
+  if (!live) return;
+  uint4* dst = h < Hq ? src
+                      : reinterpret_cast<uint4*>((h < Hq + Hkv ? kcache : vcache) + ((size_t)(p0 + t) * Hkv + (h - Hq) % Hkv) * HD);
+  dst[part] = lo;
+  dst[part + L] = hi;
 }
 
 template <int HD>
@@ -161,8 +195,9 @@ int launch_bias_add(void* y, const void* b, int64_t rows, int64_t n, cudaStream_
 int launch_prefill_qk(void* qkv, const void* q_norm, const void* k_norm, float eps, const float* rope, void* kcache,
                       void* vcache, int S, int Hq, int Hkv, int hd, int p0, cudaStream_t st) {
   B200_CHECK_ARG(hd == 64 || hd == 128, "prefill: head_dim %d not built", hd);
-  const int64_t warps = (int64_t)S * (Hq + Hkv);
-  const unsigned grid = (unsigned)((warps * 32 + 255) / 256);
+  B200_CHECK_ARG(aligned16(qkv, kcache, vcache), "prefill: rows and caches must be 16-byte aligned");   // the engine's own
+  B200_CHECK_ARG((int64_t)S * (Hq + 2 * Hkv) * (hd / 16) < (1ll << 31), "prefill: too many rows at a time");
+  const unsigned grid = (unsigned)(((int64_t)S * (Hq + 2 * Hkv) * (hd / 16) + 255) / 256);
   g_launches.fetch_add(1);
   if (hd == 64)
     prefill_qk_kernel<64><<<grid, 256, 0, st>>>((__nv_bfloat16*)qkv, (const __nv_bfloat16*)q_norm,
