@@ -368,8 +368,7 @@ static int stack_product_in(StackEngine* s, int li, const float* x, int n_tok, c
   if ((rc = launch_stack_rmsnorm(s->h, x, L.norm, nullptr, n_tok, W, d.norm_eps, d.norm_offset, s->dtype, st)) != B200_OK)
     return rc;
   if (s->fast && n_tok >= kGemmRows && gemm_shape_ok(L.n_in, W)) {
-    if ((rc = launch_gemm_bf16(s->proj, s->h, L.w_in, n_tok, L.n_in, W, st)) != B200_OK) return rc;
-    return L.b_in ? launch_stack_bias_add((__nv_bfloat16*)s->proj, L.b_in, n_tok, L.n_in, st) : B200_OK;
+    return launch_gemm_bf16_bias(s->proj, s->h, L.w_in, L.b_in, n_tok, L.n_in, W, st);
   }
   StackGemm g;
   g.a = s->h; g.lda = W; g.k1 = W;
@@ -391,10 +390,8 @@ static int stack_product_out(StackEngine* s, int li, float* x, int n_tok, cudaSt
     if ((rc = gemv_plan_set_batch(&pl, n_tok)) != B200_OK) return rc;
     return gemv_launch(pl, st, s->pdl);
   }
-  if (s->fast && n_tok >= kGemmRows && gemm_shape_ok(W, L.k_out)) {   // h is free again: it holds the bf16 product
-    if ((rc = launch_gemm_bf16(s->h, s->mid, L.w_out, n_tok, W, L.k_out, st)) != B200_OK) return rc;
-    return launch_stack_axpy(x, (const __nv_bfloat16*)s->h, s->d.residual_mult, true, (int64_t)n_tok * W, st);
-  }
+  if (s->fast && n_tok >= kGemmRows && gemm_shape_ok(W, L.k_out))
+    return launch_gemm_bf16_accum(x, s->mid, L.w_out, s->d.residual_mult, n_tok, W, L.k_out, st);
   StackGemm g;
   g.a = s->mid; g.lda = L.k_out; g.k1 = L.k_out;
   g.w = L.w_out; g.M = n_tok; g.N = W; g.K = L.k_out;
@@ -418,8 +415,7 @@ static int stack_product_mix(StackEngine* s, const float* cur, float* other, int
       if ((rc = gemv_plan_set_batch(&pl, n_tok)) != B200_OK) return rc;
       return gemv_launch(pl, st, s->pdl);
     }
-    if ((rc = launch_gemm_bf16(s->h, s->cat, s->d.mix_in, n_tok, W, 2 * W, st)) != B200_OK) return rc;
-    return launch_stack_axpy(other, (const __nv_bfloat16*)s->h, 1.f, false, (int64_t)n_tok * W, st);
+    return launch_gemm_bf16_f32(other, s->cat, s->d.mix_in, nullptr, n_tok, W, 2 * W, st);
   }
   StackGemm g;
   g.a = cur; g.a2 = s->x0; g.lda = g.lda2 = W; g.k1 = W; g.a_f32 = true;
@@ -457,6 +453,10 @@ static int stack_product_head(StackEngine* s, const float* x, const int32_t* row
     if ((rc = gemv_launch(pl, st, false)) != B200_OK) return rc;   // copies and the argmax follow: a full dependency
     return d.logit_softcap > 0.f ? launch_stack_softcap(s->logits, s->logits_bf, n_lg, d.logit_softcap, st) : B200_OK;
   }
+  // more rows than a decode batch (every position of a prompt, scoring): 2 048 rows × 2 048 columns of width 2 048 took 882 µs on the
+  // CUDA-core kernel, 22 µs on the tensor cores; the sums are fp32 in both
+  if (s->fast && n_rows > kMaxBatch && gemm_shape_ok(d.vocab, d.width) && aligned16(d.head))
+    return launch_gemm_bf16_logits(s->logits, s->logits_bf, s->hn, d.head, d.logit_softcap, n_rows, d.vocab, d.width, st);
   StackGemm g;
   g.a = s->hn; g.lda = d.width; g.k1 = d.width;
   g.w = d.head; g.M = n_rows; g.N = d.vocab; g.K = d.width;

@@ -37,6 +37,8 @@ enum GemmEpi : int {
   GEPI_STORE = 0,      // C = T(acc + bias) (fp32 bias, may be null)
   GEPI_RESIDUAL = 1,   // C = bf16(add + bf16(acc)); add [M, N] may be C itself: a linear followed by the residual's add
   GEPI_BIAS = 2,       // C = bf16(bf16(acc) + add), add [N]: a linear followed by its bias as the second rounding
+  GEPI_ACCUM = 4,      // C += mult·acc (fp32 C): a layer-stack model's residual stream
+  GEPI_LOGITS = 5,     // C = cap·tanh(acc / cap) (mult = cap; 0: acc itself), c2 = bf16(C) (fp32 C)
   GEPI_SILU = 3,       // B holds N gate rows, then N up rows: C = bf16(bf16(silu(bf16 gate)) · bf16 up)
 };
 template <typename OT>
@@ -46,7 +48,10 @@ struct GemmArgs {
   const __nv_bfloat16* add;
   int M, N, K;
   unsigned* err;
+  float mult = 0.f;
+  __nv_bfloat16* c2 = nullptr;
 };
+__device__ __forceinline__ float cap_logit(float v, float cap) { return cap > 0.f ? cap * tanhf(v / cap) : v; }
 
 // bf16(silu(bf16 g))·bf16 u of two fp32 sums each
 __device__ __forceinline__ uint32_t silu_mul2(uint32_t g0, uint32_t g1, uint32_t u0, uint32_t u1) {
@@ -243,6 +248,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
             for (int k = 0; k < 8; ++k)
               if (row0 + rr + 4 * k < p.M) add[k] = *reinterpret_cast<const uint4*>(p.add + (size_t)(row0 + rr + 4 * k) * p.N + col);
+          } else if constexpr (EPI == GEPI_ACCUM) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              if (row0 + rr + 4 * k < p.M) add[k] = *reinterpret_cast<const uint4*>(p.C + (size_t)(row0 + rr + 4 * k) * p.N + col);
           } else if constexpr (EPI == GEPI_BIAS) {
             add[0] = *reinterpret_cast<const uint4*>(p.add + col);
           }
@@ -251,6 +260,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             const int r = rr + 4 * k;
             if (row0 + r >= p.M) continue;
             uint4 v = *reinterpret_cast<const uint4*>(pw + r * 128 + ((cc ^ (r & 7)) << 4));
+            if constexpr (EPI == GEPI_ACCUM || EPI == GEPI_LOGITS) {
+              uint32_t* f = reinterpret_cast<uint32_t*>(&v);
+              const uint32_t* o = reinterpret_cast<const uint32_t*>(&add[EPI == GEPI_ACCUM ? k : 0]);
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                f[j] = __float_as_uint(EPI == GEPI_ACCUM ? fmaf(p.mult, __uint_as_float(f[j]), __uint_as_float(o[j])) : cap_logit(__uint_as_float(f[j]), p.mult));
+              if constexpr (EPI == GEPI_LOGITS)
+                *reinterpret_cast<uint2*>(p.c2 + (size_t)(row0 + r) * p.N + col) =
+                    make_uint2(pack2(__uint_as_float(f[0]), __uint_as_float(f[1])), pack2(__uint_as_float(f[2]), __uint_as_float(f[3])));
+            }
             if constexpr (EPI == GEPI_RESIDUAL || EPI == GEPI_BIAS) {
               const uint4 w = add[EPI == GEPI_BIAS ? 0 : k];
               v = make_uint4(add_bf16x2(w.x, v.x), add_bf16x2(w.y, v.y), add_bf16x2(w.z, v.z), add_bf16x2(w.w, v.w));
@@ -452,6 +471,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       if (EPI == GEPI_STORE && p.bias != nullptr) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] += p.bias[col + j];
+      }
+      if constexpr (EPI == GEPI_ACCUM) {
+        const float4 x = reinterpret_cast<const float4*>(p.C + o)[0], y = reinterpret_cast<const float4*>(p.C + o)[1];
+        v[0] = fmaf(p.mult, v[0], x.x); v[1] = fmaf(p.mult, v[1], x.y); v[2] = fmaf(p.mult, v[2], x.z); v[3] = fmaf(p.mult, v[3], x.w);
+        v[4] = fmaf(p.mult, v[4], y.x); v[5] = fmaf(p.mult, v[5], y.y); v[6] = fmaf(p.mult, v[6], y.z); v[7] = fmaf(p.mult, v[7], y.w);
+      }
+      if constexpr (EPI == GEPI_LOGITS) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = cap_logit(v[j], p.mult);
+        *reinterpret_cast<uint4*>(p.c2 + o) = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
       }
       if constexpr (sizeof(OT) == 4) {
         reinterpret_cast<float4*>(p.C + o)[0] = make_float4(v[0], v[1], v[2], v[3]);
@@ -676,6 +705,20 @@ int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t
 }
 int launch_gemm_bf16_f32(float* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   return launch_gemm_store<float>(C, A, B, bias, M, N, K, st);
+}
+
+int launch_gemm_bf16_accum(float* C, const void* A, const void* B, float mult, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
+  int rc = check_gemm(C, A, B, M, N, K);
+  if (rc != B200_OK) return rc;
+  return launch_gemm<float, GEPI_ACCUM>(GemmArgs<float>{C, nullptr, nullptr, (int)M, (int)N, (int)K, nullptr, mult}, A, B, N, false, st);
+}
+int launch_gemm_bf16_logits(float* C, void* C_bf16, const void* A, const void* B, float softcap, int64_t M, int64_t N, int64_t K,
+                            cudaStream_t st) {
+  int rc = check_gemm(C, A, B, M, N, K);
+  if (rc != B200_OK) return rc;
+  B200_CHECK_ARG(C_bf16 && aligned16(C_bf16), "gemm: bad bf16 logits");
+  return launch_gemm<float, GEPI_LOGITS>(GemmArgs<float>{C, nullptr, nullptr, (int)M, (int)N, (int)K, nullptr, softcap, (__nv_bfloat16*)C_bf16}, A,
+                                         B, N, false, st);
 }
 
 }  // namespace b200

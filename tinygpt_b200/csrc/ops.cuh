@@ -52,6 +52,10 @@ int launch_gemm_bf16_bias(void* C, const void* A, const void* B, const float* bi
 // the same products handed out as fp32 sums: C = A·Bᵀ + bias (bias may be null)
 int launch_gemm_bf16_f32(float* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st);
 
+// C += mult·(A·Bᵀ) in fp32;  C = capped A·Bᵀ in fp32 and C_bf16 = bf16(C) (softcap 0: no cap)
+int launch_gemm_bf16_accum(float* C, const void* A, const void* B, float mult, int64_t M, int64_t N, int64_t K, cudaStream_t st);
+int launch_gemm_bf16_logits(float* C, void* C_bf16, const void* A, const void* B, float softcap, int64_t M, int64_t N, int64_t K,
+                            cudaStream_t st);
 // A Linear of the prompt pass with what follows it on its store, each with its own rounding: C = bf16(A·Bᵀ), then bf16(C + bias [N]),
 // bf16(add [M, N] + C) (C may be add), or — B holding N gate rows and N up rows — bf16(bf16(silu(gate))·up).  A row's result does
 // not depend on M.
