@@ -77,6 +77,19 @@ int launch_attn_prefill_window(void* o, int64_t o_rs, const void* q, const void*
                                const void* kcache, const void* vcache, int S, int Hq, int Hkv, int hd, int p0, float scale,
                                int window, int keep_first, cudaStream_t st, int sink = 0, float softcap = 0.f,
                                const float* slopes = nullptr);
+// ---- tcgen05 prefill attention (prefill_attn_tc.cu): strides in elements; keys 0 … p0 + S − 1 of every batch element
+struct TcPrefillAttn {
+  __nv_bfloat16* o;
+  const __nv_bfloat16 *q, *k, *v;
+  const __nv_bfloat16* gate;    // per-head gate logits at the rows' stride, or null
+  int64_t o_rs, o_bs, q_rs, q_bs, kv_rs, kv_bs;
+  int B, S, Hq, Hkv, p0;
+  float scale_log2;             // score scale × log2(e)
+  int window, keep_first, sink;
+};
+bool prefill_attn_tc_ok(const TcPrefillAttn& a, int hd);     // head size, alignment and strides it takes
+bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd);   // against launch_pf's mma.sync kernel
+int launch_prefill_attn_tc(const TcPrefillAttn& a, int hd, cudaStream_t st);
 bool prefill_window_ok(int hd);   // head sizes launch_attn_prefill_window takes
 int launch_attn_causal_mma(void* o, const void* q, const void* k, const void* v, int64_t B, int64_t S, int64_t Hq,
                            int64_t Hkv, int64_t hd, cudaStream_t st);

@@ -343,7 +343,13 @@ __global__ void __launch_bounds__(kPfThreads) attn_prefill_mma_kernel(const Pref
 }
 
 template <int HD, bool SCORE = false>
-int launch_pf(const PrefillAttnParams& p, int B, cudaStream_t st) {
+int launch_pf(const PrefillAttnParams& p, int B, cudaStream_t st, bool same_bits = false) {
+  if constexpr (!SCORE && HD != 96) {
+    const TcPrefillAttn t{p.o, p.q, p.k, p.v, p.gate, p.o_rs, p.o_bs, p.q_rs, p.q_bs, p.kv_rs, p.kv_bs, B, p.S, p.Hq, p.Hkv, p.p0,
+                          p.scale_log2, p.window, p.keep_first, p.sink};
+    // "tc" | "mma" forces a side; the Llama engine's prompt pass stays on mma.sync: its keys and values keep the bits they always had
+    if (!same_bits && prefill_attn_tc_ok(t, HD) && env_choice("B200_ATTN_TC", 't', prefill_attn_tc_wins(t, HD))) return launch_prefill_attn_tc(t, HD, st);
+  }
   constexpr int smem_max = (kBM + 4 * kBN) * row_bytes<HD>();
   const int smem = SCORE && p.same ? (kBM + 2 * kBN) * row_bytes<HD>() : smem_max;
   static std::once_flag once;   // one per instantiation; the reference's server has a worker thread next to main
@@ -383,7 +389,7 @@ int launch_attn_prefill_mma(void* o, const void* qkv, const void* kcache, const 
   p.Hkv = Hkv;
   p.p0 = p0;
   p.scale_log2 = hd == 64 ? PfScale<64>::value : PfScale<128>::value;
-  return hd == 64 ? launch_pf<64>(p, 1, st) : launch_pf<128>(p, 1, st);
+  return hd == 64 ? launch_pf<64>(p, 1, st, true) : launch_pf<128>(p, 1, st, true);
 }
 
 // Layer-stack models: one sequence's rows of a step (positions p0 … p0+S-1) against that sequence's cache, with an
