@@ -690,18 +690,19 @@ int launch_gemm_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N
 int launch_gemm_bf16_bias(void* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   return launch_gemm_store<__nv_bfloat16>((__nv_bfloat16*)C, A, B, bias, M, N, K, st);
 }
-int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, LinearTail tail, const void* add, cudaStream_t st) {
+int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, LinearTail tail, const void* add, cudaStream_t st,
+                       bool whole_k) {
   int rc = check_gemm(C, A, B, M, N, K);
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG((tail == LinearTail::bias || tail == LinearTail::residual) == (add != nullptr) && aligned16(add), "linear: bad operand of the tail");
   const GemmArgs<__nv_bfloat16> p{(__nv_bfloat16*)C, nullptr, (const __nv_bfloat16*)add, (int)M, (int)N, (int)K, nullptr};
   switch (tail) {
-    case LinearTail::bias: return launch_gemm<__nv_bfloat16, GEPI_BIAS>(p, A, B, N, true, st);
-    case LinearTail::residual: return launch_gemm<__nv_bfloat16, GEPI_RESIDUAL>(p, A, B, N, true, st);
-    case LinearTail::silu_mul: return launch_gemm<__nv_bfloat16, GEPI_SILU>(p, A, B, 2 * N, true, st);
+    case LinearTail::bias: return launch_gemm<__nv_bfloat16, GEPI_BIAS>(p, A, B, N, whole_k, st);
+    case LinearTail::residual: return launch_gemm<__nv_bfloat16, GEPI_RESIDUAL>(p, A, B, N, whole_k, st);
+    case LinearTail::silu_mul: return launch_gemm<__nv_bfloat16, GEPI_SILU>(p, A, B, 2 * N, whole_k, st);
     case LinearTail::none: break;
   }
-  return launch_gemm<__nv_bfloat16, GEPI_STORE>(p, A, B, N, true, st);
+  return launch_gemm<__nv_bfloat16, GEPI_STORE>(p, A, B, N, whole_k, st);
 }
 int launch_gemm_bf16_f32(float* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   return launch_gemm_store<float>(C, A, B, bias, M, N, K, st);

@@ -389,6 +389,7 @@ KernelFn pick_r(int nseg, int pro, int epi) {
   if (nseg == 2 && pro == PRO_PLAIN && epi == EPI_SWIGLU) return gemv_batch_kernel<RPW, 2, PRO_PLAIN, EPI_SWIGLU>;
   if (nseg == 2) return (pro == PRO_RMSNORM && epi == EPI_SILU_MUL) ? gemv_batch_kernel<RPW, 2, PRO_RMSNORM, EPI_SILU_MUL> : nullptr;
   if (pro == PRO_RMSNORM && epi == EPI_PLAIN) return gemv_batch_kernel<RPW, 1, PRO_RMSNORM, EPI_PLAIN>;
+  if (pro == PRO_PLAIN && epi == EPI_PLAIN) return gemv_batch_kernel<RPW, 1, PRO_PLAIN, EPI_PLAIN>;
   if (pro == PRO_PLAIN && epi == EPI_RESIDUAL) return gemv_batch_kernel<RPW, 1, PRO_PLAIN, EPI_RESIDUAL>;
   if (pro == PRO_PLAIN && epi == EPI_BIAS_F32) return gemv_batch_kernel<RPW, 1, PRO_PLAIN, EPI_BIAS_F32>;
   if (pro == PRO_PLAIN && epi == EPI_RESID_F32) return gemv_batch_kernel<RPW, 1, PRO_PLAIN, EPI_RESID_F32>;

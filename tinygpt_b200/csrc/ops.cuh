@@ -57,10 +57,11 @@ int launch_gemm_bf16_accum(float* C, const void* A, const void* B, float mult, i
 int launch_gemm_bf16_logits(float* C, void* C_bf16, const void* A, const void* B, float softcap, int64_t M, int64_t N, int64_t K,
                             cudaStream_t st);
 // A Linear of the prompt pass with what follows it on its store, each with its own rounding: C = bf16(A·Bᵀ), then bf16(C + bias [N]),
-// bf16(add [M, N] + C) (C may be add), or — B holding N gate rows and N up rows — bf16(bf16(silu(gate))·up).  A row's result does
-// not depend on M.
+// bf16(add [M, N] + C) (C may be add), or — B holding N gate rows and N up rows — bf16(bf16(silu(gate))·up).  whole_k: a row's result
+// does not depend on M (no split of K).
 enum class LinearTail { none, bias, residual, silu_mul };
-int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, LinearTail tail, const void* add, cudaStream_t st);
+int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, LinearTail tail, const void* add, cudaStream_t st,
+                       bool whole_k = true);
 
 // ---- prefill helpers (prefill.cu)
 int launch_bias_add(void* y, const void* b, int64_t rows, int64_t n, cudaStream_t st);
