@@ -1,0 +1,59 @@
+"""One query row through b200_attn_bf16 (csrc/attn.cu attn_row_kernel) against fp64 attention, at the edges of its splits: key counts around a pass, a
+cluster's share and several passes, one and two heads per CTA, both head sizes, and the causal form (row 0 sees key 0 only).  Probabilities
+are fp32, the result bf16: 2-norm error below 2⁻⁸.  And the fused decode kernel's merge of many splits."""
+import pytest
+import torch
+
+from tinygpt_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def randn(*shape, seed, std=1.0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return (torch.randn(*shape, generator=g, device=DEV) * std).to(torch.bfloat16)
+
+
+def attend(q, k, v):
+    group = q.shape[2] // k.shape[2]
+    k, v = k.double().repeat_interleave(group, 2), v.double().repeat_interleave(group, 2)
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k) * q.shape[-1] ** -0.5
+    return torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v)
+
+
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 33, 127, 128, 129, 255, 257, 1000, 2049, 5000])
+@pytest.mark.parametrize("B,Hq,Hkv,D", [(1, 14, 2, 64), (1, 3, 1, 128), (1, 16, 8, 128), (3, 64, 8, 64), (5, 32, 8, 128)])
+def test_one_row(built_lib, n, B, Hq, Hkv, D):
+    q, k, v = randn(B, 1, Hq, D, seed=n, std=2.0), randn(B, n, Hkv, D, seed=1), randn(B, n, Hkv, D, seed=2)
+    got = ops.flash_attention(q, k, v, False)
+    want = attend(q, k, v)
+    assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -8
+    assert torch.equal(got, ops.flash_attention(q, k, v, False))
+    first = ops.flash_attention(q, k, v, True)
+    assert torch.equal(first, v[:, :1].repeat_interleave(Hq // Hkv, 2))
+
+
+def test_huge_scores_and_zeros(built_lib):
+    """Scores thousands apart (one key takes all), equal scores, and a row of zeros."""
+    q = torch.full((1, 1, 2, 64), 8.0, device=DEV, dtype=torch.bfloat16)
+    k, v = randn(1, 700, 1, 64, seed=3, std=20.0), randn(1, 700, 1, 64, seed=4)
+    want = attend(q, k, v)
+    got = ops.flash_attention(q, k, v, False)
+    assert float((got.double() - want).abs().max()) <= 2.0 ** -7 * float(v.float().abs().max())
+    flat = ops.flash_attention(q * 0, k, v, False).double()
+    assert float((flat - attend(q * 0, k, v)).abs().max()) < 2.0 ** -9
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,at", [(6, 2, 128, 1023), (6, 2, 128, 1025), (14, 2, 64, 2400), (24, 8, 128, 4000), (8, 8, 128, 3999)])
+def test_fused_decode_merges_many_splits(built_lib, Hq, Hkv, D, at):
+    ctx = 4096
+    qkv = randn((Hq + 2 * Hkv) * D, seed=5, std=1.5)
+    kc, vc = randn(ctx, Hkv, D, seed=6), randn(ctx, Hkv, D, seed=7)
+    pos = torch.tensor([at], dtype=torch.int32, device=DEV)
+    got = ops.attn_decode(qkv, kc, vc, q_heads=Hq, kv_heads=Hkv, head_dim=D, pos=pos)
+    q, k, v = (t.view(1, 1, -1, D) for t in qkv.split([Hq * D, Hkv * D, Hkv * D]))
+    want = attend(q, torch.cat([kc[None, :at], k], 1), torch.cat([vc[None, :at], v], 1)).reshape(-1)
+    assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -8
+    assert torch.equal(kc[at], k[0, 0]) and torch.equal(vc[at], v[0, 0])
+    assert torch.equal(got, ops.attn_decode(qkv, kc, vc, q_heads=Hq, kv_heads=Hkv, head_dim=D, pos=pos))

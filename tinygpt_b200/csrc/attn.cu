@@ -14,6 +14,7 @@
 // reference's.  Probabilities stay fp32 (the reference rounds P to bf16 before P·V, TFA/mma/layout.cuh:88-97); the
 // oracle models the reference's rounding and the parity tests bound the difference.
 #include "ops.cuh"
+#include "tc.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -292,6 +293,273 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_reg_kernel(const Att
   if (tid == 0) p.tickets[hg] = 0;
 }
 
+// ------------------------------------------------------------------------------- one query row over many keys
+// One new row against every key, probabilities in fp32, as (a) o = softmax(q·kᵀ)·v for Sq = 1 through the operator boundary and (b) the fused decode
+// attention over long contexts (q/k norm, rotation and the in-place append as in attn_decode_reg_kernel).
+// A cluster shares a (sequence, group of G query heads of one KV head): its CTAs take neighbouring ranges of the keys that exist now, every
+// thread holds 16-byte pieces of U keys' K and V rows while the next U are on their way, and runs an online softmax over its own
+// keys; the key groups of a warp merge by shuffles, the warps through shared memory and the CTAs through distributed shared
+// memory — no workspace, no tickets, one launch.  Bound by the latency of a few rounds of loads.
+// (a) 16 / 8 heads of 128 over 2 049 keys: 94 µs with one CTA per head walking 128 keys at a time, 8.1 µs like this (8.4 MB); 4 × 32 heads over
+// 4 096 keys 469 → 48 µs.  (b) 24 / 8 heads at position 4 000 of 4 096: 27.7 µs with one CTA per 128 keys and a merge by the last of 32,
+// 13.3 µs like this.
+struct AttnRow {
+  AttnDecodeParams d;               // decode: everything; row: qkv = q [B, Hq, HD], out, kcache / vcache and the strides
+  int nkeys;                        // row: keys to see (decode reads the position)
+  long long kv_bstride;             // elements from one batch element's keys to the next
+};
+// a load that stays where it is written: the rows of a round are requested before the first of them is used
+__device__ __forceinline__ uint4 load_ahead(const __nv_bfloat16* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+template <int HD, int G, bool DECODE>
+__global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(const AttnRow a) {
+  constexpr int LPK = HD / 8;             // lanes per key row
+  constexpr int NG = kAttnThreads / LPK;  // key rows per pass
+  constexpr int U = 4;                    // passes per round
+  constexpr int EPL = HD / 32;
+  constexpr float kScale = InvSqrtHd<HD>::value * kLog2e;
+  __shared__ float q_s[G][HD];
+  __shared__ __align__(16) __nv_bfloat16 knew[HD];
+  __shared__ __align__(16) __nv_bfloat16 vnew[HD];
+  __shared__ __align__(16) float w_acc[kAttnWarps][HD];
+  __shared__ float w_ml[kAttnWarps][2];
+  __shared__ __align__(16) float res[G][HD];
+  __shared__ __align__(16) float res_ml[G][4];
+  __shared__ float weight[G][8], total[G];   // of the cluster's CTAs; the sum of all
+  const AttnDecodeParams& p = a.d;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, part = tid % LPK, grp = tid / LPK;
+  const int h0 = blockIdx.y * G, kvh = h0 / (p.Hq / p.Hkv);
+  const long long b = blockIdx.z;
+  const int rank = (int)cluster_rank(), splits = (int)gridDim.x;
+  if (DECODE) pdl_trigger();
+  const bool append = DECODE && p.pos != nullptr;
+  const int pos = append ? *p.pos : 0;     // stable since before the producer kernel started
+  const int nkeys = append ? pos : DECODE ? p.fixed_len : a.nkeys;   // rows that are in the cache already
+  const int per = ((nkeys + splits - 1) / splits + NG - 1) / NG * NG;
+  const int k0 = min(nkeys, rank * per), k1 = min(nkeys, k0 + per);
+  const size_t base = (size_t)(b * a.kv_bstride) + (size_t)kvh * HD + part * 8, ks = (size_t)p.Hkv * HD;
+  uint4 kr[2][U], vr[2][U];
+  auto fetch = [&](int buf, int c) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const size_t j = (size_t)min(c + u * NG + grp, k1 - 1);   // past the range: its last key once more, without weight
+      kr[buf][u] = load_ahead(p.kcache + base + j * ks);
+      vr[buf][u] = load_ahead(p.vcache + base + j * ks);
+    }
+  };
+  if (k0 < k1) fetch(0, k0);               // rows of earlier tokens: nothing that the producer kernel writes
+  const __nv_bfloat16* qkv = p.qkv + b * p.qkv_bstride;
+  const bool owns_new = append && rank == splits - 1;
+  if constexpr (DECODE) {
+    float rc[EPL / 2], rs[EPL / 2];
+    if (p.rope != nullptr) {
+      const float* row = p.rope + (size_t)pos * HD * 2;
+#pragma unroll
+      for (int j = 0; j < EPL / 2; ++j) {
+        rc[j] = row[(lane + 32 * j) * 2];
+        rs[j] = row[(lane + 32 * j) * 2 + 1];
+      }
+    }
+    pdl_wait();                            // qkv of this token is complete and visible from here on
+    const int qdim = p.Hq * HD, kvdim = p.Hkv * HD;
+    for (int h = warp; h < G + 1; h += kAttnWarps) {
+      const bool is_k = h == G;
+      if (is_k && !owns_new) break;
+      const __nv_bfloat16* src = is_k ? qkv + qdim + kvh * HD : qkv + (h0 + h) * HD;
+      const __nv_bfloat16* nw = is_k ? p.k_norm : p.q_norm;
+      float x[EPL];
+#pragma unroll
+      for (int j = 0; j < EPL; ++j) x[j] = bf16_to_f(src[lane + 32 * j]);
+      if (nw != nullptr) {
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) ss += x[j] * x[j];
+        ss = warp_sum(ss);
+        const float inv = rsqrtf(ss / (float)HD + p.eps);
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) x[j] = round_bf16(x[j] * inv * bf16_to_f(nw[lane + 32 * j]));
+      }
+      if (p.rope != nullptr) {
+#pragma unroll
+        for (int j = 0; j < EPL / 2; ++j) {
+          const float x1 = x[j], x2 = x[j + EPL / 2];
+          x[j] = round_bf16(x1 * rc[j] - x2 * rs[j]);
+          x[j + EPL / 2] = round_bf16(x2 * rc[j] + x1 * rs[j]);
+        }
+      }
+      if (is_k) {
+        const size_t at = (size_t)(b * a.kv_bstride) + ((size_t)pos * p.Hkv + kvh) * HD;
+        const bool leader = h0 % (p.Hq / p.Hkv) == 0;   // one CTA writes the new cache row
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) {
+          const __nv_bfloat16 kk = f_to_bf16(x[j]), vv = qkv[qdim + kvdim + kvh * HD + lane + 32 * j];
+          knew[lane + 32 * j] = kk;
+          vnew[lane + 32 * j] = vv;
+          if (leader) {
+            p.kcache[at + lane + 32 * j] = kk;
+            p.vcache[at + lane + 32 * j] = vv;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < EPL; ++j) q_s[h][lane + 32 * j] = x[j];
+      }
+    }
+  } else {
+    for (int i = tid; i < G * HD; i += kAttnThreads) (&q_s[0][0])[i] = bf16_to_f(qkv[h0 * HD + i]);
+  }
+  __syncthreads();
+  float qf[G][8], m[G], l[G], acc[G][8];
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    m[g] = -INFINITY;
+    l[g] = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      qf[g][e] = q_s[g][part * 8 + e];
+      acc[g][e] = 0.f;
+    }
+  }
+  auto round = [&](int buf, int c) {
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      float sc[U], top = m[g];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        sc[u] = dot8(kr[buf][u], qf[g], 0.f);
+#pragma unroll
+        for (int o = LPK / 2; o > 0; o >>= 1) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o);
+        if (c + u * NG + grp >= k1) sc[u] = -INFINITY;
+        top = fmaxf(top, sc[u]);
+      }
+      const float ts = top == -INFINITY ? 0.f : top * kScale;
+      const float alpha = m[g] == -INFINITY ? 0.f : exp2f(m[g] * kScale - ts);
+      m[g] = top;
+      l[g] *= alpha;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[g][e] *= alpha;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool in = c + u * NG + grp < k1;
+        const float pr = in ? exp2f(sc[u] * kScale - ts) : 0.f;
+        l[g] += pr;
+        float vf[8];
+        unpack8(in ? vr[buf][u] : make_uint4(0, 0, 0, 0), vf);   // a key without weight meets no value
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[g][e] = fmaf(pr, vf[e], acc[g][e]);
+      }
+    }
+  };
+  for (int c = k0; c < k1; c += 2 * NG * U) {
+    if (c + NG * U < k1) fetch(1, c + NG * U);
+    round(0, c);
+    if (c + NG * U >= k1) break;
+    if (c + 2 * NG * U < k1) fetch(0, c + 2 * NG * U);
+    round(1, c + NG * U);
+  }
+  if (owns_new && warp == 0) {             // the new row, from shared memory: one more key of the first key group
+    const uint4 kn = reinterpret_cast<const uint4*>(knew)[part], vn = reinterpret_cast<const uint4*>(vnew)[part];
+    float vf[8];
+    unpack8(vn, vf);
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      float sc = dot8(kn, qf[g], 0.f);
+#pragma unroll
+      for (int o = LPK / 2; o > 0; o >>= 1) sc += __shfl_xor_sync(0xffffffffu, sc, o);
+      if (grp != 0) continue;
+      const float top = fmaxf(m[g], sc);
+      const float alpha = m[g] == -INFINITY ? 0.f : exp2f((m[g] - top) * kScale), pr = exp2f(sc * kScale - top * kScale);
+      m[g] = top;
+      l[g] = l[g] * alpha + pr;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[g][e] = fmaf(pr, vf[e], acc[g][e] * alpha);
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+#pragma unroll
+    for (int o = LPK; o < 32; o <<= 1) {   // key groups that live in the same warp
+      const float mo = __shfl_xor_sync(0xffffffffu, m[g], o), lo = __shfl_xor_sync(0xffffffffu, l[g], o);
+      const float top = fmaxf(m[g], mo);
+      const float fa = m[g] == -INFINITY ? 0.f : exp2f((m[g] - top) * kScale), fb = mo == -INFINITY ? 0.f : exp2f((mo - top) * kScale);
+      l[g] = l[g] * fa + lo * fb;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[g][e] = acc[g][e] * fa + __shfl_xor_sync(0xffffffffu, acc[g][e], o) * fb;
+      m[g] = top;
+    }
+    __syncthreads();   // the previous head's partials have been read
+    if (lane < LPK) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) w_acc[warp][lane * 8 + e] = acc[g][e];
+      if (lane == 0) {
+        w_ml[warp][0] = m[g];
+        w_ml[warp][1] = l[g];
+      }
+    }
+    __syncthreads();
+    if (tid < HD) {
+      float top = -INFINITY, num = 0.f, den = 0.f;
+#pragma unroll
+      for (int w = 0; w < kAttnWarps; ++w) top = fmaxf(top, w_ml[w][0]);
+#pragma unroll
+      for (int w = 0; w < kAttnWarps; ++w) {
+        const float f = w_ml[w][0] == -INFINITY ? 0.f : exp2f((w_ml[w][0] - top) * kScale);
+        num = fmaf(f, w_acc[w][tid], num);
+        den = fmaf(f, w_ml[w][1], den);
+      }
+      res[g][tid] = num;
+      if (tid == 0) {
+        res_ml[g][0] = top;
+        res_ml[g][1] = den;
+      }
+    }
+  }
+  __syncthreads();
+  cluster_sync_all();   // every CTA's part is in place
+  if (tid < G * 8) {    // one lane per (head, CTA)
+    const int g = tid / 8, r = tid % 8;
+    float4 ml = make_float4(-INFINITY, 0.f, 0.f, 0.f);
+    if (r < splits) ml = ld_cluster_f4(mapa_u32(smem_u32(&res_ml[g][0]), r));
+    float top = ml.x;
+    constexpr unsigned mask = (1u << (G * 8)) - 1u;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(mask, top, o));
+    const float f = ml.x == -INFINITY ? 0.f : exp2f((ml.x - top) * kScale);
+    float den = f * ml.y;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) den += __shfl_xor_sync(mask, den, o);
+    weight[g][r] = f;
+    if (r == 0) total[g] = den;
+  }
+  __syncthreads();
+  for (int i = rank * kAttnThreads + tid; i < G * HD / 4; i += splits * kAttnThreads) {   // four neighbouring outputs
+    const int g = i / (HD / 4), d = (i % (HD / 4)) * 4;
+    float4 x[8], num = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) x[r] = r < splits ? ld_cluster_f4(mapa_u32(smem_u32(&res[g][d]), r)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float f = weight[g][r];
+      num.x = fmaf(f, x[r].x, num.x);
+      num.y = fmaf(f, x[r].y, num.y);
+      num.z = fmaf(f, x[r].z, num.z);
+      num.w = fmaf(f, x[r].w, num.w);
+    }
+    const float inv = total[g] > 0.f ? 1.f / total[g] : 0.f;
+    __nv_bfloat16* o = p.out + b * p.out_bstride + (h0 + g) * HD + d;
+    o[0] = f_to_bf16(num.x * inv);
+    o[1] = f_to_bf16(num.y * inv);
+    o[2] = f_to_bf16(num.z * inv);
+    o[3] = f_to_bf16(num.w * inv);
+  }
+  __syncthreads();
+  cluster_sync_all();   // no CTA leaves while another still reads its part
+}
+
 // ------------------------------------------------------------------------------------------ general attention
 // One CTA per (q row, head, batch); keys in chunks of 128 with online softmax.  Correctness path (prefill-shaped
 // calls through b200_attn_bf16); the tensor-core prefill kernel is separate work.
@@ -356,8 +624,14 @@ __global__ void __launch_bounds__(128) attn_general_kernel(__nv_bfloat16* __rest
 
 }  // namespace
 
+// Contexts from which the cluster kernel takes over: more splits than this (1 024 tokens for heads of 128, 2 048 for heads of 64).  µs, one CTA per split /
+// cluster: position 2 200 of 2 304, 16 heads 12.8 / 9.9; 4 000 of 4 096, 24 heads 27.7 / 13.3, 32 heads 31.2 / 13.3; 500 of 4 096, 32
+// heads 14.5 / 7.4.
+constexpr int kLongSplits = 8;
+
 int64_t attn_decode_ws_floats(int Hq, int Hkv, int hd, int nsplit) {
   (void)Hkv;
+  if (nsplit > kLongSplits) return 0;      // the cluster kernel keeps its partials in shared memory
   return (int64_t)Hq * nsplit * (hd + 2);  // same size whatever the head grouping
 }
 
@@ -379,6 +653,55 @@ int attn_decode_nsplit(int hd, int max_ctx) {
   return std::max(1, (max_ctx + chunk - 1) / chunk);
 }
 
+template <int HD, int G, bool DECODE>
+static int launch_row_t(const AttnRow& a, int splits, int B, cudaStream_t st, bool pdl) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)splits, (unsigned)(a.d.Hq / G), (unsigned)B);
+  cfg.blockDim = dim3(kAttnThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)splits;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 2 : 1;
+  g_launches.fetch_add(1);
+  B200_CUDA(cudaLaunchKernelEx(&cfg, attn_row_kernel<HD, G, DECODE>, a));
+  return B200_OK;
+}
+// A CTA per query head, or per two heads of a KV head once that leaves 64 of them (K and V are read through L2 once per CTA).
+static int launch_row(const AttnRow& a, int hd, int splits, int B, bool decode, cudaStream_t st, bool pdl) {
+  const bool two = (a.d.Hq / a.d.Hkv) % 2 == 0 && (int64_t)(a.d.Hq / 2) * B >= 64;
+  if (hd == 64) {
+    if (decode) return two ? launch_row_t<64, 2, true>(a, splits, B, st, pdl) : launch_row_t<64, 1, true>(a, splits, B, st, pdl);
+    return two ? launch_row_t<64, 2, false>(a, splits, B, st, pdl) : launch_row_t<64, 1, false>(a, splits, B, st, pdl);
+  }
+  if (decode) return two ? launch_row_t<128, 2, true>(a, splits, B, st, pdl) : launch_row_t<128, 1, true>(a, splits, B, st, pdl);
+  return two ? launch_row_t<128, 2, false>(a, splits, B, st, pdl) : launch_row_t<128, 1, false>(a, splits, B, st, pdl);
+}
+// One query row: as many CTAs per cluster (≤ 8) as keep 64 keys each and no more than two CTAs per SM.
+static int launch_attn_row(void* o, const void* q, const void* k, const void* v, int64_t B, int64_t Skv, int64_t Hq, int64_t Hkv, int64_t hd,
+                           int causal, cudaStream_t st) {
+  B200_CHECK_ARG(hd == 64 || hd == 128, "attention: head_dim %lld not built (64 and 128 are)", (long long)hd);
+  B200_CHECK_ARG(B > 0 && Skv > 0 && Hkv > 0 && Hq % Hkv == 0 && Hq < 65536 && B < 65536, "attention: bad shape");
+  B200_CHECK_ARG(Skv < (1ll << 30), "attention: too many keys");
+  AttnRow a{};
+  a.d.qkv = (const __nv_bfloat16*)q;
+  a.d.out = (__nv_bfloat16*)o;
+  a.d.kcache = const_cast<__nv_bfloat16*>((const __nv_bfloat16*)k);   // read only
+  a.d.vcache = const_cast<__nv_bfloat16*>((const __nv_bfloat16*)v);
+  a.d.Hq = (int)Hq;
+  a.d.Hkv = (int)Hkv;
+  a.d.qkv_bstride = a.d.out_bstride = Hq * hd;
+  a.kv_bstride = Skv * Hkv * hd;
+  a.nkeys = causal ? 1 : (int)Skv;   // causal: the mask is top-left aligned, row 0 sees key 0
+  int splits = 1;
+  while (splits < 8 && a.nkeys >= 128 * splits && Hq * B * splits * 2 <= 296) splits *= 2;
+  return launch_row(a, (int)hd, splits, (int)B, false, st, false);
+}
+
 int launch_attn_decode(const AttnDecodeParams& p, int hd, cudaStream_t st, bool pdl) {
   B200_CHECK_ARG(hd == 64 || hd == 128, "attention: head_dim %d not built (64 and 128 are, like the reference)", hd);
   B200_CHECK_ARG(p.Hkv > 0 && p.Hq % p.Hkv == 0, "attention: Hq=%d must be a multiple of Hkv=%d", p.Hq, p.Hkv);
@@ -390,6 +713,10 @@ int launch_attn_decode(const AttnDecodeParams& p, int hd, cudaStream_t st, bool 
   B200_CHECK_ARG(p.nsplit <= 65535, "attention: context too long");
   B200_CHECK_ARG(G >= 1 && G <= 8, "attention: at most 8 query heads per CTA (got %d)", G);
   const unsigned nb = (unsigned)std::max(1, p.batch);
+  if (p.nsplit > kLongSplits) {
+    AttnRow a{p, 0, p.cache_bstride};
+    return launch_row(a, hd, 8, (int)nb, true, st, pdl);
+  }
   if (hd == 64)
     B200_CUDA(launch_pdl(attn_decode_reg_kernel<64>, dim3(p.nsplit, p.Hq / G, nb), dim3(kAttnThreads), 0, st, pdl, p, G));
   else
@@ -423,5 +750,6 @@ extern "C" int b200_attn_bf16(void* o, const void* q, const void* k, const void*
   B200_CHECK_ARG(o && q && k && v, "attention: null pointer");
   if (causal && Sq == Skv && Sq > 1 && prefill_attn_mma_enabled())
     return launch_attn_causal_mma(o, q, k, v, B, Sq, Hq, Hkv, hd, (cudaStream_t)stream);
+  if (Sq == 1) return launch_attn_row(o, q, k, v, B, Skv, Hq, Hkv, hd, causal, (cudaStream_t)stream);
   return launch_attn_general(o, q, k, v, B, Sq, Skv, Hq, Hkv, hd, causal, (cudaStream_t)stream);
 }
