@@ -15,8 +15,15 @@ from ._lib import B200Error, check, lib
 BSHD, BHSD = 1, 0  # b200_qkv_layout
 
 
+# The current stream's handle.  The raw getter (0.1 µs, what torch's own code generators use) is the handle of the same stream that
+# torch.cuda.current_stream() wraps into a Python object first (3.2 µs, a quarter of a small op's call).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _chk(t: torch.Tensor, name: str, dtype=torch.bfloat16) -> torch.Tensor:
