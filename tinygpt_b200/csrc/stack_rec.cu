@@ -106,155 +106,6 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(const AttnPrep p) {
 }
 
 // ------------------------------------------------------------------------------------------------------------ the scan
-// With a removal: one warp per (sequence, head, NC value columns): lane l holds rows l, l + 32, … of its columns of S (DR rows per lane and
-// column); 8·NC columns per CTA.  The CTA walks its sequence CH tokens at a time: the chunk's decay, key, query (and removal,
-// unit key) rows (fp32, zero past dk) and the CTA's columns of v sit in shared memory, staged once for all eight warps,
-// while the next chunk's values are already on their way into registers — the walk waits for memory once per sequence.  A
-// token costs a warp the removal's dot with the OLD columns (warp sums the update waits for, NC side by side), DR
-// multiply-adds per operand and column, and the output's dot with the NEW columns.  Columns never read each other, so
-// the result of a sequence does not depend on what else is in the step; the order of the sums inside a column is fixed by
-// dk alone (lane l sums rows l, l + 32, …, then the butterfly), whatever NC is.
-template <int DR, int NC>
-__global__ void __launch_bounds__(256, 2) lin_scan_kernel(const LinScan p) {
-  pdl_trigger();
-  pdl_wait();
-  constexpr int DK = 32 * DR;
-  // tokens per chunk: what 4 KB of one operand hold, 4 … 32 — the next chunk waits in registers, and two CTAs share an SM
-  constexpr int CH0 = 1024 / DK;
-  constexpr int CH = CH0 > 32 ? 32 : CH0 < 4 ? 4 : CH0;
-  constexpr int NV = 5;                                   // staged vectors per token: d, b, r, p, q
-  constexpr int NQ = CH * NV * DK / 256;                  // staged vector elements per thread and chunk
-  constexpr int COLS = 8 * NC;
-  constexpr int NVR = (CH * COLS + 255) / 256;            // staged values per thread and chunk
-  __shared__ float s_x[CH][NV][DK];
-  __shared__ float s_v[CH][COLS];
-  const int seg = blockIdx.x, hd = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
-  const int dk = p.dk, dv = p.dv;
-  const int j0 = blockIdx.z * COLS, jw = j0 + warp * NC;
-  const int r0 = p.seg_row0 != nullptr ? p.seg_row0[seg] : seg;
-  const int cnt = p.seg_count != nullptr ? p.seg_count[seg] : 1;
-  float* st = p.state + (int64_t)p.slot[r0] * p.slot_stride + (int64_t)hd * dk * dv;
-  const bool fresh = p.pos[r0] == 0;
-  float S[NC][DR];
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-#pragma unroll
-    for (int i = 0; i < DR; ++i) {
-      const int d = lane + 32 * i;
-      S[c][i] = (jw + c < dv && !fresh && d < dk) ? st[(int64_t)d * dv + jw + c] : 0.f;
-    }
-  }
-  const int hs = hd / p.share;   // the head whose b / r vectors this head reads
-  const float* src_d = p.d_scalar ? p.d + hd : p.d + (int64_t)hd * dk;
-  const float* src_b = p.b + (int64_t)hs * dk;
-  const float* src_r = p.r + (int64_t)hs * dk;
-  const float* src_p = p.p + (int64_t)hd * dk;
-  const float* src_q = p.q + (int64_t)(p.q_shared ? hs : hd) * dk;
-  float r_x[NQ], r_v[NVR];
-  auto fetch = [&](int c0) {
-#pragma unroll
-    for (int i = 0; i < NQ; ++i) {
-      const int e = tid + 256 * i, t = e / (NV * DK), w = (e / DK) % NV, d = e % DK;
-      float val = 0.f;
-      if (c0 + t < cnt && d < dk) {
-        const int64_t base = (int64_t)(r0 + c0 + t) * p.ld;
-        const float* src = w == 0 ? src_d : w == 1 ? src_b : w == 2 ? src_r : w == 3 ? src_p : src_q;
-        val = src[base + ((w == 0 && p.d_scalar) ? 0 : d)];
-      }
-      r_x[i] = val;
-    }
-#pragma unroll
-    for (int i = 0; i < NVR; ++i) {
-      const int e = tid + 256 * i, t = e / COLS, c = j0 + e % COLS;
-      float val = 0.f;
-      if (e < CH * COLS && c0 + t < cnt && c < dv) {
-        const int64_t base = (int64_t)(r0 + c0 + t) * p.ld;
-        val = p.v[base + (int64_t)hd * dv + c];
-        if (p.vscale != nullptr) val *= p.vscale[base + hd];
-      }
-      r_v[i] = val;
-    }
-  };
-  fetch(0);
-  for (int c0 = 0; c0 < cnt; c0 += CH) {
-    const int n = min(CH, cnt - c0);
-    __syncthreads();   // the previous chunk has been read
-#pragma unroll
-    for (int i = 0; i < NQ; ++i) (&s_x[0][0][0])[tid + 256 * i] = r_x[i];
-#pragma unroll
-    for (int i = 0; i < NVR; ++i)
-      if (tid + 256 * i < CH * COLS) (&s_v[0][0])[tid + 256 * i] = r_v[i];
-    __syncthreads();
-    if (c0 + CH < cnt) fetch(c0 + CH);
-    if (jw >= dv) continue;   // warps past the last column only help with the staging
-    for (int t4 = 0; t4 < n; t4 += 4) {   // the outputs' warp sums of four tokens run side by side, off the state's chain
-      float dot[4][NC];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int t = t4 + u;             // t < CH always (CH is a multiple of 4)
-#pragma unroll
-        for (int c = 0; c < NC; ++c) dot[u][c] = 0.f;
-        if (t >= n) continue;             // rows past the chunk's end hold zeros: they must not touch the state
-        float rem[NC], vj[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          rem[c] = 0.f;
-          vj[c] = s_v[t][warp * NC + c];
-        }
-#pragma unroll
-        for (int i = 0; i < DR; ++i) {
-          const float qq = s_x[t][4][lane + 32 * i];
-#pragma unroll
-          for (int c = 0; c < NC; ++c) rem[c] = fmaf(qq, S[c][i], rem[c]);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-          for (int c = 0; c < NC; ++c) rem[c] += __shfl_xor_sync(0xffffffffu, rem[c], o);
-        }
-#pragma unroll
-        for (int i = 0; i < DR; ++i) {
-          const int d = lane + 32 * i;
-          const float dd = s_x[t][0][d], bb = s_x[t][1][d], rr = s_x[t][2][d], pp = s_x[t][3][d];
-#pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            const float sn = fmaf(bb, vj[c], fmaf(-pp, rem[c], dd * S[c][i]));
-            S[c][i] = sn;
-            dot[u][c] = fmaf(sn, rr, dot[u][c]);
-          }
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-#pragma unroll
-          for (int c = 0; c < NC; ++c) dot[u][c] += __shfl_xor_sync(0xffffffffu, dot[u][c], o);
-        }
-      }
-      if (lane < 4 * NC) {                // lane u·NC + c hands out token t4 + u, column jw + c
-        const int u = lane / NC, c = lane % NC;
-        float mine = 0.f;
-#pragma unroll
-        for (int uu = 0; uu < 4; ++uu) {
-#pragma unroll
-          for (int cc = 0; cc < NC; ++cc) mine = (uu == u && cc == c) ? dot[uu][cc] : mine;
-        }
-        if (t4 + u < n && jw + c < dv) p.o[(int64_t)(r0 + c0 + t4 + u) * p.ld_o + (int64_t)hd * dv + jw + c] = mine;
-      }
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    if (jw + c >= dv) continue;
-#pragma unroll
-    for (int i = 0; i < DR; ++i) {
-      const int d = lane + 32 * i;
-      if (d < dk) st[(int64_t)d * dv + jw + c] = S[c][i];
-    }
-  }
-}
-
 // Without a removal no row of S waits for another: a CTA of NT threads takes kScanCols value columns of one (sequence, head), a
 // thread a tile of RS neighbouring rows and four neighbouring columns (an operand a thread reads from shared memory serves four
 // multiply-adds: the walk is bound by that traffic).  A token's output parts meet inside a warp by four shuffles per thread and,
@@ -484,6 +335,264 @@ int launch_scan_cols(const LinScan& p, cudaStream_t st) {
   if (p.read_old) return launch_scan_cols<RS, NT, 2, false>(p, st);
   if (p.d_minus_one) return launch_scan_cols<RS, NT, 1, false>(p, st);
   return p.d_scalar ? launch_scan_cols<RS, NT, 0, true>(p, st) : launch_scan_cols<RS, NT, 0, false>(p, st);
+}
+
+// With a removal every token needs the dot of its unit key with the whole column before it can touch the column: a serial chain of
+// one dot, its sum over lanes and one multiply-add per token, and few warps to hide it behind.  LN = 16 lanes share C = 2 neighbouring
+// columns (lane g holds rows 4g … 4g + 3 of every 4·LN): four shuffles to sum, and an operand that is read serves two columns —
+// shared loads and shuffles queue in one pipe, so one column per lane costs more (201 against 176 ns a token) although its chain
+// is shorter.  The decay and write of the old column and the output of the token before run beside the shuffles, the next token's
+// operands are asked for behind the last one, and the outputs of four tokens are summed together.  Keys past 256 take 32
+// lanes, 32 and less take 8: at most 16 rows a lane is what the registers hold.
+// A CTA has four such warps, one per scheduler, and a fifth that keeps kRemBuf chunks in flight: staging from the walking warps
+// costs them 60 ns a token, and bulk copies of a row were no faster than cp.async.  Columns never read each other, so the
+// result of a sequence does not depend on what else is in the step; the order of the sums inside a column is fixed by dk alone.  fp32 throughout.
+// 2 048 tokens, 16 heads, per-channel decay, against one warp per two columns with chunks staged through registers:
+// 128 × 128 1 091 → 374 µs (183 ns a token), 64 × 64 742 → 312 µs, 126 × 128 (copies of 4 bytes) 1 117 → 406 µs;
+// 64 sequences of one token 130 → 120 µs.
+constexpr int kRemBuf = 3, kRemThreads = 4 * 32 + 32;   // four warps that walk, one that stages
+template <int LN, int RPL, int C, bool SCALAR>
+struct ScanRem {
+  static constexpr int DK = LN * RPL, NV = SCALAR ? 4 : 5;   // staged vectors per token: q, b, p, r (, d)
+  static constexpr int COLS = 128 / LN * C, CH = DK <= 128 ? 16 : DK <= 256 ? 8 : 4;
+  static constexpr int FLOATS = CH * (NV * DK + COLS + 2);    // of a buffer: vectors, values (by column), value scales, scalar decays
+  static constexpr int smem = kRemBuf * FLOATS * 4;
+};
+__device__ __forceinline__ float shfl_xor_ordered(float v, int m) {   // stays in order with the loads below
+  float r;
+  asm volatile("shfl.sync.bfly.b32 %0, %1, %2, 0x1f, 0xffffffff;" : "=f"(r) : "f"(v), "r"(m));
+  return r;
+}
+__device__ __forceinline__ void lds_ordered(uint64_t& a, uint64_t& b, uint32_t addr) {
+  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
+}
+template <bool WIDE>
+__device__ __forceinline__ void copy_async(uint32_t dst, const float* src) {
+  if constexpr (WIDE) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+template <int LN, int RPL, int C, bool SCALAR>
+__global__ void __launch_bounds__(kRemThreads, 2) lin_scan_rem_kernel(const LinScan p, const bool wide) {
+  using F = ScanRem<LN, RPL, C, SCALAR>;
+  constexpr int DK = F::DK, NV = F::NV, CH = F::CH, COLS = F::COLS, NP = RPL / 2;
+  static_assert(4 * C <= LN && RPL % 4 == 0, "the outputs of four tokens are shared out over the lanes of a column");
+  pdl_trigger();
+  pdl_wait();
+  extern __shared__ __align__(16) float sm[];
+  const int seg = blockIdx.x, hd = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int dk = p.dk, dv = p.dv, z0 = blockIdx.z * COLS;
+  const int r0 = p.seg_row0 != nullptr ? p.seg_row0[seg] : seg;
+  const int cnt = p.seg_count != nullptr ? p.seg_count[seg] : 1;
+  const bool scaled = p.vscale != nullptr;
+  if (dk < DK) {   // rows past the key size: read with the others, never copied
+    for (int e = threadIdx.x; e < kRemBuf * F::FLOATS; e += kRemThreads) sm[e] = 0.f;
+    __syncthreads();
+  }
+  if (warp == 4) {
+    const int hs = hd / p.share;   // the head whose b / r vectors this head reads
+    const int64_t row0 = (int64_t)r0 * p.ld;
+    // One warp feeds four: what it issues per copy decides whether the walk waits.  Shared addresses are a register and a
+    // constant, and the tokens of a group share their row offset.
+    auto produce = [&](auto wide_copies) {
+      constexpr bool W = decltype(wide_copies)::value;
+      constexpr int STEP = W ? 128 : 32;   // floats of a row per copy of the warp
+      const int unit = W ? 4 * lane : lane;
+      const float* src[5] = {p.q + row0 + (int64_t)(p.q_shared ? hs : hd) * dk + unit, p.b + row0 + (int64_t)hs * dk + unit,
+                             p.p + row0 + (int64_t)hd * dk + unit, p.r + row0 + (int64_t)hs * dk + unit,
+                             SCALAR ? nullptr : p.d + row0 + (int64_t)hd * dk + unit};
+      const int vt = lane / COLS, vc = lane % COLS;
+      const bool v_in = z0 + vc < dv;
+      const float* v_src = p.v + row0 + (int64_t)vt * p.ld + (int64_t)hd * dv + z0 + vc;
+      const float* vs_src = scaled ? p.vscale + row0 + (int64_t)lane * p.ld + hd : nullptr;
+      const float* d_src = SCALAR ? p.d + row0 + (int64_t)lane * p.ld + hd : nullptr;
+      const uint32_t s0 = smem_u32(sm);
+      int left = cnt;
+      uint32_t at = s0;
+      auto token = [&](uint32_t x, int64_t off) {
+#pragma unroll
+        for (int w = 0; w < NV; ++w) {
+          const float* const q = src[w] + off;
+#pragma unroll
+          for (int d = 0; d < DK; d += STEP)
+            if (d + unit < dk) copy_async<W>(x + (w * DK + d) * 4, q + d);
+        }
+      };
+      auto stage = [&] {   // the next chunk of the sequence, into the next buffer; always one commit group
+        const int n = min(CH, left);
+        uint32_t x = at + unit * 4;
+        int t = 0;
+#pragma unroll 1
+        for (; t + 4 <= n; t += 4, x += 4 * NV * DK * 4)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) token(x + i * NV * DK * 4, (t + i) * p.ld);
+#pragma unroll 1
+        for (; t < n; ++t, x += NV * DK * 4) token(x, t * p.ld);
+#pragma unroll
+        for (int w = 0; w < NV; ++w) src[w] += CH * p.ld;
+        const uint32_t v = at + CH * NV * DK * 4;
+        constexpr int VT = 32 / COLS;
+#pragma unroll
+        for (int i = 0; i < CH; i += VT)
+          if (v_in && vt + i < n) copy_async<false>(v + (vc * CH + vt + i) * 4, v_src + i * p.ld);
+        v_src += CH * p.ld;
+        if (lane < n) {
+          if (scaled) copy_async<false>(v + (CH * COLS + lane) * 4, vs_src);
+          if (SCALAR) copy_async<false>(v + (CH * COLS + CH + lane) * 4, d_src);
+        }
+        if (scaled) vs_src += CH * p.ld;
+        if (SCALAR) d_src += CH * p.ld;
+        left -= n;
+        at = at == s0 + (kRemBuf - 1) * F::FLOATS * 4 ? s0 : at + F::FLOATS * 4;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+#pragma unroll 1
+      for (int k = 0; k < kRemBuf - 1; ++k) stage();
+#pragma unroll 1
+      for (int c0 = 0; c0 < cnt; c0 += CH) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRemBuf - 2) : "memory");
+        __syncthreads();   // chunk c0 is there, and the buffer of the chunk before is free
+        stage();
+      }
+    };
+    if (wide) produce(std::true_type{});
+    else produce(std::false_type{});
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    return;
+  }
+  const int gl = lane & (LN - 1), c_in = (int)threadIdx.x / LN * C, j = z0 + c_in;
+  float* st = p.state + (int64_t)p.slot[r0] * p.slot_stride + (int64_t)hd * dk * dv;
+  const bool fresh = p.pos[r0] == 0;
+  auto row_of = [&](int i) { return 4 * LN * (i >> 1) + 4 * gl + 2 * (i & 1); };   // first row of pair i
+  uint64_t S[C][NP];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int d = row_of(i);
+      const bool in = !fresh && j + c < dv;
+      S[c][i] = pair2(in && d < dk ? st[(int64_t)d * dv + j + c] : 0.f, in && d + 1 < dk ? st[(int64_t)(d + 1) * dv + j + c] : 0.f);
+    }
+  for (int c0 = 0; c0 < cnt; c0 += CH) {
+    const int n = min(CH, cnt - c0);
+    __syncthreads();
+    if (z0 + warp * (32 / LN) * C >= dv) continue;   // no column for this warp
+    const float* const x = sm + (c0 / CH % kRemBuf) * F::FLOATS;
+    const float *const v = x + CH * NV * DK + c_in * CH, *const vs = x + CH * (NV * DK + COLS), *const sd = vs + CH;
+    uint64_t q[NP], b[NP], pp[NP], r[NP], d[SCALAR ? 1 : NP];
+    uint32_t at = (uint32_t)__cvta_generic_to_shared(x) + 16 * gl;
+    auto load = [&](uint64_t(&o)[NP], int w) {
+#pragma unroll
+      for (int i = 0; i < NP; i += 2) lds_ordered(o[i], o[i + 1], at + (w * DK + 4 * LN * (i / 2)) * 4);
+    };
+    auto operands = [&] {
+      load(q, 0);
+      load(b, 1);
+      if constexpr (!SCALAR) load(d, 4);
+      load(pp, 2);
+      load(r, 3);
+    };
+    auto sum_rows = [&](const uint64_t(&w)[NP], const uint64_t(&y)[NP]) {   // this lane's rows of w · y, in two chains
+      uint64_t a0 = mul2(w[0], y[0]), a1 = mul2(w[1], y[1]);
+#pragma unroll
+      for (int i = 2; i < NP; i += 2) {
+        a0 = fma2(w[i], y[i], a0);
+        a1 = fma2(w[i + 1], y[i + 1], a1);
+      }
+      const float2 e = split2(a0), f = split2(a1);
+      return (e.x + e.y) + (f.x + f.y);
+    };
+    operands();
+    auto walk = [&](int t, auto group) {   // `group` tokens from t on
+      constexpr int U = decltype(group)::value;
+      float vj[C][U], dc[U], out[U * C];
+      if constexpr (U == 4) {
+        const float4 e = scaled ? *reinterpret_cast<const float4*>(vs + t) : make_float4(1.f, 1.f, 1.f, 1.f);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const float4 a = *reinterpret_cast<const float4*>(v + c * CH + t);
+          vj[c][0] = a.x * e.x, vj[c][1] = a.y * e.y, vj[c][2] = a.z * e.z, vj[c][3] = a.w * e.w;
+        }
+        if constexpr (SCALAR) {
+          const float4 g = *reinterpret_cast<const float4*>(sd + t);
+          dc[0] = g.x, dc[1] = g.y, dc[2] = g.z, dc[3] = g.w;
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < C; ++c) vj[c][0] = scaled ? v[c * CH + t] * vs[t] : v[c * CH + t];
+        if constexpr (SCALAR) dc[0] = sd[t];
+      }
+      uint64_t r_old[NP];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float rem[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) rem[c] = sum_rows(q, S[c]);
+#pragma unroll
+        for (int m = LN / 2; m > 0; m >>= 1)
+#pragma unroll
+          for (int c = 0; c < C; ++c) rem[c] += shfl_xor_ordered(rem[c], m);
+        uint64_t kept[C][NP];
+        const uint64_t d2 = SCALAR ? pair2(dc[u], dc[u]) : 0;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          if (u > 0) out[(u > 0 ? u - 1 : 0) * C + c] = sum_rows(r_old, S[c]);
+          const uint64_t v2 = pair2(vj[c][u], vj[c][u]);
+#pragma unroll
+          for (int i = 0; i < NP; ++i) kept[c][i] = fma2(b[i], v2, mul2(SCALAR ? d2 : d[i], S[c][i]));
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const uint64_t nr = pair2(-rem[c], -rem[c]);
+#pragma unroll
+          for (int i = 0; i < NP; ++i) S[c][i] = fma2(pp[i], nr, kept[c][i]);
+        }
+#pragma unroll
+        for (int i = 0; i < NP; ++i) r_old[i] = r[i];
+        at += t + u + 1 < n ? NV * DK * 4 : 0;
+        operands();
+      }
+#pragma unroll
+      for (int c = 0; c < C; ++c) out[(U - 1) * C + c] = sum_rows(r_old, S[c]);
+      int m = LN / 2;   // tokens and columns change hands while they are summed: lane g ends with value g / (LN / (U·C))
+#pragma unroll
+      for (int w = U * C / 2; w > 0; w >>= 1, m >>= 1) {
+        const bool hi = gl & m;
+#pragma unroll
+        for (int i = 0; i < w; ++i) out[i] = (hi ? out[w + i] : out[i]) + shfl_xor_ordered(hi ? out[i] : out[w + i], m);
+      }
+#pragma unroll
+      for (; m > 0; m >>= 1) out[0] += shfl_xor_ordered(out[0], m);
+      constexpr int each = LN / (U * C);
+      const int u = gl / each / C, c = j + gl / each % C;
+      if (gl % each == 0 && c < dv) p.o[(int64_t)(r0 + c0 + t + u) * p.ld_o + (int64_t)hd * dv + c] = out[0];
+    };
+    int t = 0;
+    for (; t + 4 <= n; t += 4) walk(t, std::integral_constant<int, 4>{});
+    for (; t < n; ++t) walk(t, std::integral_constant<int, 1>{});
+  }
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int d = row_of(i);
+      const float2 a = split2(S[c][i]);
+      if (j + c < dv && d < dk) st[(int64_t)d * dv + j + c] = a.x;
+      if (j + c < dv && d + 1 < dk) st[(int64_t)(d + 1) * dv + j + c] = a.y;
+    }
+}
+template <int LN, int RPL, int C, bool SCALAR>
+int launch_scan_rem(const LinScan& p, cudaStream_t st) {
+  using F = ScanRem<LN, RPL, C, SCALAR>;
+  static cudaError_t attr = cudaFuncSetAttribute(lin_scan_rem_kernel<LN, RPL, C, SCALAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem);
+  B200_CUDA(attr);
+  const bool wide = p.dk % 4 == 0 && p.ld % 4 == 0 && aligned16(p.b, p.r, p.p, p.q) && (SCALAR || aligned16(p.d));
+  const dim3 grid(p.n_seg, p.heads, (p.dv + F::COLS - 1) / F::COLS);
+  B200_CUDA(launch_pdl(lin_scan_rem_kernel<LN, RPL, C, SCALAR>, grid, dim3(kRemThreads), F::smem, st, stack_pdl(), p, wide));
+  return B200_OK;
+}
+template <int LN, int RPL, int C>
+int launch_scan_rem(const LinScan& p, cudaStream_t st) {
+  return p.d_scalar ? launch_scan_rem<LN, RPL, C, true>(p, st) : launch_scan_rem<LN, RPL, C, false>(p, st);
 }
 
 // ------------------------------------------------------------------------------------------- generalized delta rule
@@ -1277,21 +1386,11 @@ int launch_lin_scan(const LinScan& p, cudaStream_t st) {
     if (p.dk <= 256) return launch_scan_cols<4, 256>(p, st);
     return launch_scan_cols<8, 256>(p, st);
   }
-  // two columns per warp where the value size fills them and the registers hold them: half the CTAs stage the same rows
-  const int nc = (p.dv >= 32 && p.dk <= 256) ? 2 : 1;
-  const dim3 grid(p.n_seg, p.heads, (p.dv + 8 * nc - 1) / (8 * nc));
-#define B200_SCAN(DR)                                                                                           \
-  do {                                                                                                          \
-    if (nc == 2) B200_CUDA(launch_pdl(lin_scan_kernel<DR, 2>, grid, dim3(256), 0, st, stack_pdl(), p));          \
-    else B200_CUDA(launch_pdl(lin_scan_kernel<DR, 1>, grid, dim3(256), 0, st, stack_pdl(), p));                  \
-  } while (0)
-  if (p.dk <= 32) B200_SCAN(1);
-  else if (p.dk <= 64) B200_SCAN(2);
-  else if (p.dk <= 128) B200_SCAN(4);
-  else if (p.dk <= 256) B200_SCAN(8);
-  else B200_SCAN(16);
-#undef B200_SCAN
-  return B200_OK;
+  if (p.dk <= 32) return launch_scan_rem<8, 4, 2>(p, st);
+  if (p.dk <= 64) return launch_scan_rem<16, 4, 2>(p, st);
+  if (p.dk <= 128) return launch_scan_rem<16, 8, 2>(p, st);
+  if (p.dk <= 256) return launch_scan_rem<16, 16, 2>(p, st);
+  return launch_scan_rem<32, 16, 2>(p, st);
 }
 
 int run_delta(const DeltaRun& p, int dtype, cudaStream_t st) {
