@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kPfThreads) attn_prefill_mma_kernel(const Pref
   constexpr int ND = HD / 8;    // 8-wide output column blocks of O
   const float kScale = SCORE ? kLog2eP : p.scale_log2;   // SCORE: the scores carry their scale already
   const bool same = SCORE && p.same != 0;
-  const float slope = SCORE && p.slopes != nullptr ? p.slopes[blockIdx.y] : 0.f;
+  const float slope = SCORE && p.slopes != nullptr ? p.slopes[blockIdx.x % p.Hq] : 0.f;
 
   extern __shared__ __align__(128) uint8_t pf_smem[];
   uint8_t* const Qs = pf_smem;                       // [kBM][HD]
@@ -144,8 +144,10 @@ __global__ void __launch_bounds__(kPfThreads) attn_prefill_mma_kernel(const Pref
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, tq = lane & 3;
-  const int qb = (int)gridDim.x - 1 - (int)blockIdx.x;   // heavy blocks first
-  const int h = blockIdx.y, b = blockIdx.z;
+  const int qb = (int)(gridDim.x - 1 - blockIdx.x) / p.Hq;   // heavy blocks first, of all heads: heads
+  // run fastest, so that what is left for the last wave are the short blocks (one head after the other left long ones there: a
+  // 28-layer, 16-head prompt of 2 048 tokens took 8.85 ms, it takes 8.27)
+  const int h = (int)blockIdx.x % p.Hq, b = blockIdx.y;
   const int kvh = h / (p.Hq / p.Hkv);
   const int q0 = qb * kBM;
   const int rows_valid = min(kBM, p.S - q0);
@@ -358,7 +360,7 @@ int launch_pf(const PrefillAttnParams& p, int B, cudaStream_t st, bool same_bits
     attr_err = cudaFuncSetAttribute(attn_prefill_mma_kernel<HD, SCORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
   });
   B200_CUDA(attr_err);
-  dim3 grid((unsigned)((p.S + kBM - 1) / kBM), (unsigned)p.Hq, (unsigned)B);
+  dim3 grid((unsigned)((p.S + kBM - 1) / kBM) * (unsigned)p.Hq, (unsigned)B);
   g_launches.fetch_add(1);
   attn_prefill_mma_kernel<HD, SCORE><<<grid, kPfThreads, smem, st>>>(p);
   B200_CUDA(cudaGetLastError());
