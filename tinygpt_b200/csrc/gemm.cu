@@ -615,7 +615,9 @@ constexpr int kSplitMinKb = 8;   // k-blocks that a split takes at least: shorte
 // every SM runs several tiles (power); the rest is launch, pipeline fill and epilogue.  Measured, µs, M × N × K: 128 × 3 072 × 8 192
 // whole-K tiles 44, five splits 19; 16 × 896 × 4 864 27 → 9 (eight splits); 512 × 3 072 × 8 192 44 → 33 (pairs, two splits);
 // 2 048 × 12 288 × 2 048 persistent pairs 74, one-CTA tiles 174.  B200_GEMM = "persistent" | "tile" forces the
-// persistent pairs or one whole-K tile per CTA.
+// persistent pairs or one whole-K tile per CTA.  The products of a prompt pass (whole K) find their weights in HBM and their epilogue
+// is not hidden when a pair has one tile: 6 … 8 µs on top of the fit, so pairs start later there (24-layer, 896-wide prompt of 300
+// rows, µs: pairs 3 353, tiles 2 536; 28-layer, 2 048-wide one of 800 rows: pairs 5 724, tiles 6 604).
 struct GemmPick {
   int kind;     // 0: split-K, one CTA per tile; 1: split-K, a pair per tile; 2: persistent pairs
   int splits;
@@ -640,7 +642,7 @@ int pick_gemm(int64_t M, int64_t N, int64_t K, bool whole_k, GemmPick* out) {
   const bool tile = env_choice("B200_GEMM", 't', false), any_split = !env_choice("B200_GEMM", 'p', false);
   if (!tile) {
     const int64_t rounds = up(up(M, 256) * up(N, 256 / D), pairs);
-    consider(2, 1, 5.5 + (double)(rounds * kb) * (0.30 + 0.02 * (double)std::min<int64_t>(rounds - 1, 5)));
+    consider(2, 1, (whole_k ? 12.0 : 5.5) + (double)(rounds * kb) * (0.30 + 0.02 * (double)std::min<int64_t>(rounds - 1, 5)));
   }
   if (any_split) {
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
@@ -648,7 +650,7 @@ int pick_gemm(int64_t M, int64_t N, int64_t K, bool whole_k, GemmPick* out) {
       const int64_t t = up(M, 128) * up(N, 128 / D) * s;
       consider(0, s, (double)up(t, split_capacity<OT, EPI, false>(s)) * (5.0 + 0.15 * s + rows * (2.0 + 0.25 * s) + 0.29 * (double)up(kb, s)));
     }
-    for (int s = 1; s <= (whole_k ? 1 : 4) && (s == 1 || s * kSplitMinKb <= kb) && M > 128 && !tile; ++s) {
+    for (int s = 1; s <= 4 && (s == 1 || s * kSplitMinKb <= kb) && M > 128 && !tile && !whole_k; ++s) {
       const int64_t t = up(M, 256) * up(N, 256 / D) * 2 * s;
       consider(1, s, (double)up(t, split_capacity<OT, EPI, true>(2 * s)) * (9.5 + 1.0 * s + 0.33 * (double)up(kb, s)));
     }
