@@ -642,7 +642,9 @@ int pick_gemm(int64_t M, int64_t N, int64_t K, bool whole_k, GemmPick* out) {
   const bool tile = env_choice("B200_GEMM", 't', false), any_split = !env_choice("B200_GEMM", 'p', false);
   if (!tile) {
     const int64_t rounds = up(up(M, 256) * up(N, 256 / D), pairs);
-    consider(2, 1, (whole_k ? 12.0 : 5.5) + (double)(rounds * kb) * (0.30 + 0.02 * (double)std::min<int64_t>(rounds - 1, 5)));
+    const double tile_us = (double)kb * (0.30 + 0.02 * (double)std::min<int64_t>(rounds - 1, 5));
+    const double epilogue = whole_k && EPI == GEPI_SILU ? 13.0 : 0.0;   // of a 256 × 256 tile: longer than a short k range
+    consider(2, 1, (whole_k ? 12.0 : 5.5) + (double)rounds * std::max(tile_us, epilogue) + epilogue);
   }
   if (any_split) {
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
