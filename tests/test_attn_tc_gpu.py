@@ -40,6 +40,21 @@ def test_causal(built_lib, monkeypatch, B, S, Hq, Hkv, D):
     assert torch.equal(got, ops.flash_attention(q, k, v, True))
 
 
+@pytest.mark.parametrize("S", [65, 129, 150, 192, 321, 449])
+@pytest.mark.parametrize("D", [64, 128])
+def test_last_tile_sees_part_of_the_block(built_lib, monkeypatch, S, D):
+    """The result is read after the products of the last two key tiles, also where no softmax warp has waited for either: S % 128 in 1 … 64 (the
+    tile before the last is visible as a whole), maxima in the first tile (no rescale), two blocks beside each other on every SM."""
+    monkeypatch.setenv("B200_ATTN_TC", "tc")
+    q, k, v = randn(4, S, 96, D, seed=11), randn(4, S, 96, D, seed=12), randn(4, S, 96, D, seed=13)
+    q, k[:, 0] = q.abs(), 6.0 * D ** -0.5   # key 0: a score of about five, the others' stay below four
+    want = attend(q, k, v)
+    first = ops.flash_attention(q, k, v, True)
+    close(first, want, float(v.float().abs().max()))
+    for _ in range(20):
+        assert torch.equal(ops.flash_attention(q, k, v, True), first)
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_what_a_row_does_not_see(built_lib, monkeypatch, D):
     """Rows in front of an infinity, a NaN, or a huge key keep finite, correct results; a batch's next sequence keeps its own."""

@@ -145,8 +145,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
   uint64_t* v_empty = v_full + ST;
   uint64_t* s_full = v_empty + ST;         // [2]
   uint64_t* p_full = s_full + 2;           // [2], one arrival per softmax warp
-  uint64_t* pv_done = p_full + 2;          // one phase per tile
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
+  uint64_t* pv_done = p_full + 2;          // one phase per tile but the last
+  uint64_t* o_full = pv_done + 1;          // the last tile's product, and so all of them
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
   int* not_finite = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -179,6 +180,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
       mbar_init(&p_full[s], 4);
     }
     mbar_init(pv_done, 1);
+    mbar_init(o_full, 1);
     *not_finite = 0;
     fence_mbar_init();
   }
@@ -242,7 +244,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
           umma_bf16_ts(tmem + kColO, tmem + (uint32_t)((it & 1) * 64 + kk * 8), umma_desc_mn(v_u + s * C::TB + kk * 2048, kTBN * 128), kIdescO,
                        (it > 0 || kk > 0) ? 1u : 0u);
         umma_commit(&v_empty[s]);
-        umma_commit(pv_done);
+        umma_commit(it + 1 < n_tiles ? pv_done : o_full);
       }
     }
   } else {
@@ -335,8 +337,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[it & 1]);
     }
-    // ---- normalise and store
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_limited(pv_done, (uint32_t)((n_tiles - 1) & 1), p.err, kAttnWaitCode | 9));
+    // ---- normalise and store.  The end has a barrier of its own: a parity tells a phase from its neighbours only, and here the products
+    // of the last two tiles may both be running (inside the loop S of tile it says that the product of tile it - 2 is over).
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_limited(o_full, 0, p.err, kAttnWaitCode | 9));
     named_bar_sync(1, 128);
     const bool alone = *not_finite != 0;   // the same for all softmax threads
     if (ok) {
