@@ -15,6 +15,13 @@ def randn(*shape, seed, std=1.0):
     return (torch.randn(*shape, generator=g, device=DEV) * std).to(torch.bfloat16)
 
 
+def shifted(t):
+    """The same values two bytes off a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    buf[1:] = t.reshape(-1)
+    return buf[1:].view(t.shape)
+
+
 def attend(q, k, v):
     group = q.shape[2] // k.shape[2]
     k, v = k.double().repeat_interleave(group, 2), v.double().repeat_interleave(group, 2)
@@ -32,6 +39,17 @@ def test_one_row(built_lib, n, B, Hq, Hkv, D):
     assert torch.equal(got, ops.flash_attention(q, k, v, False))
     first = ops.flash_attention(q, k, v, True)
     assert torch.equal(first, v[:, :1].repeat_interleave(Hq // Hkv, 2))
+
+
+@pytest.mark.parametrize("which", ["q", "k", "v", "kv", "qkv"])
+@pytest.mark.parametrize("n,rows,causal", [(1, 1, False), (300, 1, False), (300, 1, True), (90, 90, True), (90, 90, False), (90, 5, False)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_views_off_a_16_byte_boundary(built_lib, which, n, rows, causal, D):
+    """Contiguous views that start two bytes off give what aligned tensors give."""
+    q, k, v = randn(2, rows, 6, D, seed=n, std=2.0), randn(2, n, 2, D, seed=1), randn(2, n, 2, D, seed=2)
+    want = ops.flash_attention(q, k, v, causal).double()
+    got = ops.flash_attention(shifted(q) if "q" in which else q, shifted(k) if "k" in which else k, shifted(v) if "v" in which else v, causal).double()
+    assert float((got - want).norm() / want.norm()) < 2.0 ** -8      # the kernels' order of sums, and P in bf16 in the prompt's
 
 
 def test_huge_scores_and_zeros(built_lib):

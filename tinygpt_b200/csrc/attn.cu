@@ -561,14 +561,14 @@ __global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(
 }
 
 // ------------------------------------------------------------------------------------------ general attention
-// One CTA per (q row, head, batch); keys in chunks of 128 with online softmax.  Correctness path (prefill-shaped
-// calls through b200_attn_bf16); the tensor-core prefill kernel is separate work.
+// One CTA per (q row, head, batch); keys in chunks of 128 with online softmax.  For what the other kernels do not take: several
+// query rows that are not a causal prompt, and tensors off a 16-byte boundary (k_wide = 0: keys read two bytes at a time).
 template <int HD>
 __global__ void __launch_bounds__(128) attn_general_kernel(__nv_bfloat16* __restrict__ o,
                                                            const __nv_bfloat16* __restrict__ q,
                                                            const __nv_bfloat16* __restrict__ k,
                                                            const __nv_bfloat16* __restrict__ v, int Sq, int Skv, int Hq,
-                                                           int Hkv, int causal) {
+                                                           int Hkv, int causal, int k_wide) {
   constexpr float kScale = InvSqrtHd<HD>::value * kLog2e;
   __shared__ float qs[HD];
   __shared__ float ps[128];
@@ -585,14 +585,21 @@ __global__ void __launch_bounds__(128) attn_general_kernel(__nv_bfloat16* __rest
     const int j = c0 + tid;
     float s = -INFINITY;
     if (j < nkeys) {
-      const uint4* kp = reinterpret_cast<const uint4*>(k + (((size_t)b * Skv + j) * Hkv + kvh) * HD);
+      const __nv_bfloat16* kp = k + (((size_t)b * Skv + j) * Hkv + kvh) * HD;
       float d = 0.f;
 #pragma unroll
       for (int piece = 0; piece < HD / 8; ++piece) {
         float qf[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) qf[e] = qs[piece * 8 + e];
-        d = dot8(kp[piece], qf, d);
+        uint4 kv;
+        if (k_wide) {
+          kv = reinterpret_cast<const uint4*>(kp)[piece];
+        } else {
+          const unsigned short* e = reinterpret_cast<const unsigned short*>(kp) + piece * 8;
+          kv = make_uint4(e[0] | (uint32_t)e[1] << 16, e[2] | (uint32_t)e[3] << 16, e[4] | (uint32_t)e[5] << 16, e[6] | (uint32_t)e[7] << 16);
+        }
+        d = dot8(kv, qf, d);
       }
       s = d;
     }
@@ -730,14 +737,15 @@ int launch_attn_general(void* o, const void* q, const void* k, const void* v, in
   B200_CHECK_ARG(B > 0 && Sq > 0 && Skv > 0 && Hkv > 0 && Hq % Hkv == 0 && Hq < 65536 && B < 65536,
                  "attention: bad shape");
   dim3 grid((unsigned)Sq, (unsigned)Hq, (unsigned)B);
+  const int k_wide = aligned16(k) ? 1 : 0;
   g_launches.fetch_add(1);
   if (hd == 64)
     attn_general_kernel<64><<<grid, 128, 0, st>>>((__nv_bfloat16*)o, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
-                                                  (const __nv_bfloat16*)v, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal);
+                                                  (const __nv_bfloat16*)v, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal, k_wide);
   else
     attn_general_kernel<128><<<grid, 128, 0, st>>>((__nv_bfloat16*)o, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
                                                    (const __nv_bfloat16*)v, (int)Sq, (int)Skv, (int)Hq, (int)Hkv,
-                                                   causal);
+                                                   causal, k_wide);
   B200_CUDA(cudaGetLastError());
   return B200_OK;
 }
@@ -748,8 +756,10 @@ extern "C" int b200_attn_bf16(void* o, const void* q, const void* k, const void*
                               int64_t Hq, int64_t Hkv, int64_t hd, int causal, void* stream) {
   using namespace b200;
   B200_CHECK_ARG(o && q && k && v, "attention: null pointer");
-  if (causal && Sq == Skv && Sq > 1 && prefill_attn_mma_enabled())
+  // A contiguous view may start anywhere: the prompt kernels read q, k and v 16 bytes at a time and store o in words, the row kernel reads k
+  // and v 16 bytes at a time; what is not aligned for them goes to the general kernel.
+  if (causal && Sq == Skv && Sq > 1 && prefill_attn_mma_enabled() && aligned16(q, k, v) && (reinterpret_cast<uintptr_t>(o) & 3) == 0)
     return launch_attn_causal_mma(o, q, k, v, B, Sq, Hq, Hkv, hd, (cudaStream_t)stream);
-  if (Sq == 1) return launch_attn_row(o, q, k, v, B, Skv, Hq, Hkv, hd, causal, (cudaStream_t)stream);
+  if (Sq == 1 && aligned16(k, v)) return launch_attn_row(o, q, k, v, B, Skv, Hq, Hkv, hd, causal, (cudaStream_t)stream);
   return launch_attn_general(o, q, k, v, B, Sq, Skv, Hq, Hkv, hd, causal, (cudaStream_t)stream);
 }
