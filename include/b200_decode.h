@@ -59,6 +59,10 @@ int b200_abi_version(void);
 const char* b200_last_error(void);
 /* Number of kernels this library has launched on this process since load (bench.py's gpu_launches claim). */
 int64_t b200_launch_count(void);
+/* The tensor-core GEMM and attention kernels give a wait that does not end within about two seconds up instead of hanging the
+ * device: they store nothing more and leave a code on the host.  B200_ERR_CUDA, once, when a stand-alone operator's kernel
+ * has done so since the last report (call it after synchronising; operators report it too); engines: b200_engine_status. */
+int b200_wait_status(void);
 /* 0 when a compute-capability 10.x device is current, else B200_ERR_NO_DEVICE. */
 int b200_device_check(void);
 
@@ -218,6 +222,11 @@ typedef struct b200_engine b200_engine;
 int b200_engine_create(const b200_model_desc* desc, const b200_weight_table* weights, b200_engine** out);
 void b200_engine_destroy(b200_engine* eng);
 
+/* B200_ERR_CUDA when a kernel of this engine gave a wait up (see b200_wait_status): logits, tokens and cache rows since then are not
+ * valid.  Holds after a synchronisation for everything enqueued before it; forward, step, decode and last_token fail the same
+ * way from then on, until b200_engine_reset starts over. */
+int b200_engine_status(const b200_engine* eng);
+
 /* New sequence: position ← 0 (the KV cache is overwritten in place). [ref: GPTModel::resetCache, GPTModel.h:91-94] */
 int b200_engine_reset(b200_engine* eng, void* stream);
 
@@ -269,6 +278,8 @@ int64_t b200_engine_generated(const b200_engine* eng);
  * the PDL wait, exit, x ready, first stage landed, first row block summed, first row block stored, unused) of the GEMV / attention launches of the most recent token into out_host; synchronises.
  * Returns the number of launches copied (0 when tracing is off). */
 int64_t b200_engine_debug_trace(b200_engine* eng, uint64_t* out_host, int64_t max_entries);
+/* Debug: the host word in which kernels of this engine (NULL: of stand-alone operators) leave their code. */
+uint32_t* b200_debug_wait_word(b200_engine* eng_or_null);
 
 /* Host-side mirrors (no device access): tokens consumed so far, and kernels per decoded token (of the batched graph
  * while the engine holds a batch: the same nodes, plus one per layer when the down projection runs in two groups). */

@@ -142,6 +142,7 @@ P, I64, I32, F = C.c_void_p, C.c_int64, C.c_int, C.c_float
 PROTOTYPES = {
     "b200_abi_version": (I32, []),
     "b200_last_error": (C.c_char_p, []),
+    "b200_wait_status": (I32, []),
     "b200_launch_count": (I64, []),
     "b200_device_check": (I32, []),
     "b200_gemv_bf16": (I32, [P, P, P, P, I64, I64, I64, P]),
@@ -162,12 +163,14 @@ PROTOTYPES = {
     "b200_attn_decode_bf16": (I32, [P, P, P, P, F, P, P, I64, P, P, I64, I64, I64, I64, P, P]),
     "b200_engine_create": (I32, [C.POINTER(ModelDesc), C.POINTER(WeightTable), C.POINTER(P)]),
     "b200_engine_destroy": (None, [P]),
+    "b200_engine_status": (I32, [P]),
     "b200_engine_reset": (I32, [P, P]),
     "b200_engine_seek": (I32, [P, I64, P]),
     "b200_engine_forward": (I32, [P, P, I64, I64, P, I32, P]),
     "b200_engine_decode": (I32, [P, I64, P, P]),
     "b200_engine_last_token": (I32, [P, P, P]),
     "b200_engine_debug_trace": (I64, [P, P, I64]),
+    "b200_debug_wait_word": (P, [P]),
     "b200_engine_position": (I64, [P]),
     "b200_engine_generated": (I64, [P]),
     "b200_engine_set_mailbox": (I32, [P, P, I64, P]),

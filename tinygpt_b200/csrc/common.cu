@@ -1,5 +1,6 @@
 // common.cu — error state, launch counter, device check and TMA descriptor encoding for the C ABI.
 #include "common.cuh"
+#include "engine.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -112,33 +113,56 @@ int make_tmap_sw128(CUtensorMap* out, int rank, const void* base, int64_t batch,
   return B200_OK;
 }
 
-// One word of mapped host memory per process.  The allocation must not disturb a capture that may be running on this thread.
-int wait_word(unsigned** out) {
-  static unsigned* word = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    void* p = nullptr;
-    if (cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
-      word = static_cast<unsigned*>(p);
-      *word = 0;
-    } else {
-      (void)cudaGetLastError();
-    }
-    cudaThreadExchangeStreamCaptureMode(&mode);
-  });
-  if (word == nullptr) {
+// The allocation must not disturb a capture that may be running on this thread.
+int wait_word_new(unsigned** out) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  void* p = nullptr;
+  const cudaError_t err = cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (err != cudaSuccess) {
+    (void)cudaGetLastError();
     set_error("no pinned host memory for the kernels' error word");
     return B200_ERR_CUDA;
   }
-  const unsigned code = *reinterpret_cast<volatile unsigned*>(word);
-  if (code != 0) {
-    *reinterpret_cast<volatile unsigned*>(word) = 0;
-    set_error("a kernel gave up waiting (code 0x%x): what it wrote is not valid", code);
-    return B200_ERR_CUDA;
-  }
-  *out = word;
+  *out = static_cast<unsigned*>(p);
+  **out = 0;
+  return B200_OK;
+}
+void wait_word_free(unsigned* word) {
+  if (word != nullptr) cudaFreeHost(word);
+}
+
+static int report_wait(unsigned code) {
+  if (code == 0) return B200_OK;
+  set_error("a kernel gave up waiting (code 0x%x): what it wrote is not valid", code);
+  return B200_ERR_CUDA;
+}
+int wait_word_check(const unsigned* word) { return word == nullptr ? B200_OK : report_wait(__atomic_load_n(word, __ATOMIC_ACQUIRE)); }
+
+static std::atomic<unsigned*> op_word{nullptr};
+int op_wait_word(unsigned** out) {
+  static std::once_flag once;
+  std::call_once(once, [] {
+    unsigned* w = nullptr;
+    if (wait_word_new(&w) == B200_OK) op_word.store(w);
+  });
+  *out = op_word.load();
+  if (*out != nullptr) return B200_OK;
+  set_error("no pinned host memory for the kernels' error word");
+  return B200_ERR_CUDA;
+}
+int op_wait_check() {
+  unsigned* w = op_word.load(std::memory_order_relaxed);
+  return w == nullptr || *(volatile unsigned*)w == 0 ? B200_OK : report_wait(__atomic_exchange_n(w, 0u, __ATOMIC_ACQ_REL));
+}
+
+static thread_local unsigned* t_wait_word = nullptr;
+WaitScope::WaitScope(unsigned* word) : outer(t_wait_word) { t_wait_word = word; }
+WaitScope::~WaitScope() { t_wait_word = outer; }
+int wait_word(unsigned** out) {
+  if (t_wait_word == nullptr) return op_wait_word(out);
+  *out = t_wait_word;
   return B200_OK;
 }
 
@@ -167,7 +191,13 @@ int b200_device_check(void) {
     b200::set_error("device %d has compute capability major %d; this library contains sm_100a code only", dev, major);
     return B200_ERR_NO_DEVICE;
   }
-  return B200_OK;
+  return b200::op_wait_check();
+}
+
+int b200_wait_status(void) { return b200::op_wait_check(); }
+uint32_t* b200_debug_wait_word(b200_engine* e) {
+  unsigned* w = e ? e->wait_word : nullptr;
+  return e == nullptr && b200::op_wait_word(&w) != B200_OK ? nullptr : w;
 }
 
 }  // extern "C"

@@ -220,9 +220,22 @@ inline bool aligned16(P... p) {
   return ((reinterpret_cast<uintptr_t>(static_cast<const void*>(p)) | ...) & 15) == 0;
 }
 
-// Word (mapped host memory) in which a kernel whose bounded wait gives up leaves a code; the next launch that asks for the word
-// reports it and fails.
-int wait_word(unsigned** out);
+// Words (mapped host memory) in which a kernel whose bounded wait gives up leaves a code.  Every engine owns one: its launches write
+// there (WaitScope), every later call of that engine fails until it is reset, and nobody else's does.  Stand-alone operators share
+// one per process; the next operator reports it, once.
+int wait_word_new(unsigned** out);
+void wait_word_free(unsigned* word);
+int wait_word_check(const unsigned* word);   // B200_ERR_CUDA while a code is there
+int op_wait_word(unsigned** out);
+int op_wait_check();                         // the operators': reports and clears
+int wait_word(unsigned** out);               // the word for a launch on this thread
+struct WaitScope {                           // launches of this thread write to `word`
+  unsigned* outer;
+  explicit WaitScope(unsigned* word);
+  ~WaitScope();
+  WaitScope(const WaitScope&) = delete;
+  WaitScope& operator=(const WaitScope&) = delete;
+};
 
 // [batch, rows, cols] bf16 (rank 3, strides in elements) or [rows, cols] (rank 2: batch 1), with boxes of 64 columns × box_rows rows,
 // 128-byte swizzle; what lies outside is zero

@@ -496,6 +496,7 @@ static int engine_build(const b200_model_desc* desc, const b200_weight_table* w,
   B200_CUDA(cudaDeviceSynchronize());  // weights may still be in flight on the loader's stream
   if ((rc = gemv_setup_attributes()) != B200_OK) return rc;
   if ((rc = attn_setup_attributes()) != B200_OK) return rc;
+  if ((rc = wait_word_new(&e->wait_word)) != B200_OK) return rc;
 
   e->nsplit = attn_decode_nsplit(d.head_dim, d.max_ctx);
   env = std::getenv("B200_TRACE");
@@ -777,6 +778,16 @@ static int engine_prefill(b200_engine* e, const int64_t* ids, int64_t S, cudaStr
 
 }  // namespace b200
 
+namespace b200 {
+// a new sequence: nothing of what a kernel that gave up has written is read again (a code is rare: waiting here is fine)
+int engine_wait_clear(unsigned* word, cudaStream_t st) {
+  if (wait_word_check(word) == B200_OK) return B200_OK;
+  B200_CUDA(cudaStreamSynchronize(st));
+  __atomic_store_n(word, 0u, __ATOMIC_RELEASE);
+  return B200_OK;
+}
+}  // namespace b200
+
 // --------------------------------------------------------------------------------------------------------- C ABI
 extern "C" {
 
@@ -800,12 +811,21 @@ void b200_engine_destroy(b200_engine* e) {
   if (e->pf_arena) cudaFree(e->pf_arena);
   if (e->trace) cudaFree(e->trace);
   b200::engine_batch_free(e);
+  b200::wait_word_free(e->wait_word);
   delete e;
+}
+
+int b200_engine_status(const b200_engine* e) {
+  using namespace b200;
+  B200_CHECK_ARG(e, "engine_status: null engine");
+  return wait_word_check(e->wait_word);
 }
 
 int b200_engine_reset(b200_engine* e, void* stream) {
   using namespace b200;
   B200_CHECK_ARG(e, "engine_reset: null engine");
+  int rc = engine_wait_clear(e->wait_word, (cudaStream_t)stream);
+  if (rc != B200_OK) return rc;
   if (e->stack) return stack_reset(e, (cudaStream_t)stream);
   B200_CUDA(cudaMemsetAsync(e->pos, 0, 16, (cudaStream_t)stream));
   e->h_pos = 0;
@@ -832,6 +852,8 @@ int b200_engine_forward(b200_engine* e, const int64_t* ids, int64_t B, int64_t S
                         void* stream) {
   using namespace b200;
   B200_CHECK_ARG(e && ids, "engine_forward: null argument");
+  if (int bad = wait_word_check(e->wait_word)) return bad;
+  const WaitScope scope(e->wait_word);
   if (e->stack) return stack_forward(e, ids, B, S, logits_out, logits_mode, (cudaStream_t)stream);
   B200_CHECK_ARG(B >= 1 && B <= kMaxBatch, "engine_forward: batch %lld not built (1 … %d sequences per step)", (long long)B,
                  kMaxBatch);
@@ -915,6 +937,8 @@ int b200_engine_forward(b200_engine* e, const int64_t* ids, int64_t B, int64_t S
 int b200_engine_decode(b200_engine* e, int64_t n_steps, int64_t* tokens_out, void* stream) {
   using namespace b200;
   B200_CHECK_ARG(e && n_steps >= 0, "engine_decode: bad argument");
+  if (int bad = wait_word_check(e->wait_word)) return bad;
+  const WaitScope scope(e->wait_word);
   if (e->stack) return stack_decode(e, n_steps, tokens_out, (cudaStream_t)stream);
   B200_CHECK_ARG(n_steps <= e->gen_cap, "engine_decode: at most %d steps per call", e->gen_cap);
   if (e->h_pos + n_steps > e->d.max_ctx) {
@@ -960,6 +984,7 @@ int b200_engine_decode(b200_engine* e, int64_t n_steps, int64_t* tokens_out, voi
 int b200_engine_last_token(b200_engine* e, int64_t* token_out, void* stream) {
   using namespace b200;
   B200_CHECK_ARG(e && token_out, "engine_last_token: null argument");
+  if (int bad = wait_word_check(e->wait_word)) return bad;
   if (e->stack) return stack_last_token(e, token_out, (cudaStream_t)stream);
   if (e->batch > 1) {   // token_out [B]
     B200_CUDA(cudaMemcpyAsync(token_out, e->b_tok, (size_t)e->batch * 8, cudaMemcpyDeviceToDevice, (cudaStream_t)stream));

@@ -10,6 +10,7 @@
 namespace b200 {
 struct StackEngine;
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
+int engine_wait_clear(unsigned* word, cudaStream_t st);
 }  // namespace b200
 
 struct b200_engine {
@@ -52,6 +53,7 @@ struct b200_engine {
   __nv_bfloat16 *pf_x = nullptr, *pf_h = nullptr, *pf_qkv = nullptr, *pf_attn = nullptr, *pf_act = nullptr;
   bool use_prefill_gemm = true;
   const void* final_norm_w = nullptr;
+  unsigned* wait_word = nullptr;       // see WaitScope
   // tensor parallel
   int tp_world = 1, tp_rank = 0;
   bool shard_attn = true;

@@ -1978,6 +1978,7 @@ static int stack_build(const b200_stack_desc* desc, b200_engine** out) {
       s->s_slot += (size_t)mlstm_state_floats(a.heads, a.dim, a.vdim);
     }
   }
+  if ((rc = wait_word_new(&e->wait_word)) != B200_OK) return rc;
   B200_CUDA(cudaDeviceSynchronize());   // weights may still be in flight on the loader's stream
   {
     int dev = 0;
@@ -2101,6 +2102,8 @@ int b200_engine_step(b200_engine* e, int64_t n_seq, const int32_t* slots, const 
     return B200_ERR_UNSUPPORTED;
   }
   B200_CHECK_ARG(n_want == 0 || (want && logits_out), "engine_step: wanted rows without an output buffer");
+  if (int bad = wait_word_check(e->wait_word)) return bad;
+  const WaitScope scope(e->wait_word);
   StackEngine* s = e->stack;
   const b200_stack_desc& d = s->d;
   cudaStream_t st = (cudaStream_t)stream;

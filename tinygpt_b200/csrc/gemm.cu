@@ -137,7 +137,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
         }
       }
-      if (!ok) drain_loads();
+      if (!ok) drain_async();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------ MMA issuer (CTA 0)
@@ -165,6 +165,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
         if (ok) umma_commit_pair(&tmem_full[acc]);
       }
+      if (!ok) drain_async();
     }
   } else {
     // ---------------------------------------------------------------------------------------------- epilogue
@@ -332,6 +333,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint64_t* empty = full + kSplitStagesMax;
   uint64_t* tmem_full = empty + kSplitStagesMax;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
+  int* gave_up = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int crank = (int)cluster_rank(), half = PAIR ? crank & 1 : 0, split = PAIR ? crank >> 1 : crank;
@@ -350,6 +352,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       mbar_init(&empty[s], 1);
     }
     mbar_init(tmem_full, 1);
+    *gave_up = 0;
     fence_mbar_init();
   }
   if (warp == 2) tmem_alloc<GROUP>(tmem_slot, BN);
@@ -388,7 +391,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           ph ^= 1;
         }
       }
-      if (!ok) drain_loads();
+      if (!ok) drain_async();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------------- MMA issuer
@@ -415,6 +418,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       if (ok) {
         if constexpr (PAIR) umma_commit_pair(tmem_full, (uint16_t)(3u << crank));
         else umma_commit(tmem_full);
+      } else {
+        drain_async();
       }
     }
   } else {
@@ -436,6 +441,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     }
   }
+  if (!ok) *gave_up = 1;
   tc_fence_before();
   __syncwarp();
   __syncthreads();
@@ -446,6 +452,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const int share = (valid + splits - 1) / splits, r_lo = split * share, r_hi = min(valid, r_lo + share);
     const uint32_t part_u = smem_u32(part);
     constexpr int G = OUT / 8;
+    int lost = 0;   // a split that gave up has no part: nothing is stored then
+#pragma unroll 4
+    for (int sp = 0; sp < splits; ++sp) lost |= ld_cluster_i32(mapa_u32(smem_u32(gave_up), (uint32_t)(PAIR ? 2 * sp + half : sp)));
     for (int it = threadIdx.x; it < (r_hi - r_lo) * G; it += kGemmThreads) {
       const int r = r_lo + it / G, c = (it % G) * 8, col = n0 + c;
       if (col >= p.N) continue;              // N is a multiple of 8: a piece lies inside the row or outside it
@@ -468,6 +477,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           u[4] += w.x; u[5] += w.y; u[6] += w.z; u[7] += w.w;
         }
       }
+      if (lost) break;
       if (EPI == GEPI_STORE && p.bias != nullptr) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] += p.bias[col + j];

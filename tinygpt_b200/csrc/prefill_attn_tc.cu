@@ -213,7 +213,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
           ph ^= 1;
         }
       }
-      if (!ok) drain_loads();
+      if (!ok) drain_async();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------------- MMA issuer
@@ -246,6 +246,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
         umma_commit(&v_empty[s]);
         umma_commit(it + 1 < n_tiles ? pv_done : o_full);
       }
+      if (!ok) drain_async();
     }
   } else {
     // ---------------------------------------------------------------------------------------------- softmax

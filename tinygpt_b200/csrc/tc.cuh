@@ -51,6 +51,11 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
+__device__ __forceinline__ int ld_cluster_i32(uint32_t addr) {
+  int v;
+  asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -92,8 +97,9 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
   }
   return true;
 }
-// what a producer that gave up does before it ends: loads may still be on their way into this CTA's shared memory
-__device__ __forceinline__ void drain_loads() {
+// what a producer or an issuer that gave up does before it ends: loads may still be on their way into this CTA's shared memory, and
+// products into its TMEM
+__device__ __forceinline__ void drain_async() {
   const unsigned long long t0 = global_timer_ns();
   while (global_timer_ns() - t0 < 1000000ull) {
   }

@@ -391,7 +391,9 @@ class DecodeEngine:
         first = torch.empty(len(prompts), 1, dtype=torch.int64, device=self.device)
         check(lib().b200_engine_last_token(self._h, first.data_ptr(), self._stream()), "b200_engine_last_token")
         rest = self.decode(max_new_tokens - 1).view(max_new_tokens - 1, -1).t()
-        return torch.cat([first, rest], dim=1).cpu().tolist()
+        out = torch.cat([first, rest], dim=1).cpu().tolist()
+        self.verify()
+        return out
 
     @staticmethod
     def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -440,6 +442,11 @@ class DecodeEngine:
 
     def reset_cache(self) -> None:
         check(lib().b200_engine_reset(self._h, self._stream()), "b200_engine_reset")
+
+    def verify(self) -> None:
+        """Raises when a kernel of this engine gave up waiting for its operands (b200_engine_status): call it where results reach the
+        host, after synchronising.  The generate_* methods do."""
+        check(lib().b200_engine_status(self._h), "b200_engine_status")
 
     def seek(self, position: int) -> None:
         """Rewind to `position` inside the cached prefix (rows below it stay valid)."""
@@ -500,6 +507,7 @@ class DecodeEngine:
         rest = self.decode(max_new_tokens - 1)                 # [n-1, B] (or [n-1] for B = 1)
         rest = rest.view(max_new_tokens - 1, -1).t()
         toks = torch.cat([first, rest], dim=1).cpu()
+        self.verify()
         return toks
 
     # ------------------------------------------------------------------------------------------ generateSync
@@ -525,6 +533,7 @@ class DecodeEngine:
             pinned_out = torch.empty(max_new_tokens, dtype=torch.int64).pin_memory()
         pinned_out[:max_new_tokens].copy_(toks, non_blocking=True)
         torch.cuda.current_stream(self.device).synchronize()
+        self.verify()
         return pinned_out[:max_new_tokens].clone()
 
     # ------------------------------------------------------------------------------------------------ sampler
@@ -633,3 +642,4 @@ class DecodeEngine:
 
     def _drain(self) -> None:
         torch.cuda.current_stream(self.device).synchronize()
+        self.verify()
