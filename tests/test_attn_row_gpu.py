@@ -63,6 +63,27 @@ def test_huge_scores_and_zeros(built_lib):
     assert float((flat - attend(q * 0, k, v)).abs().max()) < 2.0 ** -9
 
 
+@pytest.mark.parametrize("Hq,Hkv,D,ctxs", [(6, 2, 128, (1024, 1025)), (14, 2, 64, (2048, 2049, 4096))])
+@pytest.mark.parametrize("table", [False, True])
+def test_fixed_length_does_not_depend_on_the_cache(built_lib, Hq, Hkv, D, ctxs, table):
+    """Attention over the first rows of a cache that appends nothing: the same on either side of the context where the cluster kernel
+    takes over, q rotated as the last of those rows' tokens if there is a table."""
+    n = 700
+    qkv = randn((Hq + 2 * Hkv) * D, seed=9, std=1.5)
+    kc, vc = randn(max(ctxs), Hkv, D, seed=10), randn(max(ctxs), Hkv, D, seed=11)
+    ang = torch.arange(max(ctxs), device=DEV, dtype=torch.float64)[:, None] * (1e4 ** (-torch.arange(0, D, 2, device=DEV, dtype=torch.float64) / D))
+    rope = torch.stack([ang.cos().repeat(1, 2), ang.sin().repeat(1, 2)], -1).float().contiguous() if table else None
+    q = qkv[:Hq * D].view(Hq, D).float()
+    if table:
+        c, s = rope[n - 1, :D // 2, 0], rope[n - 1, :D // 2, 1]
+        lo, hi = q[:, :D // 2], q[:, D // 2:]
+        q = torch.cat([lo * c - hi * s, hi * c + lo * s], 1)
+    want = attend(q.to(torch.bfloat16)[None, None], kc[None, :n], vc[None, :n]).reshape(-1)
+    for ctx in ctxs:
+        got = ops.attn_decode(qkv, kc[:ctx].clone(), vc[:ctx].clone(), q_heads=Hq, kv_heads=Hkv, head_dim=D, fixed_len=n, rope_table=rope)
+        assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -8, ctx
+
+
 @pytest.mark.parametrize("Hq,Hkv,D,at", [(6, 2, 128, 1023), (6, 2, 128, 1025), (14, 2, 64, 2400), (24, 8, 128, 4000), (8, 8, 128, 3999)])
 def test_fused_decode_merges_many_splits(built_lib, Hq, Hkv, D, at):
     ctx = 4096

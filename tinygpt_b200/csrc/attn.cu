@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(
   const int rank = (int)cluster_rank(), splits = (int)gridDim.x;
   if (DECODE) pdl_trigger();
   const bool append = DECODE && p.pos != nullptr;
-  const int pos = append ? *p.pos : 0;     // stable since before the producer kernel started
+  const int pos = append ? *p.pos : p.fixed_len - 1;   // where q is rotated; stable since before the producer kernel started
   const int nkeys = append ? pos : DECODE ? p.fixed_len : a.nkeys;   // rows that are in the cache already
   const int per = ((nkeys + splits - 1) / splits + NG - 1) / NG * NG;
   const int k0 = min(nkeys, rank * per), k1 = min(nkeys, k0 + per);
