@@ -1,10 +1,13 @@
 """One query row through b200_attn_bf16 (csrc/attn.cu attn_row_kernel) against fp64 attention, at the edges of its splits: key counts around a pass, a
 cluster's share and several passes, one and two heads per CTA, both head sizes, and the causal form (row 0 sees key 0 only).  Probabilities
 are fp32, the result bf16: 2-norm error below 2⁻⁸.  And the fused decode kernel's merge of many splits."""
+import ctypes as C
+
 import pytest
 import torch
 
-from tinygpt_b200 import ops
+from tinygpt_b200 import engine, models, ops
+from tinygpt_b200._lib import lib
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -96,3 +99,22 @@ def test_fused_decode_merges_many_splits(built_lib, Hq, Hkv, D, at):
     assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -8
     assert torch.equal(kc[at], k[0, 0]) and torch.equal(vc[at], v[0, 0])
     assert torch.equal(got, ops.attn_decode(qkv, kc, vc, q_heads=Hq, kv_heads=Hkv, head_dim=D, pos=pos))
+
+
+@pytest.mark.parametrize("ctx", [256, 4096])
+def test_every_launch_of_a_traced_token_has_its_stamps(built_lib, monkeypatch, ctx):
+    """b200_engine_debug_trace: entry, end of the dependency wait, operands staged and exit of the GEMV and attention launches, short and long
+    contexts alike."""
+    monkeypatch.setenv("B200_TRACE", "1")
+    spec = models.TINY_QWEN2.with_ctx(ctx)
+    eng = engine.DecodeEngine(spec, {k: v.to(DEV) for k, v in models.synth_weights(spec, seed=3).items()})
+    eng.forward(torch.arange(20, device=DEV).view(1, -1))
+    eng.decode(3)
+    torch.cuda.synchronize()
+    n = 5 * spec.layers + 1
+    buf = (C.c_uint64 * (8 * n))()
+    assert lib().b200_engine_debug_trace(eng._h, buf, n) == n
+    for launch in range(n):
+        entry, waited, done, staged = buf[8 * launch:8 * launch + 4]
+        assert 0 < entry <= waited <= staged <= done, launch
+    eng.close()

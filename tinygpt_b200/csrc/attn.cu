@@ -334,6 +334,10 @@ __global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(
   const int h0 = blockIdx.y * G, kvh = h0 / (p.Hq / p.Hkv);
   const long long b = blockIdx.z;
   const int rank = (int)cluster_rank(), splits = (int)gridDim.x;
+  auto stamp = [&](int i) {                // nothing that has to stay in a register
+    if (DECODE && p.trace != nullptr && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) p.trace[i] = global_timer_ns();
+  };
+  stamp(0);
   if (DECODE) pdl_trigger();
   const bool append = DECODE && p.pos != nullptr;
   const int pos = append ? *p.pos : p.fixed_len - 1;   // where q is rotated; stable since before the producer kernel started
@@ -364,6 +368,7 @@ __global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(
       }
     }
     pdl_wait();                            // qkv of this token is complete and visible from here on
+    stamp(1);
     const int qdim = p.Hq * HD, kvdim = p.Hkv * HD;
     for (int h = warp; h < G + 1; h += kAttnWarps) {
       const bool is_k = h == G;
@@ -412,6 +417,7 @@ __global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(
     for (int i = tid; i < G * HD; i += kAttnThreads) (&q_s[0][0])[i] = bf16_to_f(qkv[h0 * HD + i]);
   }
   __syncthreads();
+  stamp(3);
   float qf[G][8], m[G], l[G], acc[G][8];
 #pragma unroll
   for (int g = 0; g < G; ++g) {
@@ -556,6 +562,7 @@ __global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(
     o[2] = f_to_bf16(num.z * inv);
     o[3] = f_to_bf16(num.w * inv);
   }
+  stamp(2);
   __syncthreads();
   cluster_sync_all();   // no CTA leaves while another still reads its part
 }
