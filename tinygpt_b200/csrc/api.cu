@@ -43,8 +43,7 @@ int b200_gemv_bf16(void* y, const void* x, const void* W, const void* bias, int6
   const bool two_passes = m <= 2 * kMaxBatch && n * k * 2 <= 5 * 1000 * 1000;
   const bool gemm = n % 8 == 0 && k % 8 == 0 && aligned16(y, x, W, bias);
   auto rest_as_gemm = [&](int64_t r) {
-    return launch_linear_bf16((__nv_bfloat16*)y + r * n, (const __nv_bfloat16*)x + r * k, W, m - r, n, k, bias ? LinearTail::bias : LinearTail::none,
-                              bias, (cudaStream_t)stream, false);
+    return launch_linear_split_bf16((__nv_bfloat16*)y + r * n, (const __nv_bfloat16*)x + r * k, W, m - r, n, k, bias, (cudaStream_t)stream);
   };
   if (m > kMaxBatch && !two_passes && gemm) return rest_as_gemm(0);
   GemvPlan plan;

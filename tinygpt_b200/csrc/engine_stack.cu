@@ -504,7 +504,7 @@ static int stack_attention(StackEngine* s, const StackAttn& a, const b200_stack_
                                          d.out_gate ? prow + a.off_g : nullptr, a.ld_proj,
                                          (const __nv_bfloat16*)a.kcache + (size_t)g.slot * a.k_slot_stride,
                                          (const __nv_bfloat16*)a.vcache + (size_t)g.slot * a.v_slot_stride, g.count, d.heads,
-                                         d.kv_heads, d.dim, g.pos0, d.scale, d.window, d.keep_first, st, d.sink, d.softcap,
+                                         d.kv_heads, d.dim, g.pos0, d.scale, d.window, d.keep_first, s->d.max_ctx, st, d.sink, d.softcap,
                                          d.slopes)) != B200_OK)
       return rc;
   }
@@ -899,7 +899,7 @@ static int stack_run_sandwich(StackEngine* s, int r, float* x, int n_tok, cudaSt
         if ((rc = launch_latent_pack(k, st)) != B200_OK) return rc;
         if ((rc = launch_attn_prefill_window((__nv_bfloat16*)s->mid + (size_t)g.row0 * L.k_out, L.k_out, s->lat_q, nullptr,
                                              (int64_t)Hh * hd, s->lat_k, s->lat_v, g.count, Hh, Hh, hd, g.pos0, L.attn.scale,
-                                             L.attn.window, 0, st)) != B200_OK)
+                                             L.attn.window, 0, s->d.max_ctx, st)) != B200_OK)
           return rc;
       }
     }

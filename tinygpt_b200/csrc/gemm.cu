@@ -8,8 +8,8 @@
 // of its own behind a Linear keeps its own rounding when it rides on the store.  Decode (m = 1) never comes
 // here — it is HBM-bound and runs on the CUDA-core GEMV (gemv.cu).
 //
-// Two kernels, chosen per shape (pick_gemm): persistent CTA pairs on 256 × 256 tiles when the tiles fill the GPU, split-K clusters
-// when they do not.  In both (192 threads, warp-specialised):
+// Two kernels, chosen per shape (pick_gemm): persistent CTA pairs on 256 × 256 tiles when the tiles fill the GPU, clusters that may
+// split K when they do not.  The engines' products never split: a row's sum has one order whatever M is.  In both (192 threads, warp-specialised):
 //   warp 0   TMA producer: 64-column k-blocks of A and B (128-byte swizzle) into a shared-memory ring, completion on `full[s]`
 //   warp 1   MMA issuer: one thread issues 4 × tcgen05.mma.kind::f16 (K16) per k-block, accumulator in TMEM; tcgen05.commit
 //            releases the stage to the producer (`empty[s]`) and signals the epilogue (`tmem_full`)
@@ -316,13 +316,14 @@ static_assert(split_ring_end(8) <= kSplitRing && split_ring_end(24) <= kSplitRin
                   split_ring_end(96) <= kSplitRing && split_ring_end(128) <= kSplitRing,
               "what the MMA reads stays inside the ring");
 
-template <typename OT, int EPI, bool PAIR>
+template <typename OT, int EPI, bool PAIR>   // more than one split: GEPI_STORE and GEPI_BIAS; PAIR: only for those
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmArgs<OT> p,
                   const int splits, const int box_rows) {
   constexpr int BN = PAIR ? 256 : 128, BMT = PAIR ? 256 : 128, LD = BN + 4, GROUP = PAIR ? 2 : 1;
   constexpr int OUT = EPI == GEPI_SILU ? BN / 2 : BN;
   constexpr uint32_t kIdesc = umma_idesc(BMT, BN);
+  static_assert(!PAIR || EPI == GEPI_STORE || EPI == GEPI_BIAS, "pairs split K");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int stages = split_stages(box_rows), a_bytes = box_rows * kBK * 2;
@@ -369,8 +370,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       uint32_t ph = 1;
       const uint32_t bytes = (uint32_t)(a_bytes + kTileBytes) * (uint32_t)GROUP;
       // the two 64-row boxes of B: neighbouring rows, or (SiLU) gate rows and the up rows that belong to them
-      const int b0 = PAIR ? n0 + half * (EPI == GEPI_SILU ? p.N : 128) : n0;
-      const int b1 = !PAIR && EPI == GEPI_SILU ? n0 + p.N : b0 + 64;
+      const int b0 = n0 + half * 128;
+      const int b1 = EPI == GEPI_SILU ? n0 + p.N : b0 + 64;
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!(ok = mbar_wait_limited(&empty[s], ph, p.err, kGemmWaitCode | 5))) break;
         uint8_t *b_dst = sB + s * kTileBytes, *a_dst = sA + s * a_bytes;
@@ -625,19 +626,20 @@ constexpr int kSplitMinKb = 8;   // k-blocks that a split takes at least: shorte
 // every SM runs several tiles (power); the rest is launch, pipeline fill and epilogue.  Measured, µs, M × N × K: 128 × 3 072 × 8 192
 // whole-K tiles 44, five splits 19; 16 × 896 × 4 864 27 → 9 (eight splits); 512 × 3 072 × 8 192 44 → 33 (pairs, two splits);
 // 2 048 × 12 288 × 2 048 persistent pairs 74, one-CTA tiles 174.  B200_GEMM = "persistent" | "tile" forces the
-// persistent pairs or one whole-K tile per CTA.  The products of a prompt pass (whole K) find their weights in HBM and their epilogue
+// persistent pairs or one whole-K tile per CTA.  The products of a prompt pass (no split) find their weights in HBM and their epilogue
 // is not hidden when a pair has one tile: 6 … 8 µs on top of the fit, so pairs start later there (24-layer, 896-wide prompt of 300
 // rows, µs: pairs 3 353, tiles 2 536; 28-layer, 2 048-wide one of 800 rows: pairs 5 724, tiles 6 604).
 struct GemmPick {
   int kind;     // 0: split-K, one CTA per tile; 1: split-K, a pair per tile; 2: persistent pairs
   int splits;
 };
-// whole_k: no splits — the order in which a row's products are summed is then the same whatever M is, so a prompt's rows have the same
-// bits in one pass, in portions and in a batch.
-template <typename OT, int EPI>
-int pick_gemm(int64_t M, int64_t N, int64_t K, bool whole_k, GemmPick* out) {
+// Without SPLIT the order in which a row's products are summed is the same whatever M is, so a prompt's rows have the same bits in one
+// pass, in portions and in a batch.  What that costs a layer-stack prompt against splits chosen by M (8 layers of 2 048, µs): 64 rows
+// 833 → 1 132, 300 rows 1 123 → 1 398, 2 048 rows none.
+template <typename OT, int EPI, bool SPLIT>
+int pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   int rc;
-  if ((rc = split_setup<OT, EPI, false>()) != B200_OK || (rc = split_setup<OT, EPI, true>()) != B200_OK) return rc;
+  if ((rc = split_setup<OT, EPI, false>()) != B200_OK) return rc;
   constexpr int D = EPI == GEPI_SILU ? 2 : 1;
   const int64_t kb = (K + kBK - 1) / kBK;
   const int pairs = std::max(1, sm_pairs());
@@ -653,30 +655,35 @@ int pick_gemm(int64_t M, int64_t N, int64_t K, bool whole_k, GemmPick* out) {
   if (!tile) {
     const int64_t rounds = up(up(M, 256) * up(N, 256 / D), pairs);
     const double tile_us = (double)kb * (0.30 + 0.02 * (double)std::min<int64_t>(rounds - 1, 5));
-    const double epilogue = whole_k && EPI == GEPI_SILU ? 13.0 : 0.0;   // of a 256 × 256 tile: longer than a short k range
-    consider(2, 1, (whole_k ? 12.0 : 5.5) + (double)rounds * std::max(tile_us, epilogue) + epilogue);
+    const double epilogue = EPI == GEPI_SILU ? 13.0 : 0.0;   // of a 256 × 256 tile: longer than a short k range
+    consider(2, 1, (SPLIT ? 5.5 : 12.0) + (double)rounds * std::max(tile_us, epilogue) + epilogue);
   }
   if (any_split) {
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
-    for (int s = 1; s <= (tile || whole_k ? 1 : 8) && (s == 1 || s * kSplitMinKb <= kb); ++s) {
+    for (int s = 1; s <= (SPLIT && !tile ? 8 : 1) && (s == 1 || s * kSplitMinKb <= kb); ++s) {
       const int64_t t = up(M, 128) * up(N, 128 / D) * s;
       consider(0, s, (double)up(t, split_capacity<OT, EPI, false>(s)) * (5.0 + 0.15 * s + rows * (2.0 + 0.25 * s) + 0.29 * (double)up(kb, s)));
     }
-    for (int s = 1; s <= 4 && (s == 1 || s * kSplitMinKb <= kb) && M > 128 && !tile && !whole_k; ++s) {
-      const int64_t t = up(M, 256) * up(N, 256 / D) * 2 * s;
-      consider(1, s, (double)up(t, split_capacity<OT, EPI, true>(2 * s)) * (9.5 + 1.0 * s + 0.33 * (double)up(kb, s)));
+    if constexpr (SPLIT) {
+      if ((rc = split_setup<OT, EPI, true>()) != B200_OK) return rc;
+      for (int s = 1; s <= 4 && (s == 1 || s * kSplitMinKb <= kb) && M > 128 && !tile; ++s) {
+        const int64_t t = up(M, 256) * up(N, 256) * 2 * s;
+        consider(1, s, (double)up(t, split_capacity<OT, EPI, true>(2 * s)) * (9.5 + 1.0 * s + 0.33 * (double)up(kb, s)));
+      }
     }
   }
   return B200_OK;
 }
 
-template <typename OT, int EPI>
-int launch_gemm(const GemmArgs<OT>& p, const void* A, const void* B, int64_t rows_b, bool whole_k, cudaStream_t st) {
+template <typename OT, int EPI, bool SPLIT = false>
+int launch_gemm(const GemmArgs<OT>& p, const void* A, const void* B, int64_t rows_b, cudaStream_t st) {
   GemmPick g{};
-  int rc = pick_gemm<OT, EPI>(p.M, p.N, p.K, whole_k, &g);
+  int rc = pick_gemm<OT, EPI, SPLIT>(p.M, p.N, p.K, &g);
   if (rc != B200_OK) return rc;
   if (g.kind == 0) return launch_split<OT, EPI, false>(p, A, B, rows_b, g.splits, st);
-  if (g.kind == 1) return launch_split<OT, EPI, true>(p, A, B, rows_b, g.splits, st);
+  if constexpr (SPLIT) {
+    if (g.kind == 1) return launch_split<OT, EPI, true>(p, A, B, rows_b, g.splits, st);
+  }
   return launch_pair<OT, EPI>(p, A, B, rows_b, st);
 }
 
@@ -693,7 +700,7 @@ template <typename OT>
 int launch_gemm_store(OT* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   int rc = check_gemm(C, A, B, M, N, K);
   if (rc != B200_OK) return rc;
-  return launch_gemm<OT, GEPI_STORE>(GemmArgs<OT>{C, bias, nullptr, (int)M, (int)N, (int)K, nullptr}, A, B, N, false, st);
+  return launch_gemm<OT, GEPI_STORE>(GemmArgs<OT>{C, bias, nullptr, (int)M, (int)N, (int)K, nullptr}, A, B, N, st);
 }
 
 }  // namespace
@@ -704,19 +711,25 @@ int launch_gemm_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N
 int launch_gemm_bf16_bias(void* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   return launch_gemm_store<__nv_bfloat16>((__nv_bfloat16*)C, A, B, bias, M, N, K, st);
 }
-int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, LinearTail tail, const void* add, cudaStream_t st,
-                       bool whole_k) {
+int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, LinearTail tail, const void* add, cudaStream_t st) {
   int rc = check_gemm(C, A, B, M, N, K);
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG((tail == LinearTail::bias || tail == LinearTail::residual) == (add != nullptr) && aligned16(add), "linear: bad operand of the tail");
   const GemmArgs<__nv_bfloat16> p{(__nv_bfloat16*)C, nullptr, (const __nv_bfloat16*)add, (int)M, (int)N, (int)K, nullptr};
   switch (tail) {
-    case LinearTail::bias: return launch_gemm<__nv_bfloat16, GEPI_BIAS>(p, A, B, N, whole_k, st);
-    case LinearTail::residual: return launch_gemm<__nv_bfloat16, GEPI_RESIDUAL>(p, A, B, N, whole_k, st);
-    case LinearTail::silu_mul: return launch_gemm<__nv_bfloat16, GEPI_SILU>(p, A, B, 2 * N, whole_k, st);
+    case LinearTail::bias: return launch_gemm<__nv_bfloat16, GEPI_BIAS>(p, A, B, N, st);
+    case LinearTail::residual: return launch_gemm<__nv_bfloat16, GEPI_RESIDUAL>(p, A, B, N, st);
+    case LinearTail::silu_mul: return launch_gemm<__nv_bfloat16, GEPI_SILU>(p, A, B, 2 * N, st);
     case LinearTail::none: break;
   }
-  return launch_gemm<__nv_bfloat16, GEPI_STORE>(p, A, B, N, whole_k, st);
+  return launch_gemm<__nv_bfloat16, GEPI_STORE>(p, A, B, N, st);
+}
+int launch_linear_split_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, const void* bias, cudaStream_t st) {
+  int rc = check_gemm(C, A, B, M, N, K);
+  if (rc != B200_OK) return rc;
+  B200_CHECK_ARG(aligned16(bias), "linear: bias must be 16-byte aligned");
+  const GemmArgs<__nv_bfloat16> p{(__nv_bfloat16*)C, nullptr, (const __nv_bfloat16*)bias, (int)M, (int)N, (int)K, nullptr};
+  return bias != nullptr ? launch_gemm<__nv_bfloat16, GEPI_BIAS, true>(p, A, B, N, st) : launch_gemm<__nv_bfloat16, GEPI_STORE, true>(p, A, B, N, st);
 }
 int launch_gemm_bf16_f32(float* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   return launch_gemm_store<float>(C, A, B, bias, M, N, K, st);
@@ -725,7 +738,7 @@ int launch_gemm_bf16_f32(float* C, const void* A, const void* B, const float* bi
 int launch_gemm_bf16_accum(float* C, const void* A, const void* B, float mult, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   int rc = check_gemm(C, A, B, M, N, K);
   if (rc != B200_OK) return rc;
-  return launch_gemm<float, GEPI_ACCUM>(GemmArgs<float>{C, nullptr, nullptr, (int)M, (int)N, (int)K, nullptr, mult}, A, B, N, false, st);
+  return launch_gemm<float, GEPI_ACCUM>(GemmArgs<float>{C, nullptr, nullptr, (int)M, (int)N, (int)K, nullptr, mult}, A, B, N, st);
 }
 int launch_gemm_bf16_logits(float* C, void* C_bf16, const void* A, const void* B, float softcap, int64_t M, int64_t N, int64_t K,
                             cudaStream_t st) {
@@ -733,7 +746,7 @@ int launch_gemm_bf16_logits(float* C, void* C_bf16, const void* A, const void* B
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(C_bf16 && aligned16(C_bf16), "gemm: bad bf16 logits");
   return launch_gemm<float, GEPI_LOGITS>(GemmArgs<float>{C, nullptr, nullptr, (int)M, (int)N, (int)K, nullptr, softcap, (__nv_bfloat16*)C_bf16}, A,
-                                         B, N, false, st);
+                                         B, N, st);
 }
 
 }  // namespace b200
@@ -741,5 +754,5 @@ int launch_gemm_bf16_logits(float* C, void* C_bf16, const void* A, const void* B
 extern "C" int b200_gemm_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, void* stream) {
   int rc = b200_device_check();
   if (rc != B200_OK) return rc;
-  return b200::launch_gemm_bf16(C, A, B, M, N, K, (cudaStream_t)stream);
+  return b200::launch_linear_split_bf16(C, A, B, M, N, K, nullptr, (cudaStream_t)stream);
 }

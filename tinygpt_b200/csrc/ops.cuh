@@ -57,11 +57,12 @@ int launch_gemm_bf16_accum(float* C, const void* A, const void* B, float mult, i
 int launch_gemm_bf16_logits(float* C, void* C_bf16, const void* A, const void* B, float softcap, int64_t M, int64_t N, int64_t K,
                             cudaStream_t st);
 // A Linear of the prompt pass with what follows it on its store, each with its own rounding: C = bf16(A·Bᵀ), then bf16(C + bias [N]),
-// bf16(add [M, N] + C) (C may be add), or — B holding N gate rows and N up rows — bf16(bf16(silu(gate))·up).  whole_k: a row's result
-// does not depend on M (no split of K).
+// bf16(add [M, N] + C) (C may be add), or — B holding N gate rows and N up rows — bf16(bf16(silu(gate))·up).
 enum class LinearTail { none, bias, residual, silu_mul };
-int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, LinearTail tail, const void* add, cudaStream_t st,
-                       bool whole_k = true);
+int launch_linear_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, LinearTail tail, const void* add, cudaStream_t st);
+// The stand-alone operators' product (bias [N] as a rounding of its own, or null): K may be split over CTAs, so the order of a row's sum
+// depends on M.  All the others above sum over the whole K in one accumulator: a row's result does not depend on the rows beside it.
+int launch_linear_split_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, const void* bias, cudaStream_t st);
 
 // ---- prefill helpers (prefill.cu)
 int launch_bias_add(void* y, const void* b, int64_t rows, int64_t n, cudaStream_t st);
@@ -76,7 +77,7 @@ int launch_attn_prefill_mma(void* o, const void* qkv, const void* kcache, const 
                             int p0, cudaStream_t st);
 int launch_attn_prefill_window(void* o, int64_t o_rs, const void* q, const void* gate_or_null, int64_t q_rs,
                                const void* kcache, const void* vcache, int S, int Hq, int Hkv, int hd, int p0, float scale,
-                               int window, int keep_first, cudaStream_t st, int sink = 0, float softcap = 0.f,
+                               int window, int keep_first, int ctx, cudaStream_t st, int sink = 0, float softcap = 0.f,
                                const float* slopes = nullptr);
 // ---- tcgen05 prefill attention (prefill_attn_tc.cu): strides in elements; keys 0 … p0 + S − 1 of every batch element
 struct TcPrefillAttn {
@@ -89,7 +90,7 @@ struct TcPrefillAttn {
   int window, keep_first, sink;
 };
 bool prefill_attn_tc_ok(const TcPrefillAttn& a, int hd);     // head size, alignment and strides it takes
-bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd);   // against launch_pf's mma.sync kernel
+bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd, int rows);   // for a prompt of so many rows, against launch_pf's mma.sync kernel
 int launch_prefill_attn_tc(const TcPrefillAttn& a, int hd, cudaStream_t st);
 bool prefill_window_ok(int hd);   // head sizes launch_attn_prefill_window takes
 int launch_attn_causal_mma(void* o, const void* q, const void* k, const void* v, int64_t B, int64_t S, int64_t Hq,

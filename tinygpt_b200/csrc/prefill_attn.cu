@@ -344,13 +344,15 @@ __global__ void __launch_bounds__(kPfThreads) attn_prefill_mma_kernel(const Pref
   }
 }
 
+// tc_rows: the prompt length for which the tcgen05 kernel has to be the faster one to be taken; 0: never
 template <int HD, bool SCORE = false>
-int launch_pf(const PrefillAttnParams& p, int B, cudaStream_t st, bool same_bits = false) {
+int launch_pf(const PrefillAttnParams& p, int B, cudaStream_t st, int tc_rows) {
   if constexpr (!SCORE && HD != 96) {
     const TcPrefillAttn t{p.o, p.q, p.k, p.v, p.gate, p.o_rs, p.o_bs, p.q_rs, p.q_bs, p.kv_rs, p.kv_bs, B, p.S, p.Hq, p.Hkv, p.p0,
                           p.scale_log2, p.window, p.keep_first, p.sink};
-    // "tc" | "mma" forces a side; the Llama engine's prompt pass stays on mma.sync: its keys and values keep the bits they always had
-    if (!same_bits && prefill_attn_tc_ok(t, HD) && env_choice("B200_ATTN_TC", 't', prefill_attn_tc_wins(t, HD))) return launch_prefill_attn_tc(t, HD, st);
+    // "tc" | "mma" forces a side
+    if (tc_rows > 0 && prefill_attn_tc_ok(t, HD) && env_choice("B200_ATTN_TC", 't', prefill_attn_tc_wins(t, HD, tc_rows)))
+      return launch_prefill_attn_tc(t, HD, st);
   }
   constexpr int smem_max = (kBM + 4 * kBN) * row_bytes<HD>();
   const int smem = SCORE && p.same ? (kBM + 2 * kBN) * row_bytes<HD>() : smem_max;
@@ -391,17 +393,21 @@ int launch_attn_prefill_mma(void* o, const void* qkv, const void* kcache, const 
   p.Hkv = Hkv;
   p.p0 = p0;
   p.scale_log2 = hd == 64 ? PfScale<64>::value : PfScale<128>::value;
-  return hd == 64 ? launch_pf<64>(p, 1, st, true) : launch_pf<128>(p, 1, st, true);
+  return hd == 64 ? launch_pf<64>(p, 1, st, 0) : launch_pf<128>(p, 1, st, 0);
 }
 
 // Layer-stack models: one sequence's rows of a step (positions p0 … p0+S-1) against that sequence's cache, with an
 // explicit score scale, a sliding window with kept first keys and a per-head sigmoid gate on the output.  q (and the
 // gate logits) are column ranges of the merged projection rows (stride q_rs), o a column range of rows of stride o_rs.
-// softcap > 0: capped scores; slopes [Hq]: a distance bias per head; vcache == kcache: the values are the keys.
+// softcap > 0: capped scores; slopes [Hq]: a distance bias per head; vcache == kcache: the values are the keys.  The kernel is chosen by
+// `ctx`, the positions that the caches are made for, as if a prompt filled them (up to 2 048 rows, the range of the fits): a choice by
+// S and p0 would give a row other bits when its prompt is cut in another way.  Long caches take tcgen05, and their short prompts pay a
+// few µs a layer for it (8 layers, 16 heads of 128, caches for 4 096, µs, mma.sync / tcgen05: 64 rows 1 094 / 1 125, 512 rows
+// 1 457 / 1 478, 1 024 rows 1 856 / 1 771, 2 048 rows 2 687 / 2 429).
 bool prefill_window_ok(int hd) { return hd == 64 || hd == 96 || hd == 128; }
 int launch_attn_prefill_window(void* o, int64_t o_rs, const void* q, const void* gate_or_null, int64_t q_rs,
                                const void* kcache, const void* vcache, int S, int Hq, int Hkv, int hd, int p0, float scale,
-                               int window, int keep_first, cudaStream_t st, int sink, float softcap, const float* slopes) {
+                               int window, int keep_first, int ctx, cudaStream_t st, int sink, float softcap, const float* slopes) {
   B200_CHECK_ARG(prefill_window_ok(hd), "prefill attention: head size %d not built", hd);
   B200_CHECK_ARG(S > 0 && Hkv > 0 && Hq % Hkv == 0 && Hq < 65536 && p0 >= 0 && window >= 0 && keep_first >= 0,
                  "prefill attention: bad shape");
@@ -430,8 +436,9 @@ int launch_attn_prefill_window(void* o, int64_t o_rs, const void* q, const void*
   p.slopes = slopes;
   p.same = kcache == vcache ? 1 : 0;
   if (softcap > 0.f || slopes != nullptr || p.same)
-    return hd == 64 ? launch_pf<64, true>(p, 1, st) : hd == 96 ? launch_pf<96, true>(p, 1, st) : launch_pf<128, true>(p, 1, st);
-  return hd == 64 ? launch_pf<64>(p, 1, st) : hd == 96 ? launch_pf<96>(p, 1, st) : launch_pf<128>(p, 1, st);
+    return hd == 64 ? launch_pf<64, true>(p, 1, st, 0) : hd == 96 ? launch_pf<96, true>(p, 1, st, 0) : launch_pf<128, true>(p, 1, st, 0);
+  const int tc_rows = std::min(ctx, 2048);
+  return hd == 64 ? launch_pf<64>(p, 1, st, tc_rows) : hd == 96 ? launch_pf<96>(p, 1, st, 0) : launch_pf<128>(p, 1, st, tc_rows);
 }
 
 // Boundary B (b200_attn_bf16, causal, Sq == Skv): separate BSHD tensors, the reference's top-left-aligned mask.
@@ -454,7 +461,7 @@ int launch_attn_causal_mma(void* o, const void* q, const void* k, const void* v,
   p.Hkv = (int)Hkv;
   p.p0 = 0;
   p.scale_log2 = hd == 64 ? PfScale<64>::value : PfScale<128>::value;
-  return hd == 64 ? launch_pf<64>(p, (int)B, st) : launch_pf<128>(p, (int)B, st);
+  return hd == 64 ? launch_pf<64>(p, (int)B, st, (int)S) : launch_pf<128>(p, (int)B, st, (int)S);
 }
 
 }  // namespace b200

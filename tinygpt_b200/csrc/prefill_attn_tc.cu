@@ -428,10 +428,10 @@ bool prefill_attn_tc_ok(const TcPrefillAttn& a, int hd) {
 // Whether this kernel beats the mma.sync one, by fits (µs) to both over 128 … 2 048 rows, 14 … 64 (head, sequence) pairs: this one takes a launch
 // and pipeline fill of 9.6 and the longest block's tiles one after another; that one the larger of its longest block's tiles and all
 // of its 64 × 64 tiles on the tensor cores, and a third of the smaller.
-bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd) {
+bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd, int rows) {
   double all = 0, longest = 0;
-  for (int r = 0; r < a.S; r += 64) {
-    const int last = a.p0 + std::min(a.S, r + 64) - 1, edge = a.window > 0 ? std::max(0, a.p0 + r - a.window + 1) / 64 : 0;
+  for (int r = 0; r < rows; r += 64) {
+    const int last = std::min(rows, r + 64) - 1, edge = a.window > 0 ? std::max(0, r - a.window + 1) / 64 : 0;
     const double tiles = last / 64 + 1 - edge + (a.window > 0 ? std::min(edge, (a.keep_first + 63) / 64) : 0);
     all += tiles;
     longest = std::max(longest, tiles);
