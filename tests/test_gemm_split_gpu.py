@@ -27,6 +27,17 @@ def test_gemm_edges(built_lib, M, N, K):
     assert_close_bf16(got.float().cpu(), want.float().cpu(), 1, f"gemm {M}x{N}x{K}", atol=1e-4, frac_exact=0.97)
 
 
+def test_more_rows_than_a_grid_has_rows_of_tiles(built_lib, monkeypatch):
+    """8.4 M rows and a few: the one-tile kernel's grid ends there, whatever was asked for."""
+    monkeypatch.setenv("B200_GEMM", "tile")
+    M = 65535 * 128 + 9
+    a, w = rand(M, 8, seed=1), rand(8, 8, seed=2)
+    got = ops.gemm(a, w)
+    tail = slice(M - 300, M)
+    assert_close_bf16(got[tail].float().cpu(), (a[tail].float() @ w.float().t()).to(torch.bfloat16).float().cpu(), 1, "gemm", atol=1e-4, frac_exact=0.97)
+    assert torch.equal(got[:128], ops.gemm(a[:128], w))
+
+
 def test_rows_outside_are_left_alone(built_lib):
     """Only rows below M and columns below N are written."""
     from tinygpt_b200._lib import check, lib

@@ -651,7 +651,9 @@ int pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
       *out = GemmPick{kind, splits};
     }
   };
-  const bool tile = env_choice("B200_GEMM", 't', false), any_split = !env_choice("B200_GEMM", 'p', false);
+  // rows of tiles run over grid.y: up to 65 535 of them, 8.4 M rows; the persistent pairs take any number
+  const bool fits = up(M, 128) <= 65535;
+  const bool tile = fits && env_choice("B200_GEMM", 't', false), any_split = fits && !env_choice("B200_GEMM", 'p', false);
   if (!tile) {
     const int64_t rounds = up(up(M, 256) * up(N, 256 / D), pairs);
     const double tile_us = (double)kb * (0.30 + 0.02 * (double)std::min<int64_t>(rounds - 1, 5));
