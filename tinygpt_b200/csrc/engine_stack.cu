@@ -583,7 +583,7 @@ static int stack_lin(StackEngine* s, const void* A, const void* Wt, const float*
   if (s->fast && M >= kGemmRows && gemm_shape_ok(N, K)) {
     if (out_t == nullptr) return launch_gemm_bf16_f32(out_f, A, Wt, bias, M, N, K, st);
     if ((rc = launch_gemm_bf16_bias(out_t, A, Wt, bias, M, N, K, st)) != B200_OK) return rc;
-    return out_f ? launch_stack_axpy(out_f, (const __nv_bfloat16*)out_t, 1.f, false, (int64_t)M * N, st) : B200_OK;
+    return out_f ? launch_stack_widen(out_f, (const __nv_bfloat16*)out_t, (int64_t)M * N, st) : B200_OK;
   }
   StackGemm g;
   g.a = A; g.lda = K; g.k1 = K;

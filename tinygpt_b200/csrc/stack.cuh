@@ -62,8 +62,8 @@ int launch_stack_embed(float* x, float* x0, const void* embed, const int32_t* to
                        float scale, int dtype, cudaStream_t st);
 
 // ---- glue of the bf16 tensor-core / weight-streaming paths (engine_stack.cu picks them per product)
-// x[i] = (add ? x[i] : 0) + mult · float(t[i])
-int launch_stack_axpy(float* x, const __nv_bfloat16* t, float mult, bool add, int64_t total, cudaStream_t st);
+// x[i] = float(t[i])
+int launch_stack_widen(float* x, const __nv_bfloat16* t, int64_t total, cudaStream_t st);
 // cat[r, :] = bf16([a[r, :] | b[r, :]]) (each `width` wide); zero_or_null[r, :] = 0
 int launch_stack_cat_cast(__nv_bfloat16* cat, const float* a, const float* b, float* zero_or_null, int64_t rows, int width,
                           cudaStream_t st);

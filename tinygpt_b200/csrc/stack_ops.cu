@@ -749,12 +749,11 @@ __global__ void __launch_bounds__(128) stack_attn_decode_kernel(const StackAttn 
   stack_attn_merge_pair<T>(p, pair, t, h, lane);
 }
 
-__global__ void __launch_bounds__(256) stack_axpy_kernel(float* __restrict__ x, const __nv_bfloat16* __restrict__ t,
-                                                         float mult, int add, int64_t total) {
+__global__ void __launch_bounds__(256) stack_widen_kernel(float* __restrict__ x, const __nv_bfloat16* __restrict__ t, int64_t total) {
   pdl_trigger();
   pdl_wait();
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x)
-    x[e] = (add ? x[e] : 0.f) + mult * __bfloat162float(t[e]);
+    x[e] = __bfloat162float(t[e]);
 }
 __global__ void __launch_bounds__(256) stack_cat_cast_kernel(__nv_bfloat16* __restrict__ cat, const float* __restrict__ a,
                                                              const float* __restrict__ b, float* __restrict__ zero,
@@ -900,9 +899,9 @@ int launch_stack_embed(float* x, float* x0, const void* embed, const int32_t* to
   return B200_OK;
 }
 
-int launch_stack_axpy(float* x, const __nv_bfloat16* t, float mult, bool add, int64_t total, cudaStream_t st) {
-  B200_CHECK_ARG(x && t && total > 0, "stack axpy: bad arguments");
-  B200_CUDA(launch_pdl(stack_axpy_kernel, dim3(grid_cap(total, 256)), dim3(256), 0, st, stack_pdl(), x, t, mult, add ? 1 : 0, total));
+int launch_stack_widen(float* x, const __nv_bfloat16* t, int64_t total, cudaStream_t st) {
+  B200_CHECK_ARG(x && t && total > 0, "stack widen: bad arguments");
+  B200_CUDA(launch_pdl(stack_widen_kernel, dim3(grid_cap(total, 256)), dim3(256), 0, st, stack_pdl(), x, t, total));
   return B200_OK;
 }
 
