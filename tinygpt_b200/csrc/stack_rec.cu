@@ -345,7 +345,8 @@ int launch_scan_cols(const LinScan& p, cudaStream_t st) {
 // operands are asked for behind the last one, and the outputs of four tokens are summed together.  Keys past 256 take 32
 // lanes, 32 and less take 8: at most 16 rows a lane is what the registers hold.
 // A CTA has four such warps, one per scheduler, and a fifth that keeps kRemBuf chunks in flight: staging from the walking warps
-// costs them 60 ns a token, and bulk copies of a row were no faster than cp.async.  Columns never read each other, so the
+// costs them 60 ns a token, and bulk copies of a row were no faster than cp.async.  The ring of keys past 64 with a decay per channel
+// (126 KB) leaves room for one CTA on an SM, the others' for two.  Columns never read each other, so the
 // result of a sequence does not depend on what else is in the step; the order of the sums inside a column is fixed by dk alone.  fp32 throughout.
 // 2 048 tokens, 16 heads, per-channel decay, against one warp per two columns with chunks staged through registers:
 // 128 × 128 1 091 → 374 µs (183 ns a token), 64 × 64 742 → 312 µs, 126 × 128 (copies of 4 bytes) 1 117 → 406 µs;
@@ -357,6 +358,7 @@ struct ScanRem {
   static constexpr int COLS = 128 / LN * C, CH = DK <= 128 ? 16 : DK <= 256 ? 8 : 4;
   static constexpr int FLOATS = CH * (NV * DK + COLS + 2);    // of a buffer: vectors, values (by column), value scales, scalar decays
   static constexpr int smem = kRemBuf * FLOATS * 4;
+  static constexpr int CTAS = 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;   // that an SM's shared memory holds
 };
 __device__ __forceinline__ float shfl_xor_ordered(float v, int m) {   // stays in order with the loads below
   float r;
@@ -372,7 +374,7 @@ __device__ __forceinline__ void copy_async(uint32_t dst, const float* src) {
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 template <int LN, int RPL, int C, bool SCALAR>
-__global__ void __launch_bounds__(kRemThreads, 2) lin_scan_rem_kernel(const LinScan p, const bool wide) {
+__global__ void __launch_bounds__(kRemThreads, (ScanRem<LN, RPL, C, SCALAR>::CTAS)) lin_scan_rem_kernel(const LinScan p, const bool wide) {
   using F = ScanRem<LN, RPL, C, SCALAR>;
   constexpr int DK = F::DK, NV = F::NV, CH = F::CH, COLS = F::COLS, NP = RPL / 2;
   static_assert(4 * C <= LN && RPL % 4 == 0, "the outputs of four tokens are shared out over the lanes of a column");
