@@ -294,14 +294,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   cluster_sync_all();
 }
 
-// ------------------------------------------------------------------------------------------------ split-K clusters
+// -------------------------------------------------------------------------------------- one tile per CTA; split-K clusters
 // The kernel for shapes with fewer tiles than the persistent pairs need: short prompts, and the o_proj / down_proj of
-// middling ones, where whole-K tiles leave most SMs idle while the few busy ones stream all of W.  One tile per cluster, 128 × 128
-// on one CTA or 256 × 256 on a CTA pair (PAIR); the cluster's `splits` CTAs (pairs) take neighbouring ranges of K, leave
-// their fp32 partial tiles in their own shared memory (the drained operand ring), and after one cluster barrier each sums
-// its share of the rows over all partials through distributed shared memory, in rank order, and stores it.  No workspace, no
-// second launch, no atomics; splits = 1 is the plain tile.  A rows past M are neither loaded nor stored (box of ≤ 128
-// rows; what the MMA reads there only reaches rows that nobody reads).
+// middling ones.  A rows past M are neither loaded nor stored (box of ≤ 128 rows; what the MMA reads there only reaches rows that
+// nobody reads).  Three forms:
+//   kWhole      one CTA, 128 × 128, the whole K; each epilogue thread takes a row from TMEM to global memory, 16 bytes at a time, and
+//               a residual's row is on its way while the products run.  As a cluster of one, through shared memory, a tile took 1.5 to 3 µs longer
+//               (µs: 37 × 2 048 × 2 048 15.1, now 13.5; 1 024 × 10 944 × 2 048 83, now 71).
+//   kSplit      a cluster per 128 × 128 tile, for operators whose whole-K tiles would leave most SMs idle while the few busy ones stream
+//               all of W: `splits` CTAs take neighbouring ranges of K, leave their fp32 partial tiles in their own shared memory
+//               (the drained operand ring), and after one cluster barrier each sums its share of the rows over all partials
+//               through distributed shared memory, in rank order, and stores it.  No workspace, no second launch, no atomics.
+//   kSplitPair  the same with 256 × 256 tiles on CTA pairs; one split is a pair's plain tile.
+enum GemmForm : int { kWhole = 0, kSplit = 1, kSplitPair = 2 };
 // The ring holds as many stages as 192 KB take: six of 128 rows of A, ten of 16 rows and fewer.
 constexpr int kSplitRing = 192 * 1024;
 constexpr int kSplitStagesMax = 10;
@@ -316,18 +321,19 @@ static_assert(split_ring_end(8) <= kSplitRing && split_ring_end(24) <= kSplitRin
                   split_ring_end(96) <= kSplitRing && split_ring_end(128) <= kSplitRing,
               "what the MMA reads stays inside the ring");
 
-template <typename OT, int EPI, bool PAIR>   // more than one split: GEPI_STORE and GEPI_BIAS; PAIR: only for those
+template <typename OT, int EPI, int FORM>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmArgs<OT> p,
                   const int splits, const int box_rows) {
+  constexpr bool PAIR = FORM == kSplitPair;
   constexpr int BN = PAIR ? 256 : 128, BMT = PAIR ? 256 : 128, LD = BN + 4, GROUP = PAIR ? 2 : 1;
   constexpr int OUT = EPI == GEPI_SILU ? BN / 2 : BN;
   constexpr uint32_t kIdesc = umma_idesc(BMT, BN);
-  static_assert(!PAIR || EPI == GEPI_STORE || EPI == GEPI_BIAS, "pairs split K");
+  static_assert(FORM == kWhole || (sizeof(OT) == 2 && (EPI == GEPI_STORE || EPI == GEPI_BIAS)), "what operators ask for");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int stages = split_stages(box_rows), a_bytes = box_rows * kBK * 2;
-  uint8_t* sB = smem;                                       // [stages][128 × 64 bf16], two boxes of 64 rows
+  uint8_t* sB = smem;                                       // [stages][128 × 64 bf16], one box or (SiLU) two of 64 rows
   uint8_t* sA = smem + stages * kTileBytes;                 // [stages][box_rows × 64 bf16]
   float* part = reinterpret_cast<float*>(smem);             // [128][LD] once the ring has drained
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kSplitRing);
@@ -369,9 +375,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       int s = 0;
       uint32_t ph = 1;
       const uint32_t bytes = (uint32_t)(a_bytes + kTileBytes) * (uint32_t)GROUP;
-      // the two 64-row boxes of B: neighbouring rows, or (SiLU) gate rows and the up rows that belong to them
-      const int b0 = n0 + half * 128;
-      const int b1 = EPI == GEPI_SILU ? n0 + p.N : b0 + 64;
+      const int b0 = n0 + half * 128;   // SiLU: 64 gate rows, and the 64 up rows that belong to them
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!(ok = mbar_wait_limited(&empty[s], ph, p.err, kGemmWaitCode | 5))) break;
         uint8_t *b_dst = sB + s * kTileBytes, *a_dst = sA + s * a_bytes;
@@ -379,12 +383,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (half == 0) mbar_arrive_expect_tx(&full[s], bytes);
           const uint32_t bar = mapa_u32(smem_u32(&full[s]), (uint32_t)(crank & ~1));
           tma_load_2d_pair(b_dst, &tmap_b, kb * kBK, b0, bar);
-          tma_load_2d_pair(b_dst + kTileBytes / 2, &tmap_b, kb * kBK, b1, bar);
           tma_load_2d_pair(a_dst, &tmap_a, kb * kBK, m0, bar);
         } else {
           mbar_arrive_expect_tx(&full[s], bytes);
           tma_load_2d(b_dst, &tmap_b, kb * kBK, b0, &full[s]);
-          tma_load_2d(b_dst + kTileBytes / 2, &tmap_b, kb * kBK, b1, &full[s]);
+          if constexpr (EPI == GEPI_SILU) tma_load_2d(b_dst + kTileBytes / 2, &tmap_b, kb * kBK, n0 + p.N, &full[s]);
           tma_load_2d(a_dst, &tmap_a, kb * kBK, m0, &full[s]);
         }
         if (++s == stages) {
@@ -423,6 +426,76 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         drain_async();
       }
     }
+  } else if constexpr (FORM == kWhole) {
+    // ---------------------------------------------------------------------------------------------- epilogue, a row per thread
+    const int q = warp & 3, row = q * 32 + lane;
+    const bool mine = row < valid;
+    const size_t o0 = (size_t)(m0 + (mine ? row : 0)) * p.N + n0;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
+    uint4 res[EPI == GEPI_RESIDUAL ? OUT / 8 : 1];
+    if constexpr (EPI == GEPI_RESIDUAL) {
+#pragma unroll
+      for (int j = 0; j < OUT / 8; ++j)
+        if (mine && n0 + 8 * j < p.N) res[j] = *reinterpret_cast<const uint4*>(p.add + o0 + 8 * j);
+    }
+    ok = __all_sync(0xffffffffu, mbar_wait_limited(tmem_full, 0, p.err, kGemmWaitCode | 7));
+    if (ok && q * 32 < valid) {
+      tc_fence_after();
+#pragma unroll(EPI == GEPI_RESIDUAL ? OUT / 32 : 1)
+      for (int c = 0; c < OUT; c += 32) {
+        uint32_t r[32], u[32];
+        float4 old[8];
+        tmem_ld32(lane_base + (uint32_t)c, r);
+        if constexpr (EPI == GEPI_SILU) tmem_ld32(lane_base + (uint32_t)(OUT + c), u);   // the up columns of these gate columns
+        if constexpr (EPI == GEPI_ACCUM) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (mine && n0 + c + 4 * j < p.N) old[j] = *reinterpret_cast<const float4*>(p.C + o0 + c + 4 * j);
+        }
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {      // N is a multiple of 8: eight columns lie inside the row or outside it
+          const int col = n0 + c + 8 * j;
+          if (!mine || col >= p.N) continue;
+          float v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * j + e]);
+          if (EPI == GEPI_STORE && p.bias != nullptr) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] += p.bias[col + e];
+          }
+          if constexpr (EPI == GEPI_ACCUM) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = fmaf(p.mult, v[e], reinterpret_cast<const float*>(old)[8 * j + e]);
+          }
+          OT* const dst = p.C + o0 + c + 8 * j;
+          if constexpr (EPI == GEPI_LOGITS) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = cap_logit(v[e], p.mult);
+            *reinterpret_cast<uint4*>(p.c2 + o0 + c + 8 * j) = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+          }
+          if constexpr (sizeof(OT) == 4) {
+            reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+            reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+          } else {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if constexpr (EPI == GEPI_SILU) w[e] = silu_mul2(r[8 * j + 2 * e], r[8 * j + 2 * e + 1], u[8 * j + 2 * e], u[8 * j + 2 * e + 1]);
+              else w[e] = pack2(v[2 * e], v[2 * e + 1]);
+            }
+            if constexpr (EPI == GEPI_RESIDUAL || EPI == GEPI_BIAS) {
+              uint4 a;
+              if constexpr (EPI == GEPI_RESIDUAL) a = res[c / 8 + j];
+              else a = *reinterpret_cast<const uint4*>(p.add + col);
+              w[0] = add_bf16x2(a.x, w[0]); w[1] = add_bf16x2(a.y, w[1]); w[2] = add_bf16x2(a.z, w[2]); w[3] = add_bf16x2(a.w, w[3]);
+            }
+            *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+        __syncwarp();
+      }
+    }
   } else {
     // ------------------------------------------------------------------------- the partial tile, into shared memory
     const int q = warp & 3, row = q * 32 + lane;
@@ -442,14 +515,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     }
   }
-  if (!ok) *gave_up = 1;
+  if (FORM != kWhole && !ok) *gave_up = 1;
   tc_fence_before();
   __syncwarp();
   __syncthreads();
-  cluster_sync_all();   // every partial of the tile is in place
+  if constexpr (FORM != kWhole) {
+    cluster_sync_all();   // every partial of the tile is in place
 
-  // ---------------------------------------------------------------------------------- sum, epilogue, store: 8 columns at a time
-  {
+    // -------------------------------------------------------------------------------- sum, epilogue, store: 8 columns at a time
     const int share = (valid + splits - 1) / splits, r_lo = split * share, r_hi = min(valid, r_lo + share);
     const uint32_t part_u = smem_u32(part);
     constexpr int G = OUT / 8;
@@ -459,59 +532,26 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     for (int it = threadIdx.x; it < (r_hi - r_lo) * G; it += kGemmThreads) {
       const int r = r_lo + it / G, c = (it % G) * 8, col = n0 + c;
       if (col >= p.N) continue;              // N is a multiple of 8: a piece lies inside the row or outside it
-      const size_t o = (size_t)(m0 + r) * p.N + col;
       uint4 add = make_uint4(0, 0, 0, 0);
-      if constexpr (EPI == GEPI_RESIDUAL) add = *reinterpret_cast<const uint4*>(p.add + o);
       if constexpr (EPI == GEPI_BIAS) add = *reinterpret_cast<const uint4*>(p.add + col);
-      float v[8], u[8];
+      float v[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = u[j] = 0.f;
+      for (int j = 0; j < 8; ++j) v[j] = 0.f;
 #pragma unroll 4
       for (int sp = 0; sp < splits; ++sp) {
         const uint32_t base = mapa_u32(part_u + (uint32_t)(r * LD + c) * 4u, (uint32_t)(PAIR ? 2 * sp + half : sp));
         const float4 x = ld_cluster_f4(base), y = ld_cluster_f4(base + 16);
         v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
         v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
-        if constexpr (EPI == GEPI_SILU) {
-          const float4 z = ld_cluster_f4(base + OUT * 4), w = ld_cluster_f4(base + OUT * 4 + 16);
-          u[0] += z.x; u[1] += z.y; u[2] += z.z; u[3] += z.w;
-          u[4] += w.x; u[5] += w.y; u[6] += w.z; u[7] += w.w;
-        }
       }
       if (lost) break;
-      if (EPI == GEPI_STORE && p.bias != nullptr) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] += p.bias[col + j];
-      }
-      if constexpr (EPI == GEPI_ACCUM) {
-        const float4 x = reinterpret_cast<const float4*>(p.C + o)[0], y = reinterpret_cast<const float4*>(p.C + o)[1];
-        v[0] = fmaf(p.mult, v[0], x.x); v[1] = fmaf(p.mult, v[1], x.y); v[2] = fmaf(p.mult, v[2], x.z); v[3] = fmaf(p.mult, v[3], x.w);
-        v[4] = fmaf(p.mult, v[4], y.x); v[5] = fmaf(p.mult, v[5], y.y); v[6] = fmaf(p.mult, v[6], y.z); v[7] = fmaf(p.mult, v[7], y.w);
-      }
-      if constexpr (EPI == GEPI_LOGITS) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = cap_logit(v[j], p.mult);
-        *reinterpret_cast<uint4*>(p.c2 + o) = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
-      }
-      if constexpr (sizeof(OT) == 4) {
-        reinterpret_cast<float4*>(p.C + o)[0] = make_float4(v[0], v[1], v[2], v[3]);
-        reinterpret_cast<float4*>(p.C + o)[1] = make_float4(v[4], v[5], v[6], v[7]);
-      } else {
-        uint32_t w[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if constexpr (EPI == GEPI_SILU) w[j] = silu_mul2(__float_as_uint(v[2 * j]), __float_as_uint(v[2 * j + 1]), __float_as_uint(u[2 * j]), __float_as_uint(u[2 * j + 1]));
-          else w[j] = pack2(v[2 * j], v[2 * j + 1]);
-        }
-        if constexpr (EPI == GEPI_RESIDUAL || EPI == GEPI_BIAS) {
-          w[0] = add_bf16x2(add.x, w[0]); w[1] = add_bf16x2(add.y, w[1]); w[2] = add_bf16x2(add.z, w[2]); w[3] = add_bf16x2(add.w, w[3]);
-        }
-        *reinterpret_cast<uint4*>(p.C + o) = make_uint4(w[0], w[1], w[2], w[3]);
-      }
+      uint4 w = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+      if constexpr (EPI == GEPI_BIAS) w = make_uint4(add_bf16x2(add.x, w.x), add_bf16x2(add.y, w.y), add_bf16x2(add.z, w.z), add_bf16x2(add.w, w.w));
+      *reinterpret_cast<uint4*>(p.C + (size_t)(m0 + r) * p.N + col) = w;
     }
+    __syncthreads();
+    cluster_sync_all();   // no CTA leaves while another still reads its partial
   }
-  __syncthreads();
-  cluster_sync_all();   // no CTA leaves while another still reads its partial
   if (warp == 2) {
     tc_fence_after();
     tmem_free<GROUP>(tmem_base, BN);
@@ -561,11 +601,11 @@ int launch_pair(const GemmArgs<OT>& args, const void* A, const void* B, int64_t 
   return B200_OK;
 }
 
-template <typename OT, int EPI, bool PAIR>
+template <typename OT, int EPI, int FORM>
 int split_setup() {
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] { attr_err = cudaFuncSetAttribute(gemm_split_kernel<OT, EPI, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem); });
+  std::call_once(once, [] { attr_err = cudaFuncSetAttribute(gemm_split_kernel<OT, EPI, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem); });
   B200_CUDA(attr_err);
   return B200_OK;
 }
@@ -582,19 +622,20 @@ struct ClusterLaunch {
     attr[0].val.clusterDim.x = cluster;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
   }
 };
 
 // CTAs of clusters of `n` ≤ 8 CTAs that the GPU holds at a time
-template <typename OT, int EPI, bool PAIR>
+template <int FORM>
 int split_capacity(int n) {
   static std::atomic<int> known[9];
   const int c = known[n].load(std::memory_order_relaxed);
   if (c != 0) return c;
   ClusterLaunch l(dim3((unsigned)n, 64), (unsigned)n, nullptr);
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, gemm_split_kernel<OT, EPI, PAIR>, &l.cfg) != cudaSuccess || clusters < 1) {
+  if (split_setup<__nv_bfloat16, GEPI_STORE, FORM>() != B200_OK ||
+      cudaOccupancyMaxActiveClusters(&clusters, gemm_split_kernel<__nv_bfloat16, GEPI_STORE, FORM>, &l.cfg) != cudaSuccess || clusters < 1) {
     (void)cudaGetLastError();
     clusters = std::max(1, 2 * sm_pairs() / n);
   }
@@ -602,19 +643,19 @@ int split_capacity(int n) {
   return clusters * n;
 }
 
-template <typename OT, int EPI, bool PAIR>
+template <typename OT, int EPI, int FORM>
 int launch_split(const GemmArgs<OT>& args, const void* A, const void* B, int64_t rows_b, int splits, cudaStream_t st) {
   GemmArgs<OT> p = args;
   int rc;
-  if ((rc = wait_word(&p.err)) != B200_OK) return rc;
-  constexpr int W = PAIR ? 2 : 1, OUT = (PAIR ? 256 : 128) / (EPI == GEPI_SILU ? 2 : 1);
+  if ((rc = split_setup<OT, EPI, FORM>()) != B200_OK || (rc = wait_word(&p.err)) != B200_OK) return rc;
+  constexpr int W = FORM == kSplitPair ? 2 : 1, OUT = 128 * W / (EPI == GEPI_SILU ? 2 : 1);
   const int box_rows = (int)std::min<int64_t>(128, ((int64_t)p.M + 7) / 8 * 8);
   CUtensorMap ta, tb;
   if ((rc = make_tmap(&ta, A, p.M, p.K, box_rows)) != B200_OK) return rc;
-  if ((rc = make_tmap(&tb, B, rows_b, p.K, 64)) != B200_OK) return rc;
+  if ((rc = make_tmap(&tb, B, rows_b, p.K, EPI == GEPI_SILU ? 64 : 128)) != B200_OK) return rc;
   ClusterLaunch l(dim3((unsigned)((p.N + OUT - 1) / OUT * splits * W), (unsigned)((p.M + 128 * W - 1) / (128 * W))), (unsigned)(splits * W), st);
   g_launches.fetch_add(1);
-  B200_CUDA(cudaLaunchKernelEx(&l.cfg, gemm_split_kernel<OT, EPI, PAIR>, ta, tb, (const GemmArgs<OT>)p, splits, box_rows));
+  B200_CUDA(cudaLaunchKernelEx(&l.cfg, gemm_split_kernel<OT, EPI, FORM>, ta, tb, (const GemmArgs<OT>)p, splits, box_rows));
   return B200_OK;
 }
 
@@ -630,16 +671,14 @@ constexpr int kSplitMinKb = 8;   // k-blocks that a split takes at least: shorte
 // is not hidden when a pair has one tile: 6 … 8 µs on top of the fit, so pairs start later there (24-layer, 896-wide prompt of 300
 // rows, µs: pairs 3 353, tiles 2 536; 28-layer, 2 048-wide one of 800 rows: pairs 5 724, tiles 6 604).
 struct GemmPick {
-  int kind;     // 0: split-K, one CTA per tile; 1: split-K, a pair per tile; 2: persistent pairs
+  int kind;     // 0: a CTA per tile (and split); 1: a pair per tile (and split); 2: persistent pairs
   int splits;
 };
 // Without SPLIT the order in which a row's products are summed is the same whatever M is, so a prompt's rows have the same bits in one
 // pass, in portions and in a batch.  What that costs a layer-stack prompt against splits chosen by M (8 layers of 2 048, µs): 64 rows
 // 833 → 1 132, 300 rows 1 123 → 1 398, 2 048 rows none.
 template <typename OT, int EPI, bool SPLIT>
-int pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
-  int rc;
-  if ((rc = split_setup<OT, EPI, false>()) != B200_OK) return rc;
+void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   constexpr int D = EPI == GEPI_SILU ? 2 : 1;
   const int64_t kb = (K + kBK - 1) / kBK;
   const int pairs = std::max(1, sm_pairs());
@@ -664,27 +703,27 @@ int pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
     for (int s = 1; s <= (SPLIT && !tile ? 8 : 1) && (s == 1 || s * kSplitMinKb <= kb); ++s) {
       const int64_t t = up(M, 128) * up(N, 128 / D) * s;
-      consider(0, s, (double)up(t, split_capacity<OT, EPI, false>(s)) * (5.0 + 0.15 * s + rows * (2.0 + 0.25 * s) + 0.29 * (double)up(kb, s)));
+      if (s == 1) consider(0, s, (double)up(t, 2 * pairs) * (5.15 + rows * 2.25 + 0.29 * (double)kb));
+      else if constexpr (SPLIT)
+        consider(0, s, (double)up(t, split_capacity<kSplit>(s)) * (5.0 + 0.15 * s + rows * (2.0 + 0.25 * s) + 0.29 * (double)up(kb, s)));
     }
     if constexpr (SPLIT) {
-      if ((rc = split_setup<OT, EPI, true>()) != B200_OK) return rc;
       for (int s = 1; s <= 4 && (s == 1 || s * kSplitMinKb <= kb) && M > 128 && !tile; ++s) {
         const int64_t t = up(M, 256) * up(N, 256) * 2 * s;
-        consider(1, s, (double)up(t, split_capacity<OT, EPI, true>(2 * s)) * (9.5 + 1.0 * s + 0.33 * (double)up(kb, s)));
+        consider(1, s, (double)up(t, split_capacity<kSplitPair>(2 * s)) * (9.5 + 1.0 * s + 0.33 * (double)up(kb, s)));
       }
     }
   }
-  return B200_OK;
 }
 
 template <typename OT, int EPI, bool SPLIT = false>
 int launch_gemm(const GemmArgs<OT>& p, const void* A, const void* B, int64_t rows_b, cudaStream_t st) {
   GemmPick g{};
-  int rc = pick_gemm<OT, EPI, SPLIT>(p.M, p.N, p.K, &g);
-  if (rc != B200_OK) return rc;
-  if (g.kind == 0) return launch_split<OT, EPI, false>(p, A, B, rows_b, g.splits, st);
+  pick_gemm<OT, EPI, SPLIT>(p.M, p.N, p.K, &g);
+  if (g.kind == 0 && g.splits == 1) return launch_split<OT, EPI, kWhole>(p, A, B, rows_b, 1, st);
   if constexpr (SPLIT) {
-    if (g.kind == 1) return launch_split<OT, EPI, true>(p, A, B, rows_b, g.splits, st);
+    if (g.kind == 0) return launch_split<OT, EPI, kSplit>(p, A, B, rows_b, g.splits, st);
+    if (g.kind == 1) return launch_split<OT, EPI, kSplitPair>(p, A, B, rows_b, g.splits, st);
   }
   return launch_pair<OT, EPI>(p, A, B, rows_b, st);
 }
