@@ -67,7 +67,7 @@ int b200_wait_status(void);
 int b200_device_check(void);
 
 /* ------------------------------------------------------------------------------------------------------------------
- * Boundary B — one entry point per TinyTorch op on the path (SURVEY.md §8a/§8b).
+ * Boundary B — one entry point per TinyTorch op on the path.
  * ---------------------------------------------------------------------------------------------------------------- */
 
 /* y[m,n] = bf16( x[m,k] · W[n,k]^T ) (fp32 accumulate, one rounding); if bias != NULL:
@@ -220,7 +220,7 @@ typedef struct b200_engine b200_engine;
 
 /* Borrow the weights (no copy), allocate the in-place KV cache [L][2][max_ctx][Hkv][hd] + workspace once,
  * encode the TMA descriptors, capture the per-token CUDA graphs.  Synchronises the device once (weights may still
- * be in flight on the loader thread's stream, see SURVEY.md §8b "Threading"). */
+ * be in flight on the loader thread's stream). */
 int b200_engine_create(const b200_model_desc* desc, const b200_weight_table* weights, b200_engine** out);
 void b200_engine_destroy(b200_engine* eng);
 

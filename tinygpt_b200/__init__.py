@@ -1,4 +1,4 @@
-"""tinygpt_b200 — B200-native decode engine behind TinyGPT's generate loop (see DESIGN.md).
+"""tinygpt_b200 — B200-native decode engine behind TinyGPT's generate loop.
 
 The package is a thin host-side mirror of the reference interfaces for the decode hot path:
   tinygpt_b200.ops      ↔ tinytorch::function::{linear, rmsNorm, ropeApply, flashAttention, siluMul, add, …}

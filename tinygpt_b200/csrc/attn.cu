@@ -46,7 +46,7 @@ struct SplitKeys {
 };
 
 // ------------------------------------------------------------------------------------------------- decode kernel
-// CTA = (KV split, group of G query heads that share one KV head).  Round 1 staged K/V of the split in shared memory
+// CTA = (KV split, group of G query heads that share one KV head).  A first version staged K/V of the split in shared memory
 // (cp.async) and ran scores / softmax / P·V as three barrier-separated phases: 2.0 µs per launch at ctx ≈ 80 for 69 KB
 // of traffic (in-kernel stamps: q/k/v staging 0.54, scores 0.54, softmax 0.64, P·V 0.3).  This kernel keeps everything
 // a thread needs in registers (measured against the staged kernel on B200: 409 vs 415 µs per Qwen2.5-0.5B token,
@@ -638,9 +638,10 @@ __global__ void __launch_bounds__(128) attn_general_kernel(__nv_bfloat16* __rest
 
 }  // namespace
 
-// Contexts from which the cluster kernel takes over: more splits than this (1 024 tokens for heads of 128, 2 048 for heads of 64).  µs, one CTA per split /
-// cluster: position 2 200 of 2 304, 16 heads 12.8 / 9.9; 4 000 of 4 096, 24 heads 27.7 / 13.3, 32 heads 31.2 / 13.3; 500 of 4 096, 32
-// heads 14.5 / 7.4.
+// Caches from which the cluster kernel takes over: more splits than this (1 024 tokens for heads of 128, 2 048 for heads of 64).  The choice is
+// by the cache, since a captured graph serves every position; it is the faster one at all of them.  Device µs with caches for 4 096 tokens, one CTA per
+// split / cluster, at positions 20, 300, 2 000 and 4 000: 16 heads of 128 5.9 / 5.1, 9.3 / 5.3, 11.4 / 8.8, 21.5 / 12.1; 32 heads of
+// 128 7.8 / 5.4, 13.8 / 5.6, 17.4 / 9.7, 33.2 / 13.1; 14 heads of 64 9.5 / 4.6, 17.4 / 4.8, 17.7 / 5.9, 21.1 / 7.2.
 constexpr int kLongSplits = 8;
 
 int64_t attn_decode_ws_floats(int Hq, int Hkv, int hd, int nsplit) {

@@ -554,8 +554,8 @@ static int engine_build(const b200_model_desc* desc, const b200_weight_table* w,
 
   // ---- shared-memory budgets = ring depth per GEMV.  Measured (B200, profiles/r02_ring_depth_sweep.txt): what decides
   // the HBM-bound models is that EVERY kernel keeps ≈ 8 stages (128 KB per SM, 19 MB chip-wide) in flight — enough to
-  // cover the HBM latency at full bandwidth.  Round 1 split 220 KB between consecutive kernels so that PDL could keep
-  // both resident; that left down_proj / o_proj with 2–4 stages and they streamed at ≈ 4 TB/s (Mistral-7B 0.60–0.79 of
+  // cover the HBM latency at full bandwidth.  Splitting 220 KB between consecutive kernels, so that PDL could keep
+  // both resident, left down_proj / o_proj with 2–4 stages and they streamed at ≈ 4 TB/s (Mistral-7B 0.60–0.79 of
   // the roofline depending on the box; 0.90 with 8 stages everywhere, Llama-3.2-3B 0.66 → 0.80, Qwen3-1.7B 0.61 →
   // 0.65).  So: every GEMV gets what it wants up to 8 stages; kernels that want less (the small models' matrices fit
   // whole) still co-reside and prefetch under PDL; the lm_head, alone at the end of the token, gets the maximum.

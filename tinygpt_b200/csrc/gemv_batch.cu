@@ -217,8 +217,7 @@ gemv_batch_kernel(const GemvParams p, const __grid_constant__ CUtensorMap tmap) 
     // and 0.65 µs for the plain staging above.  Ruled out by measurement: the norm-weight load (hoisting it above the
     // wait or above the first barrier, L2 evict_last, a copy on hot pages — no change).  Diagnosis from the stamps: with
     // k/8/32 < 8 the unroll-by-8 body of the x loop below never executes and the remainder loop runs its 3-4
-    // iterations as dependent load → use round trips (~0.4 µs each).  Issuing the lane's loads together is the next
-    // change; it was not made because it could not be validated on hardware any more this round.
+    // iterations as dependent load → use round trips (~0.4 µs each).  Issuing the lane's loads together has not been tried.
     uint4* const wv = reinterpret_cast<uint4*>(wns);
     for (int b = warp; b < nb; b += kNW) {
       const uint4* xg = reinterpret_cast<const uint4*>(p.x + (size_t)b * p.x_stride);

@@ -1,5 +1,5 @@
 // sampling.cu — temperature / top-k / top-p / min-p sampling of one token from bf16 logits, on the device, WITHOUT
-// sorting the vocabulary (SURVEY §8f rank 1).  Stand-alone op behind b200_sample_bf16 and, through
+// sorting the vocabulary.  Stand-alone op behind b200_sample_bf16 and, through
 // b200_engine_set_sampler, the last kernels of a token when any sampler knob is set.  On hardware: drawn index equal to
 // the pinned sampler oracle over 10 configurations × 5 uniform numbers × 4 vocabularies, deterministic, and every token
 // an engine draws replayable on the host (tests/test_async_sampler_gpu.py).

@@ -1,4 +1,4 @@
-"""Weight-loader fast path: HF checkpoint directory → the engine's merged, per-rank device layout (SURVEY.md §8f rank 2).
+"""Weight-loader fast path: HF checkpoint directory → the engine's merged, per-rank device layout.
 
 What the reference does  [ref: src/huggingface/ModelLoader.cpp:25-87, src/huggingface/ModelConfig.cpp:73-122,
 src/util/SafeTensors.cpp:141-229 (single file), :231-300 (index of shards), src/layer/Linear.h:64-79 (merged views)]:

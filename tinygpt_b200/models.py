@@ -3,7 +3,7 @@
 Mirrors what the reference derives from config.json (src/huggingface/ModelConfig.cpp:73-122) and the weight-name /
 merged-weight layout of its model classes (src/model/GPTModel.h:43-48, src/layer/Attention.h:61-68,
 src/layer/GatedMLP.h:44-50, src/layer/Linear.h:64-79).  No weights are available offline, so checkpoints are seeded
-synthetic tensors of the real shapes (SURVEY.md §8d).
+synthetic tensors of the real shapes.
 """
 from __future__ import annotations
 
@@ -59,18 +59,18 @@ class ModelSpec:
 
     @property
     def weight_params(self) -> int:
-        """Matrix parameters one decode step reads (tied lm_head counted once) — SURVEY.md §8a table."""
+        """Matrix parameters one decode step reads (tied lm_head counted once)."""
         return self.layers * self.per_layer_params + self.vocab * self.hidden
 
     def bytes_per_token(self, ctx: int = 0) -> int:
-        """Algorithmic HBM bytes per decoded token (SURVEY.md §8d): weights once + K/V rows read + new K/V row written."""
+        """Algorithmic HBM bytes per decoded token: weights once + K/V rows read + new K/V row written."""
         return 2 * self.weight_params + 4 * self.layers * self.kv_dim * ctx + 4 * self.layers * self.kv_dim
 
     def with_ctx(self, max_ctx: int) -> "ModelSpec":
         return replace(self, max_ctx=max_ctx)
 
 
-# The BASELINE.json configurations (standard HF configs; table in SURVEY.md §8).
+# Four models at their published sizes (standard HF configs).
 QWEN25_05B = ModelSpec("Qwen2.5-0.5B", "qwen2", 896, 24, 14, 2, 64, 4864, 151936, 1e6, 1e-6, tie=True, qkv_bias=True)
 LLAMA32_3B = ModelSpec("Llama-3.2-3B", "llama", 3072, 28, 24, 8, 128, 8192, 128256, 5e5, 1e-5, tie=True,
                        rope_scaling=RopeScaling(32.0, 4.0, 1.0, 8192))

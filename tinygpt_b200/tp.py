@@ -1,6 +1,6 @@
 """Tensor-parallel decode: one process per GPU, Megatron sharding, reductions fused into the GEMV kernels.
 
-Sharding (SURVEY.md §8e): q/k/v by head and gate/up by FFN column (column-parallel), o_proj/down_proj by input column
+Sharding: q/k/v by head and gate/up by FFN column (column-parallel), o_proj/down_proj by input column
 (row-parallel, partial hidden vectors summed across ranks), lm_head by vocabulary, embedding + norms replicated.  When
 the head counts do not divide by the world size (Qwen2.5-0.5B: 14/2 heads at 4 or 8 GPUs) attention is replicated and
 only the FFN and the vocabulary are sharded.  The reference has no tensor-parallel inference (README.md:32); the
