@@ -27,6 +27,21 @@ def test_gemm_edges(built_lib, M, N, K):
     assert_close_bf16(got.float().cpu(), want.float().cpu(), 1, f"gemm {M}x{N}x{K}", atol=1e-4, frac_exact=0.97)
 
 
+@pytest.mark.parametrize("side", ["tile", "wide"])
+@pytest.mark.parametrize("M", [1, 9, 40, 127, 129, 300])
+@pytest.mark.parametrize("N,K", [(8, 8), (136, 520), (264, 2048), (1032, 896)])
+def test_one_tile_per_cta(built_lib, monkeypatch, side, M, N, K):
+    """Whole K on one CTA, tiles of 128 and of 256 columns: ragged rows, columns and last k-block, rows and columns outside left alone."""
+    from tinygpt_b200._lib import check, lib
+    monkeypatch.setenv("B200_GEMM", side)
+    a, w = rand(M, K, seed=M + K), rand(N, K, seed=N, scale=0.02)
+    buf = torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    check(lib().b200_gemm_bf16(buf.data_ptr(), a.data_ptr(), w.data_ptr(), M, N, K, torch.cuda.current_stream().cuda_stream), "gemm")
+    want = (a.float() @ w.float().t()).to(torch.bfloat16)
+    assert_close_bf16(buf[:M].float().cpu(), want.float().cpu(), 1, f"gemm {M}x{N}x{K}", atol=1e-4, frac_exact=0.95)
+    assert bool((buf[M:] == 7.0).all())
+
+
 def test_more_rows_than_a_grid_has_rows_of_tiles(built_lib, monkeypatch):
     """8.4 M rows and a few: the one-tile kernel's grid ends there, whatever was asked for."""
     monkeypatch.setenv("B200_GEMM", "tile")

@@ -53,7 +53,7 @@ def test_prompt_rows_do_not_depend_on_the_pass(built_lib, spec, monkeypatch):
 
 
 @pytest.mark.parametrize("spec", [models.TINY_QWEN2, models.TINY_QWEN3, models.TINY_MISTRAL], ids=lambda s: s.name)
-@pytest.mark.parametrize("kernels", [("", ""), ("persistent", "tile"), ("tile", "persistent")], ids=lambda k: "-".join(k) or "default")
+@pytest.mark.parametrize("kernels", [("", ""), ("persistent", "tile"), ("tile", "persistent"), ("wide", "tile")], ids=lambda k: "-".join(k) or "default")
 def test_prompt_rows_do_not_depend_on_the_kernel(built_lib, spec, kernels, monkeypatch):
     """The same with the default attention, and with the whole prompt on the CTA pairs and its portions on one-CTA tiles, as a long prompt
     and its short portions are."""
@@ -80,15 +80,15 @@ def test_tails_on_pairs_that_run_three_tiles(built_lib, S, monkeypatch):
     eng = engine.DecodeEngine(spec, models.synth_weights(spec, seed=5, device=DEV))
     ids = torch.randint(0, spec.vocab, (1, S), generator=torch.Generator().manual_seed(S)).to(DEV)
     got = {}
-    for side in ("tile", "persistent"):
+    for side in ("tile", "wide", "persistent"):
         monkeypatch.setenv("B200_GEMM", side)
         eng.reset_cache()
         got[side] = eng.forward(ids)
-    assert torch.equal(got["tile"], got["persistent"])
+    assert torch.equal(got["tile"], got["persistent"]) and torch.equal(got["tile"], got["wide"])
     eng.close()
 
 
-@pytest.mark.parametrize("side", ["tile", "persistent"])
+@pytest.mark.parametrize("side", ["tile", "wide", "persistent"])
 def test_bias_tail_of_many_tiles(built_lib, side, monkeypatch):
     """Every row and column of a product with its bias as the second rounding: three tiles for a pair, ragged edges."""
     monkeypatch.setenv("B200_GEMM", side)

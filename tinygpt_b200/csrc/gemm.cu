@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstdlib>
 #include <mutex>
 
 namespace b200 {
@@ -297,44 +298,48 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 // -------------------------------------------------------------------------------------- one tile per CTA; split-K clusters
 // The kernel for shapes with fewer tiles than the persistent pairs need: short prompts, and the o_proj / down_proj of
 // middling ones.  A rows past M are neither loaded nor stored (box of ≤ 128 rows; what the MMA reads there only reaches rows that
-// nobody reads).  Three forms:
+// nobody reads).  The forms:
 //   kWhole      one CTA, 128 × 128, the whole K; each epilogue thread takes a row from TMEM to global memory, 16 bytes at a time, and
 //               a residual's row is on its way while the products run.  As a cluster of one, through shared memory, a tile took 1.5 to 3 µs longer
 //               (µs: 37 × 2 048 × 2 048 15.1, now 13.5; 1 024 × 10 944 × 2 048 83, now 71).
+//   kWide       the same with 256 columns: half the tiles, for row counts at which pairs of 256 rows leave a second round to a few of them
 //   kSplit      a cluster per 128 × 128 tile, for operators whose whole-K tiles would leave most SMs idle while the few busy ones stream
 //               all of W: `splits` CTAs take neighbouring ranges of K, leave their fp32 partial tiles in their own shared memory
 //               (the drained operand ring), and after one cluster barrier each sums its share of the rows over all partials
 //               through distributed shared memory, in rank order, and stores it.  No workspace, no second launch, no atomics.
 //   kSplitPair  the same with 256 × 256 tiles on CTA pairs; one split is a pair's plain tile.
-enum GemmForm : int { kWhole = 0, kSplit = 1, kSplitPair = 2 };
+enum GemmForm : int { kWhole = 0, kSplit = 1, kSplitPair = 2, kWide = 3 };
 // The ring holds as many stages as 192 KB take: six of 128 rows of A, ten of 16 rows and fewer.
 constexpr int kSplitRing = 192 * 1024;
 constexpr int kSplitStagesMax = 10;
 constexpr int kSplitSmem = kSplitRing + 1024 /*align*/ + 256 /*barriers*/;
 static_assert(128 * (256 + 4) * 4 <= kSplitRing, "a partial tile fits in the drained ring");
-__host__ __device__ constexpr int split_stages(int box_rows) {   // the MMA reads 128 rows (16 KB) from the last stage's A on
-  return (kSplitRing - kTileBytes + box_rows * kBK * 2) / (box_rows * kBK * 2 + kTileBytes) < kSplitStagesMax
-             ? (kSplitRing - kTileBytes + box_rows * kBK * 2) / (box_rows * kBK * 2 + kTileBytes) : kSplitStagesMax;
+__host__ __device__ constexpr int split_stages(int box_rows, int b_bytes) {   // the MMA reads 128 rows (16 KB) from the last stage's A on
+  return (kSplitRing - kTileBytes + box_rows * kBK * 2) / (box_rows * kBK * 2 + b_bytes) < kSplitStagesMax
+             ? (kSplitRing - kTileBytes + box_rows * kBK * 2) / (box_rows * kBK * 2 + b_bytes) : kSplitStagesMax;
 }
-constexpr int split_ring_end(int box_rows) { return split_stages(box_rows) * kTileBytes + (split_stages(box_rows) - 1) * box_rows * kBK * 2 + kTileBytes; }
-static_assert(split_ring_end(8) <= kSplitRing && split_ring_end(24) <= kSplitRing && split_ring_end(64) <= kSplitRing &&
-                  split_ring_end(96) <= kSplitRing && split_ring_end(128) <= kSplitRing,
-              "what the MMA reads stays inside the ring");
+constexpr bool split_ring_holds(int b_bytes) {
+  for (int r = 8; r <= 128; r += 8)
+    if (split_stages(r, b_bytes) * b_bytes + (split_stages(r, b_bytes) - 1) * r * kBK * 2 + kTileBytes > kSplitRing) return false;
+  return true;
+}
+static_assert(split_ring_holds(kTileBytes) && split_ring_holds(2 * kTileBytes), "what the MMA reads stays inside the ring");
 
 template <typename OT, int EPI, int FORM>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmArgs<OT> p,
                   const int splits, const int box_rows) {
-  constexpr bool PAIR = FORM == kSplitPair;
-  constexpr int BN = PAIR ? 256 : 128, BMT = PAIR ? 256 : 128, LD = BN + 4, GROUP = PAIR ? 2 : 1;
+  constexpr bool PAIR = FORM == kSplitPair, STRAIGHT = FORM == kWhole || FORM == kWide;
+  constexpr int BN = PAIR || FORM == kWide ? 256 : 128, BMT = PAIR ? 256 : 128, LD = BN + 4, GROUP = PAIR ? 2 : 1;
+  constexpr int B_BYTES = BN / GROUP * kBK * 2;   // of a k-block, per CTA
   constexpr int OUT = EPI == GEPI_SILU ? BN / 2 : BN;
   constexpr uint32_t kIdesc = umma_idesc(BMT, BN);
-  static_assert(FORM == kWhole || (sizeof(OT) == 2 && (EPI == GEPI_STORE || EPI == GEPI_BIAS)), "what operators ask for");
+  static_assert(STRAIGHT || (sizeof(OT) == 2 && (EPI == GEPI_STORE || EPI == GEPI_BIAS)), "what operators ask for");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int stages = split_stages(box_rows), a_bytes = box_rows * kBK * 2;
-  uint8_t* sB = smem;                                       // [stages][128 × 64 bf16], one box or (SiLU) two of 64 rows
-  uint8_t* sA = smem + stages * kTileBytes;                 // [stages][box_rows × 64 bf16]
+  const int stages = split_stages(box_rows, B_BYTES), a_bytes = box_rows * kBK * 2;
+  uint8_t* sB = smem;                                       // [stages][BN / GROUP × 64 bf16], one box or (SiLU) two
+  uint8_t* sA = smem + stages * B_BYTES;                    // [stages][box_rows × 64 bf16]
   float* part = reinterpret_cast<float*>(smem);             // [128][LD] once the ring has drained
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kSplitRing);
   uint64_t* empty = full + kSplitStagesMax;
@@ -374,11 +379,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 1;
-      const uint32_t bytes = (uint32_t)(a_bytes + kTileBytes) * (uint32_t)GROUP;
-      const int b0 = n0 + half * 128;   // SiLU: 64 gate rows, and the 64 up rows that belong to them
+      const uint32_t bytes = (uint32_t)(a_bytes + B_BYTES) * (uint32_t)GROUP;
+      const int b0 = n0 + half * 128;   // SiLU: gate rows, and the up rows that belong to them
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!(ok = mbar_wait_limited(&empty[s], ph, p.err, kGemmWaitCode | 5))) break;
-        uint8_t *b_dst = sB + s * kTileBytes, *a_dst = sA + s * a_bytes;
+        uint8_t *b_dst = sB + s * B_BYTES, *a_dst = sA + s * a_bytes;
         if constexpr (PAIR) {
           if (half == 0) mbar_arrive_expect_tx(&full[s], bytes);
           const uint32_t bar = mapa_u32(smem_u32(&full[s]), (uint32_t)(crank & ~1));
@@ -387,7 +392,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         } else {
           mbar_arrive_expect_tx(&full[s], bytes);
           tma_load_2d(b_dst, &tmap_b, kb * kBK, b0, &full[s]);
-          if constexpr (EPI == GEPI_SILU) tma_load_2d(b_dst + kTileBytes / 2, &tmap_b, kb * kBK, n0 + p.N, &full[s]);
+          if constexpr (EPI == GEPI_SILU) tma_load_2d(b_dst + B_BYTES / 2, &tmap_b, kb * kBK, n0 + p.N, &full[s]);
           tma_load_2d(a_dst, &tmap_a, kb * kBK, m0, &full[s]);
         }
         if (++s == stages) {
@@ -405,7 +410,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!(ok = mbar_wait_limited(&full[s], ph, p.err, kGemmWaitCode | 6))) break;
         tc_fence_after();
-        const uint32_t a_addr = smem_u32(sA + s * a_bytes), b_addr = smem_u32(sB + s * kTileBytes);
+        const uint32_t a_addr = smem_u32(sA + s * a_bytes), b_addr = smem_u32(sB + s * B_BYTES);
 #pragma unroll
         for (int k = 0; k < kBK / 16; ++k) {   // 16 bf16 = 32 bytes further along K inside the 128-byte swizzle row
           const uint32_t accumulate = (kb > kb0 || k > 0) ? 1u : 0u;
@@ -426,7 +431,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         drain_async();
       }
     }
-  } else if constexpr (FORM == kWhole) {
+  } else if constexpr (STRAIGHT) {
     // ---------------------------------------------------------------------------------------------- epilogue, a row per thread
     const int q = warp & 3, row = q * 32 + lane;
     const bool mine = row < valid;
@@ -461,8 +466,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
           for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * j + e]);
           if (EPI == GEPI_STORE && p.bias != nullptr) {
+            float b[8];
+            if ((reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
+              reinterpret_cast<float4*>(b)[0] = reinterpret_cast<const float4*>(p.bias + col)[0];
+              reinterpret_cast<float4*>(b)[1] = reinterpret_cast<const float4*>(p.bias + col)[1];
+            } else {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] += p.bias[col + e];
+              for (int e = 0; e < 8; ++e) b[e] = p.bias[col + e];
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] += b[e];
           }
           if constexpr (EPI == GEPI_ACCUM) {
 #pragma unroll
@@ -515,11 +528,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     }
   }
-  if (FORM != kWhole && !ok) *gave_up = 1;
+  if (!STRAIGHT && !ok) *gave_up = 1;
   tc_fence_before();
   __syncwarp();
   __syncthreads();
-  if constexpr (FORM != kWhole) {
+  if constexpr (!STRAIGHT) {
     cluster_sync_all();   // every partial of the tile is in place
 
     // -------------------------------------------------------------------------------- sum, epilogue, store: 8 columns at a time
@@ -648,11 +661,11 @@ int launch_split(const GemmArgs<OT>& args, const void* A, const void* B, int64_t
   GemmArgs<OT> p = args;
   int rc;
   if ((rc = split_setup<OT, EPI, FORM>()) != B200_OK || (rc = wait_word(&p.err)) != B200_OK) return rc;
-  constexpr int W = FORM == kSplitPair ? 2 : 1, OUT = 128 * W / (EPI == GEPI_SILU ? 2 : 1);
+  constexpr int W = FORM == kSplitPair ? 2 : 1, BN = FORM == kSplitPair || FORM == kWide ? 256 : 128, OUT = BN / (EPI == GEPI_SILU ? 2 : 1);
   const int box_rows = (int)std::min<int64_t>(128, ((int64_t)p.M + 7) / 8 * 8);
   CUtensorMap ta, tb;
   if ((rc = make_tmap(&ta, A, p.M, p.K, box_rows)) != B200_OK) return rc;
-  if ((rc = make_tmap(&tb, B, rows_b, p.K, EPI == GEPI_SILU ? 64 : 128)) != B200_OK) return rc;
+  if ((rc = make_tmap(&tb, B, rows_b, p.K, EPI == GEPI_SILU ? BN / 2 : BN / W)) != B200_OK) return rc;
   ClusterLaunch l(dim3((unsigned)((p.N + OUT - 1) / OUT * splits * W), (unsigned)((p.M + 128 * W - 1) / (128 * W))), (unsigned)(splits * W), st);
   g_launches.fetch_add(1);
   B200_CUDA(cudaLaunchKernelEx(&l.cfg, gemm_split_kernel<OT, EPI, FORM>, ta, tb, (const GemmArgs<OT>)p, splits, box_rows));
@@ -666,12 +679,13 @@ constexpr int kSplitMinKb = 8;   // k-blocks that a split takes at least: shorte
 // configurations: a k-block is 0.29 µs for either tile, a pair's grows to 0.40 µs when
 // every SM runs several tiles (power); the rest is launch, pipeline fill and epilogue.  Measured, µs, M × N × K: 128 × 3 072 × 8 192
 // whole-K tiles 44, five splits 19; 16 × 896 × 4 864 27 → 9 (eight splits); 512 × 3 072 × 8 192 44 → 33 (pairs, two splits);
-// 2 048 × 12 288 × 2 048 persistent pairs 74, one-CTA tiles 174.  B200_GEMM = "persistent" | "tile" forces the
-// persistent pairs or one whole-K tile per CTA.  The products of a prompt pass (no split) find their weights in HBM and their epilogue
+// 2 048 × 12 288 × 2 048 persistent pairs 74, one-CTA tiles 174; 300 × 10 944 × 2 048, where 86 tiles are two rounds of pairs and 258 tiles two
+// of single CTAs, but 129 wide ones a single round: 26.0, 28.4, 20.3.  B200_GEMM = "persistent" | "tile" | "wide" forces the
+// persistent pairs or one whole-K tile of 128 or 256 columns per CTA.  The products of a prompt pass (no split) find their weights in HBM and their epilogue
 // is not hidden when a pair has one tile: 6 … 8 µs on top of the fit, so pairs start later there (24-layer, 896-wide prompt of 300
 // rows, µs: pairs 3 353, tiles 2 536; 28-layer, 2 048-wide one of 800 rows: pairs 5 724, tiles 6 604).
 struct GemmPick {
-  int kind;     // 0: a CTA per tile (and split); 1: a pair per tile (and split); 2: persistent pairs
+  int kind;     // 0: a CTA per tile (and split); 1: a pair per tile (and split); 2: persistent pairs; 3: a CTA per wide tile
   int splits;
 };
 // Without SPLIT the order in which a row's products are summed is the same whatever M is, so a prompt's rows have the same bits in one
@@ -692,18 +706,25 @@ void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   };
   // rows of tiles run over grid.y: up to 65 535 of them, 8.4 M rows; the persistent pairs take any number
   const bool fits = up(M, 128) <= 65535;
-  const bool tile = fits && env_choice("B200_GEMM", 't', false), any_split = fits && !env_choice("B200_GEMM", 'p', false);
+  const char* env = std::getenv("B200_GEMM");   // looked up once: routed experts' products wait for the host
+  const char forced = env != nullptr ? env[0] : 0;
+  const bool tile = fits && forced == 't', wide = fits && forced == 'w', any_split = fits && !wide && forced != 'p';
+  if (wide) consider(3, 1, 0.0);
   if (!tile) {
     const int64_t rounds = up(up(M, 256) * up(N, 256 / D), pairs);
     const double tile_us = (double)kb * (0.30 + 0.02 * (double)std::min<int64_t>(rounds - 1, 5));
     const double epilogue = EPI == GEPI_SILU ? 13.0 : 0.0;   // of a 256 × 256 tile: longer than a short k range
     consider(2, 1, (SPLIT ? 5.5 : 12.0) + (double)rounds * std::max(tile_us, epilogue) + epilogue);
   }
+  if (any_split && !tile) {
+    const int64_t t = up(M, 128) * up(N, 256 / D);
+    consider(3, 1, (double)up(t, 2 * pairs) * (7.6 + (t >= 100 ? 0.44 : 0.36) * (double)kb + (EPI == GEPI_SILU ? 2.0 : 0.0)));
+  }
   if (any_split) {
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
     for (int s = 1; s <= (SPLIT && !tile ? 8 : 1) && (s == 1 || s * kSplitMinKb <= kb); ++s) {
       const int64_t t = up(M, 128) * up(N, 128 / D) * s;
-      if (s == 1) consider(0, s, (double)up(t, 2 * pairs) * (5.15 + rows * 2.25 + 0.29 * (double)kb));
+      if (s == 1) consider(0, s, (double)up(t, 2 * pairs) * (4.3 + rows * 0.8 + 0.295 * (double)kb + (EPI == GEPI_SILU ? 1.5 : 0.0)));
       else if constexpr (SPLIT)
         consider(0, s, (double)up(t, split_capacity<kSplit>(s)) * (5.0 + 0.15 * s + rows * (2.0 + 0.25 * s) + 0.29 * (double)up(kb, s)));
     }
@@ -720,6 +741,7 @@ template <typename OT, int EPI, bool SPLIT = false>
 int launch_gemm(const GemmArgs<OT>& p, const void* A, const void* B, int64_t rows_b, cudaStream_t st) {
   GemmPick g{};
   pick_gemm<OT, EPI, SPLIT>(p.M, p.N, p.K, &g);
+  if (g.kind == 3) return launch_split<OT, EPI, kWide>(p, A, B, rows_b, 1, st);
   if (g.kind == 0 && g.splits == 1) return launch_split<OT, EPI, kWhole>(p, A, B, rows_b, 1, st);
   if constexpr (SPLIT) {
     if (g.kind == 0) return launch_split<OT, EPI, kSplit>(p, A, B, rows_b, g.splits, st);
