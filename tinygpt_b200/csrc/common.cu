@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 namespace b200 {
 
@@ -113,24 +114,34 @@ int make_tmap_sw128(CUtensorMap* out, int rank, const void* base, int64_t batch,
   return B200_OK;
 }
 
-// The allocation must not disturb a capture that may be running on this thread.
+// Words come from pages of 1 024 that stay with the process: pinning memory takes a millisecond, an engine comes and goes more often.
+static std::mutex word_mutex;
+static std::vector<unsigned*> free_words;
 int wait_word_new(unsigned** out) {
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  cudaThreadExchangeStreamCaptureMode(&mode);
-  void* p = nullptr;
-  const cudaError_t err = cudaHostAlloc(&p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
-  cudaThreadExchangeStreamCaptureMode(&mode);
-  if (err != cudaSuccess) {
-    (void)cudaGetLastError();
-    set_error("no pinned host memory for the kernels' error word");
-    return B200_ERR_CUDA;
+  std::lock_guard<std::mutex> lock(word_mutex);
+  if (free_words.empty()) {
+    constexpr int kWords = 1024;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // the allocation must not disturb a capture that may be running on this thread
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    const cudaError_t err = cudaHostAlloc(&p, kWords * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (err != cudaSuccess) {
+      (void)cudaGetLastError();
+      set_error("no pinned host memory for the kernels' error words");
+      return B200_ERR_CUDA;
+    }
+    for (int i = kWords - 1; i >= 0; --i) free_words.push_back(static_cast<unsigned*>(p) + i);
   }
-  *out = static_cast<unsigned*>(p);
-  **out = 0;
+  *out = free_words.back();
+  free_words.pop_back();
+  __atomic_store_n(*out, 0u, __ATOMIC_RELEASE);
   return B200_OK;
 }
-void wait_word_free(unsigned* word) {
-  if (word != nullptr) cudaFreeHost(word);
+void wait_word_free(unsigned* word) {   // nothing that writes to it is in flight any more
+  if (word == nullptr) return;
+  std::lock_guard<std::mutex> lock(word_mutex);
+  free_words.push_back(word);
 }
 
 static int report_wait(unsigned code) {
