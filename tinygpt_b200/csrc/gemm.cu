@@ -683,14 +683,14 @@ constexpr int kSplitMinKb = 8;   // k-blocks that a split takes at least: shorte
 // of single CTAs, but 129 wide ones a single round: 26.0, 28.4, 20.3.  B200_GEMM = "persistent" | "tile" | "wide" forces the
 // persistent pairs or one whole-K tile of 128 or 256 columns per CTA.  The products of a prompt pass (no split) find their weights in HBM and their epilogue
 // is not hidden when a pair has one tile: 6 … 8 µs on top of the fit, so pairs start later there (24-layer, 896-wide prompt of 300
-// rows, µs: pairs 3 353, tiles 2 536; 28-layer, 2 048-wide one of 800 rows: pairs 5 724, tiles 6 604).
+// rows, µs: pairs 3 366, tiles 2 400; 28-layer, 2 048-wide one of 800 rows: pairs 5 717, tiles 6 019).
 struct GemmPick {
   int kind;     // 0: a CTA per tile (and split); 1: a pair per tile (and split); 2: persistent pairs; 3: a CTA per wide tile
   int splits;
 };
 // Without SPLIT the order in which a row's products are summed is the same whatever M is, so a prompt's rows have the same bits in one
 // pass, in portions and in a batch.  What that costs a layer-stack prompt against splits chosen by M (8 layers of 2 048, µs): 64 rows
-// 833 → 1 132, 300 rows 1 123 → 1 398, 2 048 rows none.
+// 833 → 1 087, 300 rows 1 123 → 1 301, 2 048 rows none.
 template <typename OT, int EPI, bool SPLIT>
 void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   constexpr int D = EPI == GEPI_SILU ? 2 : 1;
