@@ -358,9 +358,10 @@ struct ScanRem {
   static constexpr int COLS = 128 / LN * C, CH = DK <= 128 ? 16 : DK <= 256 ? 8 : 4;
   static constexpr int FLOATS = CH * (NV * DK + COLS + 2);    // of a buffer: vectors, values (by column), value scales, scalar decays
   static constexpr int smem = kRemBuf * FLOATS * 4;
-  // registers for as many CTAs as an SM's shared memory holds; keys of up to 128 need fewer than two allow, and what the compiler makes of
-  // a bound of two is the faster code (2 048 tokens, 16 heads of 128 × 128: 377 against 381 µs)
-  static constexpr int CTAS = RPL > 8 && 2 * (smem + 1024) > 228 * 1024 ? 1 : 2;
+  // The launch bound.  Where the ring leaves room for one CTA, a bound of one allows 255 registers instead of 168.  Keys of 129 … 256 with a
+  // decay per channel use 238 (1 024 tokens, 8 heads of 256 × 128: 312 → 301 µs); the other forms need no more than 168, or are faster with
+  // a few spills (4 heads of 512 × 128 357 against 364 µs, 16 heads of 128 × 128 over 2 048 tokens 377 against 381).
+  static constexpr int CTAS = RPL > 8 && LN <= 16 && 2 * (smem + 1024) > 228 * 1024 ? 1 : 2;
 };
 __device__ __forceinline__ float shfl_xor_ordered(float v, int m) {   // stays in order with the loads below
   float r;
