@@ -87,4 +87,12 @@ def test_operators_report_their_own_once(built_lib):
     assert torch.equal(ops.gemm(a, a), want)
     word().value = 0x6E000007
     assert lib().b200_wait_status() != 0 and lib().b200_wait_status() == 0
+    word().value = 0xA7000001
+    other = llama()                            # an engine neither minds nor takes the report
+    assert lib().b200_device_check() == 0
+    q = torch.ones(1, 8, 2, 64, dtype=torch.bfloat16, device=DEV)
+    with pytest.raises(B200Error, match="0xa7000001"):
+        ops.flash_attention(q, q, q, True)
+    ops.flash_attention(q, q, q, True)
+    other.close()
     eng.close()

@@ -35,7 +35,7 @@ int b200_gemv_bf16(void* y, const void* x, const void* W, const void* bias, int6
   using namespace b200;
   B200_CHECK_ARG(y && x && W, "gemv: null pointer");
   B200_CHECK_ARG(m >= 1 && m <= 4096, "gemv: m=%lld out of range (this entry point is the decode GEMV)", (long long)m);
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   if ((rc = gemv_setup_attributes()) != B200_OK) return rc;
   // More rows than one decode batch: the tensor-core GEMM, where its alignment rules hold — two passes of eight rows over W stay ahead of it
@@ -78,7 +78,7 @@ int b200_gemv_fused_bf16(void* y, const void* x, const void* W, int64_t n, int64
   B200_CHECK_ARG(!(silu_mul && (bias || residual)), "gemv_fused: silu_mul excludes bias/residual");
   B200_CHECK_ARG(!(bias && residual), "gemv_fused: bias and residual are exclusive");
   B200_CHECK_ARG((nseg == 2) == (silu_mul != 0), "gemv_fused: nseg == 2 exactly when silu_mul");
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   if ((rc = gemv_setup_attributes()) != B200_OK) return rc;
   GemvPlan plan;
@@ -110,7 +110,7 @@ int b200_attn_decode_bf16(void* out, const void* qkv, const void* q_norm, const 
   using namespace b200;
   B200_CHECK_ARG(out && qkv && kcache && vcache && workspace, "attn_decode: null pointer");
   B200_CHECK_ARG(pos != nullptr || (fixed_len >= 1 && fixed_len <= max_ctx), "attn_decode: fixed_len out of range");
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   if ((rc = attn_setup_attributes()) != B200_OK) return rc;
   AttnDecodeParams a{};
@@ -140,7 +140,7 @@ extern "C" {
 
 int b200_stack_rmsnorm(void* y, const float* x, const float* w, int64_t rows, int64_t dim, float eps, float offset,
                        int dtype, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(dim > 0 && dim < (1ll << 31) && rows < (1ll << 31), "stack_rmsnorm: size out of range");
   return b200::launch_stack_rmsnorm(y, x, w, nullptr, rows, (int)dim, eps, offset, dtype, (cudaStream_t)stream);
@@ -148,7 +148,7 @@ int b200_stack_rmsnorm(void* y, const float* x, const float* w, int64_t rows, in
 
 int b200_stack_linear(void* C, const void* A, const void* W, const float* bias, int64_t M, int64_t N, int64_t K, int dtype,
                       void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(M > 0 && N > 0 && K > 0 && M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31),
                  "stack_linear: size out of range");
@@ -175,7 +175,7 @@ int b200_stack_attention(void* out, int64_t ld_out, const void* proj, int64_t ld
                          const void* kcache, const void* vcache, int64_t k_slot_stride, int64_t v_slot_stride,
                          const int32_t* slot, const int32_t* pos, int64_t n_tok, const b200_attn_desc* attn, int dtype,
                          void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(attn && n_tok > 0 && n_tok < (1ll << 31), "stack_attention: bad arguments");
   b200::StackAttn p = stack_attn_args(proj, ld_proj, kcache, vcache, k_slot_stride, v_slot_stride, slot, pos, n_tok, attn);
@@ -187,7 +187,7 @@ int b200_stack_attention(void* out, int64_t ld_out, const void* proj, int64_t ld
 int b200_stack_kv_store(void* kcache, void* vcache, int64_t k_slot_stride, int64_t v_slot_stride, const void* proj,
                         int64_t ld_proj, int64_t off_k, int64_t off_v, const int32_t* slot, const int32_t* pos,
                         int64_t n_tok, const b200_attn_desc* attn, int dtype, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(attn && n_tok > 0 && n_tok < (1ll << 31), "stack_kv_store: bad arguments");
   b200::StackAttn p = stack_attn_args(proj, ld_proj, kcache, vcache, k_slot_stride, v_slot_stride, slot, pos, n_tok, attn);
@@ -197,7 +197,7 @@ int b200_stack_kv_store(void* kcache, void* vcache, int64_t k_slot_stride, int64
 
 int b200_stack_act_mul(void* y, int64_t ld_y, const void* g, const void* u, int64_t ld_gu, int64_t rows, int64_t n, int act,
                        int dtype, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(n > 0 && n < (1ll << 31), "stack_act_mul: size out of range");
   return b200::launch_stack_act_mul(y, ld_y, g, u, ld_gu, rows, (int)n, act, dtype, (cudaStream_t)stream);
@@ -205,7 +205,7 @@ int b200_stack_act_mul(void* y, int64_t ld_y, const void* g, const void* u, int6
 
 int b200_stack_rms_add(float* x, const float* y, const float* w, int64_t rows, int64_t dim, float eps, float mult,
                        void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(dim > 0 && dim < (1ll << 31) && rows < (1ll << 31), "stack_rms_add: size out of range");
   return b200::launch_stack_rms_add(x, y, w, rows, (int)dim, eps, mult, (cudaStream_t)stream);
@@ -231,7 +231,7 @@ struct Scratch {
 
 int b200_stack_norm(void* y, float* xadd, const float* x, const float* w, int64_t rows, int64_t dim, float eps, int kind,
                     int add, int dtype, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(dim > 0 && dim < (1ll << 31) && rows > 0 && rows < (1ll << 31), "stack_norm: size out of range");
   if (add) return b200::launch_stack_norm_add(xadd, x, false, w, rows, (int)dim, eps, 1.f, kind, (cudaStream_t)stream);
@@ -241,7 +241,7 @@ int b200_stack_norm(void* y, float* xadd, const float* x, const float* w, int64_
 int b200_stack_latent_attention(void* out, int64_t ld_out, const void* proj, int64_t ld_proj, int64_t off_down, void* cache,
                                 int64_t slot_stride, const int32_t* slot, const int32_t* pos, int64_t n_tok,
                                 const b200_attn_desc* attn, const b200_latent_desc* lat, float eps, int dtype, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(attn && lat && n_tok > 0 && n_tok < (1 << 24), "stack_latent_attention: bad arguments");
   B200_CHECK_ARG(dtype == B200_BF16 || dtype == B200_F32, "stack_latent_attention: unknown dtype");
@@ -262,7 +262,7 @@ int b200_stack_mlstm(float* out, const void* proj, int64_t ld_proj, int64_t off_
                      const float* gates, float* state, int64_t slot_stride, const int32_t* row0, const int32_t* count,
                      const int32_t* slot, const int32_t* pos, int64_t n_seq, int64_t n_rows, const b200_attn_desc* sizes,
                      float gate_cap, int dtype, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(sizes && n_seq > 0 && n_rows >= n_seq && n_rows < (1 << 24), "stack_mlstm: bad arguments");
   b200::MlstmRun p;
@@ -284,7 +284,7 @@ int64_t b200_stack_mlstm_state_floats(int64_t heads, int64_t dim, int64_t vdim) 
 
 int b200_stack_moe(float* y, const void* h, int64_t rows, int64_t width, const b200_moe_desc* moe, int32_t* chosen,
                    float* scores, int dtype, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(moe && rows > 0 && rows < (1 << 22) && width > 0 && width < (1 << 24) && moe->top > 0 && moe->experts > 0,
                  "stack_moe: bad arguments");
@@ -314,7 +314,7 @@ int b200_stack_lin_scan(float* out, const float* d, const float* p, const float*
                         const float* vscale, int64_t ld, int64_t heads, int64_t dk, int64_t dv, int64_t share, int64_t d_scalar,
                         float* state, int64_t slot_stride, const int32_t* row0, const int32_t* count, const int32_t* slot,
                         const int32_t* pos, int64_t n_seq, int64_t n_rows, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(n_seq > 0 && n_rows >= n_seq && n_rows < (1 << 24) && heads > 0 && heads < (1 << 16) && dk > 0 && dv > 0 &&
                      dv < (1 << 20),
@@ -331,7 +331,7 @@ int b200_stack_lin_scan(float* out, const float* d, const float* p, const float*
 int b200_stack_attn_prep(void* proj, int64_t ld_proj, int64_t off_q, int64_t off_k, int64_t off_v, const int32_t* pos,
                          int64_t n_tok, const b200_attn_desc* attn, const b200_attn_prep_desc* prep, void* vkeep,
                          int64_t ld_keep, float eps, int dtype, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(attn && prep && n_tok > 0 && n_tok < (1 << 24), "stack_attn_prep: bad arguments");
   b200::AttnPrep a;
@@ -342,7 +342,7 @@ int b200_stack_attn_prep(void* proj, int64_t ld_proj, int64_t off_q, int64_t off
 }
 
 int b200_stack_glu_clamp(void* y, const void* gu, int64_t rows, int64_t n, float limit, int dtype, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(n > 0 && n < (1ll << 30) && rows > 0, "stack_glu_clamp: size out of range");
   return b200::launch_stack_glu_clamp(y, n, gu, 2 * n, rows, (int)n, limit, dtype, (cudaStream_t)stream);
@@ -352,7 +352,7 @@ int b200_stack_glu_clamp(void* y, const void* gu, int64_t rows, int64_t n, float
 int b200_stack_hyper_step(void* h, float* x, const float* y, const float* in, const b200_hyper_desc* prev, float mult,
                           const float* norm_w, float eps, float offset, int64_t rows, int64_t streams, int64_t width, int dtype,
                           void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(h && rows > 0 && rows < (1 << 24) && width > 0 && width < (1 << 24) && (y == nullptr || prev), "stack_hyper_step: bad arguments");
   b200::HyperStep p;
@@ -365,7 +365,7 @@ int b200_stack_hyper_step(void* h, float* x, const float* y, const float* in, co
 int b200_stack_input_conv(void* h, void* mix, const float* hn, const float* w, const float* mu, int64_t taps, const float* state,
                           int64_t slot_stride, const int32_t* slot, const int32_t* pos, int64_t rows, int64_t width, int dtype,
                           void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(rows > 0 && rows < (1 << 24) && width > 0 && width < (1 << 24), "stack_input_conv: bad arguments");
   b200::InputConv c;
@@ -376,7 +376,7 @@ int b200_stack_input_conv(void* h, void* mix, const float* hn, const float* w, c
 int b200_stack_pool_attention(void* out, const void* q, const void* kcache, const void* vcache, int64_t k_slot_stride,
                               int64_t v_slot_stride, int64_t max_ctx, const int32_t* slot, const int32_t* pos, int64_t n_tok,
                               const b200_attn_desc* attn, const b200_pool_attn_desc* pool, int64_t splits, int dtype, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(attn && pool && n_tok > 0 && n_tok < (1 << 16) && max_ctx > 0 && max_ctx < (1 << 24) && attn->heads > 0 && attn->vdim > 0 &&
                      attn->window >= 0 && pool->pool >= 0 && splits >= 1 && splits <= b200::kPoolMaxSplits,
@@ -404,7 +404,7 @@ int b200_stack_pool_attention(void* out, const void* q, const void* kcache, cons
 int b200_stack_bonus_scan(float* out, const float* d, const float* k, const float* r, const float* v, const float* bonus, int64_t ld,
                           int64_t heads, int64_t dk, int64_t dv, float* state, int64_t slot_stride, const int32_t* row0,
                           const int32_t* count, const int32_t* slot, const int32_t* pos, int64_t n_seq, int64_t n_rows, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(n_seq > 0 && n_rows >= n_seq && n_rows < (1 << 24) && heads > 0 && heads < (1 << 16) && dk > 0 && dv > 0 && dv < (1 << 20),
                  "stack_bonus_scan: bad arguments");
@@ -421,7 +421,7 @@ int b200_stack_mamba1_scan(void* out, const void* z, const void* xc, const float
                            const b200_mamba1_desc* desc, float* state, int64_t slot_stride, const int32_t* row0,
                            const int32_t* count, const int32_t* slot, const int32_t* pos, int64_t n_seq, int64_t n_rows, int dtype,
                            void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(desc && n_seq > 0 && n_rows >= n_seq && n_rows < (1 << 24), "stack_mamba1_scan: bad arguments");
   b200::Mamba1Run m;

@@ -764,6 +764,7 @@ extern "C" int b200_attn_bf16(void* o, const void* q, const void* k, const void*
                               int64_t Hq, int64_t Hkv, int64_t hd, int causal, void* stream) {
   using namespace b200;
   B200_CHECK_ARG(o && q && k && v, "attention: null pointer");
+  if (int bad = op_wait_check()) return bad;
   // A contiguous view may start anywhere: the prompt kernels read q, k and v 16 bytes at a time and store o in words, the row kernel reads k
   // and v 16 bytes at a time; what is not aligned for them goes to the general kernel.
   if (causal && Sq == Skv && Sq > 1 && prefill_attn_mma_enabled() && aligned16(q, k, v) && (reinterpret_cast<uintptr_t>(o) & 3) == 0)

@@ -168,6 +168,11 @@ int op_wait_check() {
   return w == nullptr || *(volatile unsigned*)w == 0 ? B200_OK : report_wait(__atomic_exchange_n(w, 0u, __ATOMIC_ACQ_REL));
 }
 
+int op_check() {
+  const int rc = b200_device_check();
+  return rc != B200_OK ? rc : op_wait_check();
+}
+
 static thread_local unsigned* t_wait_word = nullptr;
 WaitScope::WaitScope(unsigned* word) : outer(t_wait_word) { t_wait_word = word; }
 WaitScope::~WaitScope() { t_wait_word = outer; }
@@ -202,7 +207,7 @@ int b200_device_check(void) {
     b200::set_error("device %d has compute capability major %d; this library contains sm_100a code only", dev, major);
     return B200_ERR_NO_DEVICE;
   }
-  return b200::op_wait_check();
+  return B200_OK;
 }
 
 int b200_wait_status(void) { return b200::op_wait_check(); }

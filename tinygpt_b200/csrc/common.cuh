@@ -228,6 +228,7 @@ void wait_word_free(unsigned* word);
 int wait_word_check(const unsigned* word);   // B200_ERR_CUDA while a code is there
 int op_wait_word(unsigned** out);
 int op_wait_check();                         // the operators': reports and clears
+int op_check();                              // what a stand-alone operator asks first: b200_device_check, then op_wait_check
 int wait_word(unsigned** out);               // the word for a launch on this thread
 struct WaitScope {                           // launches of this thread write to `word`
   unsigned* outer;

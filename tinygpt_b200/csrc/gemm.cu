@@ -815,7 +815,7 @@ int launch_gemm_bf16_logits(float* C, void* C_bf16, const void* A, const void* B
 }  // namespace b200
 
 extern "C" int b200_gemm_bf16(void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   return b200::launch_linear_split_bf16(C, A, B, M, N, K, nullptr, (cudaStream_t)stream);
 }

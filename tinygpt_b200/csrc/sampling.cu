@@ -372,7 +372,7 @@ int64_t b200_sample_workspace_bytes(void) { return b200::sample_workspace_bytes(
 
 int b200_sample_bf16(int64_t* token_out, const void* logits, int64_t V, float temperature, int64_t top_k, float top_p,
                      float min_p, float u, void* workspace, void* stream) {
-  int rc = b200_device_check();
+  int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   return b200::launch_sample(token_out, logits, V, temperature, top_k, top_p, min_p, u, workspace, (cudaStream_t)stream,
                              nullptr, 0ull, false);
