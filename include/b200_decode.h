@@ -74,7 +74,7 @@ int b200_device_check(void);
  * y = bf16( float(y) + float(bias[n]) )  — the reference's second rounding for 3-D Linear inputs.
  * [ref: TT/Operation/OpLinalg.cpp:244-277 matmul + addInplace; TT/Operation/OpLinalgCuda.cuh:276-293
  *  gemmStridedBatchedCudaBF16Impl; caller TT/Function/FuncNNLayer.h:14-18 FuncLinear]
- * Requirements: k % 8 == 0, W 16-byte aligned.  m = 1 (decode) streams W once; m ≤ 8 share one pass over W (m ≤ 16 two, for a
+ * Requirements: k % 8 == 0, x and W 16-byte aligned.  m = 1 (decode) streams W once; m ≤ 8 share one pass over W (m ≤ 16 two, for a
  * small W); more rows take the tensor-core GEMM. */
 int b200_gemv_bf16(void* y, const void* x, const void* W, const void* bias_or_null, int64_t m, int64_t n, int64_t k,
                    void* stream);

@@ -55,6 +55,15 @@ def test_views_off_a_16_byte_boundary(built_lib, which, n, rows, causal, D):
     assert float((got - want).norm() / want.norm()) < 2.0 ** -8      # the kernels' order of sums, and P in bf16 in the prompt's
 
 
+@pytest.mark.parametrize("ctx", [256, 2304])
+def test_decode_caches_off_a_16_byte_boundary_are_refused(built_lib, ctx):
+    from tinygpt_b200._lib import B200Error
+    qkv, cache = randn(10 * 64, seed=1), randn(ctx, 2, 64, seed=2)
+    for k, v in ((shifted(cache), cache), (cache, shifted(cache))):
+        with pytest.raises(B200Error, match="aligned"):
+            ops.attn_decode(qkv, k, v, q_heads=6, kv_heads=2, head_dim=64, fixed_len=9)
+
+
 def test_huge_scores_and_zeros(built_lib):
     """Scores thousands apart (one key takes all), equal scores, and a row of zeros."""
     q = torch.full((1, 1, 2, 64), 8.0, device=DEV, dtype=torch.bfloat16)

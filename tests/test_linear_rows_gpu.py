@@ -34,3 +34,13 @@ def test_rows(built_lib, m, n, k, bias):
     check(lib().b200_gemv_bf16(guard.data_ptr(), x.data_ptr(), w.data_ptr(), b.data_ptr() if bias else None, m, n, k,
                                torch.cuda.current_stream().cuda_stream), "gemv")
     assert torch.equal(guard[:m], got) and bool((guard[m:] == 3.0).all())
+
+
+@pytest.mark.parametrize("m", [1, 5, 40])
+def test_rows_off_a_16_byte_boundary_are_refused(built_lib, m):
+    """x is read 16 bytes at a time: a view that starts elsewhere is an error on the host."""
+    from tinygpt_b200._lib import B200Error
+    x, w = rand(m * 72 + 1, seed=1)[1:].view(m, 72), rand(13, 72, seed=2)
+    with pytest.raises(B200Error, match="aligned"):
+        ops.linear(x, w)
+    assert torch.equal(ops.linear(x.clone(), w), ops.linear(x.clone(), w))

@@ -35,6 +35,7 @@ int b200_gemv_bf16(void* y, const void* x, const void* W, const void* bias, int6
   using namespace b200;
   B200_CHECK_ARG(y && x && W, "gemv: null pointer");
   B200_CHECK_ARG(m >= 1 && m <= 4096, "gemv: m=%lld out of range (this entry point is the decode GEMV)", (long long)m);
+  B200_CHECK_ARG(aligned16(x), "gemv: x must be 16-byte aligned");
   int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   if ((rc = gemv_setup_attributes()) != B200_OK) return rc;
@@ -78,6 +79,7 @@ int b200_gemv_fused_bf16(void* y, const void* x, const void* W, int64_t n, int64
   B200_CHECK_ARG(!(silu_mul && (bias || residual)), "gemv_fused: silu_mul excludes bias/residual");
   B200_CHECK_ARG(!(bias && residual), "gemv_fused: bias and residual are exclusive");
   B200_CHECK_ARG((nseg == 2) == (silu_mul != 0), "gemv_fused: nseg == 2 exactly when silu_mul");
+  B200_CHECK_ARG(aligned16(x, norm_w), "gemv_fused: x and the norm weight must be 16-byte aligned");
   int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   if ((rc = gemv_setup_attributes()) != B200_OK) return rc;
@@ -110,6 +112,7 @@ int b200_attn_decode_bf16(void* out, const void* qkv, const void* q_norm, const 
   using namespace b200;
   B200_CHECK_ARG(out && qkv && kcache && vcache && workspace, "attn_decode: null pointer");
   B200_CHECK_ARG(pos != nullptr || (fixed_len >= 1 && fixed_len <= max_ctx), "attn_decode: fixed_len out of range");
+  B200_CHECK_ARG(aligned16(kcache, vcache), "attn_decode: caches must be 16-byte aligned");
   int rc = b200::op_check();
   if (rc != B200_OK) return rc;
   if ((rc = attn_setup_attributes()) != B200_OK) return rc;
