@@ -9,7 +9,9 @@
 //   warp 1    MMA issuer (one thread): S = Q·Kᵀ of the next tile goes out before P·V of this one, so the tensor pipe works
 //             while the softmax warps hold a tile; S is double-buffered in TMEM, O stays in TMEM
 //   warps 2-5 softmax, one row per thread: S from TMEM, row maximum and sum without shuffles, P (bf16) back into the TMEM columns
-//             of S as the A operand of P·V; O is rescaled in TMEM where a row's maximum grew
+//             of S as the A operand of P·V; O is rescaled in TMEM where a row's maximum grew (nearly every tile of 32 rows), behind the
+//             exponentials: by then the product before is over and S's registers are free for two loads of O in flight
+//             (16 heads of 128 over 2 048 rows 51.1 → 48.1 µs)
 // Late query blocks (most keys) of all heads are scheduled first.
 //
 // A key that a row does not see has P = 0, and 0 · V is 0 only for finite V: tiles that some row of the block sees in part are looked
@@ -18,7 +20,7 @@
 //
 // Bound by the chain of tiles that a late block waits for: about 1.1 µs each, most of it the latency of TMEM loads, maxima, 64
 // exponentials and TMEM stores of one warp (issue slots 26 %, tensor pipe 20 % busy).  µs, mma.sync → here, same error against 64 bits:
-// 16 heads of 128 over 2 048 rows 112 → 50, 24 heads 146 → 53; 14 heads of 64 over 2 048 rows 51 → 41; 16 heads of 128 over 512
+// 16 heads of 128 over 2 048 rows 112 → 48, 24 heads 146 → 53; 14 heads of 64 over 2 048 rows 51 → 41; 16 heads of 128 over 512
 // rows 17.8 → 18.2, which is where the dispatch stops (prefill_attn_tc_wins).
 #include "ops.cuh"
 #include "tc.cuh"
@@ -295,28 +297,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
         for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(s0[j + e]), __uint_as_float(s1[j + e])));
       }
       const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      if (it == 0) {
-        m = top;
-      } else {
-        const bool grow = top > m;
-        if (__any_sync(0xffffffffu, grow)) {
-          ok = __all_sync(0xffffffffu, mbar_wait_limited(pv_done, (uint32_t)((it - 1) & 1), p.err, kAttnWaitCode | 8));
-          if (!ok) break;
-          tc_fence_after();
-          const float alpha = grow ? ex2f((m - top) * k_scale) : 1.f;
-          if (grow) m = top;
-          l *= alpha;
-#pragma unroll 1
-          for (int c = 0; c < HD; c += 32) {
-            uint32_t o[32];
-            tmem_ld32(lane_base + kColO + c, o);
-            tmem_wait_ld();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
-            tmem_st32(lane_base + kColO + c, o);
-          }
-        }
-      }
+      const bool grow = top > m;
+      const bool rescale = it > 0 && __any_sync(0xffffffffu, grow);
+      const float alpha = grow && it > 0 ? ex2f((m - top) * k_scale) : 1.f;
+      if (grow) m = top;
+      l *= alpha;
       const float ms = m == -INFINITY ? 0.f : m * k_scale;
       const uint64_t neg = pack_f2(-ms, -ms);
       uint64_t sum[2] = {0, 0};
@@ -334,6 +319,25 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
       sum[0] = add_f2(sum[0], sum[1]);
       l += lo_f2(sum[0]) + hi_f2(sum[0]);
       tmem_st32(sbuf, pk);
+      if (rescale) {
+        ok = __all_sync(0xffffffffu, mbar_wait_limited(pv_done, (uint32_t)((it - 1) & 1), p.err, kAttnWaitCode | 8));
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < HD; c += 64) {
+          uint32_t o0[32], o1[32];
+          tmem_ld32(lane_base + kColO + c, o0);
+          tmem_ld32(lane_base + kColO + c + 32, o1);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            o0[j] = __float_as_uint(__uint_as_float(o0[j]) * alpha);
+            o1[j] = __float_as_uint(__uint_as_float(o1[j]) * alpha);
+          }
+          tmem_st32(lane_base + kColO + c, o0);
+          tmem_st32(lane_base + kColO + c + 32, o1);
+        }
+      }
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
