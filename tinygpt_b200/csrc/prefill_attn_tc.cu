@@ -3,25 +3,30 @@
 // fp32, P rounded to bf16, bf16 P·V products summed in fp32), same masks (causal over a cached prefix, sliding window with
 // kept first keys), sink and per-head gate.
 //
-// Shape of the work: a CTA takes 128 query rows of one query head, keys in tiles of 64 in ascending order, two CTAs per SM
-// (96 KB of shared memory, 256 TMEM columns each) so that one CTA's softmax runs beside the other's products:
+// Shape of the work: 128 query rows of one query head against keys in tiles of 64 in ascending order, by one CTA or by a cluster of two that
+// share the tiles by parity (attn_tc_halves), two CTAs per SM (96 KB of shared memory, 256 TMEM columns each) so that one CTA's softmax
+// runs beside the other's products:
 //   warp 0    TMA producer: the Q block once, then K and V tiles (128-byte swizzle; rows past the sequence are zero-filled)
 //   warp 1    MMA issuer (one thread): S = Q·Kᵀ of the next tile goes out before P·V of this one, so the tensor pipe works
 //             while the softmax warps hold a tile; S is double-buffered in TMEM, O stays in TMEM
 //   warps 2-5 softmax, one row per thread: S from TMEM, row maximum and sum without shuffles, P (bf16) back into the TMEM columns
 //             of S as the A operand of P·V; O is rescaled in TMEM where a row's maximum grew (nearly every tile of 32 rows), behind the
 //             exponentials: by then the product before is over and S's registers are free for two loads of O in flight
-//             (16 heads of 128 over 2 048 rows 51.1 → 48.1 µs)
-// Late query blocks (most keys) of all heads are scheduled first.
+// Late query blocks (most keys) of all heads are scheduled first.  Two CTAs of a cluster end with a maximum, a sum and 128 columns of O per row
+// each: one hands the other half of its columns through distributed shared memory, and each finishes its own half.
 //
 // A key that a row does not see has P = 0, and 0 · V is 0 only for finite V: tiles that some row of the block sees in part are looked
 // through, and a block that meets an infinity or a NaN there is computed again key by key (see_alone), so that nothing a row
 // does not see reaches it.
 //
-// Bound by the chain of tiles that a late block waits for: about 1.1 µs each, most of it the latency of TMEM loads, maxima, 64
-// exponentials and TMEM stores of one warp (issue slots 26 %, tensor pipe 20 % busy).  µs, mma.sync → here, same error against 64 bits:
-// 16 heads of 128 over 2 048 rows 112 → 48, 24 heads 146 → 53; 14 heads of 64 over 2 048 rows 51 → 41; 16 heads of 128 over 512
-// rows 17.8 → 18.2, which is where the dispatch stops (prefill_attn_tc_wins).
+// Bound, per pair of CTAs on an SM, by the products of 64 keys (820 of 1 000 cycles a tile: an MMA of N = 64 takes as long as one of
+// N = 128) and, on small calls, by what a CTA does once: barriers, TMEM and the first loads 3 000 cycles, the end 3 000.  128-key tiles
+// (P then shares the only S buffer) and eight softmax warps of 64 keys were no faster: 43 and 40 µs where this form took 38.
+// Masks as bits (they were two comparisons per key: 4 000 to 7 000 cycles a tile), results stored in whole rows through shared memory
+// (straight from the lanes a store touches 32 rows), the first loads in front of the TMEM allocation, waits whose first look is inline.
+// µs, mma.sync / here at first / now, same error against 64 bits: 16 heads of 128 over 2 048 rows 80 / 51 / 34.6, 24 heads
+// 122 / 53 / 41.4, 32 heads 152 / 71 / 52.5; 16 heads over 512 rows 18.9 / 18.2 / 10.6; 14 heads of 64 over 2 048 rows 50 / 41 / 29.2,
+// four sequences of 333 rows 12.8 / - / 9.9.
 #include "ops.cuh"
 #include "tc.cuh"
 
@@ -73,6 +78,11 @@ __device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+__device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 __device__ __forceinline__ float lo_f2(uint64_t a) { return __uint_as_float((uint32_t)a); }
 __device__ __forceinline__ float hi_f2(uint64_t a) { return __uint_as_float((uint32_t)(a >> 32)); }
 __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int32_t c0, int32_t c1, int32_t c2, uint64_t* bar) {
@@ -81,12 +91,26 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
-// D[tmem] (+)= A[tmem]·B[smem]
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// Products whose operands are the same in the whole warp, issued where `one` is set.  D[tmem] (+)= A·B with A in shared memory or in TMEM
+__device__ __forceinline__ void umma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t a_hi, uint32_t b_hi, uint32_t idesc,
+                                        uint32_t accumulate, uint32_t one) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\tmov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %4};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}"
+      ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(a_hi), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(one)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate, uint32_t one) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 b, {%2, %3};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+      ::"r"(d), "r"(a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(one)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint64_t* bar, uint32_t one) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(one)
       : "memory");
 }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -100,11 +124,20 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
       : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// [keys][64 columns] rows of 128 bytes, 128-byte swizzle, as a B operand whose N runs along the columns (MN-major): 64-column blocks
-// `blk` bytes apart (bits 16-29), groups of 8 keys 1 024 bytes apart (bits 32-45)
-__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t smem_addr, uint32_t blk) {
-  return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)(blk >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+// Matrix descriptors in halves: the lower one holds the address (and, from bit 16 on, the distance of 64-column blocks of an operand whose N
+// runs along the columns: V's [keys][64 columns] rows of 128 bytes, MN-major), the upper one is the same for all (umma_desc)
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr) { return (smem_addr & 0x3FFFFu) >> 4; }
+
+// A wait that gave up says so to the whole CTA and sets `dead`: its role goes on without waiting (what follows neither hangs nor leaves
+// the buffers), and nothing is stored.  The first look is inline and has no loop around it.
+__device__ __noinline__ bool wait_slow(uint64_t* bar, uint32_t parity, unsigned* err, unsigned code, volatile int* gave_up) {
+  if (mbar_wait_limited(bar, parity, err, code)) return false;
+  *gave_up = 1;
+  __threadfence_block();
+  return true;
 }
+__device__ __forceinline__ uint32_t bits_below(int n) { return n >= 32 ? ~0u : n <= 0 ? 0u : (1u << n) - 1; }
 
 // One row, the keys it sees one after another (P rounded to bf16 like above): the way out for a block whose partly visible tiles hold
 // infinities or NaNs in V.  Slow and rare.
@@ -128,7 +161,7 @@ __device__ __noinline__ void see_alone(const TcAttn& p, int b, int h, int kvh, i
   }
 }
 
-template <int HD>
+template <int HD, int SPLIT>
 __global__ void __launch_bounds__(kTThreads, 2)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                const TcAttn p) {
@@ -152,9 +185,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
   uint64_t* o_full = pv_done + 1;          // the last tile's product, and so all of them
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
   int* not_finite = reinterpret_cast<int*>(tmem_slot + 1);
+  int* gave_up = not_finite + 1;
+  float4* part = reinterpret_cast<float4*>(sQ);   // [128 rows]: maximum, sum, V is not finite, gave up
+  float4* give = reinterpret_cast<float4*>(sK);   // [HD / 8][128 rows]: the columns that the other CTA finishes
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.x, qb = (int)gridDim.y - 1 - (int)blockIdx.y, b = blockIdx.z;
+  const int half = SPLIT == 2 ? (int)cluster_rank() : 0;
+  const int h = blockIdx.x / SPLIT, qb = (int)gridDim.y - 1 - (int)blockIdx.y, b = blockIdx.z;
   const int kvh = h / (p.Hq / p.Hkv);
   const int q0 = qb * kTBM;
   const int rows_valid = min(kTBM, p.S - q0);
@@ -163,10 +200,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
   // tiles to visit: with a window those of the kept first keys, then from the first row's window edge up to the diagonal
   const int t_lo = p.window > 0 ? max(0, first_pos - p.window + 1) / kTBN : 0;
   const int n_keep = p.window > 0 ? min(t_lo, (p.keep_first + kTBN - 1) / kTBN) : 0;
-  const int n_tiles = T - t_lo + n_keep;
-  auto tile_of = [&](int it) { return it < n_keep ? it : t_lo + (it - n_keep); };
-  bool ok = true;
+  // this CTA's share of them: all, or the tiles of its parity.  By the tile's place in the cache, so that a row's sums are the same however
+  // its prompt is cut
+  const int own_keep = SPLIT == 2 ? (n_keep + 1 - half) >> 1 : n_keep, own_lo = SPLIT == 2 ? t_lo + ((t_lo ^ half) & 1) : t_lo;
+  const int n_tiles = own_keep + (max(T - own_lo, 0) + SPLIT - 1) / SPLIT;
+  auto tile_of = [&](int it) { return it < own_keep ? half + SPLIT * it : own_lo + SPLIT * (it - own_keep); };
+  bool dead = false;
+  auto wait_for = [&](uint64_t* bar, uint32_t parity, unsigned code) {
+    if (!mbar_try_wait(bar, parity) && !dead) dead = wait_slow(bar, parity, p.err, code, gave_up);
+  };
 
+  auto load_k = [&](int it, int s) {
+    mbar_arrive_expect_tx(&k_full[s], C::TB);
+#pragma unroll
+    for (int c = 0; c < NB; ++c) tma_load_3d(sK + s * C::TB + c * kTBN * 128, &tk, kvh * HD + c * 64, tile_of(it) * kTBN, b, &k_full[s]);
+  };
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tq);
     tma_prefetch_desc(&tk);
@@ -185,7 +233,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
     mbar_init(pv_done, 1);
     mbar_init(o_full, 1);
     *not_finite = 0;
+    *gave_up = 0;
     fence_mbar_init();
+    if (n_tiles > 0) {   // on their way while TMEM is allocated
+      load_k(0, 0);
+      mbar_arrive_expect_tx(q_full, C::QB);
+#pragma unroll
+      for (int c = 0; c < NB; ++c) tma_load_3d(sQ + c * kTBM * 128, &tq, h * HD + c * 64, q0, b, q_full);
+    }
   }
   if (warp == 2) tmem_alloc<1>(tmem_slot, kCols);
   tc_fence_before();
@@ -193,64 +248,67 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
+  float4 mine{};   // of a row: maximum, sum, V is not finite, gave up
   if (warp == 0) {
     // ------------------------------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      mbar_arrive_expect_tx(q_full, C::QB);
-#pragma unroll
-      for (int c = 0; c < NB; ++c) tma_load_3d(sQ + c * kTBM * 128, &tq, h * HD + c * 64, q0, b, q_full);
       int s = 0;
       uint32_t ph = 1;
       for (int it = 0; it < n_tiles; ++it) {
-        const int k0 = tile_of(it) * kTBN;
-        if (!(ok = mbar_wait_limited(&k_empty[s], ph, p.err, kAttnWaitCode | 1))) break;
-        mbar_arrive_expect_tx(&k_full[s], C::TB);
-#pragma unroll
-        for (int c = 0; c < NB; ++c) tma_load_3d(sK + s * C::TB + c * kTBN * 128, &tk, kvh * HD + c * 64, k0, b, &k_full[s]);
-        if (!(ok = mbar_wait_limited(&v_empty[s], ph, p.err, kAttnWaitCode | 2))) break;
+        if (it > 0) {
+          wait_for(&k_empty[s], ph, kAttnWaitCode | 1);
+          load_k(it, s);
+        }
+        wait_for(&v_empty[s], ph, kAttnWaitCode | 2);
         mbar_arrive_expect_tx(&v_full[s], C::TB);
 #pragma unroll
-        for (int c = 0; c < NB; ++c) tma_load_3d(sV + s * C::TB + c * kTBN * 128, &tv, kvh * HD + c * 64, k0, b, &v_full[s]);
+        for (int c = 0; c < NB; ++c) tma_load_3d(sV + s * C::TB + c * kTBN * 128, &tv, kvh * HD + c * 64, tile_of(it) * kTBN, b, &v_full[s]);
         if (++s == ST) {
           s = 0;
           ph ^= 1;
         }
       }
-      if (!ok) drain_async();
+      if (dead) drain_async();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      const uint32_t q_u = smem_u32(sQ), k_u = smem_u32(sK), v_u = smem_u32(sV);
-      auto scores = [&](int it) -> bool {   // S[it & 1] = Q·Kᵀ of tile it
-        const int s = it % ST;
-        if (!mbar_wait_limited(&k_full[s], (uint32_t)((it / ST) & 1), p.err, kAttnWaitCode | 3)) return false;
-        tc_fence_after();
+    // The whole warp walks the loop and one thread's predicate issues: descriptors then live in uniform registers.
+    const uint32_t one = lane == 0;
+    const uint32_t q_u = desc_lo(smem_u32(sQ)), k_u = desc_lo(smem_u32(sK)), v_u = desc_lo(smem_u32(sV));
+    auto scores = [&](int it) {   // S[it & 1] = Q·Kᵀ of tile it
+      const int s = it % ST;
+      wait_for(&k_full[s], (uint32_t)((it / ST) & 1), kAttnWaitCode | 3);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t ks = k_u + s * (C::TB >> 4), d = tmem + (uint32_t)((it & 1) * 64);
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk)
-          umma_bf16(tmem + (uint32_t)((it & 1) * 64), umma_desc(q_u + (kk / 4) * kTBM * 128 + (kk % 4) * 32),
-                    umma_desc(k_u + s * C::TB + (kk / 4) * kTBN * 128 + (kk % 4) * 32), kIdescS, kk > 0 ? 1u : 0u);
-        umma_commit(&k_empty[s]);
-        umma_commit(&s_full[it & 1]);
-        return true;
-      };
-      ok = mbar_wait_limited(q_full, 0, p.err, kAttnWaitCode | 4) && scores(0);
-      for (int it = 0; it < n_tiles && ok; ++it) {
-        // the buffer that tile it + 1 overwrites held P of tile it - 1: its product went out before, and products run in order
-        if (it + 1 < n_tiles && !(ok = scores(it + 1))) break;
-        const int s = it % ST;
-        if (!(ok = mbar_wait_limited(&p_full[it & 1], (uint32_t)((it >> 1) & 1), p.err, kAttnWaitCode | 5))) break;
-        if (!(ok = mbar_wait_limited(&v_full[s], (uint32_t)((it / ST) & 1), p.err, kAttnWaitCode | 6))) break;
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < kTBN / 16; ++kk)   // 16 keys: 8 columns of P, 2 048 bytes further down V's rows
-          umma_bf16_ts(tmem + kColO, tmem + (uint32_t)((it & 1) * 64 + kk * 8), umma_desc_mn(v_u + s * C::TB + kk * 2048, kTBN * 128), kIdescO,
-                       (it > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&v_empty[s]);
-        umma_commit(it + 1 < n_tiles ? pv_done : o_full);
-      }
-      if (!ok) drain_async();
+      for (int kk = 0; kk < HD / 16; ++kk)
+        umma_ss(d, q_u + (((kk / 4) * kTBM * 128 + (kk % 4) * 32) >> 4), ks + (((kk / 4) * kTBN * 128 + (kk % 4) * 32) >> 4), kDescHi, kDescHi,
+                kIdescS, kk > 0 ? 1u : 0u, one);
+      umma_commit_if(&k_empty[s], one);
+      umma_commit_if(&s_full[it & 1], one);
+    };
+    if (n_tiles > 0) {
+      wait_for(q_full, 0, kAttnWaitCode | 4);
+      scores(0);
     }
+    for (int it = 0; it < n_tiles; ++it) {
+      // the buffer that tile it + 1 overwrites held P of tile it - 1: its product went out before, and products run in order
+      if (it + 1 < n_tiles) scores(it + 1);
+      const int s = it % ST;
+      wait_for(&v_full[s], (uint32_t)((it / ST) & 1), kAttnWaitCode | 6);
+      wait_for(&p_full[it & 1], (uint32_t)((it >> 1) & 1), kAttnWaitCode | 5);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t vs = v_u + s * (C::TB >> 4), ps = tmem + (uint32_t)((it & 1) * 64);
+#pragma unroll
+      for (int kk = 0; kk < kTBN / 16; ++kk)   // 16 keys: 8 columns of P, 2 048 bytes further down V's rows
+        umma_ts(tmem + kColO, ps + kk * 8, vs + (kk * 2048 >> 4) + ((kTBN * 128 >> 4) << 16), kDescHi, kIdescO,
+                (it > 0 || kk > 0) ? 1u : 0u, one);
+      umma_commit_if(&v_empty[s], one);
+      umma_commit_if(it + 1 < n_tiles ? pv_done : o_full, one);
+    }
+    if (dead) drain_async();
   } else {
     // ---------------------------------------------------------------------------------------------- softmax
     const int q = warp & 3, row = q * 32 + lane;
@@ -260,25 +318,27 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
     const uint64_t scale2 = pack_f2(k_scale, k_scale);
     float m = -INFINITY, l = 0.f;
     for (int it = 0; it < n_tiles; ++it) {
-      ok = __all_sync(0xffffffffu, mbar_wait_limited(&s_full[it & 1], (uint32_t)((it >> 1) & 1), p.err, kAttnWaitCode | 7));
-      if (!ok) break;
+      wait_for(&s_full[it & 1], (uint32_t)((it >> 1) & 1), kAttnWaitCode | 7);
+      __syncwarp();
       tc_fence_after();
-      uint32_t s0[32], s1[32];
+      uint32_t s[2][32];
       const uint32_t sbuf = lane_base + (uint32_t)((it & 1) * 64);
-      tmem_ld32(sbuf, s0);
-      tmem_ld32(sbuf + 32, s1);
+      tmem_ld32(sbuf, s[0]);
+      tmem_ld32(sbuf + 32, s[1]);
       tmem_wait_ld();
       const int kbase = tile_of(it) * kTBN;
       if (kbase + kTBN - 1 > first_pos || (p.window > 0 && last_pos - kbase >= p.window)) {
+        // the keys this row sees, a bit each (comparing them one by one took 4 000 to 7 000 cycles a tile, more than three whole tiles)
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int j0 = kbase + j, j1 = kbase + 32 + j;
-          if (j0 > rpos || (p.window > 0 && rpos - j0 >= p.window && j0 >= p.keep_first)) s0[j] = 0xff800000u;
-          if (j1 > rpos || (p.window > 0 && rpos - j1 >= p.window && j1 >= p.keep_first)) s1[j] = 0xff800000u;
+        for (int i = 0; i < 2; ++i) {
+          const int k0 = kbase + i * 32;
+          const uint32_t seen = bits_below(rpos + 1 - k0) &
+                                (p.window > 0 ? ~bits_below(rpos + 1 - p.window - k0) | bits_below(p.keep_first - k0) : ~0u);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) s[i][j] = seen & (1u << j) ? s[i][j] : 0xff800000u;
         }
         const int vs = it % ST;
-        ok = __all_sync(0xffffffffu, mbar_wait_limited(&v_full[vs], (uint32_t)((it / ST) & 1), p.err, kAttnWaitCode | 10));
-        if (!ok) break;
+        wait_for(&v_full[vs], (uint32_t)((it / ST) & 1), kAttnWaitCode | 10);
         const uint4* vt = reinterpret_cast<const uint4*>(sV + vs * C::TB);
         bool bad = false;
 #pragma unroll
@@ -286,15 +346,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
           const uint4 w = vt[j * 128 + row];
           const uint32_t x[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) bad = bad || (x[e] & 0x7f80u) == 0x7f80u || (x[e] & 0x7f800000u) == 0x7f800000u;
+          for (int e = 0; e < 4; ++e) bad |= (x[e] & 0x7f80u) == 0x7f80u | (x[e] & 0x7f800000u) == 0x7f800000u;
         }
         if (bad) *not_finite = 1;
+        __syncwarp();
       }
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int j = 0; j < 32; j += 4) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(s0[j + e]), __uint_as_float(s1[j + e])));
+        for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(s[0][j + e]), __uint_as_float(s[1][j + e])));
       }
       const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       const bool grow = top > m;
@@ -308,8 +369,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
       uint32_t pk[32];
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const uint64_t za = fma_f2(pack_f2(__uint_as_float(s0[2 * j]), __uint_as_float(s0[2 * j + 1])), scale2, neg);
-        const uint64_t zb = fma_f2(pack_f2(__uint_as_float(s1[2 * j]), __uint_as_float(s1[2 * j + 1])), scale2, neg);
+        const uint64_t za = fma_f2(pack_f2(__uint_as_float(s[0][2 * j]), __uint_as_float(s[0][2 * j + 1])), scale2, neg);
+        const uint64_t zb = fma_f2(pack_f2(__uint_as_float(s[1][2 * j]), __uint_as_float(s[1][2 * j + 1])), scale2, neg);
         const float a0 = ex2f(lo_f2(za)), a1 = ex2f(hi_f2(za)), b0 = ex2f(lo_f2(zb)), b1 = ex2f(hi_f2(zb));
         sum[0] = add_f2(sum[0], pack_f2(a0, a1));
         sum[1] = add_f2(sum[1], pack_f2(b0, b1));
@@ -320,22 +381,26 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
       l += lo_f2(sum[0]) + hi_f2(sum[0]);
       tmem_st32(sbuf, pk);
       if (rescale) {
-        ok = __all_sync(0xffffffffu, mbar_wait_limited(pv_done, (uint32_t)((it - 1) & 1), p.err, kAttnWaitCode | 8));
-        if (!ok) break;
+        wait_for(pv_done, (uint32_t)((it - 1) & 1), kAttnWaitCode | 8);
+        __syncwarp();
         tc_fence_after();
+        const uint64_t alpha2 = pack_f2(alpha, alpha);
 #pragma unroll 1
         for (int c = 0; c < HD; c += 64) {
-          uint32_t o0[32], o1[32];
-          tmem_ld32(lane_base + kColO + c, o0);
-          tmem_ld32(lane_base + kColO + c + 32, o1);
+          uint32_t o[2][32];
+          tmem_ld32(lane_base + kColO + c, o[0]);
+          tmem_ld32(lane_base + kColO + c + 32, o[1]);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            o0[j] = __float_as_uint(__uint_as_float(o0[j]) * alpha);
-            o1[j] = __float_as_uint(__uint_as_float(o1[j]) * alpha);
-          }
-          tmem_st32(lane_base + kColO + c, o0);
-          tmem_st32(lane_base + kColO + c + 32, o1);
+          for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              const uint64_t y = mul_f2(pack_f2(__uint_as_float(o[i][j]), __uint_as_float(o[i][j + 1])), alpha2);
+              o[i][j] = (uint32_t)y;
+              o[i][j + 1] = (uint32_t)(y >> 32);
+            }
+          tmem_st32(lane_base + kColO + c, o[0]);
+          tmem_st32(lane_base + kColO + c + 32, o[1]);
         }
       }
       tmem_wait_st();
@@ -343,16 +408,56 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[it & 1]);
     }
-    // ---- normalise and store.  The end has a barrier of its own: a parity tells a phase from its neighbours only, and here the products
-    // of the last two tiles may both be running (inside the loop S of tile it says that the product of tile it - 2 is over).
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_limited(o_full, 0, p.err, kAttnWaitCode | 9));
-    named_bar_sync(1, 128);
-    const bool alone = *not_finite != 0;   // the same for all softmax threads
-    if (ok) {
-      tc_fence_after();
+    // ---- the end has a barrier of its own: a parity tells a phase from its neighbours only, and here the products of the last two tiles may
+    // both be running (inside the loop S of tile it says that the product of tile it - 2 is over).
+    if (n_tiles > 0) wait_for(o_full, 0, kAttnWaitCode | 9);
+    __syncwarp();
+    tc_fence_after();
+    named_bar_sync(1, 128);   // every load and product of this CTA is over
+    mine = make_float4(m, l, *not_finite != 0 ? 1.f : 0.f, dead || *gave_up != 0 ? 1.f : 0.f);
+    if constexpr (SPLIT == 2) {   // the other CTA's columns, the maxima and the sums go where Q and K were
+      part[row] = mine;
+      if (n_tiles > 0) {
+#pragma unroll 1
+        for (int c = 0; c < HD / 2; c += 32) {
+          uint32_t o[32];
+          tmem_ld32(lane_base + kColO + (half ^ 1) * (HD / 2) + c, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            give[(c / 4 + j) * kTBM + row] = make_float4(__uint_as_float(o[4 * j]), __uint_as_float(o[4 * j + 1]), __uint_as_float(o[4 * j + 2]),
+                                                         __uint_as_float(o[4 * j + 3]));
+        }
+      }
+    }
+  }
+  __syncwarp();
+  if constexpr (SPLIT == 2) cluster_sync_all();   // both halves have written
+  if (warp >= 2) {
+    // ---- merge, normalise and store this CTA's columns
+    constexpr int W = HD / SPLIT, CH = W / 8;   // columns; 16-byte pieces of a row of results
+    const int q = warp & 3, row = q * 32 + lane;
+    const int r = q0 + min(row, rows_valid - 1);
+    const uint32_t o_at = tmem + ((uint32_t)(q * 32) << 16) + kColO + half * W;
+    const float k_scale = p.scale_log2;
+    float4 other = make_float4(-INFINITY, 0.f, 0.f, 0.f), y[SPLIT == 2 ? W / 4 : 1];
+    if constexpr (SPLIT == 2) {
+      const uint32_t take = mapa_u32(smem_u32(&give[row]), (uint32_t)(half ^ 1));
+      other = ld_cluster_f4(mapa_u32(smem_u32(&part[row]), (uint32_t)(half ^ 1)));
+#pragma unroll
+      for (int j = 0; j < W / 4; ++j) y[j] = ld_cluster_f4(take + j * kTBM * 16);
+      cluster_arrive();   // the other half may leave; its wait lies behind the store
+    }
+    const bool alone = __any_sync(0xffffffffu, mine.z + other.z != 0.f);
+    float m = fmaxf(mine.x, other.x);
+    // a half whose tiles the row does not see has no maximum and a sum of 0, or of NaN where its scores were
+    const float fm = SPLIT == 1 ? 1.f : mine.x == -INFINITY ? mine.y : ex2f((mine.x - m) * k_scale);
+    const float fo = SPLIT == 1 ? 0.f : other.x == -INFINITY ? other.y : ex2f((other.x - m) * k_scale);
+    float l = SPLIT == 1 ? mine.y : mine.y * fm + other.y * fo;
+    if (__all_sync(0xffffffffu, mine.w + other.w == 0.f)) {
       if (alone) {
         float ml[2] = {-INFINITY, 0.f}, none[32];
-        see_alone<HD>(p, b, h, kvh, q0 + min(row, rows_valid - 1), ml, -1, none);
+        see_alone<HD>(p, b, h, kvh, r, ml, -1, none);
         m = ml[0];
         l = ml[1];
       }
@@ -360,49 +465,68 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
       float inv = l > 0.f ? 1.f / l : 0.f;
       if (p.gate != nullptr && row < rows_valid)
         inv *= 1.f / (1.f + expf(-bf16_to_f(p.gate[(size_t)b * p.q_bs + (size_t)(q0 + row) * p.q_rs + h])));
-      __nv_bfloat16* dst = p.o + (size_t)b * p.o_bs + (size_t)(q0 + min(row, rows_valid - 1)) * p.o_rs + (size_t)h * HD;
-#pragma unroll 1
-      for (int c = 0; c < HD; c += 32) {
+      // through shared memory (where V was), so that a store covers whole rows: straight from the lanes it touches 32 of them
+      uint8_t* const mid = sV + q * (32 * W * 2);
+      auto place = [&](int rw, int c) { return mid + rw * (W * 2) + (c ^ ((CH >= 8 ? rw : rw >> 1) & (CH >= 8 ? 7 : 3))) * 16; };
+      const uint32_t km = fm != 0.f ? ~0u : 0u, ko = fo != 0.f ? ~0u : 0u;   // what a half of weight 0 holds is not looked at
+      const float wm = fm * inv, wo = fo * inv;
+      auto mix = [&](uint32_t a, float b) {
+        if constexpr (SPLIT == 1) return __uint_as_float(a) * inv;
+        return __uint_as_float(a & km) * wm + __uint_as_float(__float_as_uint(b) & ko) * wo;
+      };
+#pragma unroll
+      for (int c = 0; c < W; c += 32) {
         uint32_t o[32];
-        tmem_ld32(lane_base + kColO + c, o);
+        tmem_ld32(o_at + c, o);
         tmem_wait_ld();
-        if (alone) {
-          float ml[2] = {m, l}, acc[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) acc[j] = 0.f;
-          see_alone<HD>(p, b, h, kvh, q0 + min(row, rows_valid - 1), ml, c, acc);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(acc[j]);
-        }
-        if (row < rows_valid) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint4 v;
-            v.x = pack2(__uint_as_float(o[8 * j]) * inv, __uint_as_float(o[8 * j + 1]) * inv);
-            v.y = pack2(__uint_as_float(o[8 * j + 2]) * inv, __uint_as_float(o[8 * j + 3]) * inv);
-            v.z = pack2(__uint_as_float(o[8 * j + 4]) * inv, __uint_as_float(o[8 * j + 5]) * inv);
-            v.w = pack2(__uint_as_float(o[8 * j + 6]) * inv, __uint_as_float(o[8 * j + 7]) * inv);
-            *reinterpret_cast<uint4*>(dst + c + 8 * j) = v;
-          }
+        for (int j = 0; j < 4; ++j) {
+          const float4 ya = y[SPLIT == 2 ? c / 4 + 2 * j : 0], yb = y[SPLIT == 2 ? c / 4 + 2 * j + 1 : 0];
+          uint4 v;
+          v.x = pack2(mix(o[8 * j], ya.x), mix(o[8 * j + 1], ya.y));
+          v.y = pack2(mix(o[8 * j + 2], ya.z), mix(o[8 * j + 3], ya.w));
+          v.z = pack2(mix(o[8 * j + 4], yb.x), mix(o[8 * j + 5], yb.y));
+          v.w = pack2(mix(o[8 * j + 6], yb.z), mix(o[8 * j + 7], yb.w));
+          *reinterpret_cast<uint4*>(place(lane, c / 8 + j)) = v;
         }
       }
+      if (alone) {
+#pragma unroll 1
+        for (int c = 0; c < W; c += 32) {
+          float ml[2] = {m, l}, x[32];
+          for (int e = 0; e < 32; ++e) x[e] = 0.f;
+          see_alone<HD>(p, b, h, kvh, r, ml, half * W + c, x);
+          for (int e = 0; e < 32; ++e) reinterpret_cast<__nv_bfloat16*>(place(lane, (c + e) / 8))[e & 7] = f_to_bf16(x[e] * inv);
+        }
+      }
+      __syncwarp();
+      __nv_bfloat16* const dst = p.o + (size_t)b * p.o_bs + (size_t)h * HD + half * W + (lane % CH) * 8;
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const int rw = i * (32 / CH) + lane / CH;
+        if (q * 32 + rw < rows_valid)
+          *reinterpret_cast<uint4*>(dst + (size_t)(q0 + q * 32 + rw) * p.o_rs) = *reinterpret_cast<const uint4*>(place(rw, lane % CH));
+      }
     }
+    tc_fence_before();
+    __syncwarp();
+  } else if constexpr (SPLIT == 2) {
+    cluster_arrive();
   }
-  tc_fence_before();
-  __syncwarp();
-  __syncthreads();
+  if constexpr (SPLIT == 2) cluster_wait();   // neither half leaves while the other still reads
+  __syncthreads();                            // nor frees its TMEM before its own warps have read
   if (warp == 2) {
     tc_fence_after();
     tmem_free<1>(tmem, kCols);
   }
 }
 
-template <int HD>
+template <int HD, int SPLIT>
 int launch_tc(const TcPrefillAttn& a, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(attn_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::smem);
+    attr_err = cudaFuncSetAttribute(attn_tc_kernel<HD, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::smem);
   });
   B200_CUDA(attr_err);
   TcAttn p{};
@@ -417,10 +541,19 @@ int launch_tc(const TcPrefillAttn& a, cudaStream_t st) {
   if ((rc = make_tmap_sw128(&tq, 3, a.q, a.B, a.S, (int64_t)a.Hq * HD, a.q_bs, a.q_rs, kTBM)) != B200_OK) return rc;
   if ((rc = make_tmap_sw128(&tk, 3, a.k, a.B, keys, (int64_t)a.Hkv * HD, a.kv_bs, a.kv_rs, kTBN)) != B200_OK) return rc;
   if ((rc = make_tmap_sw128(&tv, 3, a.v, a.B, keys, (int64_t)a.Hkv * HD, a.kv_bs, a.kv_rs, kTBN)) != B200_OK) return rc;
-  const dim3 grid((unsigned)a.Hq, (unsigned)((a.S + kTBM - 1) / kTBM), (unsigned)a.B);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)a.Hq * SPLIT, (unsigned)((a.S + kTBM - 1) / kTBM), (unsigned)a.B);
+  cfg.blockDim = dim3(kTThreads);
+  cfg.dynamicSmemBytes = TcCfg<HD>::smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = SPLIT == 2 ? 1 : 0;
   g_launches.fetch_add(1);
-  attn_tc_kernel<HD><<<grid, kTThreads, TcCfg<HD>::smem, st>>>(tq, tk, tv, p);
-  B200_CUDA(cudaGetLastError());
+  B200_CUDA(cudaLaunchKernelEx(&cfg, attn_tc_kernel<HD, SPLIT>, tq, tk, tv, p));
   return B200_OK;
 }
 
@@ -430,23 +563,26 @@ bool prefill_attn_tc_ok(const TcPrefillAttn& a, int hd) {
   return (hd == 64 || hd == 128) && (a.S + kTBM - 1) / kTBM < 65536 && a.B < 65536 && aligned16(a.o, a.q, a.k, a.v) && a.q_rs % 8 == 0 &&
          a.q_bs % 8 == 0 && a.kv_rs % 8 == 0 && a.kv_bs % 8 == 0 && a.o_rs % 8 == 0 && a.o_bs % 8 == 0;
 }
-// Whether this kernel beats the mma.sync one, by fits (µs) to both over 128 … 2 048 rows, 14 … 64 (head, sequence) pairs: this one takes a launch
-// and pipeline fill of 9.6 and the longest block's tiles one after another; that one the larger of its longest block's tiles and all
-// of its 64 × 64 tiles on the tensor cores, and a third of the smaller.
+// Whether this kernel beats the mma.sync one: where the longest block walks enough tiles of 64 keys.  µs here / there: one to four sequences, 16 … 32 heads
+// of 128, 128 rows (two tiles) 7.7 / 6.9 … 7.9 / 9.3, 200 rows (four) 8.7 / 10.4 … 11.9 / 20.5; 14 heads of 64, 256 rows (four)
+// 6.9 / 6.9 and 7.8 / 8.2, 333 rows (six) 7.5 / 8.8 and 9.9 / 12.8.
 bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd, int rows) {
-  double all = 0, longest = 0;
-  for (int r = 0; r < rows; r += 64) {
-    const int last = std::min(rows, r + 64) - 1, edge = a.window > 0 ? std::max(0, r - a.window + 1) / 64 : 0;
-    const double tiles = last / 64 + 1 - edge + (a.window > 0 ? std::min(edge, (a.keep_first + 63) / 64) : 0);
-    all += tiles;
-    longest = std::max(longest, tiles);
-  }
-  all *= (double)a.B * a.Hq;
-  const double chain = (hd == 64 ? 1.0 : 1.75) * longest, work = (hd == 64 ? 0.0066 : 0.0133) * all;
-  const double mma = 3.3 + std::max(chain, work) + 0.3 * std::min(chain, work);
-  const double here = std::max(9.6 + (hd == 64 ? 0.98 : 1.1) * longest, 5.0 + 0.0038 * all);
-  return here < mma;
+  const int last = (rows - 1) / 64 * 64;   // first row of the last block
+  const int edge = a.window > 0 ? std::max(0, last - a.window + 1) / 64 : 0;
+  const int tiles = last / 64 + 1 - edge + (a.window > 0 ? std::min(edge, (a.keep_first + 63) / 64) : 0);
+  return tiles >= (hd == 64 ? 5 : 4);
 }
-int launch_prefill_attn_tc(const TcPrefillAttn& a, int hd, cudaStream_t st) { return hd == 64 ? launch_tc<64>(a, st) : launch_tc<128>(a, st); }
+// Two CTAs per 128 rows of a head while all of them still run at once (two to an SM): the longest chain of tiles is half as long.  Beyond that the
+// second CTA's start and end cost more than the chain.  µs, one / two: 16 heads of 128 512 rows 12.9 / 10.6, 1 024 rows (128 blocks)
+// 20.5 / 15.7, 1 536 rows (192) 27.2 / 27.0, 2 048 rows 34.6 / 35.5; 32 heads 512 rows (128) 13.4 / 12.7, 768 rows (192) 17.7 / 22.0; a single
+// tile or two of them per block 5.7 / 7.4.
+static bool attn_tc_halves(const TcPrefillAttn& a, int rows) {
+  return rows > kTBM && (int64_t)a.B * a.Hq * ((rows + kTBM - 1) / kTBM) <= 148;
+}
+int launch_prefill_attn_tc(const TcPrefillAttn& a, int hd, int rows, cudaStream_t st) {
+  const bool two = attn_tc_halves(a, rows);
+  if (hd == 64) return two ? launch_tc<64, 2>(a, st) : launch_tc<64, 1>(a, st);
+  return two ? launch_tc<128, 2>(a, st) : launch_tc<128, 1>(a, st);
+}
 
 }  // namespace b200
