@@ -127,8 +127,13 @@ __device__ __forceinline__ void cap_scores(float (&s)[8][4], float scale, float 
   }
 }
 
+// Bound by the rate of mma.sync: a tensor core takes one m16n8k16 in 16 cycles (512 multiply-adds per cycle and SM, an eighth of tcgen05's), 61 of
+// the 64 µs of 16 heads of 128 over 2 048 rows; short prompts by the longest block's chain of tiles.  The launch bound asks for one CTA: two fit
+// all the same (239 registers), and the schedule with 177, which the compiler chooses by itself, takes 80 µs (512 rows 18.9 → 14.2, 14 heads of 64
+// over 1 024 rows 21.8 → 19.9).  Heads of 64 keep to the 168 registers with which three fit.  Two row tiles per warp, which halve the reads of
+// keys and values, were slower: 107 µs, and no faster with 32 heads (129 against 123).
 template <int HD, bool SCORE>
-__global__ void __launch_bounds__(kPfThreads) attn_prefill_mma_kernel(const PrefillAttnParams p) {
+__global__ void __launch_bounds__(kPfThreads, HD == 64 ? 3 : 1) attn_prefill_mma_kernel(const PrefillAttnParams p) {
   constexpr int CH = HD / 8;    // 16-byte chunks per row
   constexpr int TB = kBN * row_bytes<HD>();   // bytes of a key / value tile
   constexpr int KS = HD / 16;   // k-steps of Q·Kᵀ
