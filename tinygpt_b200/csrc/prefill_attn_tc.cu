@@ -24,9 +24,9 @@
 // (P then shares the only S buffer) and eight softmax warps of 64 keys were no faster: 43 and 40 µs where this form took 38.
 // Masks as bits (they were two comparisons per key: 4 000 to 7 000 cycles a tile), results stored in whole rows through shared memory
 // (straight from the lanes a store touches 32 rows), the first loads in front of the TMEM allocation, waits whose first look is inline.
-// µs, mma.sync / here at first / now, same error against 64 bits: 16 heads of 128 over 2 048 rows 80 / 51 / 34.6, 24 heads
-// 122 / 53 / 41.4, 32 heads 152 / 71 / 52.5; 16 heads over 512 rows 18.9 / 18.2 / 10.6; 14 heads of 64 over 2 048 rows 50 / 41 / 29.2,
-// four sequences of 333 rows 12.8 / - / 9.9.
+// µs, mma.sync / here at first / now, same error against 64 bits: 16 heads of 128 over 2 048 rows 64 / 51 / 34.6, 24 heads
+// 98 / 53 / 41.4, 32 heads 123 / 71 / 52.5; 16 heads over 512 rows 14.2 / 18.2 / 10.6; 14 heads of 64 over 2 048 rows 48 / 41 / 29.2,
+// four sequences of 333 rows 12.1 / - / 9.9.
 #include "ops.cuh"
 #include "tc.cuh"
 
@@ -563,14 +563,16 @@ bool prefill_attn_tc_ok(const TcPrefillAttn& a, int hd) {
   return (hd == 64 || hd == 128) && (a.S + kTBM - 1) / kTBM < 65536 && a.B < 65536 && aligned16(a.o, a.q, a.k, a.v) && a.q_rs % 8 == 0 &&
          a.q_bs % 8 == 0 && a.kv_rs % 8 == 0 && a.kv_bs % 8 == 0 && a.o_rs % 8 == 0 && a.o_bs % 8 == 0;
 }
-// Whether this kernel beats the mma.sync one: where the longest block walks enough tiles of 64 keys.  µs here / there: one to four sequences, 16 … 32 heads
-// of 128, 128 rows (two tiles) 7.7 / 6.9 … 7.9 / 9.3, 200 rows (four) 8.7 / 10.4 … 11.9 / 20.5; 14 heads of 64, 256 rows (four)
-// 6.9 / 6.9 and 7.8 / 8.2, 333 rows (six) 7.5 / 8.8 and 9.9 / 12.8.
+// Whether this kernel beats the mma.sync one: where the longest block walks enough tiles of 64 keys, or a few of them in more blocks than that one
+// runs at once.  µs here / there: 16 heads of 128, one sequence 192 rows (three tiles) 8.5 / 7.3, 256 rows 8.5 / 8.6, 320 rows (five)
+// 9.3 / 10.0, two sequences 11.9 / 11.2, four 12.9 / 14.2; four sequences of 32 heads 128 rows (256 blocks of 64) 8.1 / 8.2, 160 rows
+// (384) 10.0 / 12.1, of 24 heads 160 rows (288) 9.9 / 9.8, 256 rows (384) 12.3 / 15.5; 14 heads of 64, one, two and four sequences: 320 rows (five)
+// 7.4 / 7.1, 8.9 / 7.3, 9.8 / 9.5, 333 rows (six) 7.4 / 7.8, 8.9 / 9.0, 10.1 / 12.1.
 bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd, int rows) {
   const int last = (rows - 1) / 64 * 64;   // first row of the last block
   const int edge = a.window > 0 ? std::max(0, last - a.window + 1) / 64 : 0;
   const int tiles = last / 64 + 1 - edge + (a.window > 0 ? std::min(edge, (a.keep_first + 63) / 64) : 0);
-  return tiles >= (hd == 64 ? 5 : 4);
+  return tiles >= (hd == 64 ? 6 : 5) || (hd == 128 && tiles >= 3 && (int64_t)a.B * a.Hq * (last / 64 + 1) > 296);
 }
 // Two CTAs per 128 rows of a head while all of them still run at once (two to an SM): the longest chain of tiles is half as long.  Beyond that the
 // second CTA's start and end cost more than the chain.  µs, one / two: 16 heads of 128 512 rows 12.9 / 10.6, 1 024 rows (128 blocks)
