@@ -296,67 +296,102 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_reg_kernel(const Att
 // ------------------------------------------------------------------------------- one query row over many keys
 // One new row against every key, probabilities in fp32, as (a) o = softmax(q·kᵀ)·v for Sq = 1 through the operator boundary and (b) the fused decode
 // attention over long contexts (q/k norm, rotation and the in-place append as in attn_decode_reg_kernel).
-// A cluster shares a (sequence, group of G query heads of one KV head): its CTAs take neighbouring ranges of the keys that exist now, every
-// thread holds 16-byte pieces of U keys' K and V rows while the next U are on their way, and runs an online softmax over its own
-// keys; the key groups of a warp merge by shuffles, the warps through shared memory and the CTAs through distributed shared
-// memory — no workspace, no tickets, one launch.  Bound by the latency of a few rounds of loads.
-// (a) 16 / 8 heads of 128 over 2 049 keys: 94 µs with one CTA per head walking 128 keys at a time, 8.1 µs like this (8.4 MB); 4 × 32 heads over
-// 4 096 keys 469 → 48 µs.  (b) 24 / 8 heads at position 4 000 of 4 096: 27.7 µs with one CTA per 128 keys and a merge by the last of 32,
-// 13.3 µs like this.
+// A cluster shares a (sequence, group of up to eight query heads of one KV head): its CTAs take neighbouring ranges of the keys, so that a key
+// and a value are read once for all of the group's heads.  A CTA walks its range in units of 128 keys, sixteen a warp; the K and V rows come
+// through a ring in shared memory (cp.async, 96 KB, all of it asked for at once and, for cached rows, before the kernel in front has ended).
+// Inside its sixteen keys a warp works alone, without a barrier:
+//   scores  K·qᵀ on mma.sync, the heads as its eight columns: exact products of bf16, summed in fp32
+//   softmax online, from the score fragments
+//   P·V     fp32 multiply-adds, a lane four columns, the probabilities broadcast from shared memory
+// The warps merge through shared memory, and every CTA sends each of the others its share of the result through distributed shared memory:
+// one cluster barrier, no workspace, no tickets, one launch.  Bound by launch, one round trip of loads and the merge.
+//
+// Against eight CTAs per one or two heads, which read K and V once per head in eight dependent rounds of register loads: device µs, rotating caches of 4 096
+// tokens, positions 100 / 1 000 / 2 000 / 4 000: 16 / 8 heads of 128 5.1 / 6.6 / 8.7 / 12.2 → 5.4 / 5.8 / 6.7 / 9.9, 24 / 8 heads 5.3 / 6.8 / 9.2 / 13.0 →
+// 5.8 / 6.0 / 7.3 / 10.9, 14 / 2 heads of 64 4.6 / 5.3 / 5.9 / 7.2 → 5.2 / 5.2 / 5.6 / 6.9.  Where it counts, inside a token, the loads run beside the
+// kernel in front: 28 layers, 2 048 wide, ctx 4 096 802 / 866 / 919 / 1 014 → 787 / 811 / 838 / 909 µs a token, 24 layers, 896 wide 440 / 449 / 461 / 501 →
+// 427 / 431 / 436 / 460.  Eight CTAs at most instead of sixteen: 0.3 µs less at short positions, 0.7 … 2 more at long ones, and tokens behind
+// in both (4 000: 1 021).  Barriers over the whole CTA in every unit: 6.9 µs at position 100.
 struct AttnRow {
   AttnDecodeParams d;               // decode: everything; row: qkv = q [B, Hq, HD], out, kcache / vcache and the strides
   int nkeys;                        // row: keys to see (decode reads the position)
   long long kv_bstride;             // elements from one batch element's keys to the next
+  int G, per_kv;                    // query heads of a CTA; CTAs (clusters) per KV head
+  int log_splits;
 };
-// a load that stays where it is written: the rows of a round are requested before the first of them is used
-__device__ __forceinline__ uint4 load_ahead(const __nv_bfloat16* p) {
-  uint4 v;
-  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
+constexpr int kUnit = 128, kMaxSplits = 16;
+template <int HD>
+struct KeyRing {
+  static constexpr int RB = HD * 2, SLOT = kUnit * RB, NS = HD == 128 ? 3 : 6;   // bytes of a row and of a unit's K or V; slots
+  static constexpr int smem = NS * SLOT;
+};
+template <bool DECODE>
+__device__ __forceinline__ void row_stamp(const AttnDecodeParams& p, int i) {   // nothing that has to stay in a register
+  if (DECODE && p.trace != nullptr && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) p.trace[i] = global_timer_ns();
 }
-template <int HD, int G, bool DECODE>
-__global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(const AttnRow a) {
-  constexpr int LPK = HD / 8;             // lanes per key row
-  constexpr int NG = kAttnThreads / LPK;  // key rows per pass
-  constexpr int U = 4;                    // passes per round
-  constexpr int EPL = HD / 32;
+template <int HD, int GM, bool DECODE>
+__global__ void __launch_bounds__(kAttnThreads, 2) attn_row_kernel(const AttnRow a) {
+  using R = KeyRing<HD>;
+  constexpr int LQ = HD / 4;   // column quads
+  constexpr int EPL = HD / 32, QP = HD + 8;
   constexpr float kScale = InvSqrtHd<HD>::value * kLog2e;
-  __shared__ float q_s[G][HD];
+  static_assert(kAttnWarps * GM * HD * 4 <= R::smem, "the warps' sums fit where the keys were");
+  extern __shared__ __align__(128) uint8_t ring[];
+  __shared__ __align__(16) __nv_bfloat16 q_s[8][QP];
   __shared__ __align__(16) __nv_bfloat16 knew[HD];
   __shared__ __align__(16) __nv_bfloat16 vnew[HD];
-  __shared__ __align__(16) float w_acc[kAttnWarps][HD];
-  __shared__ float w_ml[kAttnWarps][2];
-  __shared__ __align__(16) float res[G][HD];
-  __shared__ __align__(16) float res_ml[G][4];
-  __shared__ float weight[G][8], total[G];   // of the cluster's CTAs; the sum of all
+  __shared__ __align__(16) float ps[kUnit][GM];
+  __shared__ __align__(16) float2 w_ml[kAttnWarps][8];
+  __shared__ __align__(16) float4 part[GM * LQ + kMaxSplits];   // [CTA][its share of this CTA's columns]
+  __shared__ __align__(16) float2 part_ml[kMaxSplits][GM];
   const AttnDecodeParams& p = a.d;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, part = tid % LPK, grp = tid / LPK;
-  const int h0 = blockIdx.y * G, kvh = h0 / (p.Hq / p.Hkv);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3, G = a.G;
+  const int h0 = blockIdx.y * G, kvh = a.per_kv == 1 ? blockIdx.y : blockIdx.y / a.per_kv;
   const long long b = blockIdx.z;
-  const int rank = (int)cluster_rank(), splits = (int)gridDim.x;
-  auto stamp = [&](int i) {                // nothing that has to stay in a register
-    if (DECODE && p.trace != nullptr && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) p.trace[i] = global_timer_ns();
-  };
-  stamp(0);
+  const int rank = (int)cluster_rank(), splits = 1 << a.log_splits;
+  row_stamp<DECODE>(p, 0);
   if (DECODE) pdl_trigger();
+  cluster_arrive_relaxed();                // this CTA runs: the others may write to it once they have waited for that
   const bool append = DECODE && p.pos != nullptr;
   const int pos = append ? *p.pos : p.fixed_len - 1;   // where q is rotated; stable since before the producer kernel started
-  const int nkeys = append ? pos : DECODE ? p.fixed_len : a.nkeys;   // rows that are in the cache already
-  const int per = ((nkeys + splits - 1) / splits + NG - 1) / NG * NG;
-  const int k0 = min(nkeys, rank * per), k1 = min(nkeys, k0 + per);
-  const size_t base = (size_t)(b * a.kv_bstride) + (size_t)kvh * HD + part * 8, ks = (size_t)p.Hkv * HD;
-  uint4 kr[2][U], vr[2][U];
-  auto fetch = [&](int buf, int c) {
+  const int cached = append ? pos : DECODE ? p.fixed_len : a.nkeys;   // rows that are in the cache already
+  const int nkeys = cached + (append ? 1 : 0);
+  const int per = (((nkeys + splits - 1) >> a.log_splits) + 15) & ~15;
+  const int k0 = min(nkeys, rank * per), n = min(nkeys, k0 + per) - k0, n_cached = min(cached, k0 + n) - k0;   // this CTA's keys
+  const int units = (n - warp * 16 + kUnit - 1) / kUnit;   // with a key for this warp
+  constexpr int PC = HD / 8, RP = 32 / PC;   // 16-byte pieces of a row; rows that a warp copies at once
+  constexpr uint32_t WB = 16 * R::RB;        // a warp's part of a slot
+  const int c0 = lane % PC, r0 = lane / PC;
+  const int64_t ks = (int64_t)p.Hkv * HD, first = (int64_t)b * a.kv_bstride + kvh * HD + (k0 + warp * 16 + r0) * ks + c0 * 8;
+  const __nv_bfloat16 *k_src = p.kcache + first, *v_src = p.vcache + first;
+  const uint32_t ring_u = smem_u32(ring) + warp * WB;
+  // place of 16-byte piece c of row r: pieces of eight rows change places, so that both ways of reading spread over the banks
+  auto piece_at = [&](int r, int c) { return (uint32_t)(r * R::RB + ((c ^ (r & 7)) << 4)); };
+  auto load = [&](int s) {   // K (even) or V (odd) of this warp's keys of unit s / 2, zeros behind the last; always one commit group
+    const int rows = n_cached - (s >> 1) * kUnit - warp * 16 - r0;
+    if (rows + r0 > 0) {
+      const __nv_bfloat16* src = ((s & 1) ? v_src : k_src) + (int64_t)(s >> 1) * kUnit * ks;
+      const uint32_t dst = ring_u + (uint32_t)(s % R::NS) * R::SLOT;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const size_t j = (size_t)min(c + u * NG + grp, k1 - 1);   // past the range: its last key once more, without weight
-      kr[buf][u] = load_ahead(p.kcache + base + j * ks);
-      vr[buf][u] = load_ahead(p.vcache + base + j * ks);
+      for (int r = 0; r < 16; r += RP)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                     ::"r"(dst + piece_at(r + r0, c0)), "l"(r < rows ? src + r * ks : p.kcache), "r"(r < rows ? 16 : 0) : "memory");
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  if (k0 < k1) fetch(0, k0);               // rows of earlier tokens: nothing that the producer kernel writes
-  const __nv_bfloat16* qkv = p.qkv + b * p.qkv_bstride;
-  const bool owns_new = append && rank == splits - 1;
+  float q_in[DECODE ? 1 : GM * HD / kAttnThreads + 1];
+  if constexpr (!DECODE) {
+#pragma unroll
+    for (int i = 0; i < GM * HD / kAttnThreads + 1; ++i) {
+      const int e = i * kAttnThreads + tid;
+      q_in[i] = e < G * HD ? bf16_to_f(p.qkv[b * p.qkv_bstride + h0 * HD + e]) : 0.f;
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < R::NS; ++s) load(s);   // rows of earlier tokens: nothing that the producer kernel writes
+  [[maybe_unused]] const __nv_bfloat16* qkv = p.qkv + b * p.qkv_bstride;
+  const bool owns_new = append && n > n_cached;
+  for (int i = G * (QP / 2) + tid; i < 8 * (QP / 2); i += kAttnThreads) reinterpret_cast<uint32_t*>(&q_s[0][0])[i] = 0;   // columns without a head
   if constexpr (DECODE) {
     float rc[EPL / 2], rs[EPL / 2];
     if (p.rope != nullptr) {
@@ -368,7 +403,7 @@ __global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(
       }
     }
     pdl_wait();                            // qkv of this token is complete and visible from here on
-    stamp(1);
+    row_stamp<DECODE>(p, 1);
     const int qdim = p.Hq * HD, kvdim = p.Hkv * HD;
     for (int h = warp; h < G + 1; h += kAttnWarps) {
       const bool is_k = h == G;
@@ -397,7 +432,7 @@ __global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(
       }
       if (is_k) {
         const size_t at = (size_t)(b * a.kv_bstride) + ((size_t)pos * p.Hkv + kvh) * HD;
-        const bool leader = h0 % (p.Hq / p.Hkv) == 0;   // one CTA writes the new cache row
+        const bool leader = (int)blockIdx.y == kvh * a.per_kv;   // one CTA writes the new cache row
 #pragma unroll
         for (int j = 0; j < EPL; ++j) {
           const __nv_bfloat16 kk = f_to_bf16(x[j]), vv = qkv[qdim + kvdim + kvh * HD + lane + 32 * j];
@@ -410,161 +445,181 @@ __global__ void __launch_bounds__(kAttnThreads, G == 1 ? 1 : 2) attn_row_kernel(
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < EPL; ++j) q_s[h][lane + 32 * j] = x[j];
+        for (int j = 0; j < EPL; ++j) q_s[h][lane + 32 * j] = f_to_bf16(x[j]);   // rounded before: exact
       }
     }
   } else {
-    for (int i = tid; i < G * HD; i += kAttnThreads) (&q_s[0][0])[i] = bf16_to_f(qkv[h0 * HD + i]);
+#pragma unroll
+    for (int i = 0; i < GM * HD / kAttnThreads + 1; ++i) {
+      const int e = i * kAttnThreads + tid;
+      if (e < G * HD) q_s[e / HD][e % HD] = f_to_bf16(q_in[i]);
+    }
   }
   __syncthreads();
-  stamp(3);
-  float qf[G][8], m[G], l[G], acc[G][8];
+  row_stamp<DECODE>(p, 3);
+  uint32_t qb[HD / 16][2];   // q as the B operand: column g = head, rows of two neighbouring channels
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
-    m[g] = -INFINITY;
-    l[g] = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      qf[g][e] = q_s[g][part * 8 + e];
-      acc[g][e] = 0.f;
-    }
+  for (int kk = 0; kk < HD / 16; ++kk) {
+    qb[kk][0] = *reinterpret_cast<const uint32_t*>(&q_s[g][kk * 16 + tq * 2]);
+    qb[kk][1] = *reinterpret_cast<const uint32_t*>(&q_s[g][kk * 16 + tq * 2 + 8]);
   }
-  auto round = [&](int buf, int c) {
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // of heads 2·tq and 2·tq + 1; l: this lane's keys
+  const int dq = lane % LQ, kg = lane / LQ;                 // P·V: this lane's columns, and (heads of 64) its half of the keys
+  float acc[GM][4];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      float sc[U], top = m[g];
+  for (int h = 0; h < GM; ++h)
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        sc[u] = dot8(kr[buf][u], qf[g], 0.f);
-#pragma unroll
-        for (int o = LPK / 2; o > 0; o >>= 1) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o);
-        if (c + u * NG + grp >= k1) sc[u] = -INFINITY;
-        top = fmaxf(top, sc[u]);
+    for (int e = 0; e < 4; ++e) acc[h][e] = 0.f;
+  float(*const pw)[GM] = ps + warp * 16;
+  for (int u = 0; u < units; ++u) {
+    const int nv = min(16, n - u * kUnit - warp * 16);
+    const bool has_new = owns_new && u * kUnit + warp * 16 + nv == n;
+    const uint32_t kslot = (uint32_t)(2 * u % R::NS) * R::SLOT, vslot = (uint32_t)((2 * u + 1) % R::NS) * R::SLOT;
+    auto put_new = [&](uint32_t slot, const __nv_bfloat16* row) {
+      if (nv == 1 && n_cached == n - 1 && u * kUnit + warp * 16 == n_cached) {   // a warp without a cached key has not cleared its rows
+        for (int e = lane; e < (int)WB / 16; e += 32) reinterpret_cast<uint4*>(ring + warp * WB + slot)[e] = make_uint4(0, 0, 0, 0);
+        __syncwarp();
       }
-      const float ts = top == -INFINITY ? 0.f : top * kScale;
-      const float alpha = m[g] == -INFINITY ? 0.f : exp2f(m[g] * kScale - ts);
-      m[g] = top;
-      l[g] *= alpha;
+      if (lane < HD / 8) *reinterpret_cast<uint4*>(ring + warp * WB + slot + piece_at(nv - 1, lane)) = reinterpret_cast<const uint4*>(row)[lane];
+    };
+    asm volatile("cp.async.wait_group %0;" ::"n"(R::NS - 1) : "memory");
+    if (has_new) put_new(kslot, knew);
+    __syncwarp();
+    float c[2][4] = {};   // keys g and g + 8 of the warp's sixteen, heads 2·tq and 2·tq + 1; two chains
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[g][e] *= alpha;
+    for (int kk = 0; kk < HD / 16; ++kk) {
+      uint32_t ka[4];
+      float(&d)[4] = c[kk & 1];
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(ka[0]), "=r"(ka[1]), "=r"(ka[2]), "=r"(ka[3]) : "r"(ring_u + kslot + piece_at(lane & 15, 2 * kk + (lane >> 4))) : "memory");
+      asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                   : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                   : "r"(ka[0]), "r"(ka[1]), "r"(ka[2]), "r"(ka[3]), "r"(qb[kk][0]), "r"(qb[kk][1]));
+    }
+    load(2 * u + R::NS);   // K has been read
+    float pr[4], alpha[2];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const bool in = c + u * NG + grp < k1;
-        const float pr = in ? exp2f(sc[u] * kScale - ts) : 0.f;
-        l[g] += pr;
-        float vf[8];
-        unpack8(in ? vr[buf][u] : make_uint4(0, 0, 0, 0), vf);   // a key without weight meets no value
+    for (int e = 0; e < 2; ++e) {
+      const float s0 = g < nv ? c[0][e] + c[1][e] : -INFINITY, s1 = g + 8 < nv ? c[0][2 + e] + c[1][2 + e] : -INFINITY;
+      float t = fmaxf(s0, s1);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[g][e] = fmaf(pr, vf[e], acc[g][e]);
+      for (int o = 4; o < 32; o <<= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
+      t = fmaxf(t, m[e]);
+      const float ts = t == -INFINITY ? 0.f : t * kScale;
+      alpha[e] = u == 0 || m[e] == -INFINITY ? 0.f : exp2f(m[e] * kScale - ts);
+      m[e] = t;
+      pr[e] = g < nv ? exp2f(s0 * kScale - ts) : 0.f;
+      pr[2 + e] = g + 8 < nv ? exp2f(s1 * kScale - ts) : 0.f;
+      l[e] = l[e] * alpha[e] + (pr[e] + pr[2 + e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (2 * tq + e < GM) {
+        pw[g][2 * tq + e] = pr[e];
+        pw[g + 8][2 * tq + e] = pr[2 + e];
+      }
+    if (u > 0) {
+#pragma unroll
+      for (int h = 0; h < GM; ++h) {
+        const float f = __shfl_sync(0xffffffffu, alpha[h & 1], h >> 1);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[h][e] *= f;
       }
     }
-  };
-  for (int c = k0; c < k1; c += 2 * NG * U) {
-    if (c + NG * U < k1) fetch(1, c + NG * U);
-    round(0, c);
-    if (c + NG * U >= k1) break;
-    if (c + 2 * NG * U < k1) fetch(0, c + 2 * NG * U);
-    round(1, c + NG * U);
-  }
-  if (owns_new && warp == 0) {             // the new row, from shared memory: one more key of the first key group
-    const uint4 kn = reinterpret_cast<const uint4*>(knew)[part], vn = reinterpret_cast<const uint4*>(vnew)[part];
-    float vf[8];
-    unpack8(vn, vf);
+    asm volatile("cp.async.wait_group %0;" ::"n"(R::NS - 1) : "memory");
+    if (has_new) put_new(vslot, vnew);
+    __syncwarp();
+    const uint8_t* const vt = ring + warp * WB + vslot + (dq & 1) * 8;
+#pragma unroll 4
+    for (int k = kg; k < 16; k += 32 / LQ) {   // keys behind the last: a weight of 0 and rows of zeros
+      const uint2 w = *reinterpret_cast<const uint2*>(vt + piece_at(k, dq >> 1));
+      const float v[4] = {__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u)};
+      float pk[GM];
+      if constexpr (GM >= 4) {
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      float sc = dot8(kn, qf[g], 0.f);
+        for (int h = 0; h < GM; h += 4) *reinterpret_cast<float4*>(&pk[h]) = *reinterpret_cast<const float4*>(&pw[k][h]);
+      } else {
 #pragma unroll
-      for (int o = LPK / 2; o > 0; o >>= 1) sc += __shfl_xor_sync(0xffffffffu, sc, o);
-      if (grp != 0) continue;
-      const float top = fmaxf(m[g], sc);
-      const float alpha = m[g] == -INFINITY ? 0.f : exp2f((m[g] - top) * kScale), pr = exp2f(sc * kScale - top * kScale);
-      m[g] = top;
-      l[g] = l[g] * alpha + pr;
+        for (int h = 0; h < GM; ++h) pk[h] = pw[k][h];
+      }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[g][e] = fmaf(pr, vf[e], acc[g][e] * alpha);
+      for (int h = 0; h < GM; ++h)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[h][e] = fmaf(pk[h], v[e], acc[h][e]);
     }
     __syncwarp();
+    load(2 * u + 1 + R::NS);
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");   // only empty groups are left
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
+  for (int e = 0; e < 2; ++e)
 #pragma unroll
-    for (int o = LPK; o < 32; o <<= 1) {   // key groups that live in the same warp
-      const float mo = __shfl_xor_sync(0xffffffffu, m[g], o), lo = __shfl_xor_sync(0xffffffffu, l[g], o);
-      const float top = fmaxf(m[g], mo);
-      const float fa = m[g] == -INFINITY ? 0.f : exp2f((m[g] - top) * kScale), fb = mo == -INFINITY ? 0.f : exp2f((mo - top) * kScale);
-      l[g] = l[g] * fa + lo * fb;
+    for (int o = 4; o < 32; o <<= 1) l[e] += __shfl_xor_sync(0xffffffffu, l[e], o);
+  if (g == 0) {
+    w_ml[warp][2 * tq] = make_float2(m[0], l[0]);
+    w_ml[warp][2 * tq + 1] = make_float2(m[1], l[1]);
+  }
+  __syncthreads();                                     // every warp's keys are read: the ring takes the sums
+  float4* const sums = reinterpret_cast<float4*>(ring);   // [warp][GM][LQ]
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[g][e] = acc[g][e] * fa + __shfl_xor_sync(0xffffffffu, acc[g][e], o) * fb;
-      m[g] = top;
+  for (int h = 0; h < GM; ++h) {
+    if constexpr (LQ == 16) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[h][e] += __shfl_xor_sync(0xffffffffu, acc[h][e], 16);
     }
-    __syncthreads();   // the previous head's partials have been read
-    if (lane < LPK) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) w_acc[warp][lane * 8 + e] = acc[g][e];
-      if (lane == 0) {
-        w_ml[warp][0] = m[g];
-        w_ml[warp][1] = l[g];
-      }
-    }
-    __syncthreads();
-    if (tid < HD) {
-      float top = -INFINITY, num = 0.f, den = 0.f;
-#pragma unroll
-      for (int w = 0; w < kAttnWarps; ++w) top = fmaxf(top, w_ml[w][0]);
-#pragma unroll
-      for (int w = 0; w < kAttnWarps; ++w) {
-        const float f = w_ml[w][0] == -INFINITY ? 0.f : exp2f((w_ml[w][0] - top) * kScale);
-        num = fmaf(f, w_acc[w][tid], num);
-        den = fmaf(f, w_ml[w][1], den);
-      }
-      res[g][tid] = num;
-      if (tid == 0) {
-        res_ml[g][0] = top;
-        res_ml[g][1] = den;
-      }
-    }
+    if (kg == 0) sums[(warp * GM + h) * LQ + dq] = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
   }
   __syncthreads();
-  cluster_sync_all();   // every CTA's part is in place
-  if (tid < G * 8) {    // one lane per (head, CTA)
-    const int g = tid / 8, r = tid % 8;
-    float4 ml = make_float4(-INFINITY, 0.f, 0.f, 0.f);
-    if (r < splits) ml = ld_cluster_f4(mapa_u32(smem_u32(&res_ml[g][0]), r));
+  cluster_wait();                                      // every CTA runs
+  const int share = (G * LQ + splits - 1) / splits;    // column quads that a CTA finishes
+  for (int i = tid; i < G * LQ; i += kAttnThreads) {
+    const int h = i / LQ, to = i / share;
+    float2 ml[kAttnWarps];
+    float4 x[kAttnWarps];
+    float top = -INFINITY, den = 0.f;
+#pragma unroll
+    for (int w = 0; w < kAttnWarps; ++w) {
+      ml[w] = w_ml[w][h];
+      x[w] = sums[(w * GM + h) * LQ + i % LQ];
+      top = fmaxf(top, ml[w].x);
+    }
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < kAttnWarps; ++w) {
+      const float f = ml[w].x == -INFINITY ? 0.f : exp2f((ml[w].x - top) * kScale);
+      den = fmaf(f, ml[w].y, den);
+      t.x = fmaf(f, x[w].x, t.x);
+      t.y = fmaf(f, x[w].y, t.y);
+      t.z = fmaf(f, x[w].z, t.z);
+      t.w = fmaf(f, x[w].w, t.w);
+    }
+    st_cluster_f4(mapa_u32(smem_u32(&part[rank * share + i - to * share]), to), t);
+    // with the first of this head's columns that go there, the maximum and the sum
+    if (i == max(h * LQ, to * share)) st_cluster_f2(mapa_u32(smem_u32(&part_ml[rank][h]), to), make_float2(top, den));
+  }
+  cluster_sync_all();                                  // every CTA's parts are in place
+  const int r = tid & (splits - 1), j = tid >> a.log_splits, i = rank * share + j;   // a lane per CTA and four neighbouring outputs
+  if (j < share && i < G * LQ) {
+    const unsigned mask = __activemask();
+    const float2 ml = part_ml[r][i / LQ];
+    const float4 x = part[r * share + j];
     float top = ml.x;
-    constexpr unsigned mask = (1u << (G * 8)) - 1u;
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(mask, top, o));
+    for (int o = splits >> 1; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(mask, top, o));
     const float f = ml.x == -INFINITY ? 0.f : exp2f((ml.x - top) * kScale);
-    float den = f * ml.y;
+    float den = f * ml.y, num[4] = {f * x.x, f * x.y, f * x.z, f * x.w};
+    for (int o = splits >> 1; o > 0; o >>= 1) {
+      den += __shfl_xor_sync(mask, den, o);
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) den += __shfl_xor_sync(mask, den, o);
-    weight[g][r] = f;
-    if (r == 0) total[g] = den;
-  }
-  __syncthreads();
-  for (int i = rank * kAttnThreads + tid; i < G * HD / 4; i += splits * kAttnThreads) {   // four neighbouring outputs
-    const int g = i / (HD / 4), d = (i % (HD / 4)) * 4;
-    float4 x[8], num = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int r = 0; r < 8; ++r) x[r] = r < splits ? ld_cluster_f4(mapa_u32(smem_u32(&res[g][d]), r)) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const float f = weight[g][r];
-      num.x = fmaf(f, x[r].x, num.x);
-      num.y = fmaf(f, x[r].y, num.y);
-      num.z = fmaf(f, x[r].z, num.z);
-      num.w = fmaf(f, x[r].w, num.w);
+      for (int e = 0; e < 4; ++e) num[e] += __shfl_xor_sync(mask, num[e], o);
     }
-    const float inv = total[g] > 0.f ? 1.f / total[g] : 0.f;
-    __nv_bfloat16* o = p.out + b * p.out_bstride + (h0 + g) * HD + d;
-    o[0] = f_to_bf16(num.x * inv);
-    o[1] = f_to_bf16(num.y * inv);
-    o[2] = f_to_bf16(num.z * inv);
-    o[3] = f_to_bf16(num.w * inv);
+    const float inv = den > 0.f ? 1.f / den : 0.f;
+    __nv_bfloat16* o = p.out + b * p.out_bstride + h0 * HD + i * 4;
+    if (r == 0) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = f_to_bf16(num[e] * inv);
+    }
   }
-  stamp(2);
-  __syncthreads();
-  cluster_sync_all();   // no CTA leaves while another still reads its part
+  row_stamp<DECODE>(p, 2);
 }
 
 // ------------------------------------------------------------------------------------------ general attention
@@ -639,9 +694,9 @@ __global__ void __launch_bounds__(128) attn_general_kernel(__nv_bfloat16* __rest
 }  // namespace
 
 // Caches from which the cluster kernel takes over: more splits than this (1 024 tokens for heads of 128, 2 048 for heads of 64).  The choice is
-// by the cache, since a captured graph serves every position; it is the faster one at all of them.  Device µs with caches for 4 096 tokens, one CTA per
-// split / cluster, at positions 20, 300, 2 000 and 4 000: 16 heads of 128 5.9 / 5.1, 9.3 / 5.3, 11.4 / 8.8, 21.5 / 12.1; 32 heads of
-// 128 7.8 / 5.4, 13.8 / 5.6, 17.4 / 9.7, 33.2 / 13.1; 14 heads of 64 9.5 / 4.6, 17.4 / 4.8, 17.7 / 5.9, 21.1 / 7.2.
+// by the cache, since a captured graph serves every position.  Device µs with caches for 4 096 tokens, one CTA per
+// split / cluster, at positions 20, 300, 2 000 and 4 000: 16 heads of 128 5.9 / 5.5, 9.3 / 5.6, 11.4 / 6.7, 21.5 / 9.9; 32 heads of
+// 128 7.8 / 5.9, 13.8 / 5.9, 17.4 / 7.3, 33.2 / 10.9; 14 heads of 64 9.5 / 5.1, 17.4 / 5.2, 17.7 / 5.6, 21.1 / 6.9.
 constexpr int kLongSplits = 8;
 
 int64_t attn_decode_ws_floats(int Hq, int Hkv, int hd, int nsplit) {
@@ -668,11 +723,19 @@ int attn_decode_nsplit(int hd, int max_ctx) {
   return std::max(1, (max_ctx + chunk - 1) / chunk);
 }
 
-template <int HD, int G, bool DECODE>
+template <int HD, int GM, bool DECODE>
 static int launch_row_t(const AttnRow& a, int splits, int B, cudaStream_t st, bool pdl) {
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(attn_row_kernel<HD, GM, DECODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, KeyRing<HD>::smem);
+    if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(attn_row_kernel<HD, GM, DECODE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  });
+  B200_CUDA(attr_err);
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)splits, (unsigned)(a.d.Hq / G), (unsigned)B);
+  cfg.gridDim = dim3((unsigned)splits, (unsigned)(a.d.Hq / a.G), (unsigned)B);
   cfg.blockDim = dim3(kAttnThreads);
+  cfg.dynamicSmemBytes = KeyRing<HD>::smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -683,20 +746,30 @@ static int launch_row_t(const AttnRow& a, int splits, int B, cudaStream_t st, bo
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 2 : 1;
   g_launches.fetch_add(1);
-  B200_CUDA(cudaLaunchKernelEx(&cfg, attn_row_kernel<HD, G, DECODE>, a));
+  B200_CUDA(cudaLaunchKernelEx(&cfg, attn_row_kernel<HD, GM, DECODE>, a));
   return B200_OK;
 }
-// A CTA per query head, or per two heads of a KV head once that leaves 64 of them (K and V are read through L2 once per CTA).
-static int launch_row(const AttnRow& a, int hd, int splits, int B, bool decode, cudaStream_t st, bool pdl) {
-  const bool two = (a.d.Hq / a.d.Hkv) % 2 == 0 && (int64_t)(a.d.Hq / 2) * B >= 64;
-  if (hd == 64) {
-    if (decode) return two ? launch_row_t<64, 2, true>(a, splits, B, st, pdl) : launch_row_t<64, 1, true>(a, splits, B, st, pdl);
-    return two ? launch_row_t<64, 2, false>(a, splits, B, st, pdl) : launch_row_t<64, 1, false>(a, splits, B, st, pdl);
-  }
-  if (decode) return two ? launch_row_t<128, 2, true>(a, splits, B, st, pdl) : launch_row_t<128, 1, true>(a, splits, B, st, pdl);
-  return two ? launch_row_t<128, 2, false>(a, splits, B, st, pdl) : launch_row_t<128, 1, false>(a, splits, B, st, pdl);
+template <int HD, bool DECODE>
+static int launch_row_g(const AttnRow& a, int splits, int B, cudaStream_t st, bool pdl) {
+  if (a.G == 1) return launch_row_t<HD, 1, DECODE>(a, splits, B, st, pdl);
+  if (a.G == 2) return launch_row_t<HD, 2, DECODE>(a, splits, B, st, pdl);
+  return a.G <= 4 ? launch_row_t<HD, 4, DECODE>(a, splits, B, st, pdl) : launch_row_t<HD, 8, DECODE>(a, splits, B, st, pdl);
 }
-// One query row: as many CTAs per cluster (≤ 8) as keep 64 keys each and no more than two CTAs per SM.
+// The heads of a CTA: the largest divisor of the group up to eight.  The CTAs of a cluster: as many (a power of two up to 16) as the SMs hold
+// clusters of at once, two CTAs to an SM (14 of 16 CTAs, 33 of 8, 71 of 4, 148 of 2), while each keeps 64 of `keys` keys.
+static int launch_row(AttnRow& a, int hd, int64_t keys, int B, bool decode, cudaStream_t st, bool pdl) {
+  const int group = a.d.Hq / a.d.Hkv;
+  a.G = 1;
+  for (int g = 2; g <= 8; ++g)
+    if (group % g == 0) a.G = g;
+  const int64_t clusters = (int64_t)(a.d.Hq / a.G) * B;
+  const int most = clusters <= 14 ? 16 : clusters <= 33 ? 8 : clusters <= 71 ? 4 : clusters <= 148 ? 2 : 1;
+  int splits = 1;
+  while (splits < most && keys >= 128 * splits) splits *= 2, ++a.log_splits;
+  a.per_kv = group / a.G;
+  if (hd == 64) return decode ? launch_row_g<64, true>(a, splits, B, st, pdl) : launch_row_g<64, false>(a, splits, B, st, pdl);
+  return decode ? launch_row_g<128, true>(a, splits, B, st, pdl) : launch_row_g<128, false>(a, splits, B, st, pdl);
+}
 static int launch_attn_row(void* o, const void* q, const void* k, const void* v, int64_t B, int64_t Skv, int64_t Hq, int64_t Hkv, int64_t hd,
                            int causal, cudaStream_t st) {
   B200_CHECK_ARG(hd == 64 || hd == 128, "attention: head_dim %lld not built (64 and 128 are)", (long long)hd);
@@ -712,9 +785,7 @@ static int launch_attn_row(void* o, const void* q, const void* k, const void* v,
   a.d.qkv_bstride = a.d.out_bstride = Hq * hd;
   a.kv_bstride = Skv * Hkv * hd;
   a.nkeys = causal ? 1 : (int)Skv;   // causal: the mask is top-left aligned, row 0 sees key 0
-  int splits = 1;
-  while (splits < 8 && a.nkeys >= 128 * splits && Hq * B * splits * 2 <= 296) splits *= 2;
-  return launch_row(a, (int)hd, splits, (int)B, false, st, false);
+  return launch_row(a, (int)hd, a.nkeys, (int)B, false, st, false);
 }
 
 int launch_attn_decode(const AttnDecodeParams& p, int hd, cudaStream_t st, bool pdl) {
@@ -729,8 +800,8 @@ int launch_attn_decode(const AttnDecodeParams& p, int hd, cudaStream_t st, bool 
   B200_CHECK_ARG(G >= 1 && G <= 8, "attention: at most 8 query heads per CTA (got %d)", G);
   const unsigned nb = (unsigned)std::max(1, p.batch);
   if (p.nsplit > kLongSplits) {
-    AttnRow a{p, 0, p.cache_bstride};
-    return launch_row(a, hd, 8, (int)nb, true, st, pdl);
+    AttnRow a{p, 0, p.cache_bstride, 1, 1, 0};
+    return launch_row(a, hd, p.max_ctx, (int)nb, true, st, pdl);
   }
   if (hd == 64)
     B200_CUDA(launch_pdl(attn_decode_reg_kernel<64>, dim3(p.nsplit, p.Hq / G, nb), dim3(kAttnThreads), 0, st, pdl, p, G));
