@@ -7,6 +7,7 @@ from pathlib import Path
 import os
 
 LIB_PATH = Path(os.environ.get("B200_LIB") or (Path(__file__).resolve().parent / "lib" / "libb200decode.so"))
+NATIVE_PATH = LIB_PATH.with_name("b200ops.so")   # it loads the library that lies beside it
 IPC_HANDLE_BYTES = 64
 
 _lib = None
@@ -227,6 +228,27 @@ def lib() -> C.CDLL:
             fn.argtypes = args
         _lib = h
     return _lib
+
+
+_native = None
+
+
+def native():
+    """lib/b200ops.so: the operators of ops.py as native functions over torch tensors (csrc/torch_ops.cpp)."""
+    global _native
+    if _native is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries come first)
+        lib()
+        if not NATIVE_PATH.exists():
+            raise B200Error(f"{NATIVE_PATH} is missing: build it with `python -m tinygpt_b200.build`. There is no other path to the operators.")
+        loader = importlib.machinery.ExtensionFileLoader("b200ops", str(NATIVE_PATH))
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200ops", loader))
+        loader.exec_module(mod)
+        _native = mod
+    return _native
 
 
 def check(rc: int, what: str = "") -> None:

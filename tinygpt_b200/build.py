@@ -2,7 +2,8 @@
 
     python -m tinygpt_b200.build [--force] [--verbose]
 
-Output: tinygpt_b200/lib/libb200decode.so  (C ABI declared in include/b200_decode.h).
+Output: tinygpt_b200/lib/libb200decode.so  (C ABI declared in include/b200_decode.h) and, linked to it and to torch,
+tinygpt_b200/lib/b200ops.so  (the operators of ops.py as native functions, csrc/torch_ops.cpp).
 """
 from __future__ import annotations
 
@@ -20,6 +21,7 @@ CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 OBJ_DIR = LIB_DIR / "obj"
 LIB_PATH = LIB_DIR / "libb200decode.so"
+NATIVE_PATH = LIB_DIR / "b200ops.so"
 
 SOURCES = ["common.cu", "gemv.cu", "gemv_batch.cu", "gemm.cu", "prefill.cu", "prefill_attn.cu", "prefill_attn_tc.cu", "sampling.cu", "ops.cu", "attn.cu", "engine.cu", "api.cu", "tp.cu", "stack_ops.cu",
            "stack_mix.cu", "stack_rec.cu", "stack_hyper.cu", "stack_pool.cu", "stack_pool_mma.cu", "engine_stack.cu"]
@@ -43,11 +45,24 @@ def _nvcc() -> str:
 
 def _digest() -> str:
     h = hashlib.sha256()
-    for p in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + [ROOT / "include" / "b200_decode.h"]):
+    for p in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.cpp")) + [ROOT / "include" / "b200_decode.h"]):
         h.update(p.name.encode())
         h.update(p.read_bytes())
     h.update(" ".join(NVCC_FLAGS).encode())
     return h.hexdigest()
+
+
+def _native_command() -> list[str]:
+    """g++ for the torch extension: torch's own headers and libraries, the library beside it at load time."""
+    import sysconfig
+
+    import torch
+    home = Path(torch.__file__).parent
+    nvcc_home = Path(_nvcc()).resolve().parent.parent
+    includes = [home / "include", home / "include/torch/csrc/api/include", nvcc_home / "include", sysconfig.get_paths()["include"]]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *[x for i in includes for x in ("-isystem", str(i))], "-I", str(ROOT / "include"), str(CSRC / "torch_ops.cpp"), "-o", str(NATIVE_PATH),
+            f"-L{home / 'lib'}", f"-L{LIB_DIR}", "-lb200decode", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -55,7 +70,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     OBJ_DIR.mkdir(exist_ok=True)
     stamp = LIB_DIR / "build.stamp"
     digest = _digest()
-    if not force and LIB_PATH.exists() and stamp.exists() and stamp.read_text().strip() == digest:
+    if not force and LIB_PATH.exists() and NATIVE_PATH.exists() and stamp.exists() and stamp.read_text().strip() == digest:
         return LIB_PATH
     nvcc = _nvcc()
     log_lines: list[str] = []
@@ -76,6 +91,11 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     log_lines.append(f"$ {' '.join(cmd)}\n{r.stdout}{r.stderr}")
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    cmd = _native_command()
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    log_lines.append(f"$ {' '.join(cmd)}\n{r.stdout}{r.stderr}")
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on torch_ops.cpp:\n{r.stdout}\n{r.stderr}")
     (LIB_DIR / "build.log").write_text("\n".join(log_lines))
     stamp.write_text(digest)
     if verbose:

@@ -10,7 +10,7 @@ from typing import Optional
 
 import torch
 
-from ._lib import B200Error, check, lib
+from ._lib import B200Error, check, lib, native
 
 BSHD, BHSD = 1, 0  # b200_qkv_layout
 
@@ -38,9 +38,27 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
+class _Native:
+    """The functions of lib/b200ops.so (csrc/torch_ops.cpp): each makes the plain case of the operator of its name here one native call and
+    answers None for all else, which then goes the way below.  Loaded with the first call."""
+
+    def __getattr__(self, name):
+        self.__dict__.update({k: f for k, f in vars(native()).items() if not k.startswith("_")})
+        return self.__dict__[name]
+
+
+_fast = _Native()
+_Tensor = torch.Tensor
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """function::linear(x, W, b) = op::matmul(x, W, false, true, b)  [ref: TT/Function/FuncNNLayer.h:14-18].
     x [..., k] bf16, W [n, k] bf16 → [..., n] bf16."""
+    y = _fast.linear(x, weight, bias)
+    if y.__class__ is _Tensor:
+        return y
+    if y is not None:
+        check(y, "b200_gemv_bf16")
     x, weight = _chk(x, "linear.x"), _chk(weight, "linear.weight")
     if bias is not None:
         bias = _chk(bias, "linear.bias")
@@ -56,6 +74,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
 
 def gemm(a: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """Batched Linear without bias on the tcgen05 tensor cores: a [..., k] · W[n, k]ᵀ → [..., n] (prefill, m > 1)."""
+    c = _fast.gemm(a, weight)
+    if c.__class__ is _Tensor:
+        return c
+    if c is not None:
+        check(c, "b200_gemm_bf16")
     a, weight = _chk(a, "gemm.a"), _chk(weight, "gemm.weight")
     n, k = weight.shape
     if a.shape[-1] != k:
@@ -68,6 +91,11 @@ def gemm(a: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
 
 def rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], eps: float) -> torch.Tensor:
     """function::rmsNorm(x, {dim}, w, eps)  [ref: TT/Function/FuncNNLayer.h:220-227]."""
+    y = _fast.rms_norm(x, weight, eps)
+    if y.__class__ is _Tensor:
+        return y
+    if y is not None:
+        check(y, "b200_rmsnorm_bf16")
     x = _chk(x, "rms_norm.x")
     if weight is not None:
         weight = _chk(weight, "rms_norm.weight")
@@ -107,6 +135,11 @@ def rope_init(head_dim: int, ctx: int, theta: float, scaling=None, device="cuda"
 
 def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, is_causal: bool = False) -> torch.Tensor:
     """function::flashAttention(q, k, v, isCausal), BSHD  [ref: TT/Function/FuncNNLayer.h:270-277]."""
+    o = _fast.flash_attention(q, k, v, is_causal)
+    if o.__class__ is _Tensor:
+        return o
+    if o is not None:
+        check(o, "b200_attn_bf16")
     q, k, v = _chk(q, "flash_attention.q"), _chk(k, "flash_attention.k"), _chk(v, "flash_attention.v")
     B, Sq, Hq, D = q.shape
     Skv, Hkv = k.shape[1], k.shape[2]
@@ -118,6 +151,11 @@ def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, is_causal
 
 def silu_mul(x: torch.Tensor) -> torch.Tensor:
     """function::siluMul(x): last dim = [gate | up]  [ref: TT/Function/FuncFused.h:14-21]."""
+    y = _fast.silu_mul(x)
+    if y.__class__ is _Tensor:
+        return y
+    if y is not None:
+        check(y, "b200_silu_mul_bf16")
     x = _chk(x, "silu_mul.x")
     I = x.shape[-1] // 2
     if x.shape[-1] % 2:
@@ -130,6 +168,11 @@ def silu_mul(x: torch.Tensor) -> torch.Tensor:
 
 def add(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """function::add(a, b) with alpha = 1, same shapes  [ref: TT/Function/FuncElemWise.h:74]."""
+    y = _fast.add(a, b)
+    if y.__class__ is _Tensor:
+        return y
+    if y is not None:
+        check(y, "b200_add_bf16")
     a, b = _chk(a, "add.a"), _chk(b, "add.b")
     if a.shape != b.shape:
         raise B200Error("add: the decode path only adds same-shape tensors")
@@ -166,6 +209,11 @@ def argmax(logits: torch.Tensor, keepdim: bool = True) -> torch.Tensor:
 # ---- fused building blocks (the kernels the engine actually runs)
 def gemv_fused(x, weight, *, norm_weight=None, eps=0.0, bias=None, residual=None, silu_mul=False) -> torch.Tensor:
     """[RMSNorm] → GEMV → {bias | residual | SiLU·mul over merged gate|up} in ONE launch (m = 1)."""
+    y = _fast.gemv_fused(x, weight, norm_weight, eps, bias, residual, silu_mul)
+    if y.__class__ is _Tensor:
+        return y
+    if y is not None:
+        check(y, "b200_gemv_fused_bf16")
     x, weight = _chk(x, "gemv_fused.x"), _chk(weight, "gemv_fused.weight")
     rows, k = weight.shape
     nseg = 2 if silu_mul else 1
@@ -180,6 +228,11 @@ def gemv_fused(x, weight, *, norm_weight=None, eps=0.0, bias=None, residual=None
 def attn_decode(qkv, kcache, vcache, *, q_heads, kv_heads, head_dim, pos=None, fixed_len=0, rope_table=None,
                 q_norm=None, k_norm=None, eps=0.0) -> torch.Tensor:
     """Fused decode attention of one layer (see include/b200_decode.h b200_attn_decode_bf16)."""
+    out = _fast.attn_decode(qkv, kcache, vcache, q_heads, kv_heads, head_dim, pos, fixed_len, rope_table, q_norm, k_norm, eps)
+    if out.__class__ is _Tensor:
+        return out
+    if out is not None:
+        check(out, "b200_attn_decode_bf16")
     qkv, kcache, vcache = _chk(qkv, "attn_decode.qkv"), _chk(kcache, "attn_decode.kcache"), _chk(vcache, "attn_decode.vcache")
     max_ctx = kcache.shape[0]
     n, tickets = lib().b200_attn_decode_workspace_bytes(q_heads, kv_heads, head_dim, max_ctx), (4 * q_heads + 15) // 16 * 16
