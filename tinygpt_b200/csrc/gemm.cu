@@ -9,11 +9,15 @@
 // here — it is HBM-bound and runs on the CUDA-core GEMV (gemv.cu).
 //
 // Two kernels, chosen per shape (pick_gemm): persistent CTA pairs on 256 × 256 tiles when the tiles fill the GPU, clusters that may
-// split K when they do not.  The engines' products never split: a row's sum has one order whatever M is.  In both (192 threads, warp-specialised):
+// split K when they do not.  The engines' products never split: a row's sum has one order whatever M is.  In both (warp-specialised, 192 threads
+// or 320):
 //   warp 0   TMA producer: 64-column k-blocks of A and B (128-byte swizzle) into a shared-memory ring, completion on `full[s]`
 //   warp 1   MMA issuer: one thread issues 4 × tcgen05.mma.kind::f16 (K16) per k-block, accumulator in TMEM; tcgen05.commit
-//            releases the stage to the producer (`empty[s]`) and signals the epilogue (`tmem_full`)
-//   warps 2-5 epilogue: tcgen05.ld 32x32b (each warp owns the TMEM lane quarter warp_id % 4)
+//            releases the stage to the producer (`empty[s]`) and signals the epilogue (`tmem_full`).  It looks at the next stage's barrier
+//            before it issues, and builds half descriptors: 64 cycles a k-block, where a wait of its own (210) and whole descriptors (305)
+//            took longer than the products of any tile (512 at 256 columns a pair).  µs, 2 048 rows: 3 072 × 8 192 85 → 75 (with 192-column
+//            tiles), 16 384 × 3 072 137 → 133, 12 288 × 2 048 76 → 70.5; 17 × 2 048 × 6 144 on one-CTA tiles 27 → 23
+//   the other warps: epilogue, tcgen05.ld 32x32b (each warp owns the TMEM lane quarter warp_id % 4)
 // TMA zero-fills out-of-range rows/columns, so M, N, K need not be multiples of the tile.  Every wait is bounded: one that gives up
 // leaves a code in the host-visible word of wait_word() and lets the kernel end.
 #include "ops.cuh"
@@ -22,6 +26,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
+#include <cstring>
 #include <mutex>
 
 namespace b200 {
@@ -60,32 +65,37 @@ __device__ __forceinline__ uint32_t silu_mul2(uint32_t g0, uint32_t g1, uint32_t
 }
 
 // ------------------------------------------------------------------------------------------- persistent CTA pairs
-// One tcgen05.mma.cta_group::2 covers a 256 × 256 tile (M256 N256 K16): CTA r of the pair holds rows 128·r of A and half of B's
-// 256 rows, so per 64-wide k-block an SM loads 32 KB where two one-CTA 128 × 256 tiles take 48 KB each.  Persistent pairs (grid =
+// One tcgen05.mma.cta_group::2 covers a 256 × bn tile (M256 K16, bn = 256, 224 or 192): CTA r of the pair holds rows 128·r of A and half of
+// B's rows, so per 64-wide k-block an SM loads 32 KB at most where two one-CTA 128 × 256 tiles take 48 KB each.  Persistent pairs (grid =
 // min(tiles, #SMs / 2) pairs) walk tiles m-fastest, so pairs that run side by side share weight rows in L2; the fp32
-// accumulator is double-buffered in TMEM (2 × 256 columns): the epilogue of tile i drains one buffer while the MMA warp
-// fills the other.  The epilogue turns rows of TMEM lanes into whole 128-byte row pieces through a swizzled 4 KB patch per
-// warp and stores 16 bytes per lane along the row.  Bound by the tensor pipe under the power cap: 2 048 × 12 288 × 2 048 in 74 µs
-// (1.39 PFLOP/s; one-CTA 128 × 256 tiles: 80 µs), 2 048 × 16 384 × 3 072 in 138 µs (1.49 PFLOP/s).
+// accumulator is double-buffered in TMEM (256 columns apart): the epilogue of tile i drains one buffer while the MMA warp
+// fills the other.  Eight epilogue warps, two to a quarter of the rows, turn rows of TMEM lanes into whole 128-byte row pieces through a swizzled
+// 4 KB patch per warp and store 16 bytes per lane along the row (four of them took 13 µs for SiLU products of a 256 × 256 tile, as long as
+// K = 2 048).  Bound by the tensor pipe under the power cap (a k-block of 256 columns takes 512 cycles, its products' own time; 192 columns
+// take 406, 128 no less: operands from L2, 70 bytes per cycle and SM).  The width is what wastes least in the last round of tiles, any
+// width sums the same bits: 2 048 × 3 072 × 8 192 is 96 tiles of 256 (two rounds of 74 pairs, 83.6 µs) or 128 of 192 (75.0),
+// 2 048 × 12 288 × 2 048 384 (six rounds, 73.1) or 440 of 224 (six, 70.4), 2 048 × 16 400 × 2 048 520 (eight, 95.9) or 592 of 224 (92.7).
 constexpr int kPairBN = 256;
 constexpr int kPairStages = 6;
 constexpr int kPairStageBytes = 2 * kTileBytes;
 constexpr int kPairPatch = 4096;   // 32 rows × 128 bytes per epilogue warp
-constexpr int kPairSmem = kPairStages * kPairStageBytes + 4 * kPairPatch + 1024 /*align*/ + 256 /*barriers*/;
+constexpr int kPairEpiWarps = 8, kPairThreads = 64 + 32 * kPairEpiWarps;
+constexpr int kPairSmem = kPairStages * kPairStageBytes + kPairEpiWarps * kPairPatch + 1024 /*align*/ + 256 /*barriers*/;
 
 template <typename OT, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmArgs<OT> p) {
-  constexpr int BN = kPairBN, ST = kPairStages, HB = BN / 2;
-  constexpr int OUT = EPI == GEPI_SILU ? HB : BN;   // output columns of a tile
-  constexpr uint32_t kIdesc = umma_idesc(256, BN);
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmArgs<OT> p, const int bn) {
+  constexpr int BN = kPairBN, ST = kPairStages;     // BN: columns from one accumulator to the next
+  const int HB = bn / 2;
+  const int OUT = EPI == GEPI_SILU ? HB : bn;       // output columns of a tile
+  const uint32_t idesc = umma_idesc(256, bn);
   constexpr int kCols = 2 * BN;                     // TMEM: two accumulators
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sA = smem;                               // [stages][128 × 64 bf16]
   uint8_t* sB = smem + ST * kTileBytes;             // [stages][128 × 64 bf16]
   uint8_t* patch = smem + ST * kPairStageBytes;     // [4 warps][32 rows × 128 bytes]
-  uint64_t* full = reinterpret_cast<uint64_t*>(patch + 4 * kPairPatch);   // CTA 0's count the pair's bytes
+  uint64_t* full = reinterpret_cast<uint64_t*>(patch + kPairEpiWarps * kPairPatch);   // CTA 0's count the pair's bytes
   uint64_t* empty = full + ST;
   uint64_t* tmem_full = empty + ST;                 // [2]
   uint64_t* tmem_empty = tmem_full + 2;             // [2], CTA 0's: one arrival per epilogue warp of the pair
@@ -107,7 +117,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
-      mbar_init(&tmem_empty[a], 8);
+      mbar_init(&tmem_empty[a], 2 * kPairEpiWarps);
     }
     fence_mbar_init();
   }
@@ -128,7 +138,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const int n0 = (t / mt) * OUT + rank * (EPI == GEPI_SILU ? p.N : HB);
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!(ok = mbar_wait_limited(&empty[s], ph, p.err, kGemmWaitCode | 1))) break;
-          if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * kPairStageBytes);
+          if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * (kTileBytes + HB * kBK * 2));
           const uint32_t bar = mapa_u32(smem_u32(&full[s]), 0);
           tma_load_2d_pair(sA + s * kTileBytes, &tmap_a, kb * kBK, m0, bar);
           tma_load_2d_pair(sB + s * kTileBytes, &tmap_b, kb * kBK, n0, bar);
@@ -142,27 +152,30 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------ MMA issuer (CTA 0)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
+      const uint32_t a0 = desc_lo(smem_u32(sA)), b0 = desc_lo(smem_u32(sB));
       int s = 0;
       uint32_t ph = 0;
       int i = 0;
+      bool ready = false;   // of the next stage, looked at before the products of this one go out
       for (int t = pair; t < tiles && ok; t += pairs, ++i) {
         const int acc = i & 1;
         if (!(ok = mbar_wait_limited(&tmem_empty[acc], (uint32_t)(((i >> 1) & 1) ^ 1), p.err, kGemmWaitCode | 2))) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (!(ok = mbar_wait_limited(&full[s], ph, p.err, kGemmWaitCode | 3))) break;
+          if (!ready && !(ok = mbar_wait_limited(&full[s], ph, p.err, kGemmWaitCode | 3))) break;
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + s * kTileBytes), b_addr = smem_u32(sB + s * kTileBytes);
-#pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)
-            umma_bf16_pair(tmem_d, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), kIdesc, (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(&empty[s]);
+          const uint32_t a = a0 + s * (kTileBytes >> 4), b = b0 + s * (kTileBytes >> 4);
+          uint64_t* const done = &empty[s];
           if (++s == ST) {
             s = 0;
             ph ^= 1;
           }
+          ready = mbar_test(&full[s], ph);
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k) umma_lo<2>(tmem_d, a + 2 * k, b + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(done);
         }
         if (ok) umma_commit_pair(&tmem_full[acc]);
       }
@@ -172,8 +185,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     // ---------------------------------------------------------------------------------------------- epilogue
     constexpr int CW = 128 / (int)sizeof(OT);       // columns of a patch row
     constexpr int VW = 16 / (int)sizeof(OT);        // columns per lane when the patch is read back
-    const int q = warp & 3;
-    uint8_t* const pw = patch + q * kPairPatch;
+    const int q = warp & 3, grp = (warp - 2) >> 2;  // two warps share a quarter of the lanes and take its column chunks in turn
+    uint8_t* const pw = patch + (warp - 2) * kPairPatch;
     const int rr = lane >> 3, cc = lane & 7;        // read-back: lane takes 16-byte piece cc of rows rr, rr + 4, …
     const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
     int i = 0;
@@ -183,8 +196,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       ok = __all_sync(0xffffffffu, mbar_wait_limited(&tmem_full[acc], (uint32_t)((i >> 1) & 1), p.err, kGemmWaitCode | 4));
       if (!ok) break;
       tc_fence_after();
+      const int n_end = min(p.N, n0 + OUT);
+      if (grp * CW >= OUT && lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty[acc]), 0));   // no chunk for this warp
 #pragma unroll 1
-      for (int c = 0; c < OUT; c += CW) {
+      for (int c = grp * CW; c < OUT; c += 2 * CW) {   // of a last chunk that reaches past the tile, what lies there is not stored
         if constexpr (EPI == GEPI_SILU) {           // 64 columns: gate at c, up at HB + c
           uint32_t g[32], u[32];
 #pragma unroll
@@ -237,14 +252,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           for (int j = 0; j < 8; ++j)
             *reinterpret_cast<uint4*>(pw + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
         }
-        if (c + CW >= OUT) {   // this warp holds the tile's last columns: the accumulator may be filled again
+        if (c + 2 * CW >= OUT) {   // this warp holds the tile's last columns: the accumulator may be filled again
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty[acc]), 0));
         }
         __syncwarp();
         const int col = n0 + c + cc * VW;
-        if (col < p.N) {       // N is a multiple of 8: a 16-byte piece lies inside the row or outside it
+        if (col < n_end) {     // N and the tile are multiples of 8: a 16-byte piece lies inside the row or outside it
           uint4 add[8];
           if constexpr (EPI == GEPI_RESIDUAL) {
 #pragma unroll
@@ -404,25 +419,26 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------------- MMA issuer
-    if (lane == 0 && half == 0) {
+    if (half == 0 && elect_one()) {
+      const uint32_t a0 = desc_lo(smem_u32(sA)), b0 = desc_lo(smem_u32(sB));
       int s = 0;
       uint32_t ph = 0;
+      bool ready = false;
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!(ok = mbar_wait_limited(&full[s], ph, p.err, kGemmWaitCode | 6))) break;
+        if (!ready && !(ok = mbar_wait_limited(&full[s], ph, p.err, kGemmWaitCode | 6))) break;
         tc_fence_after();
-        const uint32_t a_addr = smem_u32(sA + s * a_bytes), b_addr = smem_u32(sB + s * B_BYTES);
-#pragma unroll
-        for (int k = 0; k < kBK / 16; ++k) {   // 16 bf16 = 32 bytes further along K inside the 128-byte swizzle row
-          const uint32_t accumulate = (kb > kb0 || k > 0) ? 1u : 0u;
-          if constexpr (PAIR) umma_bf16_pair(tmem_base, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), kIdesc, accumulate);
-          else umma_bf16(tmem_base, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), kIdesc, accumulate);
-        }
-        if constexpr (PAIR) umma_commit_pair(&empty[s], (uint16_t)(3u << crank));
-        else umma_commit(&empty[s]);
+        const uint32_t a = a0 + s * (uint32_t)(a_bytes >> 4), b = b0 + s * (B_BYTES >> 4);
+        uint64_t* const done = &empty[s];
         if (++s == stages) {
           s = 0;
           ph ^= 1;
         }
+        ready = mbar_test(&full[s], ph);
+#pragma unroll
+        for (int k = 0; k < kBK / 16; ++k)   // 16 bf16 = 32 bytes further along K inside the 128-byte swizzle row
+          umma_lo<GROUP>(tmem_base, a + 2 * k, b + 2 * k, kIdesc, (kb > kb0 || k > 0) ? 1u : 0u);
+        if constexpr (PAIR) umma_commit_pair(done, (uint16_t)(3u << crank));
+        else umma_commit(done);
       }
       if (ok) {
         if constexpr (PAIR) umma_commit_pair(tmem_full, (uint16_t)(3u << crank));
@@ -593,7 +609,7 @@ int sm_pairs() {
 }
 
 template <typename OT, int EPI>
-int launch_pair(const GemmArgs<OT>& args, const void* A, const void* B, int64_t rows_b, cudaStream_t st) {
+int launch_pair(const GemmArgs<OT>& args, const void* A, const void* B, int64_t rows_b, int bn, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] { attr_err = cudaFuncSetAttribute(gemm_pair_kernel<OT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem); });
@@ -603,13 +619,13 @@ int launch_pair(const GemmArgs<OT>& args, const void* A, const void* B, int64_t 
   if ((rc = wait_word(&p.err)) != B200_OK) return rc;
   CUtensorMap ta, tb;
   if ((rc = make_tmap(&ta, A, p.M, p.K, 128)) != B200_OK) return rc;
-  if ((rc = make_tmap(&tb, B, rows_b, p.K, 128)) != B200_OK) return rc;
-  constexpr int OUT = EPI == GEPI_SILU ? kPairBN / 2 : kPairBN;
+  if ((rc = make_tmap(&tb, B, rows_b, p.K, bn / 2)) != B200_OK) return rc;
+  const int OUT = EPI == GEPI_SILU ? bn / 2 : bn;
   const int64_t tiles = (int64_t)((p.M + 255) / 256) * ((p.N + OUT - 1) / OUT);
   const int pairs = sm_pairs();
   B200_CHECK_ARG(pairs > 0 && tiles < (1ll << 30), "gemm: no device, or shape out of range");
   g_launches.fetch_add(1);
-  gemm_pair_kernel<OT, EPI><<<(unsigned)(2 * std::min<int64_t>(tiles, pairs)), kGemmThreads, kPairSmem, st>>>(ta, tb, p);
+  gemm_pair_kernel<OT, EPI><<<(unsigned)(2 * std::min<int64_t>(tiles, pairs)), kPairThreads, kPairSmem, st>>>(ta, tb, p, bn);
   B200_CUDA(cudaGetLastError());
   return B200_OK;
 }
@@ -675,22 +691,22 @@ int launch_split(const GemmArgs<OT>& args, const void* A, const void* B, int64_t
 constexpr int kSplitMinKb = 8;   // k-blocks that a split takes at least: shorter ones save less than their sum costs
 
 // Which kernel, by what each would take (µs): rounds of resident tiles × (k-blocks × the time of one + what a tile costs
-// besides).  The constants are fits to graph-timed launches over M = 16 … 2 048 and the (N, K) of the four model
-// configurations: a k-block is 0.29 µs for either tile, a pair's grows to 0.40 µs when
-// every SM runs several tiles (power); the rest is launch, pipeline fill and epilogue.  Measured, µs, M × N × K: 128 × 3 072 × 8 192
-// whole-K tiles 44, five splits 19; 16 × 896 × 4 864 27 → 9 (eight splits); 512 × 3 072 × 8 192 44 → 33 (pairs, two splits);
-// 2 048 × 12 288 × 2 048 persistent pairs 74, one-CTA tiles 174; 300 × 10 944 × 2 048, where 86 tiles are two rounds of pairs and 258 tiles two
-// of single CTAs, but 129 wide ones a single round: 26.0, 28.4, 20.3.  B200_GEMM = "persistent" | "tile" | "wide" forces the
+// besides).  The constants are fits to graph-timed launches over M = 17 … 2 048 and the (N, K) of the four model
+// configurations: a k-block is 0.205 µs on a 128 × 128 tile, 0.33 µs on a 128 × 256 one, 0.25 µs on a pair's, which grows to 0.39 µs when
+// every SM runs several tiles (power, L2); the rest is launch, pipeline fill and epilogue.  Measured, µs, M × N × K, one-CTA tiles / wide ones /
+// pairs / splits: 40 × 2 048 × 6 144 23.2 / 34.0 / 26.9 / 11.0; 128 × 16 384 × 3 072 22.3 / 27.3 / 24.7; 300 × 12 288 × 2 048, where 96 tiles are
+// two rounds of pairs and 288 two of single CTAs, but 144 wide ones a single round, 26.2 / 22.1 / 23.6; 2 048 × 2 048 × 2 048 21.6 / 16.2 / 17.0;
+// 2 048 × 12 288 × 2 048 123 / 108 / 71.  B200_GEMM = "persistent" (with a width: "persistent192") | "tile" | "wide" forces the
 // persistent pairs or one whole-K tile of 128 or 256 columns per CTA.  The products of a prompt pass (no split) find their weights in HBM and their epilogue
-// is not hidden when a pair has one tile: 6 … 8 µs on top of the fit, so pairs start later there (24-layer, 896-wide prompt of 300
-// rows, µs: pairs 3 366, tiles 2 400; 28-layer, 2 048-wide one of 800 rows: pairs 5 717, tiles 6 019).
+// is not hidden when a pair has one tile: 5 µs on top of the fit, so pairs start later there (ms a prompt, tiles / pairs / the choice: 24 layers,
+// 896 wide, 60 rows 1.76 / 2.31 / 1.75, 300 rows 2.15 / 2.67 / 2.05; 28 layers, 2 048 wide, 500 rows 3.68 / 4.03 / 3.59, 1 000 rows 5.62 / 4.84 / 4.56).
 struct GemmPick {
   int kind;     // 0: a CTA per tile (and split); 1: a pair per tile (and split); 2: persistent pairs; 3: a CTA per wide tile
   int splits;
+  int bn;       // kind 2: columns of a tile
 };
 // Without SPLIT the order in which a row's products are summed is the same whatever M is, so a prompt's rows have the same bits in one
-// pass, in portions and in a batch.  What that costs a layer-stack prompt against splits chosen by M (8 layers of 2 048, µs): 64 rows
-// 833 → 1 087, 300 rows 1 123 → 1 301, 2 048 rows none.
+// pass, in portions and in a batch.
 template <typename OT, int EPI, bool SPLIT>
 void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   constexpr int D = EPI == GEPI_SILU ? 2 : 1;
@@ -698,10 +714,10 @@ void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   const int pairs = std::max(1, sm_pairs());
   auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
   double best = 1e30;
-  auto consider = [&](int kind, int splits, double cost) {
+  auto consider = [&](int kind, int splits, double cost, int bn = 0) {
     if (cost < best) {
       best = cost;
-      *out = GemmPick{kind, splits};
+      *out = GemmPick{kind, splits, bn};
     }
   };
   // rows of tiles run over grid.y: up to 65 535 of them, 8.4 M rows; the persistent pairs take any number
@@ -711,27 +727,33 @@ void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   const bool tile = fits && forced == 't', wide = fits && forced == 'w', any_split = fits && !wide && forced != 'p';
   if (wide) consider(3, 1, 0.0);
   if (!tile) {
-    const int64_t rounds = up(up(M, 256) * up(N, 256 / D), pairs);
-    const double tile_us = (double)kb * (0.30 + 0.02 * (double)std::min<int64_t>(rounds - 1, 5));
-    const double epilogue = EPI == GEPI_SILU ? 13.0 : 0.0;   // of a 256 × 256 tile: longer than a short k range
-    consider(2, 1, (SPLIT ? 5.5 : 12.0) + (double)rounds * std::max(tile_us, epilogue) + epilogue);
+    const int only = forced == 'p' ? std::atoi(env + std::strcspn(env, "0123456789")) : 0;   // "persistent224": that width
+    for (int bn = kPairBN; bn >= 192; bn -= 32) {
+      if (only != 0 && bn != only) continue;
+      const int64_t t = up(M, 256) * up(N, bn / D), rounds = up(t, pairs);
+      const double block = 0.25 + 0.10 * std::min(1.0, (double)t / 64.0) + 0.02 * (double)std::min<int64_t>(rounds - 1, 2);
+      const double tile_us = (double)kb * block * std::max(0.79, (double)bn / kPairBN);
+      const double epilogue = EPI == GEPI_SILU ? 6.5 * bn / kPairBN : 0.0;   // longer than a short k range
+      consider(2, 1, (SPLIT ? 5.2 : 10.5) + (double)rounds * std::max(tile_us, epilogue) + epilogue, bn);
+    }
   }
   if (any_split && !tile) {
     const int64_t t = up(M, 128) * up(N, 256 / D);
-    consider(3, 1, (double)up(t, 2 * pairs) * (7.6 + (t >= 100 ? 0.44 : 0.36) * (double)kb + (EPI == GEPI_SILU ? 2.0 : 0.0)));
+    const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
+    consider(3, 1, (double)up(t, 2 * pairs) * (4.0 + 2.2 * rows + (t >= 100 ? 0.42 : 0.33) * (double)kb + (EPI == GEPI_SILU ? 2.0 : 0.0)));
   }
   if (any_split) {
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
     for (int s = 1; s <= (SPLIT && !tile ? 8 : 1) && (s == 1 || s * kSplitMinKb <= kb); ++s) {
       const int64_t t = up(M, 128) * up(N, 128 / D) * s;
-      if (s == 1) consider(0, s, (double)up(t, 2 * pairs) * (4.3 + rows * 0.8 + 0.295 * (double)kb + (EPI == GEPI_SILU ? 1.5 : 0.0)));
+      if (s == 1) consider(0, s, (double)up(t, 2 * pairs) * (3.6 + rows * 1.4 + 0.205 * (double)kb + (EPI == GEPI_SILU ? 1.5 : 0.0)));
       else if constexpr (SPLIT)
-        consider(0, s, (double)up(t, split_capacity<kSplit>(s)) * (5.0 + 0.15 * s + rows * (2.0 + 0.25 * s) + 0.29 * (double)up(kb, s)));
+        consider(0, s, (double)up(t, split_capacity<kSplit>(s)) * (5.0 + 0.15 * s + rows * (2.0 + 0.25 * s) + 0.23 * (double)up(kb, s)));
     }
     if constexpr (SPLIT) {
       for (int s = 1; s <= 4 && (s == 1 || s * kSplitMinKb <= kb) && M > 128 && !tile; ++s) {
         const int64_t t = up(M, 256) * up(N, 256) * 2 * s;
-        consider(1, s, (double)up(t, split_capacity<kSplitPair>(2 * s)) * (9.5 + 1.0 * s + 0.33 * (double)up(kb, s)));
+        consider(1, s, (double)up(t, split_capacity<kSplitPair>(2 * s)) * (9.5 + 1.0 * s + 0.30 * (double)up(kb, s)));
       }
     }
   }
@@ -747,7 +769,7 @@ int launch_gemm(const GemmArgs<OT>& p, const void* A, const void* B, int64_t row
     if (g.kind == 0) return launch_split<OT, EPI, kSplit>(p, A, B, rows_b, g.splits, st);
     if (g.kind == 1) return launch_split<OT, EPI, kSplitPair>(p, A, B, rows_b, g.splits, st);
   }
-  return launch_pair<OT, EPI>(p, A, B, rows_b, st);
+  return launch_pair<OT, EPI>(p, A, B, rows_b, g.bn, st);
 }
 
 int check_gemm(const void* C, const void* A, const void* B, int64_t M, int64_t N, int64_t K) {

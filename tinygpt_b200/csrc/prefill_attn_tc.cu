@@ -91,26 +91,12 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
-// Products whose operands are the same in the whole warp, issued where `one` is set.  D[tmem] (+)= A·B with A in shared memory or in TMEM
-__device__ __forceinline__ void umma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t a_hi, uint32_t b_hi, uint32_t idesc,
-                                        uint32_t accumulate, uint32_t one) {
+// D[tmem] (+)= A[tmem]·B[smem], B's descriptor by its lower half: the address and, from bit 16 on, the distance of 64-column blocks of an operand
+// whose N runs along the columns (V's [keys][64 columns] rows of 128 bytes, MN-major)
+__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\tmov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %4};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}"
-      ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(a_hi), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(one)
-      : "memory");
-}
-__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate, uint32_t one) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 b, {%2, %3};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
-      ::"r"(d), "r"(a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(one)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit_if(uint64_t* bar, uint32_t one) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(one)
+      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 b, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}" ::"r"(d), "r"(a), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -124,11 +110,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
       : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// Matrix descriptors in halves: the lower one holds the address (and, from bit 16 on, the distance of 64-column blocks of an operand whose N
-// runs along the columns: V's [keys][64 columns] rows of 128 bytes, MN-major), the upper one is the same for all (umma_desc)
-constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr) { return (smem_addr & 0x3FFFFu) >> 4; }
-
 // A wait that gave up says so to the whole CTA and sets `dead`: its role goes on without waiting (what follows neither hangs nor leaves
 // the buffers), and nothing is stored.  The first look is inline and has no loop around it.
 __device__ __noinline__ bool wait_slow(uint64_t* bar, uint32_t parity, unsigned* err, unsigned code, volatile int* gave_up) {
@@ -272,43 +253,40 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------------- MMA issuer
-    // The whole warp walks the loop and one thread's predicate issues: descriptors then live in uniform registers.
-    const uint32_t one = lane == 0;
-    const uint32_t q_u = desc_lo(smem_u32(sQ)), k_u = desc_lo(smem_u32(sK)), v_u = desc_lo(smem_u32(sV));
-    auto scores = [&](int it) {   // S[it & 1] = Q·Kᵀ of tile it
-      const int s = it % ST;
-      wait_for(&k_full[s], (uint32_t)((it / ST) & 1), kAttnWaitCode | 3);
-      __syncwarp();
-      tc_fence_after();
-      const uint32_t ks = k_u + s * (C::TB >> 4), d = tmem + (uint32_t)((it & 1) * 64);
+    if (n_tiles > 0 && elect_one()) {
+      const uint32_t q_u = desc_lo(smem_u32(sQ)), k_u = desc_lo(smem_u32(sK)), v_u = desc_lo(smem_u32(sV));
+      bool k_ready = false;   // of the tile after the next, looked at before the products of this one go out
+      auto scores = [&](int it) {   // S[it & 1] = Q·Kᵀ of tile it
+        const int s = it % ST;
+        if (!k_ready) wait_for(&k_full[s], (uint32_t)((it / ST) & 1), kAttnWaitCode | 3);
+        tc_fence_after();
+        const uint32_t ks = k_u + s * (C::TB >> 4), d = tmem + (uint32_t)((it & 1) * 64);
 #pragma unroll
-      for (int kk = 0; kk < HD / 16; ++kk)
-        umma_ss(d, q_u + (((kk / 4) * kTBM * 128 + (kk % 4) * 32) >> 4), ks + (((kk / 4) * kTBN * 128 + (kk % 4) * 32) >> 4), kDescHi, kDescHi,
-                kIdescS, kk > 0 ? 1u : 0u, one);
-      umma_commit_if(&k_empty[s], one);
-      umma_commit_if(&s_full[it & 1], one);
-    };
-    if (n_tiles > 0) {
+        for (int kk = 0; kk < HD / 16; ++kk)
+          umma_lo<1>(d, q_u + (((kk / 4) * kTBM * 128 + (kk % 4) * 32) >> 4), ks + (((kk / 4) * kTBN * 128 + (kk % 4) * 32) >> 4), kIdescS,
+                     kk > 0 ? 1u : 0u);
+        umma_commit(&k_empty[s]);
+        umma_commit(&s_full[it & 1]);
+      };
       wait_for(q_full, 0, kAttnWaitCode | 4);
       scores(0);
-    }
-    for (int it = 0; it < n_tiles; ++it) {
-      // the buffer that tile it + 1 overwrites held P of tile it - 1: its product went out before, and products run in order
-      if (it + 1 < n_tiles) scores(it + 1);
-      const int s = it % ST;
-      wait_for(&v_full[s], (uint32_t)((it / ST) & 1), kAttnWaitCode | 6);
-      wait_for(&p_full[it & 1], (uint32_t)((it >> 1) & 1), kAttnWaitCode | 5);
-      __syncwarp();
-      tc_fence_after();
-      const uint32_t vs = v_u + s * (C::TB >> 4), ps = tmem + (uint32_t)((it & 1) * 64);
+      for (int it = 0; it < n_tiles; ++it) {
+        // the buffer that tile it + 1 overwrites held P of tile it - 1: its product went out before, and products run in order
+        if (it + 1 < n_tiles) scores(it + 1);
+        const int s = it % ST, next = it + 2;
+        wait_for(&v_full[s], (uint32_t)((it / ST) & 1), kAttnWaitCode | 6);
+        wait_for(&p_full[it & 1], (uint32_t)((it >> 1) & 1), kAttnWaitCode | 5);
+        tc_fence_after();
+        k_ready = mbar_test(&k_full[next % ST], (uint32_t)((next / ST) & 1));
+        const uint32_t vs = v_u + s * (C::TB >> 4), ps = tmem + (uint32_t)((it & 1) * 64);
 #pragma unroll
-      for (int kk = 0; kk < kTBN / 16; ++kk)   // 16 keys: 8 columns of P, 2 048 bytes further down V's rows
-        umma_ts(tmem + kColO, ps + kk * 8, vs + (kk * 2048 >> 4) + ((kTBN * 128 >> 4) << 16), kDescHi, kIdescO,
-                (it > 0 || kk > 0) ? 1u : 0u, one);
-      umma_commit_if(&v_empty[s], one);
-      umma_commit_if(it + 1 < n_tiles ? pv_done : o_full, one);
+        for (int kk = 0; kk < kTBN / 16; ++kk)   // 16 keys: 8 columns of P, 2 048 bytes further down V's rows
+          umma_ts(tmem + kColO, ps + kk * 8, vs + (kk * 2048 >> 4) + ((kTBN * 128 >> 4) << 16), kIdescO, (it > 0 || kk > 0) ? 1u : 0u);
+        umma_commit(&v_empty[s]);
+        umma_commit(it + 1 < n_tiles ? pv_done : o_full);
+      }
+      if (dead) drain_async();
     }
-    if (dead) drain_async();
   } else {
     // ---------------------------------------------------------------------------------------------- softmax
     const int q = warp & 3, row = q * 32 + lane;
