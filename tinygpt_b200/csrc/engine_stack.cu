@@ -181,15 +181,19 @@ constexpr int kGemmRows = 32;
 
 namespace {
 
-// rows of a [B, S] id matrix (columns s0 … s0+cs) → the step's row list; positions continue each slot's cache
+// rows of a [B, S] id matrix (columns s0 … s0+cs) → the step's row list; positions continue each slot's cache.  Wanted rows: every one (all), then
+// the B last ones (last)
 __global__ void stack_meta_from_ids_kernel(const int64_t* __restrict__ ids, int B, int S, int s0, int cs,
-                                           const int* __restrict__ pos_dev, int32_t* tok, int32_t* slot, int32_t* pos) {
+                                           const int* __restrict__ pos_dev, int32_t* tok, int32_t* slot, int32_t* pos, int32_t* want,
+                                           int all, int last) {
   const int n = B * cs;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const int b = e / cs, t = e % cs;
     tok[e] = (int32_t)ids[(int64_t)b * S + s0 + t];
     slot[e] = b;
     pos[e] = pos_dev[b] + s0 + t;
+    if (all) want[e] = e;
+    if (last && t == cs - 1) want[(all ? n : 0) + b] = e;
   }
 }
 // one decode token per active row: the slot's current token at the slot's position, which then advances
@@ -210,14 +214,6 @@ __global__ void stack_meta_decode_kernel(const int* __restrict__ row_slot, int r
 __global__ void stack_set_pos_kernel(const int32_t* __restrict__ upd, int n, int* pos_dev) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) pos_dev[upd[2 * i]] = upd[2 * i + 1];
-}
-__global__ void stack_iota_last_kernel(int32_t* want, int B, int cs) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < B) want[b] = b * cs + cs - 1;
-}
-__global__ void stack_iota_kernel(int32_t* want, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) want[i] = i;
 }
 
 }  // namespace
@@ -1383,17 +1379,11 @@ int stack_forward(b200_engine* e, const int64_t* ids, int64_t B, int64_t S, void
     const int n_tok = cs * (int)B;
     const bool last = s0 + cs == S;
     B200_CUDA(launch_pdl(stack_meta_from_ids_kernel, dim3((n_tok + 255) / 256), dim3(256), 0, st, false, ids, (int)B, (int)S,
-                         (int)s0, cs, (const int*)s->pos_dev, s->m_tok, s->m_slot, s->m_pos));
+                         (int)s0, cs, (const int*)s->pos_dev, s->m_tok, s->m_slot, s->m_pos, s->m_want, (int)all, (int)last));
     // rows: every token of the chunk when all positions are asked for, then (last chunk) the B last positions
-    int n_rows = 0;
-    if (all) {
-      n_rows = n_tok;
-      B200_CUDA(launch_pdl(stack_iota_kernel, dim3((n_tok + 255) / 256), dim3(256), 0, st, false, s->m_want, n_tok));
-    }
+    int n_rows = all ? n_tok : 0;
     if (last) {
       head_row0 = n_rows;
-      B200_CUDA(launch_pdl(stack_iota_last_kernel, dim3(((int)B + 63) / 64), dim3(64), 0, st, false, s->m_want + n_rows,
-                           (int)B, cs));
       n_rows += (int)B;
     }
     s->segs.clear();

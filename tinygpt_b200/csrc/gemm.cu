@@ -722,6 +722,7 @@ void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   };
   // rows of tiles run over grid.y: up to 65 535 of them, 8.4 M rows; the persistent pairs take any number
   const bool fits = up(M, 128) <= 65535;
+  const double f32_us = sizeof(OT) == 4 ? 2.5 : 0.0;   // 128 columns of fp32 results, a row per thread (2 049 × 2 048 × 2 048 logits: wide 24.9, pairs 22.1)
   const char* env = std::getenv("B200_GEMM");   // looked up once: routed experts' products wait for the host
   const char forced = env != nullptr ? env[0] : 0;
   const bool tile = fits && forced == 't', wide = fits && forced == 'w', any_split = fits && !wide && forced != 'p';
@@ -740,13 +741,13 @@ void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   if (any_split && !tile) {
     const int64_t t = up(M, 128) * up(N, 256 / D);
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
-    consider(3, 1, (double)up(t, 2 * pairs) * (4.0 + 2.2 * rows + (t >= 100 ? 0.42 : 0.33) * (double)kb + (EPI == GEPI_SILU ? 2.0 : 0.0)));
+    consider(3, 1, (double)up(t, 2 * pairs) * (4.0 + 2.2 * rows + (t >= 100 ? 0.42 : 0.33) * (double)kb + (EPI == GEPI_SILU ? 2.0 : f32_us * 2)));
   }
   if (any_split) {
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
     for (int s = 1; s <= (SPLIT && !tile ? 8 : 1) && (s == 1 || s * kSplitMinKb <= kb); ++s) {
       const int64_t t = up(M, 128) * up(N, 128 / D) * s;
-      if (s == 1) consider(0, s, (double)up(t, 2 * pairs) * (3.6 + rows * 1.4 + 0.205 * (double)kb + (EPI == GEPI_SILU ? 1.5 : 0.0)));
+      if (s == 1) consider(0, s, (double)up(t, 2 * pairs) * (3.6 + rows * 1.4 + 0.205 * (double)kb + (EPI == GEPI_SILU ? 1.5 : f32_us)));
       else if constexpr (SPLIT)
         consider(0, s, (double)up(t, split_capacity<kSplit>(s)) * (5.0 + 0.15 * s + rows * (2.0 + 0.25 * s) + 0.23 * (double)up(kb, s)));
     }

