@@ -1,0 +1,97 @@
+"""Operators launched beside the end of the one in front (programmatic dependent launch): what each reads was written by the operator, or the torch
+kernel, right before it — activations, weights, caches and positions alike.  Against the same calls with a synchronisation between, bit for bit."""
+import pytest
+import torch
+
+from tinygpt_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def maker(seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return lambda *s, k=1.0: (torch.randn(*s, generator=g, device="cuda") * k).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 7, 16, 40, 130, 300, 1000])
+def test_chain_of_operators(built_lib, rows):
+    r = maker(3)
+    x0 = r(rows, 512)
+    layers = [(r(2048, 512, k=.04), r(512, 1024, k=.03), r(512, k=.1) + 1, r(512, 512, k=.04)) for _ in range(4)]
+    kc, vc = r(1, 700, 2, 64), r(1, 700, 2, 64)
+
+    def chain(sync):
+        def s(t):
+            if sync:
+                torch.cuda.synchronize()
+            return t
+        x = x0
+        for w1, w2, n, wq in layers:
+            h = s(ops.rms_norm(x, n, 1e-6))
+            h = s(ops.gemm(h, w1)) if rows > 8 else s(ops.linear(h, w1))
+            x = s(ops.add(x, s(ops.linear(s(ops.silu_mul(h)), w2))))
+            q = s(ops.linear(x, wq)).view(1, rows, 8, 64)
+            x = s(ops.add(x, s(ops.flash_attention(q, q[:, :, :4], q[:, :, 4:], True)).view(rows, -1)))
+            if rows == 1:
+                y = s(ops.gemv_fused(x.view(-1), w1, norm_weight=n, eps=1e-6, silu_mul=True))
+                x = s(ops.gemv_fused(y, w2, residual=x.view(-1))).view(1, -1)
+                x = s(ops.add(x, s(ops.flash_attention(x.view(1, 1, 8, 64), kc, vc)).view(1, -1)))
+        return x
+
+    want = chain(True)
+    assert bool(torch.isfinite(want.float()).all())
+    for _ in range(20):
+        assert torch.equal(chain(False), want)
+
+
+def test_weights_that_were_just_written(built_lib):
+    r = maker(4)
+    for rows in (1, 8, 300):
+        w, x = r(1152, 896), r(rows, 896)
+        want = ops.linear(x, w + w), ops.linear(x, w)
+        torch.cuda.synchronize()
+        for _ in range(30):
+            w2 = ops.add(w, w)               # an operator in front
+            a = ops.linear(x, w2)
+            w2.mul_(0.5)                     # a torch kernel in front
+            assert torch.equal(a, want[0]) and torch.equal(ops.linear(x, w2), want[1])
+
+
+@pytest.mark.parametrize("ctx", [512, 2304])
+def test_decode_steps_behind_each_other(built_lib, ctx):
+    """Each step appends the row that the next one reads, at a position written right before it."""
+    r = maker(5)
+    kc, vc, qkv = r(ctx, 2, 64), r(ctx, 2, 64), r(10 * 64)
+
+    def steps(sync):
+        k, v, out, x = kc.clone(), vc.clone(), [], qkv
+        for t in range(30):
+            pos = torch.tensor([200 + t], dtype=torch.int32, device="cuda")
+            x = ops.add(x, qkv) if t % 2 else qkv
+            if sync:
+                torch.cuda.synchronize()
+            out.append(ops.attn_decode(x, k, v, q_heads=6, kv_heads=2, head_dim=64, pos=pos))
+        return torch.stack(out), k, v
+
+    want = steps(True)
+    for _ in range(10):
+        assert all(torch.equal(a, b) for a, b in zip(steps(False), want))
+
+
+def test_captured_operators_have_plain_edges(built_lib):
+    """A captured graph ends with the operators' own kernels: what is enqueued behind its launch sees their results."""
+    r = maker(6)
+    x, w = r(8, 2048), r(4096, 2048, k=.02)
+    want = ops.linear(x, w)
+    st = torch.cuda.Stream()
+    st.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(st):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            y = ops.linear(ops.add(x, x), w)
+        for i in range(50):
+            y.zero_()
+            graph.replay()
+            assert torch.equal(y.clone(), ops.linear(x + x, w)), i
+    torch.cuda.synchronize()
+    assert torch.equal(ops.linear(x, w), want)

@@ -50,6 +50,8 @@ int b200_gemv_bf16(void* y, const void* x, const void* W, const void* bias, int6
   GemvPlan plan;
   if ((rc = gemv_make_plan(&plan, W, n, n, k, 1, PRO_PLAIN, EPI_PLAIN, num_sms_cached())) != B200_OK) return rc;
   plan.p.bias = (const __nv_bfloat16*)bias;
+  plan.p.late = 1;
+  const bool pdl = op_pdl((cudaStream_t)stream);
   // Up to eight rows share one pass over W (tensor-core GEMV): 8 rows × 4 096 × 2 048 32.6 µs as eight launches, 5.9 µs as one.  Rows too
   // long for two activation vectors beside the ring go one by one.
   int64_t r = 0;
@@ -61,13 +63,13 @@ int b200_gemv_bf16(void* y, const void* x, const void* W, const void* bias, int6
     if (batch.sub > 0 && gemm) return rest_as_gemm(r);   // two launches would stream W twice (8 × 4 096 × 14 336: 46 µs, GEMM 25 µs)
     batch.p.x = (const __nv_bfloat16*)x + r * k;
     batch.p.y = (__nv_bfloat16*)y + r * n;
-    if ((rc = gemv_launch(batch, (cudaStream_t)stream, false)) != B200_OK) return rc;
+    if ((rc = gemv_launch(batch, (cudaStream_t)stream, pdl)) != B200_OK) return rc;
     r += rows;
   }
   for (; r < m; ++r) {
     plan.p.x = (const __nv_bfloat16*)x + r * k;
     plan.p.y = (__nv_bfloat16*)y + r * n;
-    if ((rc = gemv_launch(plan, (cudaStream_t)stream, false)) != B200_OK) return rc;
+    if ((rc = gemv_launch(plan, (cudaStream_t)stream, pdl)) != B200_OK) return rc;
   }
   return B200_OK;
 }
@@ -97,7 +99,8 @@ int b200_gemv_fused_bf16(void* y, const void* x, const void* W, int64_t n, int64
   plan.p.bias = (const __nv_bfloat16*)bias;
   plan.p.residual = (const __nv_bfloat16*)residual;
   plan.p.y = (__nv_bfloat16*)y;
-  return gemv_launch(plan, (cudaStream_t)stream, false);
+  plan.p.late = 1;
+  return gemv_launch(plan, (cudaStream_t)stream, op_pdl((cudaStream_t)stream));
 }
 
 int64_t b200_attn_decode_workspace_bytes(int64_t Hq, int64_t Hkv, int64_t hd, int64_t max_ctx) {
@@ -133,7 +136,8 @@ int b200_attn_decode_bf16(void* out, const void* qkv, const void* q_norm, const 
   a.Hkv = (int)Hkv;
   a.nsplit = attn_decode_nsplit((int)hd, (int)max_ctx);
   a.max_ctx = (int)max_ctx;
-  return launch_attn_decode(a, (int)hd, (cudaStream_t)stream, false);
+  a.late = 1;
+  return launch_attn_decode(a, (int)hd, (cudaStream_t)stream, op_pdl((cudaStream_t)stream));
 }
 
 }  // extern "C"

@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_reg_kernel(const Att
   const bool kv_leader = (h0 % group) == 0;
   if (p.trace != nullptr && hg == 0 && split == 0 && blockIdx.z == 0 && tid == 0) p.trace[0] = global_timer_ns();
   pdl_trigger();
+  if (p.late) pdl_wait();
   const bool append = (p.pos != nullptr);
   const int pos = append ? *p.pos : p.fixed_len - 1;   // stable since before the producer kernel started (engine.cu)
   const int L = pos + 1;
@@ -350,7 +351,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_row_kernel(const AttnRow
   const long long b = blockIdx.z;
   const int rank = (int)cluster_rank(), splits = 1 << a.log_splits;
   row_stamp<DECODE>(p, 0);
-  if (DECODE) pdl_trigger();
+  pdl_trigger();
+  if (!DECODE || p.late) pdl_wait();
   cluster_arrive_relaxed();                // this CTA runs: the others may write to it once they have waited for that
   const bool append = DECODE && p.pos != nullptr;
   const int pos = append ? *p.pos : p.fixed_len - 1;   // where q is rotated; stable since before the producer kernel started
@@ -785,7 +787,7 @@ static int launch_attn_row(void* o, const void* q, const void* k, const void* v,
   a.d.qkv_bstride = a.d.out_bstride = Hq * hd;
   a.kv_bstride = Skv * Hkv * hd;
   a.nkeys = causal ? 1 : (int)Skv;   // causal: the mask is top-left aligned, row 0 sees key 0
-  return launch_row(a, (int)hd, a.nkeys, (int)B, false, st, false);
+  return launch_row(a, (int)hd, a.nkeys, (int)B, false, st, op_pdl(st));
 }
 
 int launch_attn_decode(const AttnDecodeParams& p, int hd, cudaStream_t st, bool pdl) {

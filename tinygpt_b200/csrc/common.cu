@@ -168,6 +168,15 @@ int op_wait_check() {
   return w == nullptr || *(volatile unsigned*)w == 0 ? B200_OK : report_wait(__atomic_exchange_n(w, 0u, __ATOMIC_ACQ_REL));
 }
 
+bool op_pdl(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {   // the legacy stream beside a capture
+    (void)cudaGetLastError();
+    return false;
+  }
+  return s == cudaStreamCaptureStatusNone;
+}
+
 int op_check() {
   const int rc = b200_device_check();
   return rc != B200_OK ? rc : op_wait_check();

@@ -50,7 +50,10 @@ extern std::atomic<int64_t> g_launches;
 
 // Kernel launch through cudaLaunchKernelEx with the programmatic-dependent-launch attribute (PDL): the kernel may
 // start while its predecessor on the stream is still running and must call pdl_wait() before touching anything the
-// predecessor writes.  Weight prefetch (TMA into shared memory) is issued BEFORE pdl_wait().
+// predecessor writes.  Weight prefetch (TMA into shared memory) is issued BEFORE pdl_wait() by the engines' launches.  A stand-alone operator's
+// operands may all come from the kernel in front: it waits before it reads any (the kernels' `late`), and only its launch, barriers, tensor
+// memory and descriptors run beside that kernel's end.
+bool op_pdl(cudaStream_t st);   // whether an operator may be launched so: not while the stream is captured (see engine_launch_token's note)
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                               bool pdl, Args&&... args) {

@@ -56,6 +56,7 @@ struct GemmArgs {
   unsigned* err;
   float mult = 0.f;
   __nv_bfloat16* c2 = nullptr;
+  int pdl = 0;                   // 1: launched beside the end of the kernel in front, whose end it waits for
 };
 __device__ __forceinline__ float cap_logit(float v, float cap) { return cap > 0.f ? cap * tanhf(v / cap) : v; }
 
@@ -108,6 +109,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const int kblocks = (p.K + kBK - 1) / kBK;
   bool ok = true;
 
+  if (p.pdl) pdl_trigger();
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
@@ -127,6 +129,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   cluster_sync_all();   // the pair's barriers exist
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (p.pdl) pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------------------------------------ TMA producer
@@ -371,6 +374,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int valid = max(0, min(128, p.M - m0));             // rows of this CTA that exist
   bool ok = true;
 
+  if (p.pdl) pdl_trigger();
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
@@ -388,6 +392,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   if constexpr (PAIR) cluster_sync_all();   // the pair's barriers exist
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (p.pdl) pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------------------------------------ TMA producer
@@ -624,9 +629,7 @@ int launch_pair(const GemmArgs<OT>& args, const void* A, const void* B, int64_t 
   const int64_t tiles = (int64_t)((p.M + 255) / 256) * ((p.N + OUT - 1) / OUT);
   const int pairs = sm_pairs();
   B200_CHECK_ARG(pairs > 0 && tiles < (1ll << 30), "gemm: no device, or shape out of range");
-  g_launches.fetch_add(1);
-  gemm_pair_kernel<OT, EPI><<<(unsigned)(2 * std::min<int64_t>(tiles, pairs)), kPairThreads, kPairSmem, st>>>(ta, tb, p, bn);
-  B200_CUDA(cudaGetLastError());
+  B200_CUDA(launch_pdl(gemm_pair_kernel<OT, EPI>, dim3((unsigned)(2 * std::min<int64_t>(tiles, pairs))), dim3(kPairThreads), kPairSmem, st, p.pdl != 0, ta, tb, p, bn));
   return B200_OK;
 }
 
@@ -641,8 +644,8 @@ int split_setup() {
 
 struct ClusterLaunch {
   cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute attr[1];
-  ClusterLaunch(dim3 grid, unsigned cluster, cudaStream_t st) {
+  cudaLaunchAttribute attr[2];
+  ClusterLaunch(dim3 grid, unsigned cluster, cudaStream_t st, bool pdl = false) {
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kGemmThreads);
     cfg.dynamicSmemBytes = kSplitSmem;
@@ -650,8 +653,10 @@ struct ClusterLaunch {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = cluster;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = cluster > 1 ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = cluster > 1 ? attr : attr + 1;
+    cfg.numAttrs = (cluster > 1 ? 1 : 0) + (pdl ? 1 : 0);
   }
 };
 
@@ -682,7 +687,7 @@ int launch_split(const GemmArgs<OT>& args, const void* A, const void* B, int64_t
   CUtensorMap ta, tb;
   if ((rc = make_tmap(&ta, A, p.M, p.K, box_rows)) != B200_OK) return rc;
   if ((rc = make_tmap(&tb, B, rows_b, p.K, EPI == GEPI_SILU ? BN / 2 : BN / W)) != B200_OK) return rc;
-  ClusterLaunch l(dim3((unsigned)((p.N + OUT - 1) / OUT * splits * W), (unsigned)((p.M + 128 * W - 1) / (128 * W))), (unsigned)(splits * W), st);
+  ClusterLaunch l(dim3((unsigned)((p.N + OUT - 1) / OUT * splits * W), (unsigned)((p.M + 128 * W - 1) / (128 * W))), (unsigned)(splits * W), st, p.pdl != 0);
   g_launches.fetch_add(1);
   B200_CUDA(cudaLaunchKernelEx(&l.cfg, gemm_split_kernel<OT, EPI, FORM>, ta, tb, (const GemmArgs<OT>)p, splits, box_rows));
   return B200_OK;
@@ -814,7 +819,8 @@ int launch_linear_split_bf16(void* C, const void* A, const void* B, int64_t M, i
   int rc = check_gemm(C, A, B, M, N, K);
   if (rc != B200_OK) return rc;
   B200_CHECK_ARG(aligned16(bias), "linear: bias must be 16-byte aligned");
-  const GemmArgs<__nv_bfloat16> p{(__nv_bfloat16*)C, nullptr, (const __nv_bfloat16*)bias, (int)M, (int)N, (int)K, nullptr};
+  GemmArgs<__nv_bfloat16> p{(__nv_bfloat16*)C, nullptr, (const __nv_bfloat16*)bias, (int)M, (int)N, (int)K, nullptr};
+  p.pdl = op_pdl(st);
   return bias != nullptr ? launch_gemm<__nv_bfloat16, GEPI_BIAS, true>(p, A, B, N, st) : launch_gemm<__nv_bfloat16, GEPI_STORE, true>(p, A, B, N, st);
 }
 int launch_gemm_bf16_f32(float* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st) {

@@ -72,6 +72,7 @@ gemv_stream_kernel(const GemvParams p, const __grid_constant__ CUtensorMap tmap)
   }
   __syncthreads();
   pdl_trigger();  // dependents only prefetch weights before their own griddepcontrol.wait
+  if (p.late) pdl_wait();
 
   if (warp == kNW) {
     // ------------------------------------------------------------------ producer: one thread drives the TMA ring

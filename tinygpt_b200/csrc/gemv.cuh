@@ -66,6 +66,7 @@ struct GemvParams {
   int seg_rows;                   // row offset of segment 1 inside W (NSEG == 2: gate rows | up rows)
   int rowblocks;                  // ceil(n / (8 * RPW))
   int stages;                     // depth of the shared-memory ring
+  int late;                       // 1 (operators): nothing is read before the kernel in front has ended
   unsigned long long* trace;      // debug (B200_TRACE=1): CTA 0 stores globaltimer at entry / after the PDL wait / at exit
   int* pos_inc;                   // engine: when set, CTA 0 advances the token position after its last row block
   // ---- tensor-parallel exchange (peer-mapped windows over NVLink).  Low-latency protocol: every fp32 partial travels

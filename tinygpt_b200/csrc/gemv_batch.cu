@@ -79,6 +79,10 @@ gemv_batch_kernel(const GemvParams p, const __grid_constant__ CUtensorMap tmap) 
   const int my_rbs = (p.rowblocks - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
   if (p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0) p.trace[0] = global_timer_ns();   // B200_TRACE=1
+  if (p.late) {
+    pdl_trigger();
+    pdl_wait();
+  }
   // The RMSNorm weight does not depend on the producer kernel: its loads (k ≤ 4096 stays in registers) are issued
   // first, before the dependency wait (like gemv_stream_kernel).
   constexpr int kMaxHoist = 2;

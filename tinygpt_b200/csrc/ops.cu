@@ -452,7 +452,7 @@ int launch_argmax(int64_t* idx, const void* logits, int64_t rows, int64_t V, voi
 extern "C" {
 
 int b200_rmsnorm_bf16(void* y, const void* x, const void* w, int64_t rows, int64_t dim, float eps, void* stream) {
-  return b200::launch_rmsnorm(y, x, w, rows, dim, eps, (cudaStream_t)stream, false);
+  return b200::launch_rmsnorm(y, x, w, rows, dim, eps, (cudaStream_t)stream, b200::op_pdl((cudaStream_t)stream));
 }
 
 int b200_rope_bf16(void* y, const void* x, const float* table, int64_t B, int64_t S, int64_t heads, int64_t hd,
@@ -477,11 +477,11 @@ int b200_rope_init_f32(float* table, int64_t hd, int64_t ctx, float theta, float
 }
 
 int b200_silu_mul_bf16(void* y, const void* gate_up, int64_t rows, int64_t I, void* stream) {
-  return b200::launch_silu_mul(y, gate_up, rows, I, (cudaStream_t)stream, false);
+  return b200::launch_silu_mul(y, gate_up, rows, I, (cudaStream_t)stream, b200::op_pdl((cudaStream_t)stream));
 }
 
 int b200_add_bf16(void* y, const void* a, const void* b, int64_t n, void* stream) {
-  return b200::launch_add(y, a, b, n, (cudaStream_t)stream, false);
+  return b200::launch_add(y, a, b, n, (cudaStream_t)stream, b200::op_pdl((cudaStream_t)stream));
 }
 
 int b200_embedding_bf16(void* y, const void* table, const int64_t* ids, int64_t n_ids, int64_t V, int64_t H,

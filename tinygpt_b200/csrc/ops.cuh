@@ -88,6 +88,7 @@ struct TcPrefillAttn {
   int B, S, Hq, Hkv, p0;
   float scale_log2;             // score scale × log2(e)
   int window, keep_first, sink;
+  int pdl;                      // 1: launched beside the end of the kernel in front, whose end it waits for
 };
 bool prefill_attn_tc_ok(const TcPrefillAttn& a, int hd);     // head size, alignment and strides it takes
 bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd, int rows);   // for a prompt of so many rows, against launch_pf's mma.sync kernel
@@ -115,6 +116,7 @@ struct AttnDecodeParams {
   __nv_bfloat16* out;            // [Hq*hd]
   float* ws;                     // split partials: [Hq / G][nsplit][G][hd + 2] floats (G = query heads per CTA)
   unsigned int* tickets;         // [Hq], zero-initialised, self-resetting
+  int late;                      // 1 (operators): nothing is read before the kernel in front has ended
   int heads_per_cta;             // 0 = choose from max_ctx (attn_heads_per_cta)
   unsigned long long* trace;     // debug timestamps (see GemvParams::trace)
   int Hq, Hkv, nsplit, max_ctx;  // nsplit = attn_decode_nsplit(hd, max_ctx): fixed 256 (hd 64) / 128 (hd 128) keys per split

@@ -83,6 +83,7 @@ struct PrefillAttnParams {
   float scale, cap;
   const float* slopes;
   int same;                     // SCORE kernels: the values are the keys (v == k): one tile serves both
+  int pdl;                      // 1: launched beside the end of the kernel in front, whose end it waits for
 };
 
 // bytes of a tile row in shared memory: whole groups of eight 16-byte chunks
@@ -142,6 +143,10 @@ __global__ void __launch_bounds__(kPfThreads, HD == 64 ? 3 : 1) attn_prefill_mma
   const bool same = SCORE && p.same != 0;
   const float slope = SCORE && p.slopes != nullptr ? p.slopes[blockIdx.x % p.Hq] : 0.f;
 
+  if (p.pdl) {
+    pdl_trigger();
+    pdl_wait();
+  }
   extern __shared__ __align__(128) uint8_t pf_smem[];
   uint8_t* const Qs = pf_smem;                       // [kBM][HD]
   uint8_t* const Ks = Qs + kBM * row_bytes<HD>();    // [2][kBN][HD]
@@ -354,7 +359,7 @@ template <int HD, bool SCORE = false>
 int launch_pf(const PrefillAttnParams& p, int B, cudaStream_t st, int tc_rows) {
   if constexpr (!SCORE && HD != 96) {
     const TcPrefillAttn t{p.o, p.q, p.k, p.v, p.gate, p.o_rs, p.o_bs, p.q_rs, p.q_bs, p.kv_rs, p.kv_bs, B, p.S, p.Hq, p.Hkv, p.p0,
-                          p.scale_log2, p.window, p.keep_first, p.sink};
+                          p.scale_log2, p.window, p.keep_first, p.sink, p.pdl};
     // "tc" | "mma" forces a side
     if (tc_rows > 0 && prefill_attn_tc_ok(t, HD) && env_choice("B200_ATTN_TC", 't', prefill_attn_tc_wins(t, HD, tc_rows)))
       return launch_prefill_attn_tc(t, HD, tc_rows, st);
@@ -368,9 +373,7 @@ int launch_pf(const PrefillAttnParams& p, int B, cudaStream_t st, int tc_rows) {
   });
   B200_CUDA(attr_err);
   dim3 grid((unsigned)((p.S + kBM - 1) / kBM) * (unsigned)p.Hq, (unsigned)B);
-  g_launches.fetch_add(1);
-  attn_prefill_mma_kernel<HD, SCORE><<<grid, kPfThreads, smem, st>>>(p);
-  B200_CUDA(cudaGetLastError());
+  B200_CUDA(launch_pdl(attn_prefill_mma_kernel<HD, SCORE>, grid, dim3(kPfThreads), (size_t)smem, st, p.pdl != 0, p));
   return B200_OK;
 }
 
@@ -465,6 +468,7 @@ int launch_attn_causal_mma(void* o, const void* q, const void* k, const void* v,
   p.Hq = (int)Hq;
   p.Hkv = (int)Hkv;
   p.p0 = 0;
+  p.pdl = op_pdl(st);
   p.scale_log2 = hd == 64 ? PfScale<64>::value : PfScale<128>::value;
   return hd == 64 ? launch_pf<64>(p, (int)B, st, (int)S) : launch_pf<128>(p, (int)B, st, (int)S);
 }
