@@ -177,6 +177,11 @@ bool op_pdl(cudaStream_t st) {
   return s == cudaStreamCaptureStatusNone;
 }
 
+static thread_local bool t_pdl = false;
+PdlScope::PdlScope(bool on) : outer(t_pdl) { t_pdl = on; }
+PdlScope::~PdlScope() { t_pdl = outer; }
+bool pdl_scope() { return t_pdl; }
+
 int op_check() {
   const int rc = b200_device_check();
   return rc != B200_OK ? rc : op_wait_check();

@@ -233,6 +233,15 @@ int op_wait_word(unsigned** out);
 int op_wait_check();                         // the operators': reports and clears
 int op_check();                              // what a stand-alone operator asks first: b200_device_check, then op_wait_check
 int wait_word(unsigned** out);               // the word for a launch on this thread
+// A prompt pass of an engine, whose GEMMs, norms, rotations and attentions of this thread are launched beside the end of the kernel in front
+struct PdlScope {
+  bool outer;
+  explicit PdlScope(bool on);
+  ~PdlScope();
+  PdlScope(const PdlScope&) = delete;
+  PdlScope& operator=(const PdlScope&) = delete;
+};
+bool pdl_scope();
 struct WaitScope {                           // launches of this thread write to `word`
   unsigned* outer;
   explicit WaitScope(unsigned* word);

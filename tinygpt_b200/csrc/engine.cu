@@ -713,10 +713,12 @@ static int prefill_chunk(b200_engine* e, const int64_t* ids, int S, int p0, bool
   const int H = d.hidden, nqkv = e->qdim + 2 * e->kvdim;
   const size_t kv_layer = (size_t)d.max_ctx * e->Hkv_l * d.head_dim;
   int rc;
+  const bool pdl = e->use_pdl && op_pdl(st);
+  const PdlScope overlap(pdl);
   if ((rc = launch_embedding(e->pf_x, e->embed, ids, S, d.vocab, H, st, false)) != B200_OK) return rc;
   for (int l = 0; l < d.layers; ++l) {
     const b200_layer_weights& lw = e->lw[l];
-    if ((rc = launch_rmsnorm(e->pf_h, e->pf_x, lw.input_norm, S, H, d.rms_eps, st, false)) != B200_OK) return rc;
+    if ((rc = launch_rmsnorm(e->pf_h, e->pf_x, lw.input_norm, S, H, d.rms_eps, st, pdl)) != B200_OK) return rc;
     // a bias that is not 16-byte aligned (a caller's own view) cannot ride on the store
     const bool bias_tail = d.qkv_bias && aligned16(lw.qkv_b);
     if ((rc = launch_linear_bf16(e->pf_qkv, e->pf_h, lw.qkv_w, S, nqkv, H, bias_tail ? LinearTail::bias : LinearTail::none,
@@ -731,7 +733,7 @@ static int prefill_chunk(b200_engine* e, const int64_t* ids, int S, int p0, bool
     if ((rc = launch_attn_prefill(e->pf_attn, e->pf_qkv, kc, vc, S, e->Hq_l, e->Hkv_l, d.head_dim, p0, st)) != B200_OK)
       return rc;
     if ((rc = launch_linear_bf16(e->pf_x, e->pf_attn, lw.o_w, S, H, e->qdim, LinearTail::residual, e->pf_x, st)) != B200_OK) return rc;
-    if ((rc = launch_rmsnorm(e->pf_h, e->pf_x, lw.post_norm, S, H, d.rms_eps, st, false)) != B200_OK) return rc;
+    if ((rc = launch_rmsnorm(e->pf_h, e->pf_x, lw.post_norm, S, H, d.rms_eps, st, pdl)) != B200_OK) return rc;
     if ((rc = launch_linear_bf16(e->pf_act, e->pf_h, lw.gate_up_w, S, e->I_l, H, LinearTail::silu_mul, nullptr, st)) != B200_OK) return rc;
     if ((rc = launch_linear_bf16(e->pf_x, e->pf_act, lw.down_w, S, H, e->I_l, LinearTail::residual, e->pf_x, st)) != B200_OK) return rc;
   }

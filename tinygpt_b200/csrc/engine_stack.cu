@@ -1180,6 +1180,7 @@ static int stack_run_hyper(StackEngine* s, int r, float* x, int n_tok, cudaStrea
 // One pass: n_tok rows {m_tok, m_slot, m_pos} through every run, then the head for the n_rows rows listed in m_want.
 // rows_in_order: m_want is 0 … n_rows-1 (decode steps), so the head may read the stream directly.
 static int stack_pass(b200_engine* e, int n_tok, int n_rows, cudaStream_t st, bool rows_in_order = false) {
+  const PdlScope overlap(stack_pdl() && op_pdl(st));
   StackEngine* s = e->stack;
   const b200_stack_desc& d = s->d;
   const int W = d.width, dt = s->dtype;

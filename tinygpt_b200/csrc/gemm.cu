@@ -109,7 +109,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const int kblocks = (p.K + kBK - 1) / kBK;
   bool ok = true;
 
-  if (p.pdl) pdl_trigger();
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
@@ -129,7 +128,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   cluster_sync_all();   // the pair's barriers exist
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (p.pdl) pdl_wait();
+  if (p.pdl) {
+    pdl_wait();
+    pdl_trigger();   // behind the wait: what starts beside this product finds all that lies before it done
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------------------------------------ TMA producer
@@ -374,7 +376,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int valid = max(0, min(128, p.M - m0));             // rows of this CTA that exist
   bool ok = true;
 
-  if (p.pdl) pdl_trigger();
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
@@ -392,7 +393,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   if constexpr (PAIR) cluster_sync_all();   // the pair's barriers exist
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (p.pdl) pdl_wait();
+  if (p.pdl) {
+    pdl_wait();
+    pdl_trigger();   // behind the wait: what starts beside this product finds all that lies before it done
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------------------------------------ TMA producer
@@ -766,7 +770,9 @@ void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
 }
 
 template <typename OT, int EPI, bool SPLIT = false>
-int launch_gemm(const GemmArgs<OT>& p, const void* A, const void* B, int64_t rows_b, cudaStream_t st) {
+int launch_gemm(const GemmArgs<OT>& args, const void* A, const void* B, int64_t rows_b, cudaStream_t st) {
+  GemmArgs<OT> p = args;
+  if (pdl_scope()) p.pdl = 1;
   GemmPick g{};
   pick_gemm<OT, EPI, SPLIT>(p.M, p.N, p.K, &g);
   if (g.kind == 3) return launch_split<OT, EPI, kWide>(p, A, B, rows_b, 1, st);

@@ -31,6 +31,8 @@ __global__ void __launch_bounds__(256) prefill_qk_kernel(__nv_bfloat16* __restri
                                                          const float* __restrict__ rope, __nv_bfloat16* __restrict__ kcache,
                                                          __nv_bfloat16* __restrict__ vcache, int S, int Hq, int Hkv, int p0) {
   constexpr int L = HD / 16;   // lanes per head
+  pdl_wait();
+  pdl_trigger();
   const int heads = Hq + 2 * Hkv;
   const unsigned item = (blockIdx.x * blockDim.x + threadIdx.x) / L;
   const int part = threadIdx.x % L;
@@ -198,16 +200,12 @@ int launch_prefill_qk(void* qkv, const void* q_norm, const void* k_norm, float e
   B200_CHECK_ARG(aligned16(qkv, kcache, vcache), "prefill: rows and caches must be 16-byte aligned");   // the engine's own
   B200_CHECK_ARG((int64_t)S * (Hq + 2 * Hkv) * (hd / 16) < (1ll << 31), "prefill: too many rows at a time");
   const unsigned grid = (unsigned)(((int64_t)S * (Hq + 2 * Hkv) * (hd / 16) + 255) / 256);
-  g_launches.fetch_add(1);
   if (hd == 64)
-    prefill_qk_kernel<64><<<grid, 256, 0, st>>>((__nv_bfloat16*)qkv, (const __nv_bfloat16*)q_norm,
-                                                 (const __nv_bfloat16*)k_norm, eps, rope, (__nv_bfloat16*)kcache,
-                                                 (__nv_bfloat16*)vcache, S, Hq, Hkv, p0);
+    B200_CUDA(launch_pdl(prefill_qk_kernel<64>, dim3(grid), dim3(256), 0, st, pdl_scope(), (__nv_bfloat16*)qkv, (const __nv_bfloat16*)q_norm,
+                         (const __nv_bfloat16*)k_norm, eps, rope, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, S, Hq, Hkv, p0));
   else
-    prefill_qk_kernel<128><<<grid, 256, 0, st>>>((__nv_bfloat16*)qkv, (const __nv_bfloat16*)q_norm,
-                                                  (const __nv_bfloat16*)k_norm, eps, rope, (__nv_bfloat16*)kcache,
-                                                  (__nv_bfloat16*)vcache, S, Hq, Hkv, p0);
-  B200_CUDA(cudaGetLastError());
+    B200_CUDA(launch_pdl(prefill_qk_kernel<128>, dim3(grid), dim3(256), 0, st, pdl_scope(), (__nv_bfloat16*)qkv, (const __nv_bfloat16*)q_norm,
+                         (const __nv_bfloat16*)k_norm, eps, rope, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, S, Hq, Hkv, p0));
   return B200_OK;
 }
 

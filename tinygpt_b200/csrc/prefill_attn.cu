@@ -144,8 +144,8 @@ __global__ void __launch_bounds__(kPfThreads, HD == 64 ? 3 : 1) attn_prefill_mma
   const float slope = SCORE && p.slopes != nullptr ? p.slopes[blockIdx.x % p.Hq] : 0.f;
 
   if (p.pdl) {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
   }
   extern __shared__ __align__(128) uint8_t pf_smem[];
   uint8_t* const Qs = pf_smem;                       // [kBM][HD]
@@ -401,6 +401,7 @@ int launch_attn_prefill_mma(void* o, const void* qkv, const void* kcache, const 
   p.Hkv = Hkv;
   p.p0 = p0;
   p.scale_log2 = hd == 64 ? PfScale<64>::value : PfScale<128>::value;
+  p.pdl = pdl_scope();
   return hd == 64 ? launch_pf<64>(p, 1, st, 0) : launch_pf<128>(p, 1, st, 0);
 }
 
@@ -443,6 +444,7 @@ int launch_attn_prefill_window(void* o, int64_t o_rs, const void* q, const void*
   p.cap = softcap;
   p.slopes = slopes;
   p.same = kcache == vcache ? 1 : 0;
+  p.pdl = pdl_scope();
   if (softcap > 0.f || slopes != nullptr || p.same)
     return hd == 64 ? launch_pf<64, true>(p, 1, st, 0) : hd == 96 ? launch_pf<96, true>(p, 1, st, 0) : launch_pf<128, true>(p, 1, st, 0);
   const int tc_rows = std::min(ctx, 2048);
