@@ -420,8 +420,12 @@ static int stack_product_mix(StackEngine* s, const float* cur, float* other, int
   return launch_stack_gemm(g, s->dtype, st);
 }
 
+static bool stack_head_gemm(const StackEngine* s, int n_rows) {
+  return s->fast && n_rows > kMaxBatch && gemm_shape_ok(s->d.vocab, s->d.width) && aligned16(s->d.head);
+}
 // logits (fp32) and logits_bf (bf16) = rmsnorm(x[rows])·(offset + w) · headᵀ; rows == null: the stream's rows in order
-static int stack_product_head(StackEngine* s, const float* x, const int32_t* rows, int n_rows, cudaStream_t st) {
+// out: where the bf16 rows of a head GEMM go instead, without their fp32 sums (which only a step hands out)
+static int stack_product_head(StackEngine* s, const float* x, const int32_t* rows, int n_rows, cudaStream_t st, void* out) {
   const b200_stack_desc& d = s->d;
   int rc;
   const int64_t n_lg = (int64_t)n_rows * d.vocab;
@@ -451,8 +455,8 @@ static int stack_product_head(StackEngine* s, const float* x, const int32_t* row
   }
   // more rows than a decode batch (every position of a prompt, scoring): 2 048 rows × 2 048 columns of width 2 048 took 882 µs on the
   // CUDA-core kernel, 22 µs on the tensor cores; the sums are fp32 in both
-  if (s->fast && n_rows > kMaxBatch && gemm_shape_ok(d.vocab, d.width) && aligned16(d.head))
-    return launch_gemm_bf16_logits(s->logits, s->logits_bf, s->hn, d.head, d.logit_softcap, n_rows, d.vocab, d.width, st);
+  if (stack_head_gemm(s, n_rows))
+    return launch_gemm_bf16_logits(out ? nullptr : s->logits, out ? out : s->logits_bf, s->hn, d.head, d.logit_softcap, n_rows, d.vocab, d.width, st);
   StackGemm g;
   g.a = s->hn; g.lda = d.width; g.k1 = d.width;
   g.w = d.head; g.M = n_rows; g.N = d.vocab; g.K = d.width;
@@ -1179,7 +1183,7 @@ static int stack_run_hyper(StackEngine* s, int r, float* x, int n_tok, cudaStrea
 
 // One pass: n_tok rows {m_tok, m_slot, m_pos} through every run, then the head for the n_rows rows listed in m_want.
 // rows_in_order: m_want is 0 … n_rows-1 (decode steps), so the head may read the stream directly.
-static int stack_pass(b200_engine* e, int n_tok, int n_rows, cudaStream_t st, bool rows_in_order = false) {
+static int stack_pass(b200_engine* e, int n_tok, int n_rows, cudaStream_t st, bool rows_in_order = false, void* head_out = nullptr) {
   const PdlScope overlap(stack_pdl() && op_pdl(st));
   StackEngine* s = e->stack;
   const b200_stack_desc& d = s->d;
@@ -1249,15 +1253,14 @@ static int stack_pass(b200_engine* e, int n_tok, int n_rows, cudaStream_t st, bo
     if ((rc = launch_hyper_step(p, dt, st)) != B200_OK) return rc;
     cur = s->x0;
   }
-  if (n_rows > 0 && (rc = stack_product_head(s, cur, rows_in_order ? nullptr : s->m_want, n_rows, st)) != B200_OK) return rc;
+  if (n_rows > 0 && (rc = stack_product_head(s, cur, rows_in_order ? nullptr : s->m_want, n_rows, st, head_out)) != B200_OK) return rc;
   return B200_OK;
 }
 
-// greedy / sampled token of logits rows [row0, row0 + n) → the slots in `slots` (row order)
-static int stack_publish(b200_engine* e, int row0, const std::vector<int>& slots, cudaStream_t st) {
+// greedy / sampled token of the logits rows lg, lg + ld, … → the slots in `slots` (row order)
+static int stack_publish(b200_engine* e, const __nv_bfloat16* lg, int64_t ld, const std::vector<int>& slots, cudaStream_t st) {
   StackEngine* s = e->stack;
   const int n = (int)slots.size();
-  const __nv_bfloat16* lg = s->logits_bf + (size_t)row0 * s->d.vocab;
   int rc;
   if (e->sampler_on) {
     for (int r = 0; r < n; ++r) {
@@ -1267,7 +1270,7 @@ static int stack_publish(b200_engine* e, int row0, const std::vector<int>& slots
       pub.gen_log = s->gen_log + (size_t)sl * s->gen_cap;
       pub.gen_count = s->gen_count + sl;
       pub.gen_cap = s->gen_cap;
-      if ((rc = launch_sample(nullptr, lg + (size_t)r * s->d.vocab, s->d.vocab, e->s_temperature, e->s_top_k, e->s_top_p,
+      if ((rc = launch_sample(nullptr, lg + (size_t)r * ld, s->d.vocab, e->s_temperature, e->s_top_k, e->s_top_p,
                               e->s_min_p, 0.f, s->sample_ws, st, &pub, e->s_seed, true)) != B200_OK)
         return rc;
     }
@@ -1278,7 +1281,7 @@ static int stack_publish(b200_engine* e, int row0, const std::vector<int>& slots
     pub.gen_count = s->gen_count;
     pub.gen_cap = s->gen_cap;
     pub.row_slot = s->row_slot;
-    if ((rc = launch_argmax(s->amax_out, lg, n, s->d.vocab, s->argmax_ws, st, false, &pub)) != B200_OK) return rc;
+    if ((rc = launch_argmax(s->amax_out, lg, n, s->d.vocab, s->argmax_ws, st, false, &pub, ld)) != B200_OK) return rc;
   }
   return B200_OK;
 }
@@ -1374,23 +1377,31 @@ int stack_forward(b200_engine* e, const int64_t* ids, int64_t B, int64_t S, void
   if ((rc = stack_workspace(s, ws_tok, (all ? ws_tok : 0) + (int)B)) != B200_OK) return rc;
   if ((rc = stack_set_active(s, slots, st)) != B200_OK) return rc;
   const size_t vb = (size_t)d.vocab * 2;
-  int head_row0 = 0;   // first of the B rows that hold the sequences' last positions
+  const __nv_bfloat16* last_row = s->logits_bf;   // of the first sequence; the others' follow last_ld further on each
+  int64_t last_ld = d.vocab;
   for (int64_t s0 = 0; s0 < S; s0 += cs_max) {
     const int cs = (int)std::min<int64_t>(cs_max, S - s0);
     const int n_tok = cs * (int)B;
     const bool last = s0 + cs == S;
     B200_CUDA(launch_pdl(stack_meta_from_ids_kernel, dim3((n_tok + 255) / 256), dim3(256), 0, st, false, ids, (int)B, (int)S,
                          (int)s0, cs, (const int*)s->pos_dev, s->m_tok, s->m_slot, s->m_pos, s->m_want, (int)all, (int)last));
-    // rows: every token of the chunk when all positions are asked for, then (last chunk) the B last positions
+    // rows: every token of the chunk when all positions are asked for, then (last chunk) the B last positions.  Where the head is a GEMM whose
+    // rows lie in logits_out as they come, it stores there, bf16 alone, and the last positions are read from there: the fp32 sums, the copy and
+    // the tile that a row of its own had opened were 7 of 286 µs in one layer of 2 048 over 2 048 tokens and as many words
+    uint8_t* const out = (uint8_t*)logits_out + (size_t)s0 * vb;
+    const bool direct = all && (B == 1 || cs == S) && aligned16(out) && stack_head_gemm(s, n_tok);
     int n_rows = all ? n_tok : 0;
-    if (last) {
-      head_row0 = n_rows;
+    if (last && direct) {
+      last_row = (const __nv_bfloat16*)out + (size_t)(cs - 1) * d.vocab;
+      last_ld = (int64_t)cs * d.vocab;
+    } else if (last) {
+      last_row = s->logits_bf + (size_t)n_rows * d.vocab;
       n_rows += (int)B;
     }
     s->segs.clear();
     for (int b = 0; b < B; ++b) s->segs.push_back({b * cs, cs, b, (int)s->h_pos[b] + (int)s0});
-    if ((rc = stack_pass(e, n_tok, n_rows, st)) != B200_OK) return rc;
-    if (all)   // rows are [b][t of this chunk] → logits_out [B][S][V]
+    if ((rc = stack_pass(e, n_tok, n_rows, st, false, direct ? out : (uint8_t*)s->logits_bf)) != B200_OK) return rc;
+    if (all && !direct)   // rows are [b][t of this chunk] → logits_out [B][S][V]
       B200_CUDA(cudaMemcpy2DAsync((uint8_t*)logits_out + (size_t)s0 * vb, (size_t)S * vb, s->logits_bf, (size_t)cs * vb,
                                   (size_t)cs * vb, (size_t)B, cudaMemcpyDeviceToDevice, st));
   }
@@ -1408,7 +1419,7 @@ int stack_forward(b200_engine* e, const int64_t* ids, int64_t B, int64_t S, void
   e->batch = (int)B;
   // the greedy token of every sequence's last position becomes its slot's current token
   stack_count_generated(s, slots, 1);
-  return stack_publish(e, head_row0, slots, st);
+  return stack_publish(e, last_row, last_ld, slots, st);
 }
 
 // one greedy decode step of the active batch: row list from the slots' device state, the pass, the publication
@@ -1419,7 +1430,7 @@ static int stack_decode_step(b200_engine* e, int B, cudaStream_t st) {
                        s->pos_dev, (const int64_t*)s->cur_tok, s->m_tok, s->m_slot, s->m_pos, s->m_want));
   s->segs.clear();
   if ((rc = stack_pass(e, B, B, st, true)) != B200_OK) return rc;
-  return stack_publish(e, 0, s->active, st);
+  return stack_publish(e, s->logits_bf, s->d.vocab, s->active, st);
 }
 
 static int stack_capture_decode(b200_engine* e, int B) {
@@ -2177,7 +2188,7 @@ int b200_engine_step(b200_engine* e, int64_t n_seq, const int32_t* slots, const 
     }
     if (greedy && tail) {
       stack_count_generated(s, act_slots, 1);
-      if ((rc = stack_publish(e, n_user, act_slots, st)) != B200_OK) return rc;
+      if ((rc = stack_publish(e, s->logits_bf + (size_t)n_user * s->d.vocab, s->d.vocab, act_slots, st)) != B200_OK) return rc;
     }
   }
   std::vector<int32_t> upd;

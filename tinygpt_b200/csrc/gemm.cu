@@ -44,7 +44,7 @@ enum GemmEpi : int {
   GEPI_RESIDUAL = 1,   // C = bf16(add + bf16(acc)); add [M, N] may be C itself: a linear followed by the residual's add
   GEPI_BIAS = 2,       // C = bf16(bf16(acc) + add), add [N]: a linear followed by its bias as the second rounding
   GEPI_ACCUM = 4,      // C += mult·acc (fp32 C): a layer-stack model's residual stream
-  GEPI_LOGITS = 5,     // C = cap·tanh(acc / cap) (mult = cap; 0: acc itself), c2 = bf16(C) (fp32 C)
+  GEPI_LOGITS = 5,     // C = cap·tanh(acc / cap) (mult = cap; 0: acc itself); fp32 C: and c2 = bf16(C)
   GEPI_SILU = 3,       // B holds N gate rows, then N up rows: C = bf16(bf16(silu(bf16 gate)) · bf16 up)
 };
 template <typename OT>
@@ -244,6 +244,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
               if (n0 + c + 32 + j < p.N) b[j] = __float_as_uint(__uint_as_float(b[j]) + p.bias[n0 + c + 32 + j]);
             }
           }
+          if (EPI == GEPI_LOGITS && p.mult > 0.f) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              a[j] = __float_as_uint(cap_logit(__uint_as_float(a[j]), p.mult));
+              b[j] = __float_as_uint(cap_logit(__uint_as_float(b[j]), p.mult));
+            }
+          }
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const uint32_t* v = j < 4 ? a + 8 * j : b + 8 * (j - 4);
@@ -292,7 +299,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             const int r = rr + 4 * k;
             if (row0 + r >= p.M) continue;
             uint4 v = *reinterpret_cast<const uint4*>(pw + r * 128 + ((cc ^ (r & 7)) << 4));
-            if constexpr (EPI == GEPI_ACCUM || EPI == GEPI_LOGITS) {
+            if constexpr (EPI == GEPI_ACCUM || (EPI == GEPI_LOGITS && sizeof(OT) == 4)) {
               uint32_t* f = reinterpret_cast<uint32_t*>(&v);
               const uint32_t* o = reinterpret_cast<const uint32_t*>(&add[EPI == GEPI_ACCUM ? k : 0]);
 #pragma unroll
@@ -528,7 +535,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if constexpr (EPI == GEPI_LOGITS) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) v[e] = cap_logit(v[e], p.mult);
-            *reinterpret_cast<uint4*>(p.c2 + o0 + c + 8 * j) = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+            if constexpr (sizeof(OT) == 4) *reinterpret_cast<uint4*>(p.c2 + o0 + c + 8 * j) = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
           }
           if constexpr (sizeof(OT) == 4) {
             reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
@@ -861,9 +868,12 @@ int launch_gemm_bf16_accum(float* C, const void* A, const void* B, float mult, i
 }
 int launch_gemm_bf16_logits(float* C, void* C_bf16, const void* A, const void* B, float softcap, int64_t M, int64_t N, int64_t K,
                             cudaStream_t st) {
-  int rc = check_gemm(C, A, B, M, N, K);
+  int rc = check_gemm(C_bf16, A, B, M, N, K);
   if (rc != B200_OK) return rc;
-  B200_CHECK_ARG(C_bf16 && aligned16(C_bf16), "gemm: bad bf16 logits");
+  if (C == nullptr)
+    return launch_gemm<__nv_bfloat16, GEPI_LOGITS>(GemmArgs<__nv_bfloat16>{(__nv_bfloat16*)C_bf16, nullptr, nullptr, (int)M, (int)N, (int)K, nullptr, softcap},
+                                                   A, B, N, st);
+  B200_CHECK_ARG(aligned16(C), "gemm: bad fp32 logits");
   return launch_gemm<float, GEPI_LOGITS>(GemmArgs<float>{C, nullptr, nullptr, (int)M, (int)N, (int)K, nullptr, softcap, (__nv_bfloat16*)C_bf16}, A,
                                          B, N, st);
 }

@@ -228,7 +228,7 @@ __device__ __forceinline__ void argmax_merge(float& v, int64_t& i, float ov, int
 }
 
 __global__ void __launch_bounds__(256) argmax_kernel(int64_t* __restrict__ out, const __nv_bfloat16* __restrict__ logits,
-                                                     int64_t V, float* __restrict__ ws_val, int64_t* __restrict__ ws_idx,
+                                                     int64_t V, int64_t ld, float* __restrict__ ws_val, int64_t* __restrict__ ws_idx,
                                                      unsigned int* __restrict__ ticket, const ArgmaxPublish pub) {
   __shared__ float sv[8];
   __shared__ int64_t si[8];
@@ -237,11 +237,11 @@ __global__ void __launch_bounds__(256) argmax_kernel(int64_t* __restrict__ out, 
   pdl_wait();
   const int row = blockIdx.y;
   const int chunks = gridDim.x;
-  const __nv_bfloat16* lg = logits + (size_t)row * V;
+  const __nv_bfloat16* lg = logits + (size_t)row * ld;
   float v = -INFINITY;
   int64_t idx = -1;
   // eight logits a load where rows allow it (one at a time a thread waits for eight round trips in turn: 2 048 logits 8.1 → 6.0 µs)
-  const bool wide = V % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+  const bool wide = V % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
   if (wide) {
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < V / 8; j += (int64_t)chunks * blockDim.x) {
       float x[8];
@@ -434,7 +434,7 @@ int64_t argmax_workspace_bytes(int64_t rows, int64_t V) {
 }
 
 int launch_argmax(int64_t* idx, const void* logits, int64_t rows, int64_t V, void* workspace, cudaStream_t st,
-                  bool pdl, const ArgmaxPublish* pub) {
+                  bool pdl, const ArgmaxPublish* pub, int64_t ld) {
   B200_CHECK_ARG(idx && logits && workspace && rows > 0 && V > 0 && rows < 65536, "argmax: bad arguments");
   const int c = argmax_chunks(V);
   uint8_t* ws = (uint8_t*)workspace;
@@ -442,7 +442,7 @@ int launch_argmax(int64_t* idx, const void* logits, int64_t rows, int64_t V, voi
   float* wv = (float*)(ws + argmax_ticket_bytes(rows));
   int64_t* wi = (int64_t*)((uint8_t*)wv + ((rows * c * 4 + 15) / 16) * 16);
   B200_CUDA(launch_pdl(argmax_kernel, dim3(c, (unsigned)rows), dim3(256), 0, st, pdl, idx,
-                       (const __nv_bfloat16*)logits, V, wv, wi, ticket, pub ? *pub : ArgmaxPublish{}));
+                       (const __nv_bfloat16*)logits, V, ld > 0 ? ld : V, wv, wi, ticket, pub ? *pub : ArgmaxPublish{}));
   return B200_OK;
 }
 

@@ -37,7 +37,7 @@ struct ArgmaxPublish {
   const unsigned long long* tp_epoch = nullptr;   // tag = *tp_epoch + 1
 };
 int launch_argmax(int64_t* idx, const void* logits, int64_t rows, int64_t V, void* workspace, cudaStream_t st,
-                  bool pdl, const ArgmaxPublish* pub);
+                  bool pdl, const ArgmaxPublish* pub, int64_t ld = 0);   // ld: from row to row (0: V)
 
 // ---- device sampler (sampling.cu): temperature / top-k / top-p / min-p + inverse-CDF draw without sorting
 int64_t sample_workspace_bytes();
@@ -52,7 +52,7 @@ int launch_gemm_bf16_bias(void* C, const void* A, const void* B, const float* bi
 // the same products handed out as fp32 sums: C = A·Bᵀ + bias (bias may be null)
 int launch_gemm_bf16_f32(float* C, const void* A, const void* B, const float* bias, int64_t M, int64_t N, int64_t K, cudaStream_t st);
 
-// C += mult·(A·Bᵀ) in fp32;  C = capped A·Bᵀ in fp32 and C_bf16 = bf16(C) (softcap 0: no cap)
+// C += mult·(A·Bᵀ) in fp32;  C = capped A·Bᵀ in fp32 (null: not wanted) and C_bf16 = bf16(C) (softcap 0: no cap)
 int launch_gemm_bf16_accum(float* C, const void* A, const void* B, float mult, int64_t M, int64_t N, int64_t K, cudaStream_t st);
 int launch_gemm_bf16_logits(float* C, void* C_bf16, const void* A, const void* B, float softcap, int64_t M, int64_t N, int64_t K,
                             cudaStream_t st);
