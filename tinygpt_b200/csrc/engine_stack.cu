@@ -141,7 +141,7 @@ struct StackEngine {
   int lat_heads_max = 0, lat_rank_max = 0, lat_hd_max = 0, lat_hv_max = 0;
   __nv_bfloat16 *lat_c = nullptr, *lat_kp = nullptr, *lat_k = nullptr, *lat_v = nullptr, *lat_q = nullptr;   // one sequence's expanded keys / values
   int qa_max = 0, ol_max = 0, rec_o_max = 0, moe_e_max = 0, moe_top_max = 0, moe_ff_max = 0, lin_max = 0;
-  bool any_rec = false, any_moe = false;
+  bool any_rec = false, any_moe = false, any_mix = false;   // any_mix: some run mixes the embedding in, so x0 keeps it
   bool h_ready = false;            // the previous sublayer's fused post-norm already left this run's normed input in h
   // ---- post-norm blocks: the scan's fp32 operand rows, the decay projection's two stages, the kept values of a pass
   float *rec_f = nullptr, *rec_wl = nullptr;
@@ -1191,7 +1191,7 @@ static int stack_pass(b200_engine* e, int n_tok, int n_rows, cudaStream_t st, bo
   int rc;
   const bool hyper = d.block == B200_BLOCK_HYPER;
   if ((rc = hyper ? launch_hyper_embed(s->x, d.embed, s->m_tok, n_tok, d.vocab, W, s->streams, d.embed_scale, dt, st)
-                  : launch_stack_embed(s->x, s->x0, d.embed, s->m_tok, n_tok, d.vocab, W, d.embed_scale, dt, st)) != B200_OK)
+                  : launch_stack_embed(s->x, s->any_mix ? s->x0 : nullptr, d.embed, s->m_tok, n_tok, d.vocab, W, d.embed_scale, dt, st)) != B200_OK)
     return rc;
   s->hy_y = nullptr;
   float *cur = s->x, *other = s->x_alt;
@@ -1727,6 +1727,7 @@ static int stack_build(const b200_stack_desc* desc, b200_engine** out) {
   s->layers.assign(d.layers_host, d.layers_host + d.n_layers);
   s->run_layer.assign(d.run_layer_host, d.run_layer_host + d.n_runs);
   s->run_mix.assign(d.run_mix_host, d.run_mix_host + d.n_runs);
+  for (int m : s->run_mix) s->any_mix = s->any_mix || m != 0;
   s->d.layers_host = nullptr;
   s->d.run_layer_host = s->d.run_mix_host = nullptr;
   const bool hyper = d.block == B200_BLOCK_HYPER;

@@ -57,7 +57,7 @@ int launch_stack_rms_add(float* x, const float* y, const float* w, int64_t rows,
                          cudaStream_t st);
 int launch_stack_act_mul(void* y, int64_t ld_y, const void* g, const void* u, int64_t ld_gu, int64_t rows, int n, int act,
                          int dtype, cudaStream_t st);
-// x0[t, :] = float(embed[tok[t], :]) · scale, and x = x0
+// x[t, :] = float(embed[tok[t], :]) · scale, and x0 = x where it is kept (x0 may be null)
 int launch_stack_embed(float* x, float* x0, const void* embed, const int32_t* tok, int64_t n_tok, int vocab, int width,
                        float scale, int dtype, cudaStream_t st);
 

@@ -307,6 +307,8 @@ __global__ void __launch_bounds__(256) stack_act_mul_vec_kernel(__nv_bfloat16* _
   }
 }
 
+// Bound by its stores; x0 is kept only for a model that mixes the embedding in again (8 layers of 2 048, 2 048 tokens, with / without 1 717 / 1 648 µs
+// a prompt: 16.8 MB less in L2).  Eight values at a time were no faster.
 template <typename T>
 __global__ void __launch_bounds__(128) stack_embed_kernel(float* __restrict__ x, float* __restrict__ x0,
                                                           const T* __restrict__ embed, const int32_t* __restrict__ tok,
@@ -319,7 +321,7 @@ __global__ void __launch_bounds__(128) stack_embed_kernel(float* __restrict__ x,
   for (int i = threadIdx.x; i < width; i += blockDim.x) {
     const float v = ldf<T>(row + i) * scale;
     x[(int64_t)blockIdx.x * width + i] = v;
-    x0[(int64_t)blockIdx.x * width + i] = v;
+    if (x0 != nullptr) x0[(int64_t)blockIdx.x * width + i] = v;
   }
 }
 
@@ -889,7 +891,7 @@ int launch_stack_act_mul(void* y, int64_t ld_y, const void* g, const void* u, in
 int launch_stack_embed(float* x, float* x0, const void* embed, const int32_t* tok, int64_t n_tok, int vocab, int width,
                        float scale, int dtype, cudaStream_t st) {
   STACK_DTYPE_CHECK(dtype);
-  B200_CHECK_ARG(x && x0 && embed && tok && n_tok > 0, "stack embed: bad arguments");
+  B200_CHECK_ARG(x && embed && tok && n_tok > 0, "stack embed: bad arguments");
   if (dtype == B200_F32)
     B200_CUDA(launch_pdl(stack_embed_kernel<float>, dim3((unsigned)n_tok), dim3(128), 0, st, stack_pdl(), x, x0,
                          (const float*)embed, tok, vocab, width, scale));
