@@ -478,6 +478,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_row_kernel(const AttnRow
     const bool has_new = owns_new && u * kUnit + warp * 16 + nv == n;
     const uint32_t kslot = (uint32_t)(2 * u % R::NS) * R::SLOT, vslot = (uint32_t)((2 * u + 1) % R::NS) * R::SLOT;
     auto put_new = [&](uint32_t slot, const __nv_bfloat16* row) {
+      __syncwarp();   // a lane has waited for its own copies only: the zeros of this row are another's at most places
       if (nv == 1 && n_cached == n - 1 && u * kUnit + warp * 16 == n_cached) {   // a warp without a cached key has not cleared its rows
         for (int e = lane; e < (int)WB / 16; e += 32) reinterpret_cast<uint4*>(ring + warp * WB + slot)[e] = make_uint4(0, 0, 0, 0);
         __syncwarp();
