@@ -499,7 +499,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_row_kernel(const AttnRow
                    : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                    : "r"(ka[0]), "r"(ka[1]), "r"(ka[2]), "r"(ka[3]), "r"(qb[kk][0]), "r"(qb[kk][1]));
     }
-    load(2 * u + R::NS);   // K has been read
+    __syncwarp();   // every lane's rows of K have been read
+    load(2 * u + R::NS);
     float pr[4], alpha[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
