@@ -13,6 +13,7 @@
 // Numerics: q·k and P·V accumulate in fp32 over bf16 inputs; rounding points of q/k (after norm, after RoPE) are the
 // reference's.  Probabilities stay fp32 (the reference rounds P to bf16 before P·V, TFA/mma/layout.cuh:88-97); the
 // oracle models the reference's rounding and the parity tests bound the difference.
+#include "key_range.cuh"
 #include "ops.cuh"
 #include "tc.cuh"
 
@@ -357,9 +358,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_row_kernel(const AttnRow
   const bool append = DECODE && p.pos != nullptr;
   const int pos = append ? *p.pos : p.fixed_len - 1;   // where q is rotated; stable since before the producer kernel started
   const int cached = append ? pos : DECODE ? p.fixed_len : a.nkeys;   // rows that are in the cache already
-  const int nkeys = cached + (append ? 1 : 0);
-  const int per = (((nkeys + splits - 1) >> a.log_splits) + 15) & ~15;
-  const int k0 = min(nkeys, rank * per), n = min(nkeys, k0 + per) - k0, n_cached = min(cached, k0 + n) - k0;   // this CTA's keys
+  const KeyRange keys = key_range(cached, append, rank, a.log_splits);
+  const int k0 = keys.first, n = keys.n, n_cached = keys.n_cached;   // this CTA's keys
   const int units = (n - warp * 16 + kUnit - 1) / kUnit;   // with a key for this warp
   constexpr int PC = HD / 8, RP = 32 / PC;   // 16-byte pieces of a row; rows that a warp copies at once
   constexpr uint32_t WB = 16 * R::RB;        // a warp's part of a slot
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_row_kernel(const AttnRow
 #pragma unroll
   for (int s = 0; s < R::NS; ++s) load(s);   // rows of earlier tokens: nothing that the producer kernel writes
   [[maybe_unused]] const __nv_bfloat16* qkv = p.qkv + b * p.qkv_bstride;
-  const bool owns_new = append && n > n_cached;
+  const bool owns_new = keys.owns_new;
   for (int i = G * (QP / 2) + tid; i < 8 * (QP / 2); i += kAttnThreads) reinterpret_cast<uint32_t*>(&q_s[0][0])[i] = 0;   // columns without a head
   if constexpr (DECODE) {
     float rc[EPL / 2], rs[EPL / 2];
