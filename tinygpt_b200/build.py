@@ -43,13 +43,29 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found: the B200 library cannot be built (there is no CPU fallback)")
 
 
-def _digest() -> str:
+def _hash(paths, *also: str) -> str:
     h = hashlib.sha256()
-    for p in sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.cpp")) + [ROOT / "include" / "b200_decode.h"]):
+    for p in sorted([*paths, ROOT / "include" / "b200_decode.h"]):
         h.update(p.name.encode())
         h.update(p.read_bytes())
-    h.update(" ".join(NVCC_FLAGS).encode())
+    for text in also:
+        h.update(text.encode())
     return h.hexdigest()
+
+
+def _digest() -> str:
+    return _hash([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")], " ".join(NVCC_FLAGS))
+
+
+def _cxx_flags() -> list[str]:
+    import torch
+    return ["-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+
+
+def _native_digest() -> str:
+    """The extension is bound to the torch and the Python that it was compiled against.  Without paths: the built files travel with the tree."""
+    import torch
+    return _hash([CSRC / "torch_ops.cpp"], torch.__version__, str(torch.version.git_version), sys.version, *_cxx_flags())
 
 
 def _native_command() -> list[str]:
@@ -60,18 +76,27 @@ def _native_command() -> list[str]:
     home = Path(torch.__file__).parent
     nvcc_home = Path(_nvcc()).resolve().parent.parent
     includes = [home / "include", home / "include/torch/csrc/api/include", nvcc_home / "include", sysconfig.get_paths()["include"]]
-    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-            *[x for i in includes for x in ("-isystem", str(i))], "-I", str(ROOT / "include"), str(CSRC / "torch_ops.cpp"), "-o", str(NATIVE_PATH),
-            f"-L{home / 'lib'}", f"-L{LIB_DIR}", "-lb200decode", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
+    return ["g++", *_cxx_flags(), *[x for i in includes for x in ("-isystem", str(i))], "-I", str(ROOT / "include"), str(CSRC / "torch_ops.cpp"),
+            "-o", str(NATIVE_PATH), f"-L{home / 'lib'}", f"-L{LIB_DIR}", "-lb200decode", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
+    """Both files, each when it or what it is made from has changed since its stamp was written; the library first, which needs no torch."""
     LIB_DIR.mkdir(exist_ok=True)
     OBJ_DIR.mkdir(exist_ok=True)
-    stamp = LIB_DIR / "build.stamp"
-    digest = _digest()
-    if not force and LIB_PATH.exists() and NATIVE_PATH.exists() and stamp.exists() and stamp.read_text().strip() == digest:
-        return LIB_PATH
+    for made, digest, stamp, make in ((LIB_PATH, _digest, "build", _build_library), (NATIVE_PATH, _native_digest, "native", _build_native)):
+        stamp, now = LIB_DIR / f"{stamp}.stamp", digest()
+        if not force and made.exists() and stamp.exists() and stamp.read_text().strip() == now:
+            continue
+        log = make()
+        stamp.with_suffix(".log").write_text(log)
+        stamp.write_text(now)
+        if verbose:
+            print(log)
+    return LIB_PATH
+
+
+def _build_library() -> str:
     nvcc = _nvcc()
     log_lines: list[str] = []
 
@@ -91,16 +116,15 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     log_lines.append(f"$ {' '.join(cmd)}\n{r.stdout}{r.stderr}")
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    return "\n".join(log_lines)
+
+
+def _build_native() -> str:
     cmd = _native_command()
     r = subprocess.run(cmd, capture_output=True, text=True)
-    log_lines.append(f"$ {' '.join(cmd)}\n{r.stdout}{r.stderr}")
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on torch_ops.cpp:\n{r.stdout}\n{r.stderr}")
-    (LIB_DIR / "build.log").write_text("\n".join(log_lines))
-    stamp.write_text(digest)
-    if verbose:
-        print("\n".join(log_lines))
-    return LIB_PATH
+    return f"$ {' '.join(cmd)}\n{r.stdout}{r.stderr}"
 
 
 if __name__ == "__main__":
