@@ -17,6 +17,27 @@ def test_cpu_tensors_are_refused(built_lib):
             call()
 
 
+def test_a_library_under_another_name_and_place(built_lib, tmp_path):
+    """B200_LIB names the library that the native operators call too; no other is loaded, and nothing need lie beside it."""
+    import os
+    import shutil
+    import subprocess
+    import sys
+    other = tmp_path / "other_name.so"
+    shutil.copy(built_lib, other)
+    code = """
+import torch
+from tinygpt_b200 import ops
+from tinygpt_b200._lib import B200Error
+x = torch.zeros(2, 8, dtype=torch.bfloat16)
+assert ops._fast.linear(x, x, None) is None and ops._fast.attn_decode(x, x, x, 1, 1, 64, None, 1, None, None, None, 0.0) is None
+maps = open("/proc/self/maps").read()
+assert "other_name.so" in maps and "libb200decode.so" not in maps
+"""
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, B200_LIB=str(other)), capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+
 @pytest.mark.gpu
 class TestOnDevice:
     def setup_method(self):

@@ -6,8 +6,9 @@ from pathlib import Path
 
 import os
 
-LIB_PATH = Path(os.environ.get("B200_LIB") or (Path(__file__).resolve().parent / "lib" / "libb200decode.so"))
-NATIVE_PATH = LIB_PATH.with_name("b200ops.so")   # it loads the library that lies beside it
+LIB_DIR = Path(__file__).resolve().parent / "lib"
+LIB_PATH = Path(os.environ.get("B200_LIB") or LIB_DIR / "libb200decode.so")
+NATIVE_PATH = LIB_DIR / "b200ops.so"   # calls the library that lib() has loaded, wherever that lies
 IPC_HANDLE_BYTES = 64
 
 _lib = None
@@ -241,12 +242,13 @@ def native():
         import importlib.util
 
         import torch  # noqa: F401  (its libraries come first)
-        lib()
+        handle = lib()._handle
         if not NATIVE_PATH.exists():
             raise B200Error(f"{NATIVE_PATH} is missing: build it with `python -m tinygpt_b200.build`. There is no other path to the operators.")
         loader = importlib.machinery.ExtensionFileLoader("b200ops", str(NATIVE_PATH))
         mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200ops", loader))
         loader.exec_module(mod)
+        mod._bind(handle)
         _native = mod
     return _native
 

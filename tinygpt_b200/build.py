@@ -2,7 +2,7 @@
 
     python -m tinygpt_b200.build [--force] [--verbose]
 
-Output: tinygpt_b200/lib/libb200decode.so  (C ABI declared in include/b200_decode.h) and, linked to it and to torch,
+Output: tinygpt_b200/lib/libb200decode.so  (C ABI declared in include/b200_decode.h) and, linked to torch alone,
 tinygpt_b200/lib/b200ops.so  (the operators of ops.py as native functions, csrc/torch_ops.cpp).
 """
 from __future__ import annotations
@@ -69,7 +69,7 @@ def _native_digest() -> str:
 
 
 def _native_command() -> list[str]:
-    """g++ for the torch extension: torch's own headers and libraries, the library beside it at load time."""
+    """g++ for the torch extension: torch's own headers and libraries.  The library's functions come from the one that _lib.py loads."""
     import sysconfig
 
     import torch
@@ -77,7 +77,7 @@ def _native_command() -> list[str]:
     nvcc_home = Path(_nvcc()).resolve().parent.parent
     includes = [home / "include", home / "include/torch/csrc/api/include", nvcc_home / "include", sysconfig.get_paths()["include"]]
     return ["g++", *_cxx_flags(), *[x for i in includes for x in ("-isystem", str(i))], "-I", str(ROOT / "include"), str(CSRC / "torch_ops.cpp"),
-            "-o", str(NATIVE_PATH), f"-L{home / 'lib'}", f"-L{LIB_DIR}", "-lb200decode", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
+            "-o", str(NATIVE_PATH), f"-L{home / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:

@@ -16,9 +16,29 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <dlfcn.h>
+
 #include "b200_decode.h"
 
 namespace {
+
+// The C ABI of the library that _lib.py has loaded, whatever its file is called: this module is linked to none.
+#define B200_FUNCTIONS(F) \
+  F(gemv_bf16) F(gemm_bf16) F(rmsnorm_bf16) F(silu_mul_bf16) F(add_bf16) F(attn_bf16) F(gemv_fused_bf16) F(attn_decode_workspace_bytes) F(attn_decode_bf16)
+struct {
+#define B200_FIELD(f) decltype(&b200_##f) f;
+  B200_FUNCTIONS(B200_FIELD)
+} abi;
+
+PyObject* bind(PyObject*, PyObject* handle) {   // what dlopen gave; before any other function here
+  void* const lib = PyLong_AsVoidPtr(handle);
+  if (lib == nullptr) return PyErr_Occurred() ? nullptr : PyErr_Format(PyExc_ValueError, "no library");
+#define B200_BIND(f)                                                             \
+  abi.f = reinterpret_cast<decltype(abi.f)>(dlsym(lib, "b200_" #f));             \
+  if (abi.f == nullptr) return PyErr_Format(PyExc_AttributeError, "the library does not export b200_" #f);
+  B200_FUNCTIONS(B200_BIND)
+  Py_RETURN_NONE;
+}
 
 // an ordinary contiguous CUDA tensor of this type, or null
 const at::Tensor* plain(PyObject* o, at::ScalarType type = at::kBFloat16) {
@@ -65,7 +85,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {   // x, wei
   const int64_t n = w->size(0), k = w->size(1);
   if (k < 1 || x->size(-1) != k || x->numel() < 1) Py_RETURN_NONE;
   const int64_t m = x->numel() / k;
-  return run(*x, with_last(*x, n), [&](void* y, void* st) { return b200_gemv_bf16(y, x->data_ptr(), w->data_ptr(), ptr(b), m, n, k, st); });
+  return run(*x, with_last(*x, n), [&](void* y, void* st) { return abi.gemv_bf16(y, x->data_ptr(), w->data_ptr(), ptr(b), m, n, k, st); });
   END_HANDLE_TH_ERRORS
 }
 
@@ -76,7 +96,7 @@ PyObject* gemm(PyObject*, PyObject* const* a, Py_ssize_t n_args) {   // a, weigh
   const int64_t n = w->size(0), k = w->size(1);
   if (k < 1 || x->size(-1) != k || x->numel() < 1) Py_RETURN_NONE;
   const int64_t m = x->numel() / k;
-  return run(*x, with_last(*x, n), [&](void* y, void* st) { return b200_gemm_bf16(y, x->data_ptr(), w->data_ptr(), m, n, k, st); });
+  return run(*x, with_last(*x, n), [&](void* y, void* st) { return abi.gemm_bf16(y, x->data_ptr(), w->data_ptr(), m, n, k, st); });
   END_HANDLE_TH_ERRORS
 }
 
@@ -86,7 +106,7 @@ PyObject* rms_norm(PyObject*, PyObject* const* a, Py_ssize_t n_args) {   // x, w
   if (n_args != 3 || modes() || !(x = plain(a[0])) || !plain_or_none(a[1], w) || !PyFloat_Check(a[2]) || x->dim() < 1 || x->numel() < 1) Py_RETURN_NONE;
   const int64_t dim = x->size(-1);
   const float eps = (float)PyFloat_AS_DOUBLE(a[2]);
-  return run(*x, x->sizes(), [&](void* y, void* st) { return b200_rmsnorm_bf16(y, x->data_ptr(), ptr(w), x->numel() / dim, dim, eps, st); });
+  return run(*x, x->sizes(), [&](void* y, void* st) { return abi.rmsnorm_bf16(y, x->data_ptr(), ptr(w), x->numel() / dim, dim, eps, st); });
   END_HANDLE_TH_ERRORS
 }
 
@@ -95,7 +115,7 @@ PyObject* silu_mul(PyObject*, PyObject* const* a, Py_ssize_t n_args) {   // x
   const at::Tensor* x;
   if (n_args != 1 || modes() || !(x = plain(a[0])) || x->dim() < 1 || x->numel() < 1 || x->size(-1) % 2 != 0) Py_RETURN_NONE;
   const int64_t n = x->size(-1) / 2;
-  return run(*x, with_last(*x, n), [&](void* y, void* st) { return b200_silu_mul_bf16(y, x->data_ptr(), x->numel() / (2 * n), n, st); });
+  return run(*x, with_last(*x, n), [&](void* y, void* st) { return abi.silu_mul_bf16(y, x->data_ptr(), x->numel() / (2 * n), n, st); });
   END_HANDLE_TH_ERRORS
 }
 
@@ -103,7 +123,7 @@ PyObject* add(PyObject*, PyObject* const* a, Py_ssize_t n_args) {   // a, b of o
   HANDLE_TH_ERRORS
   const at::Tensor *x, *z;
   if (n_args != 2 || modes() || !(x = plain(a[0])) || !(z = plain(a[1])) || x->sizes() != z->sizes()) Py_RETURN_NONE;
-  return run(*x, x->sizes(), [&](void* y, void* st) { return b200_add_bf16(y, x->data_ptr(), z->data_ptr(), x->numel(), st); });
+  return run(*x, x->sizes(), [&](void* y, void* st) { return abi.add_bf16(y, x->data_ptr(), z->data_ptr(), x->numel(), st); });
   END_HANDLE_TH_ERRORS
 }
 
@@ -115,7 +135,7 @@ PyObject* flash_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {   
   const int64_t B = q->size(0), Sq = q->size(1), Hq = q->size(2), D = q->size(3), Skv = k->size(1), Hkv = k->size(2);
   const int causal = a[3] == Py_True;
   return run(*q, q->sizes(), [&](void* y, void* st) {
-    return b200_attn_bf16(y, q->data_ptr(), k->data_ptr(), v->data_ptr(), B, Sq, Skv, Hq, Hkv, D, causal, st);
+    return abi.attn_bf16(y, q->data_ptr(), k->data_ptr(), v->data_ptr(), B, Sq, Skv, Hq, Hkv, D, causal, st);
   });
   END_HANDLE_TH_ERRORS
 }
@@ -130,7 +150,7 @@ PyObject* gemv_fused(PyObject*, PyObject* const* a, Py_ssize_t n_args) {   // x,
   const int64_t n = w->size(0) / nseg, k = w->size(1);
   const float eps = (float)PyFloat_AS_DOUBLE(a[3]);
   return run(*x, {n}, [&](void* y, void* st) {
-    return b200_gemv_fused_bf16(y, x->data_ptr(), w->data_ptr(), n, k, nseg, ptr(norm), eps, ptr(b), ptr(r), silu, st);
+    return abi.gemv_fused_bf16(y, x->data_ptr(), w->data_ptr(), n, k, nseg, ptr(norm), eps, ptr(b), ptr(r), silu, st);
   });
   END_HANDLE_TH_ERRORS
 }
@@ -150,18 +170,19 @@ PyObject* attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     Py_RETURN_NONE;
   }
   const int64_t ctx = kc->size(0), tickets = (4 * Hq + 15) / 16 * 16;
-  if (Hq < 1 || Hq > (1 << 20) || hd < 1 || hd > 1024 || b200_attn_decode_workspace_bytes(Hq, Hkv, hd, ctx) != tickets) Py_RETURN_NONE;
+  if (Hq < 1 || Hq > (1 << 20) || hd < 1 || hd > 1024 || abi.attn_decode_workspace_bytes(Hq, Hkv, hd, ctx) != tickets) Py_RETURN_NONE;
   const float eps = (float)PyFloat_AS_DOUBLE(a[11]);
   return run(*qkv, {Hq * hd}, [&](void* y, void* st) {   // no tickets are taken and no partials written: any address will do
-    return b200_attn_decode_bf16(y, qkv->data_ptr(), ptr(qn), ptr(kn), eps, (const float*)ptr(rope), (const int32_t*)ptr(pos), len, kc->data_ptr(),
+    return abi.attn_decode_bf16(y, qkv->data_ptr(), ptr(qn), ptr(kn), eps, (const float*)ptr(rope), (const int32_t*)ptr(pos), len, kc->data_ptr(),
                                  vc->data_ptr(), Hq, Hkv, hd, ctx, y, st);
   });
   END_HANDLE_TH_ERRORS
 }
 
 #define B200_OP(f) {#f, (PyCFunction)(void (*)(void))f, METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {B200_OP(linear), B200_OP(gemm),            B200_OP(rms_norm),   B200_OP(silu_mul),   B200_OP(add),
-                         B200_OP(flash_attention), B200_OP(gemv_fused), B200_OP(attn_decode), {nullptr, nullptr, 0, nullptr}};
+PyMethodDef methods[] = {{"_bind", bind, METH_O, nullptr}, B200_OP(linear),     B200_OP(gemm),        B200_OP(rms_norm),
+                         B200_OP(silu_mul),                B200_OP(add),        B200_OP(flash_attention),
+                         B200_OP(gemv_fused),              B200_OP(attn_decode), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "b200ops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
