@@ -1,7 +1,7 @@
 """Batched decode (B ≤ 8 sequences at the same position — GPTEngine::generateSync's left-padded batch,
 src/engine/GPTEngine.cpp:101-174): one weight pass per step for the whole batch (csrc/gemv_batch.cu: the B activation vectors
 are the n = 8 operand of tensor-core MMAs), attention with grid.z = B, per-sequence KV caches.  Everything but the
-GEMV's k-sum is the batch-1 arithmetic, so a batched run must agree with B independent batch-1 runs inside the
+GEMV's k-sum (and, over caches of more than eight splits, the number of key ranges) is the batch-1 arithmetic, so a batched run must agree with B independent batch-1 runs inside the
 summation-order floor — the gate of the TP-vs-single-GPU and engine-vs-reference-CUDA tests — with greedy ids equal
 wherever the top-2 margin is decisive."""
 import pytest

@@ -13,6 +13,7 @@
 // Numerics: q·k and P·V accumulate in fp32 over bf16 inputs; rounding points of q/k (after norm, after RoPE) are the
 // reference's.  Probabilities stay fp32 (the reference rounds P to bf16 before P·V, TFA/mma/layout.cuh:88-97); the
 // oracle models the reference's rounding and the parity tests bound the difference.
+#include "gemv.cuh"
 #include "key_range.cuh"
 #include "ops.cuh"
 #include "tc.cuh"
@@ -760,13 +761,18 @@ static int launch_row_g(const AttnRow& a, int splits, int B, cudaStream_t st, bo
   return a.G <= 4 ? launch_row_t<HD, 4, DECODE>(a, splits, B, st, pdl) : launch_row_t<HD, 8, DECODE>(a, splits, B, st, pdl);
 }
 // The heads of a CTA: the largest divisor of the group up to eight.  The CTAs of a cluster: as many (a power of two up to 16) as the SMs hold
-// clusters of at once, two CTAs to an SM (14 of 16 CTAs, 33 of 8, 71 of 4, 148 of 2), while each keeps 64 of `keys` keys.
+// clusters of at once, two CTAs to an SM (14 of 16 CTAs, 33 of 8, 71 of 4, 148 of 2), while each keeps 64 of `keys` keys.  Every CTA is a range of keys
+// with a maximum and sums of its own, so their number is part of a sequence's bits: a decoded batch takes what the largest one would, whatever
+// its size, and the limits are constants, not the chip's.  µs a token at positions 100 / 1 000 / 3 900, caches for 4 096, CTAs by the batch's own size → by
+// the largest: 28 layers, 8 KV heads of 128, two sequences 884 / 930 / 1 137 → 876 / 991 / 1 405, four 1 032 / 1 102 / 1 431 → 906 / 1 027 / 1 445, eight
+// the same; 24 layers, 2 KV heads of 64, two 577 / 579 / 628 → 576 / 589 / 709.  Sixteen ranges for every batch, several to a CTA with the same sums: four
+// sequences 1 039 / 1 315 / 1 629, the merges of the ranges cost more than the waves they save.
 static int launch_row(AttnRow& a, int hd, int64_t keys, int B, bool decode, cudaStream_t st, bool pdl) {
   const int group = a.d.Hq / a.d.Hkv;
   a.G = 1;
   for (int g = 2; g <= 8; ++g)
     if (group % g == 0) a.G = g;
-  const int64_t clusters = (int64_t)(a.d.Hq / a.G) * B;
+  const int64_t clusters = (int64_t)(a.d.Hq / a.G) * (decode && B > 1 ? std::max(B, kMaxBatch) : B);
   const int most = clusters <= 14 ? 16 : clusters <= 33 ? 8 : clusters <= 71 ? 4 : clusters <= 148 ? 2 : 1;
   int splits = 1;
   while (splits < most && keys >= 128 * splits) splits *= 2, ++a.log_splits;
