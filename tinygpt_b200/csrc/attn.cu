@@ -604,8 +604,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_row_kernel(const AttnRow
   }
   cluster_sync_all();                                  // every CTA's parts are in place
   const int r = tid & (splits - 1), j = tid >> a.log_splits, i = rank * share + j;   // a lane per CTA and four neighbouring outputs
-  if (j < share && i < G * LQ) {
-    const unsigned mask = __activemask();
+  const bool live = j < share && i < G * LQ;
+  const unsigned mask = __ballot_sync(0xffffffffu, live);   // the lanes that sum below: all of a CTA's parts of an output, or none
+  if (live) {
     const float2 ml = part_ml[r][i / LQ];
     const float4 x = part[r * share + j];
     float top = ml.x;
