@@ -168,7 +168,13 @@ int op_wait_check() {
   return w == nullptr || *(volatile unsigned*)w == 0 ? B200_OK : report_wait(__atomic_exchange_n(w, 0u, __ATOMIC_ACQ_REL));
 }
 
+bool pdl_on() {
+  static const bool on = !env_flag("B200_NO_PDL", false);
+  return on;
+}
+
 bool op_pdl(cudaStream_t st) {
+  if (!pdl_on()) return false;
   cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {   // the legacy stream beside a capture
     (void)cudaGetLastError();

@@ -53,6 +53,7 @@ extern std::atomic<int64_t> g_launches;
 // predecessor writes.  Weight prefetch (TMA into shared memory) is issued BEFORE pdl_wait() by the engines' launches.  A stand-alone operator's
 // operands may all come from the kernel in front: it waits before it reads any (the kernels' `late`), and only its launch, barriers, tensor
 // memory and descriptors run beside that kernel's end.
+bool pdl_on();                  // unless B200_NO_PDL=1, read with the first launch that asks
 bool op_pdl(cudaStream_t st);   // whether an operator may be launched so: not while the stream is captured (see engine_launch_token's note)
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

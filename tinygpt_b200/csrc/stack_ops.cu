@@ -11,10 +11,7 @@ namespace b200 {
 // Every kernel of this file starts with griddepcontrol.launch_dependents + griddepcontrol.wait, so it may be launched
 // ahead of the end of its predecessor (programmatic dependent launch): the launch latency hides behind the predecessor's
 // tail and nothing is read or written before the predecessor's results are complete.  B200_NO_PDL=1 turns it off.
-bool stack_pdl() {
-  static const bool on = !env_flag("B200_NO_PDL", false);
-  return on;
-}
+bool stack_pdl() { return pdl_on(); }
 
 namespace {
 
