@@ -58,3 +58,13 @@ def test_fp32_tails(built_lib, monkeypatch):
         got[side] = eng.forward(toks, True)
     assert all(torch.equal(got["tile"], got[side]) for side in WIDTHS)
     eng.close()
+
+
+@pytest.mark.parametrize("side", ["persistent128", "persistent0", "persistent257"])
+def test_a_width_that_is_not_built(built_lib, monkeypatch, side):
+    """Any of those that are: the persistent pairs all the same."""
+    x, w = rand(300, 136, seed=1), rand(456, 136, seed=2, scale=136 ** -0.5)
+    monkeypatch.setenv("B200_GEMM", "persistent")
+    want = ops.gemm(x, w)
+    monkeypatch.setenv("B200_GEMM", side)
+    assert torch.equal(ops.gemm(x, w), want)

@@ -762,7 +762,8 @@ void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   const bool tile = fits && forced == 't', wide = fits && forced == 'w', any_split = fits && !wide && forced != 'p';
   if (wide) consider(3, 1, 0.0);
   if (!tile) {
-    const int only = forced == 'p' ? std::atoi(env + std::strcspn(env, "0123456789")) : 0;   // "persistent224": that width
+    int only = forced == 'p' ? std::atoi(env + std::strcspn(env, "0123456789")) : 0;   // "persistent224": that width
+    if (only != kPairBN && only != 224 && only != 192) only = 0;                       // one that is not built: any
     for (int bn = kPairBN; bn >= 192; bn -= 32) {
       if (only != 0 && bn != only) continue;
       const int64_t t = up(M, 256) * up(N, bn / D), rounds = up(t, pairs);
