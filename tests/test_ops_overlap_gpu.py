@@ -3,7 +3,7 @@ kernel, right before it — activations, weights, caches and positions alike.  A
 import pytest
 import torch
 
-from tinygpt_b200 import ops
+from tinygpt_b200 import engine, models, ops, stack_bench
 
 pytestmark = pytest.mark.gpu
 
@@ -95,6 +95,60 @@ def test_captured_operators_have_plain_edges(built_lib):
             assert torch.equal(y.clone(), ops.linear(x + x, w)), i
     torch.cuda.synchronize()
     assert torch.equal(ops.linear(x, w), want)
+
+
+def test_operators_right_behind_a_graph(built_lib):
+    """An operator, and no torch kernel, is the first thing behind a graph's launch: it sees what the graph's last kernel has written, be that an operator's, a
+    torch kernel's or the engine's."""
+    r = maker(7)
+    x, w, n = r(8, 2048), r(4096, 2048, k=.02), r(2048, k=.1) + 1
+    xs = [r(8, 2048) for _ in range(20)]
+    st = torch.cuda.Stream()
+    st.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(st):
+        want = [(ops.linear(t + t, w), ops.rms_norm(t + t, n, 1e-6), ops.add(t + t, t + t)) for t in xs]
+        ends = []
+        for end in (ops.add, torch.add):
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=st):
+                y = end(x, x)
+            ends.append((graph, y))
+        torch.cuda.synchronize()
+        for graph, y in ends:
+            for t, (lin, norm, both) in zip(xs, want):
+                for call, expect in ((lambda: ops.linear(y, w), lin), (lambda: ops.rms_norm(y, n, 1e-6), norm), (lambda: ops.add(y, y), both)):
+                    x.copy_(t)
+                    y.zero_()
+                    graph.replay()
+                    assert torch.equal(call(), expect)
+
+
+def test_engine_and_operators_without_a_kernel_between(built_lib):
+    """Operators right behind a decode step's graph read its logits; a prompt right behind the operator that wrote its ids."""
+    spec = models.TINY_QWEN2
+    eng = engine.DecodeEngine(spec, {k: v.to("cuda") for k, v in models.synth_weights(spec, seed=3, std=0.05).items()})
+    attn = models.AttnSpec(4, 2, 64, 64, 0.125, 0, 0)
+    stack = models.StackSpec(name="w", architecture="Kozusun", width=256, vocab=spec.vocab, layers=(models.StackLayerSpec(attn, 512),) * 2, embed_scale=4.0,
+                             residual_mult=0.5, norm_eps=1e-5, norm_offset=1.0, max_ctx=256, max_slots=1)
+    other = engine.DecodeEngine(stack, stack_bench.device_stack_weights(stack, torch.device("cuda"), 8))
+    r = maker(8)
+    for i in range(10):
+        rows = r(40, spec.vocab)
+        ids = ops.argmax(rows, keepdim=False).view(1, -1)
+        torch.cuda.synchronize()
+        for e in (eng, other):
+            e.reset_cache()
+            want = e.forward(ids).clone()
+            step = e.forward(ids[:, -1:]).clone()
+            torch.cuda.synchronize()
+            e.reset_cache()
+            got = e.forward(ops.argmax(rows, keepdim=False).view(1, -1))
+            assert torch.equal(got, want), i
+            logits = e.forward(ids[:, -1:])
+            twice = ops.add(logits, logits)
+            assert torch.equal(logits, step) and torch.equal(twice, step + step), i
+    eng.close()
+    other.close()
 
 
 def test_the_switch_turns_operators_overlap_off(built_lib):
