@@ -722,7 +722,7 @@ int attn_heads_per_cta(int Hq, int Hkv, int max_ctx) {
   return 1;
 }
 
-int attn_setup_attributes() { return B200_OK; }   // the decode kernel uses static shared memory only
+int attn_setup_attributes() { return B200_OK; }   // attn_decode_reg_kernel has static shared memory only; launch_row_t sets attn_row_kernel's
 
 int attn_decode_nsplit(int hd, int max_ctx) {
   const int chunk = (hd == 64) ? SplitKeys<64>::value : SplitKeys<128>::value;

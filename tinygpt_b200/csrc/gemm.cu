@@ -97,7 +97,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sA = smem;                               // [stages][128 × 64 bf16]
   uint8_t* sB = smem + ST * kTileBytes;             // [stages][128 × 64 bf16]
-  uint8_t* patch = smem + ST * kPairStageBytes;     // [4 warps][32 rows × 128 bytes]
+  uint8_t* patch = smem + ST * kPairStageBytes;     // [8 warps][32 rows × 128 bytes]
   uint64_t* full = reinterpret_cast<uint64_t*>(patch + kPairEpiWarps * kPairPatch);   // CTA 0's count the pair's bytes
   uint64_t* empty = full + ST;
   uint64_t* tmem_full = empty + ST;                 // [2]
@@ -212,9 +212,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if (!ok) break;
       tc_fence_after();
       const int n_end = min(p.N, n0 + OUT);
-      if (grp * CW >= OUT && lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tmem_empty[acc]), 0));   // no chunk for this warp
 #pragma unroll 1
-      for (int c = grp * CW; c < OUT; c += 2 * CW) {   // of a last chunk that reaches past the tile, what lies there is not stored
+      for (int c = grp * CW; c < OUT; c += 2 * CW) {   // at least one chunk a warp (OUT is 96 and more); of a last chunk that reaches past the tile, what lies there is not stored
         if constexpr (EPI == GEPI_SILU) {           // 64 columns: gate at c, up at HB + c
           uint32_t g[32], u[32];
 #pragma unroll

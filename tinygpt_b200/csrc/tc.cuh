@@ -5,20 +5,15 @@
 
 namespace b200 {
 
-// shared-memory matrix descriptor, K-major, SWIZZLE_128B: start address >> 4 (bits 0-13), LBO = 0 (bits 16-29, unused
-// for swizzled K-major), SBO = 1024 B >> 4 (bits 32-45: 8 rows × 128 B between core-matrix groups), version 1
-// (bits 46-47), layout type 2 = SWIZZLE_128B (bits 61-63).
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
-  return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
 // kind::f16 instruction descriptor: D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1), A K-major (bit 15 = 0), B K-major or
 // (b_mn) MN-major (bit 16), N >> 3 at bits 17-22, M >> 4 at bits 24-28
 __host__ __device__ constexpr uint32_t umma_idesc(int m, int n, bool b_mn = false) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// Descriptors of that form in halves: the lower one holds the address, the upper one is the same for all.  An issuing thread that builds whole
-// descriptors per product takes 76 cycles for one, with halves and the upper one a constant 50.
+// Shared-memory matrix descriptor, K-major, SWIZZLE_128B, in halves.  The lower one holds start address >> 4 (bits 0-13) and LBO = 0 (bits 16-29, unused
+// for swizzled K-major).  The upper one is the same for all: SBO = 1024 B >> 4 (bits 32-45: 8 rows × 128 B between core-matrix groups), version 1
+// (bits 46-47), layout type 2 = SWIZZLE_128B (bits 61-63).  An issuing thread that builds whole descriptors per product does not keep up with the tensor pipe.
 constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr) { return (smem_addr & 0x3FFFFu) >> 4; }
 // one lane of a converged warp
@@ -42,14 +37,6 @@ __device__ __forceinline__ void umma_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t
         : "memory");
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
@@ -89,13 +76,6 @@ __device__ __forceinline__ int ld_cluster_i32(uint32_t addr) {
   int v;
   asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
   return v;
-}
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 // arrives on the barrier at this offset in the CTAs of the mask (bits = ranks in the cluster)
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask = 3) {

@@ -156,7 +156,7 @@ PyObject* gemv_fused(PyObject*, PyObject* const* a, Py_ssize_t n_args) {   // x,
 }
 
 // qkv, kcache, vcache, q_heads, kv_heads, head_dim, pos or None, fixed_len, rope table or None, q_norm or None, k_norm or None, eps: caches whose
-// attention takes no workspace
+// attention takes no workspace.  Shorter ones take tickets that are zeroed first, a torch kernel of its own that ops.py launches.
 PyObject* attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
   const at::Tensor *qkv, *kc, *vc, *pos, *rope, *qn, *kn;
