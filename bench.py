@@ -5,7 +5,7 @@
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 --master-port P \
         bench.py --gpus N --steps K --warmup W
 
-A "step" is ONE 128-token greedy decode of one sequence (Qwen2.5-0.5B bf16, batch 1,
+A "step" is ONE 128-token greedy decode of one sequence (the headline workload: Qwen2.5-0.5B bf16, batch 1,
 128-token decode) continuing a 16-token prompt: rewind to position 16, run 128 engine steps on the device.
 `value` = decoded tokens / second with everything resident in HBM (CUDA events on the launching stream).
 `e2e`   = the same through the public API with HOST buffers: DecodeEngine.generate_sync(prompt ids on the host) —
@@ -356,7 +356,7 @@ def explain_id_agreement(eng, prompt, resident_toks, host_toks, spec):
 
 
 def measure_extra_model(name, world, rank, dev, d: Dist, steps, tp_mode):
-    """Decode tokens/s of another BASELINE config in the same job (same prompt length / token count / timing method).
+    """Decode tokens/s of another configuration in the same job (same prompt length / token count / timing method).
     N = 1: one GPU.  N > 1: tensor parallel over the N ranks plus, on rank 0, the one-GPU engine of the same model, so that
     the scaling curve of the models tensor parallelism is for comes out of one job."""
     import torch
@@ -428,7 +428,7 @@ def measure_batched_decode(spec, w, dev, hbm_peak):
 
 
 def measure_prefill_config(dev, steps=2):
-    """BASELINE config 4: Qwen3-1.7B, prefill of 2 048 prompt tokens (tcgen05 GEMMs + tensor-core causal attention) and
+    """Qwen3-1.7B, prefill of 2 048 prompt tokens (tcgen05 GEMMs + tensor-core causal attention) and
     256 decode steps at ctx 2 048 → 2 304.  Prefill against the measured cuBLAS bf16 peak, decode against HBM."""
     import torch
     from tinygpt_b200 import engine, models
@@ -533,7 +533,7 @@ def run_ours(args):
     agreement = explain_id_agreement(eng, prompt, toks, host_toks, spec) if world == 1 else {
         "free_running_equal_fraction": float((host_toks == toks.cpu()).float().mean())}
 
-    # ---- the other BASELINE configs, same job (every rank takes part under tensor parallelism)
+    # ---- the other configurations, same job (every rank takes part under tensor parallelism)
     others = []
     if not args.no_other_configs and args.model == "Qwen2.5-0.5B":
         eng_keep = eng
@@ -594,7 +594,7 @@ def run_ours(args):
         ref = CpuReference(args.model)
         v, sample = ref.step(8)
         cpu = {"value": v, "unit": "tokens/s", "cores": ref.cores, "kind": ref.kind, "sample": sample}
-        # BASELINE config 1 — GPT-2 124M fp32 `--device cpu`, 32 new tokens: the one family whose forward exists on the
+        # GPT-2 124M fp32 `--device cpu`, 32 new tokens: the one family whose forward exists on the
         # reference's CPU path unmodified (examples/inference/main.cpp:39-62); reported once, beside the headline's arm
         if ref.kind == "reference":
             try:
@@ -671,7 +671,7 @@ def main():
     ap.add_argument("--model", default="Qwen2.5-0.5B")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-other-configs", action="store_true",
-                    help="skip the other BASELINE configs (Llama-3.2-3B, Qwen3-1.7B prefill, Mistral-7B TP) in the same job")
+                    help="skip the other configurations (Llama-3.2-3B, Qwen3-1.7B prefill, Mistral-7B TP) in the same job")
     ap.add_argument("--mode", default="tp", choices=["tp", "replicas"],
                     help="N > 1: tensor parallel over one sequence (default, strong scaling) or independent replicas")
     ap.add_argument("--stack-compare", nargs="?", const="all", default=None, metavar="SIZES",

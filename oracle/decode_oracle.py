@@ -5,13 +5,12 @@ This file restates, on the CPU, the arithmetic of the reference's CUDA path for 
 in tinygpt_b200/csrc; nothing in the product path may import it (only tests/, __graft_entry__.smoke() and bench.py's
 cpu_baseline / --impl reference legs do).  The product path has no CPU fallback.
 
-Pinning status (see DESIGN.md "Oracle"):
+Pinning status:
   * pinned against the reference's own golden vectors (tests/golden/reference_vectors.json: func_rmsNorm, func_silu,
     func_linear, func_sdpAttention, TEST_Module.rope) — tests/test_oracle_golden.py;
-  * pinned against outputs of the reference itself, compiled from /root/reference by oracle/Makefile into
+  * pinned against outputs of the reference itself, compiled from its sources by oracle/Makefile into
     oracle/_ref and run on the CPU in fp32 (per-op and whole-model logits; fixtures in tests/golden/ref_cpu_*.npz);
-  * the bf16 rounding points follow the reference's CUDA sources by reading (cited per function); the reference's
-    CUDA build cannot run in the build container (no GPU) and its sources cannot travel to the GPU box, and cuBLAS'
+  * the bf16 rounding points follow the reference's CUDA sources by reading (cited per function); cuBLAS'
     summation order is not reproducible — so bf16 parity is "within tolerance", never bit-exact, except where the
     arithmetic is exact (embedding, add, argmax, KV append).
 

@@ -1,7 +1,7 @@
 // ref_cuda_main.cpp — TEST INFRASTRUCTURE.  Runs the UNMODIFIED reference's CUDA path (keith2018/TinyGPT: its modules,
 // TinyTorch CUDA ops, cuBLAS GEMMs, TinyFA attention, its KV-cache manager and its own argmax), compiled from
 // /root/reference by `make -C oracle cuda`, on a checkpoint directory written by tinygpt_b200.models.save_checkpoint:
-// the bf16 parity oracle north_star names ("logits matching the reference CUDA path … bit-exact argmax ids") and the
+// the bf16 parity oracle, and the
 // reference's own decode speed on the same GPU.  Nothing in the product links or loads this.
 //
 //   ref_cuda_decode --ckpt DIR --family {llama|qwen2|qwen3|mistral} --dims H,L,Hq,Hkv,hd,I,V,ctx --theta T --eps E

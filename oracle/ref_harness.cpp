@@ -247,7 +247,7 @@ void* ref_model_create(const RefModelDesc* d) {
       else
         m->model = std::make_unique<tinygpt::ModelQwen3>(m->qwen, cpu);
       break;
-    case 4:   // BASELINE config 1: GPT-2, the only family whose forward exists on the reference's CPU path unmodified
+    case 4:   // GPT-2, the only family whose forward exists on the reference's CPU path unmodified
       fillCommon(m->gpt2, *d);
       m->gpt2.activationFunction = "gelu_new";
       m->gpt2.layerNormEpsilon = d->rms_eps;

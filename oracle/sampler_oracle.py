@@ -1,4 +1,4 @@
-"""TEST INFRASTRUCTURE — CPU restatement of the reference's sampler (SURVEY.md §8f rank 1: the part of the async token
+"""TEST INFRASTRUCTURE — CPU restatement of the reference's sampler (the part of the async token
 pipeline that is not greedy).  Nothing in the product imports this.
 
     tinygpt::Sampler::sample           src/engine/Sampler.cpp:23-78

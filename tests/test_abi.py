@@ -120,7 +120,7 @@ def test_product_does_not_import_the_oracle():
 def test_model_byte_counts_match_survey():
     from tinygpt_b200 import models
     want = {"Qwen2.5-0.5B": 987_922_432, "Llama-3.2-3B": 6_425_149_440, "Qwen3-1.7B": 3_440_902_144,
-            "Mistral-7B-v0.3": 14_227_079_168}  # SURVEY.md §8d weights-only bytes per token
+            "Mistral-7B-v0.3": 14_227_079_168}  # weights-only bytes per token
     for name, b in want.items():
         assert 2 * models.SPECS[name].weight_params == b
 

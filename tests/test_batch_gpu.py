@@ -175,7 +175,7 @@ def test_batched_through_the_adapter_inside_the_reference(built_lib):
     sys.path.insert(0, str(Path(__file__).resolve().parent.parent / "tools"))
     import ref_cuda_parity as rp
     if not rp.REF_BIN.exists():
-        pytest.skip("oracle/_ref/ref_cuda_decode not built (needs /root/reference: make -C oracle cuda)")
+        pytest.skip("oracle/_ref/ref_cuda_decode not built (needs the reference's sources: make -C oracle cuda)")
     spec = models.TINY_QWEN2
     w = models.synth_weights(spec, seed=0)
     B, S, n = 4, 16, 8

@@ -1,18 +1,17 @@
 """Whole-token parity of the engine (boundary A) against the oracle.
 
-Tolerance.  north_star asks for logits within 1e-3 (bf16) of the reference CUDA path and bit-exact greedy ids.  An
+Tolerance.  The aim is logits within 1e-3 (bf16) of the reference CUDA path and bit-exact greedy ids.  An
 absolute 1e-3 is below ONE bf16 ulp of an O(1) logit (2^-8 … 2^-7) and, measured here, below the pipeline's own
 sensitivity to summation order: the oracle against ITSELF with fp64 instead of fp32 accumulation (same rounding
 points, teacher-forced) differs by mean 8e-3 / max 5e-2 on Qwen2.5-0.5B, because ~50 bf16 roundings of the hidden
-state amplify every 1-ulp flip.  cuBLAS' order is not reproducible either (SURVEY.md §8a a6).  The gate is therefore
+state amplify every 1-ulp flip.  cuBLAS' order is not reproducible either.  The gate is therefore
 the noise floor itself, computed inside the test:
   * floor = |oracle − oracle'| on the same forced tokens, where oracle' accumulates every Linear in fp64 and keeps the
     attention probabilities in fp32 (the reference rounds them to bf16; our kernel does not) — same rounding points
     for every stored tensor;
   * mean |engine − oracle| ≤ 1.5 × floor.mean + 1e-4  and  max |engine − oracle| ≤ 2 × floor.max + 1 ulp
     (the 1e-3 figure is reported next to it, and holds where the floor allows: the 2-layer models);
-  * greedy ids identical wherever the oracle's top-2 margin exceeds 2 × floor.max (near-ties counted and reported,
-    SURVEY.md §7 "hard parts"); the engine's argmax always equals the reference tie rule applied to its own logits;
+  * greedy ids identical wherever the oracle's top-2 margin exceeds 2 × floor.max (near-ties counted and reported); the engine's argmax always equals the reference tie rule applied to its own logits;
   * exact ties (all-equal logits) → HIGHEST index, bit-exact.
 """
 import pytest
@@ -79,7 +78,7 @@ def check_parity(name, toks_gpu, logits_gpu, toks_orc, logits_orc, logits_alt):
     print(f"[{name}] engine-vs-oracle mean|Δ|={mean_err:.3e} max|Δ|={max_err:.3e}; oracle summation-order floor "
           f"mean={floor_mean:.3e} max={floor_max:.3e}; bf16 ulp at max logit {ulp:.3e}; "
           f"bit-identical logits {float((logits_gpu == logits_orc).float().mean()):.4f}; "
-          f"north_star 1e-3 {'met' if mean_err <= 1e-3 else 'below the noise floor of this model'}")
+          f"1e-3 {'met' if mean_err <= 1e-3 else 'below the noise floor of this model'}")
     assert mean_err <= 1.5 * floor_mean + 1e-4, f"{name}: mean logit error {mean_err} vs floor {floor_mean}"
     assert max_err <= 2 * floor_max + ulp, f"{name}: max logit error {max_err} vs floor {floor_max}"
     # argmax on the engine's own logits follows the reference tie rule
@@ -145,7 +144,7 @@ def test_engine_state_and_errors(built_lib):
 
 
 def test_qwen25_05b_full_size_parity(built_lib):
-    """BASELINE config 2 at its real shape: synthetic Qwen2.5-0.5B, 16-token prompt, oracle-checked decode steps."""
+    """The headline model at its real shape: synthetic Qwen2.5-0.5B, 16-token prompt, oracle-checked decode steps."""
     spec = models.QWEN25_05B.with_ctx(256)
     check_parity(spec.name, *run_parity(spec, prompt_len=16, new_tokens=6))
 

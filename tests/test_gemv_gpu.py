@@ -1,5 +1,5 @@
 """Parity of the weight-streaming GEMV (plain and fused variants) against the oracle at every (n, k) of the decode
-path (SURVEY.md §8a) plus ragged shapes.  Tolerance: ≤ 1 bf16 ulp (fp32 summation order differs from the oracle's
+path plus ragged shapes.  Tolerance: ≤ 1 bf16 ulp (fp32 summation order differs from the oracle's
 and from cuBLAS'; products are exact), or 1e-4 absolute near zero; ≥ 98 % of elements bit-identical."""
 import pytest
 import torch

@@ -1,4 +1,4 @@
-"""Per-op parity of the sm_100a kernels (through the C ABI) against the CPU oracle — boundary B of SURVEY.md §8b.
+"""Per-op parity of the sm_100a kernels (through the C ABI) against the CPU oracle — the operator boundary.
 
 Tolerances (stated per test): exact for copy/compare ops (embedding, add, argmax, silu_mul given identical inputs up
 to expf ulp), ≤ 1 bf16 ulp where fp32 summation order or rsqrt/exp implementation differs from the oracle's."""

@@ -1,6 +1,6 @@
 """The reference's OWN CUDA path (oracle/_ref/ref_cuda_decode: unmodified TinyTorch CUDA ops + cuBLAS + TinyFA, built by
-`make -C oracle cuda` where /root/reference exists; the binary travels to the GPU box) as the parity oracle north_star
-names, and the drop-in boundary exercised INSIDE that program (integration/tinytorch_b200_adapter.h).  Skipped only
+`make -C oracle cuda` where the reference's sources are) as the parity
+oracle, and the drop-in boundary exercised INSIDE that program (integration/tinytorch_b200_adapter.h).  Skipped only
 when the binary is absent.  Full-size numbers for the four models: tools/ref_cuda_parity.py →
 profiles/r02_ref_cuda_parity.json."""
 import pytest
@@ -15,7 +15,7 @@ DEV = "cuda"
 # ------------------------------------------------------------- the reference's own CUDA path as the oracle (oracle/_ref)
 def test_engine_and_oracle_against_reference_cuda(built_lib):
     """oracle/_ref/ref_cuda_decode = the UNMODIFIED reference CUDA build (TinyTorch ops + cuBLAS + TinyFA), compiled in
-    the container that has /root/reference (`make -C oracle cuda`).  Same synthetic checkpoint, same forced tokens:
+    a container that has the reference's sources (`make -C oracle cuda`).  Same synthetic checkpoint, same forced tokens:
     engine vs reference and oracle vs reference within the summation-order floor (cuBLAS' order is not ours), greedy
     ids equal wherever the reference's own top-2 margin is decisive."""
     import sys
@@ -24,7 +24,7 @@ def test_engine_and_oracle_against_reference_cuda(built_lib):
     sys.path.insert(0, str(root / "tools"))
     import ref_cuda_parity as rp
     if not rp.REF_BIN.exists():
-        pytest.skip("oracle/_ref/ref_cuda_decode not built (needs /root/reference: make -C oracle cuda)")
+        pytest.skip("oracle/_ref/ref_cuda_decode not built (needs the reference's sources: make -C oracle cuda)")
     import tempfile
     from tinygpt_b200 import ops
     for spec in (models.TINY_QWEN2, models.TINY_LLAMA, models.TINY_QWEN3, models.TINY_MISTRAL):
@@ -53,8 +53,8 @@ def test_engine_and_oracle_against_reference_cuda(built_lib):
 
 @pytest.mark.parametrize("name,n", [("Qwen2.5-0.5B", 12), ("Qwen3-1.7B", 5), ("Llama-3.2-3B", 5), ("Mistral-7B-v0.3", 4)])
 def test_full_size_against_reference_cuda_and_its_own_noise_floor(built_lib, name, n):
-    """The four BASELINE models at FULL size (qkv bias / QK-norm / llama3 RoPE scaling + 24:8 GQA at hd 128 / untied head),
-    teacher-forced on our tokens, against the reference's own CUDA path.  north_star asks for 1e-3 on the logits; no
+    """The four models at FULL size (qkv bias / QK-norm / llama3 RoPE scaling + 24:8 GQA at hd 128 / untied head),
+    teacher-forced on our tokens, against the reference's own CUDA path.  The aim is 1e-3 on the logits; no
     two summation orders reach that on an O(1) bf16 logit (1 ulp = 0.0078 … 0.0625), and the reference does not reach it
     against ITSELF: its decode path vs its own batched path (one forward over prompt + forced tokens, other cuBLAS
     kernels) is the measured floor (0 for the shapes where cuBLAS happens to pick the same kernel twice).  Gate:
@@ -67,7 +67,7 @@ def test_full_size_against_reference_cuda_and_its_own_noise_floor(built_lib, nam
     sys.path.insert(0, str(Path(__file__).resolve().parent.parent / "tools"))
     import ref_cuda_parity as rp
     if not rp.REF_BIN.exists():
-        pytest.skip("oracle/_ref/ref_cuda_decode not built (needs /root/reference: make -C oracle cuda)")
+        pytest.skip("oracle/_ref/ref_cuda_decode not built (needs the reference's sources: make -C oracle cuda)")
     spec = models.SPECS[name].with_ctx(256)
     w = models.synth_weights(spec, seed=0, device=DEV, device_generator=True)
     prompt = torch.randint(0, spec.vocab, (16,), generator=torch.Generator().manual_seed(0)).tolist()
@@ -105,7 +105,7 @@ def test_drop_in_boundary_inside_the_real_reference(built_lib):
     sys.path.insert(0, str(Path(__file__).resolve().parent.parent / "tools"))
     import ref_cuda_parity as rp
     if not rp.REF_BIN.exists():
-        pytest.skip("oracle/_ref/ref_cuda_decode not built (needs /root/reference: make -C oracle cuda)")
+        pytest.skip("oracle/_ref/ref_cuda_decode not built (needs the reference's sources: make -C oracle cuda)")
     for spec in (models.TINY_QWEN2, models.TINY_QWEN3, models.TINY_MISTRAL):
         w = models.synth_weights(spec, seed=0)
         prompt = torch.randint(0, spec.vocab, (16,), generator=torch.Generator().manual_seed(0)).tolist()

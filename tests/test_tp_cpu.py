@@ -143,7 +143,7 @@ def test_shard_weights_partition_is_exact():
 
 def test_unshardable_configs_are_rejected():
     from tinygpt_b200._lib import B200Error
-    assert not tp.can_shard_attention(models.QWEN25_05B, 4)      # 14 / 2 heads: only 2-way (SURVEY §8e)
+    assert not tp.can_shard_attention(models.QWEN25_05B, 4)      # 14 / 2 heads: only 2-way
     assert tp.can_shard_attention(models.QWEN25_05B, 2)
     assert all(tp.can_shard_attention(models.MISTRAL_7B, n) for n in (2, 4, 8))
     with pytest.raises(B200Error):

@@ -1,4 +1,4 @@
-"""Tensor-parallel engine on 2, 4 and 8 GPUs (run with `gpurun --gpus N`; cases that need more GPUs than the box has are
+"""Tensor-parallel engine on 2, 4 and 8 GPUs (cases that need more GPUs than there are are
 skipped): logits and greedy ids against the single-GPU engine and, through it, the oracle.  Tolerance: the two row-parallel GEMVs per layer sum in a different order than the single
 GPU engine (fp32 partials per rank, then rank order), everything else is identical arithmetic — compare like
 tests/test_engine_gpu.py does, against the oracle's own summation-order floor."""
@@ -68,7 +68,7 @@ CASES = [(2, "tiny-mistral", True), (2, "tiny-qwen3", True), (2, "tiny-qwen2", T
 @pytest.mark.parametrize("world,spec_name,shard_attn", CASES, ids=lambda v: str(v))
 def test_tp_matches_single_gpu(built_lib, world, spec_name, shard_attn):
     if torch.cuda.device_count() < world:
-        pytest.skip(f"needs {world} GPUs (gpurun --gpus {world})")
+        pytest.skip(f"needs {world} GPUs")
     import torch.multiprocessing as mp
     ctx = mp.get_context("spawn")
     q = ctx.Queue()

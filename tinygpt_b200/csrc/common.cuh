@@ -21,7 +21,7 @@ void set_error(const char* fmt, ...);
 // ------------------------------------------------------------------------------- selectable code paths and their defaults
 // The environment variable overrides the default BOTH ways (the named value), so a measured alternative stays one
 // variable away.  Variants that were measured and lost (flag synchronisation, register-resident small-k GEMV loop,
-// cross-kernel L2 prefetch, whole-token persistent kernel) are not here any more: profiles/experiments/.
+// cross-kernel L2 prefetch, whole-token persistent kernel) are not here any more: profiles/not_kept.md.
 struct Defaults {
   static constexpr bool kPrefillAttnMma = true;   // B200_PREFILL_ATTN   "mma" (tensor cores) | "cuda" (CUDA cores)
   // B200_GEMM "persistent" | "tile" | "wide": chosen per shape when unset (gemm.cu pick_gemm)
@@ -189,7 +189,7 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
 // L2 eviction-priority hint for the weight stream: a decode token streams ~8 × the L2 capacity of weights, each byte
 // once.  Tagging the stream evict_first keeps the lines every kernel re-reads (activations, KV cache, code) resident:
 // measured −1.5 % per token on Qwen2.5-0.5B and Mistral-7B, −2.4 % on the batched Mistral step.  (evict_last on the RMSNorm
-// weights measured no change.)  profiles/experiments/r02_l2_hints.txt
+// weights measured no change.)
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
   uint64_t pol;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));

@@ -7,8 +7,8 @@
 // passes per step; decode is weight-bound, so B sequences should cost (almost) one.  [B ≤ 8, k] × [k, n] is GEMM-shaped
 // work: on the tensor cores the consumer side costs ~25 warp instructions per 16 KB stage whatever B is, and the step
 // stays bound by the weight stream.  (A first version repeated gemv_stream_kernel's CUDA-core arithmetic per sequence —
-// bit-identical to batch 1, but B × the FMAs per weight vector: a B = 8 step cost 4.1-4.5 × a batch-1 step.  It is kept,
-// with its numbers, under profiles/experiments/r02_batched_gemv_cuda_core/.)  The price: the k-sum of a row is taken in
+// bit-identical to batch 1, but B × the FMAs per weight vector: a B = 8 step cost 4.1-4.5 × a batch-1 step;
+// numbers in profiles/not_kept.md.)  The price: the k-sum of a row is taken in
 // tensor-core order (fp32 accumulation of exact bf16 products, 8 k-slices added in warp order), so a batched step agrees
 // with batch-1 steps to summation-order noise instead of bit for bit — exactly the relation between the reference's own
 // m = 1 and m = B paths (profiles/r02_ref_cuda_parity.json, "reference_cuda_decode_vs_its_own_batched_path").
@@ -217,7 +217,7 @@ gemv_batch_kernel(const GemvParams p, const __grid_constant__ CUtensorMap tmap) 
     // RMSNorm, one WARP per sequence: lane-strided loads, sum of squares by shuffle only, no cross-warp reduction; the
     // norm weight goes through shared memory.  The partition of the sum of squares differs from the batch-1 kernel's,
     // which is inside the summation-order tolerance this kernel already has.
-    // OPEN (profiles/r02_trace_batch_prologue.log): this prologue takes 2.5-2.7 µs per kernel against 0.8 µs at batch 1
+    // OPEN: this prologue takes 2.5-2.7 µs per kernel against 0.8 µs at batch 1
     // and 0.65 µs for the plain staging above.  Ruled out by measurement: the norm-weight load (hoisting it above the
     // wait or above the first barrier, L2 evict_last, a copy on hot pages — no change).  Diagnosis from the stamps: with
     // k/8/32 < 8 the unroll-by-8 body of the x loop below never executes and the remainder loop runs its 3-4

@@ -1,4 +1,4 @@
-"""tcgen05 prefill GEMM alone, at the Linear shapes of BASELINE config 4 (Qwen3-1.7B, 2 048 prompt tokens): TFLOP/s of
+"""tcgen05 prefill GEMM alone, at the Linear shapes of a long prompt (Qwen3-1.7B, 2 048 prompt tokens): TFLOP/s of
 the one-tile-per-CTA kernel (B200_GEMM=tile) and of the persistent 256×256 pair kernel (B200_GEMM=persistent) against the measured cuBLAS
 bf16 peak in MEASURED_PEAKS.json.  CUDA events on the current stream, operands cycled so that B never sits in L2."""
 import json

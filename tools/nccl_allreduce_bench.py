@@ -1,7 +1,6 @@
-"""What would north_star's literal design cost?  It names "a single NCCL all-reduce on the hidden vector per layer"; the
-engine instead fuses the reduction into the GEMV kernels (fp32 partials pushed into peer windows as {value, tag} words,
-DESIGN.md §6).  This measures the NCCL side of that comparison on the same box: latency of an in-graph
-`ncclAllReduce` of one hidden vector (bf16 H and fp32 H elements, H of the four BASELINE models), back to back on one
+"""What would an NCCL all-reduce of the hidden vector per reduction cost?  The
+engine fuses the reduction into the GEMV kernels (fp32 partials pushed into peer windows as {value, tag} words).  This measures the NCCL side of that comparison on the same box: latency of an in-graph
+`ncclAllReduce` of one hidden vector (bf16 H and fp32 H elements, H of the four models), back to back on one
 stream inside a CUDA graph like a decode token would issue them, so that the per-token cost of 2·L all-reduces can be
 set against the measured exchange cost of the fused path (tools/trace_tp.py).
 
@@ -23,7 +22,7 @@ def main():
     for name, (H, L) in models.items():
         for dtype in (torch.bfloat16, torch.float32):
             x = torch.ones(H, dtype=dtype, device=dev)
-            n_ar = 2 * L                       # two reductions per layer for exact parity (SURVEY §8e)
+            n_ar = 2 * L                       # two reductions per layer for exact parity
             for _ in range(5):
                 dist.all_reduce(x)
             torch.cuda.synchronize()

@@ -1,4 +1,4 @@
-"""Extract the judged metrics from .ncu-rep files into a markdown table (run here, no GPU needed)."""
+"""Extract the main metrics from .ncu-rep files into a markdown table (no GPU needed)."""
 import csv
 import subprocess
 import sys

@@ -1,4 +1,4 @@
-"""prefill S tokens (tcgen05 GEMM path) + decode N tokens, timed with CUDA events.
+"""Prefill S tokens (tcgen05 GEMM path) + decode N tokens, timed with CUDA events.
     python tools/prefill_bench.py [model] [S] [N]"""
 import os
 import sys

@@ -1,9 +1,8 @@
-"""Engine and oracle against the REFERENCE'S OWN CUDA PATH on the same GPU (north_star: "logits matching the reference
-CUDA path within 1e-3 (bf16) / bit-exact for argmax token ids on the same prompts").
+"""Engine and oracle against the REFERENCE'S OWN CUDA PATH on the same GPU (the aim: logits within 1e-3 (bf16),
+bit-exact argmax token ids on the same prompts).
 
 oracle/_ref/ref_cuda_decode is the unmodified reference (TinyTorch CUDA ops + cuBLAS + TinyFA + its KV-cache manager +
-its argmax) compiled from /root/reference by `make -C oracle cuda` in the build container; it travels to the GPU box as
-a binary.  For every model this script
+its argmax) compiled from the reference's sources by `make -C oracle cuda`.  For every model this script
   1. writes the seeded synthetic checkpoint in the reference loader's layout (models.save_checkpoint),
   2. runs our engine (free-running greedy decode, then logits teacher-forced on its own tokens),
   3. runs the reference CUDA path teacher-forced on the SAME tokens, and once free-running,
@@ -12,7 +11,7 @@ and reports |engine − reference|, |oracle − reference| (this pins the oracle
 could not be pinned without a GPU), greedy-id agreement, and the reference's own decode speed next to ours.
 
     python tools/ref_cuda_parity.py [--models tiny-qwen2,tiny-llama,tiny-qwen3,tiny-mistral,Qwen2.5-0.5B] [--new 24]
-                                    [--json gpurun_out/ref_cuda_parity.json]
+                                    [--json ref_cuda_parity.json]
 """
 from __future__ import annotations
 
@@ -125,7 +124,7 @@ def main():
     ap.add_argument("--prefill", default="", help="MODEL:TOKENS, e.g. Qwen3-1.7B:2048 — time the prefill of both paths")
     args = ap.parse_args()
     if not REF_BIN.exists():
-        raise SystemExit(f"{REF_BIN} is missing: build it in the container that has /root/reference (make -C oracle cuda)")
+        raise SystemExit(f"{REF_BIN} is missing: build it where the reference's sources are (make -C oracle cuda)")
     from helpers import orc, to_oracle_cfg
     report = []
     for name in args.models.split(","):
@@ -201,7 +200,7 @@ def main():
                     row[f"reference_with_b200_{mode}"] = {"failed": str(e)[:400]}
         report.append(row)
         print(json.dumps(row), flush=True)
-    # config 4 of BASELINE.json: prefill of a long prompt, the reference's own path vs ours (timing only)
+    # prefill of a long prompt, the reference's own path vs ours (timing only)
     if args.prefill:
         name, plen = args.prefill.split(":")
         plen = int(plen)
