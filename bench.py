@@ -578,7 +578,7 @@ def run_ours(args):
          "achieved_gbs": gu_bytes / t_gu / 1e6, "frac": gu_bytes / t_gu / 1e6 / peak,
          "how": f"{4 * spec.layers} launches back to back over the {spec.layers} layers' matrices (stand-alone op: host "
                 "launch gaps included, no PDL overlap — inside the token graph the same kernel's body is "
-                "profiles/r02_trace_*.log)"},
+                "tools/trace_decode.py)"},
     ]
     traffic = None
     tpath = ROOT / "profiles" / "traffic.json"

@@ -311,10 +311,10 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_reg_kernel(const Att
 //
 // Against eight CTAs per one or two heads, which read K and V once per head in eight dependent rounds of register loads: device µs, rotating caches of 4 096
 // tokens, positions 100 / 1 000 / 2 000 / 4 000: 16 / 8 heads of 128 5.1 / 6.6 / 8.7 / 12.2 → 5.4 / 5.8 / 6.7 / 9.9, 24 / 8 heads 5.3 / 6.8 / 9.2 / 13.0 →
-// 5.8 / 6.0 / 7.3 / 10.9, 14 / 2 heads of 64 4.6 / 5.3 / 5.9 / 7.2 → 5.2 / 5.2 / 5.6 / 6.9.  Where it counts, inside a token, the loads run beside the
-// kernel in front: 28 layers, 2 048 wide, ctx 4 096 802 / 866 / 919 / 1 014 → 787 / 811 / 838 / 909 µs a token, 24 layers, 896 wide 440 / 449 / 461 / 501 →
-// 427 / 431 / 436 / 460.  Eight CTAs at most instead of sixteen: 0.3 µs less at short positions, 0.7 … 2 more at long ones, and tokens behind
-// in both (4 000: 1 021).  Barriers over the whole CTA in every unit: 6.9 µs at position 100.
+// 5.8 / 6.0 / 7.3 / 10.9, 14 / 2 heads of 64 4.6 / 5.3 / 5.9 / 7.2 → 5.2 / 5.2 / 5.6 / 6.9.  Inside a token the loads run beside the
+// kernel in front: µs a token at positions 100 / 1 000 / 3 900, caches for 4 096, 28 layers, 2 048 wide 804 / 869 / 1 035 → 826 / 834 / 913, 24 layers, 896 wide
+// 452 / 461 / 509 → 432 / 437 / 465.  Eight CTAs at most instead of sixteen: 0.3 µs less at short positions, 0.7 … 2 more at long ones, and long
+// tokens behind (4 000: 1 021).  Barriers over the whole CTA in every unit: 6.9 µs at position 100.
 struct AttnRow {
   AttnDecodeParams d;               // decode: everything; row: qkv = q [B, Hq, HD], out, kcache / vcache and the strides
   int nkeys;                        // row: keys to see (decode reads the position)

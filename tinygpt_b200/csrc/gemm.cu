@@ -14,8 +14,8 @@
 //   warp 0   TMA producer: 64-column k-blocks of A and B (128-byte swizzle) into a shared-memory ring, completion on `full[s]`
 //   warp 1   MMA issuer: one thread issues 4 × tcgen05.mma.kind::f16 (K16) per k-block, accumulator in TMEM; tcgen05.commit
 //            releases the stage to the producer (`empty[s]`) and signals the epilogue (`tmem_full`).  It looks at the next stage's barrier
-//            before it issues, and builds half descriptors: 64 cycles a k-block, where a wait of its own (210) and whole descriptors (305)
-//            took longer than the products of any tile (512 at 256 columns a pair).  µs, 2 048 rows: 3 072 × 8 192 85 → 75 (with 192-column
+//            before it issues, and builds half descriptors: with a wait in every k-block and whole descriptors the issuer, not the products, set the
+//            pace.  µs, 2 048 rows: 3 072 × 8 192 85 → 75 (with 192-column
 //            tiles), 16 384 × 3 072 137 → 133, 12 288 × 2 048 76 → 70.5; 17 × 2 048 × 6 144 on one-CTA tiles 27 → 23
 //   the other warps: epilogue, tcgen05.ld 32x32b (each warp owns the TMEM lane quarter warp_id % 4)
 // TMA zero-fills out-of-range rows/columns, so M, N, K need not be multiples of the tile.  Every wait is bounded: one that gives up
@@ -74,8 +74,8 @@ __device__ __forceinline__ uint32_t silu_mul2(uint32_t g0, uint32_t g1, uint32_t
 // accumulator is double-buffered in TMEM (256 columns apart): the epilogue of tile i drains one buffer while the MMA warp
 // fills the other.  Eight epilogue warps, two to a quarter of the rows, turn rows of TMEM lanes into whole 128-byte row pieces through a swizzled
 // 4 KB patch per warp and store 16 bytes per lane along the row (four of them took 13 µs for SiLU products of a 256 × 256 tile, as long as
-// K = 2 048).  Bound by the tensor pipe under the power cap (a k-block of 256 columns takes 512 cycles, its products' own time; 192 columns
-// take 406, 128 no less: operands from L2, 70 bytes per cycle and SM).  The width is what wastes least in the last round of tiles, any
+// K = 2 048).  Bound by the tensor pipe under the power cap (87 % of the active cycles, at 224 and 192 columns;
+// profiles/prompt_kernels_ncu.md).  The width is what wastes least in the last round of tiles, any
 // width sums the same bits: 2 048 × 3 072 × 8 192 is 96 tiles of 256 (two rounds of 74 pairs, 83.6 µs) or 128 of 192 (75.0),
 // 2 048 × 12 288 × 2 048 384 (six rounds, 73.1) or 440 of 224 (six, 70.4), 2 048 × 16 400 × 2 048 520 (eight, 95.9) or 592 of 224 (92.7).
 constexpr int kPairBN = 256;

@@ -128,9 +128,9 @@ __device__ __forceinline__ void cap_scores(float (&s)[8][4], float scale, float 
   }
 }
 
-// Bound by the rate of mma.sync: a tensor core takes one m16n8k16 in 16 cycles (512 multiply-adds per cycle and SM, an eighth of tcgen05's), 61 of
-// the 64 µs of 16 heads of 128 over 2 048 rows; short prompts by the longest block's chain of tiles.  The launch bound asks for one CTA: two fit
-// all the same (239 registers), and the schedule with 177, which the compiler chooses by itself, takes 80 µs (512 rows 18.9 → 14.2, 14 heads of 64
+// Bound by two CTAs of four warps an SM, whose products, softmax and shared loads take turns: 16 heads of 128 over 2 048 rows 64 µs with the tensor pipe 52 % and
+// the issue slots 44 % busy (profiles/prompt_kernels_ncu.md); short prompts by the longest block's chain of tiles.  The launch bound asks for one CTA: two fit
+// all the same (239 registers), and the schedule that the compiler chooses without it takes 80 µs (512 rows 18.9 → 14.2, 14 heads of 64
 // over 1 024 rows 21.8 → 19.9).  Heads of 64 keep to the 168 registers with which three fit.  Two row tiles per warp, which halve the reads of
 // keys and values, were slower: 107 µs, and no faster with 32 heads (129 against 123).
 template <int HD, bool SCORE>

@@ -19,10 +19,11 @@
 // through, and a block that meets an infinity or a NaN there is computed again key by key (see_alone), so that nothing a row
 // does not see reaches it.
 //
-// Bound, per pair of CTAs on an SM, by the products of 64 keys (820 of 1 000 cycles a tile: an MMA of N = 64 takes as long as one of
-// N = 128) and, on small calls, by what a CTA does once: barriers, TMEM and the first loads 3 000 cycles, the end 3 000.  128-key tiles
+// Bound by the chain of a block's tiles, S → softmax → P·V in turn, and by how long and short blocks come to lie on the SMs: 16 heads of 128 over 2 048
+// rows keep the tensor pipe 28 % and the issue slots 30 % busy (a tile's products take 640 cycles, those of N = 64 three quarters of what
+// N = 128 takes; profiles/prompt_kernels_ncu.md).  Small calls by what a CTA does once: barriers, TMEM and the first loads, the merge and the stores.  128-key tiles
 // (P then shares the only S buffer) and eight softmax warps of 64 keys were no faster: 43 and 40 µs where this form took 38.
-// Masks as bits (they were two comparisons per key: 4 000 to 7 000 cycles a tile), results stored in whole rows through shared memory
+// Masks as bits (two comparisons per key took longer than whole tiles), results stored in whole rows through shared memory
 // (straight from the lanes a store touches 32 rows), the first loads in front of the TMEM allocation, waits whose first look is inline.
 // µs, mma.sync / here at first / now, same error against 64 bits: 16 heads of 128 over 2 048 rows 64 / 51 / 34.6, 24 heads
 // 98 / 53 / 41.4, 32 heads 123 / 71 / 52.5; 16 heads over 512 rows 14.2 / 18.2 / 10.6; 14 heads of 64 over 2 048 rows 48 / 41 / 29.2,
@@ -309,7 +310,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
       tmem_wait_ld();
       const int kbase = tile_of(it) * kTBN;
       if (kbase + kTBN - 1 > first_pos || (p.window > 0 && last_pos - kbase >= p.window)) {
-        // the keys this row sees, a bit each (comparing them one by one took 4 000 to 7 000 cycles a tile, more than three whole tiles)
+        // the keys this row sees, a bit each (comparing them one by one took longer than a whole tile)
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const int k0 = kbase + i * 32;
@@ -565,7 +566,7 @@ bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd, int rows) {
   const int tiles = last / 64 + 1 - edge + (a.window > 0 ? std::min(edge, (a.keep_first + 63) / 64) : 0);
   return tiles >= (hd == 64 ? 6 : 5) || (hd == 128 && tiles >= 3 && (int64_t)a.B * a.Hq * (last / 64 + 1) > 296);
 }
-// Two CTAs per 128 rows of a head while all of them still run at once (two to an SM): the longest chain of tiles is half as long.  Beyond that the
+// Two CTAs per 128 rows of a head while all of them still run at once (two to an SM; a constant, since the two forms sum in other orders): the longest chain of tiles is half as long.  Beyond that the
 // second CTA's start and end cost more than the chain.  µs, one / two: 16 heads of 128 512 rows 12.9 / 10.6, 1 024 rows (128 blocks)
 // 20.5 / 15.7, 1 536 rows (192) 27.2 / 27.0, 2 048 rows 34.6 / 35.5; 32 heads 512 rows (128) 13.4 / 12.7, 768 rows (192) 17.7 / 22.0; a single
 // tile or two of them per block 5.7 / 7.4.
