@@ -577,8 +577,8 @@ def run_ours(args):
         {"kernel": "gemv_stream_kernel gate|up (RMSNorm prologue, SiLU·mul epilogue)", "bytes": gu_bytes, "ms": t_gu,
          "achieved_gbs": gu_bytes / t_gu / 1e6, "frac": gu_bytes / t_gu / 1e6 / peak,
          "how": f"{4 * spec.layers} launches back to back over the {spec.layers} layers' matrices (stand-alone op: host "
-                "launch gaps included, no PDL overlap — inside the token graph the same kernel's body is "
-                "tools/trace_decode.py)"},
+                "launch gaps included, no PDL overlap — tools/trace_decode.py shows the same kernel "
+                "inside the token graph)"},
     ]
     traffic = None
     tpath = ROOT / "profiles" / "traffic.json"
