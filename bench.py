@@ -346,7 +346,7 @@ def explain_id_agreement(eng, prompt, resident_toks, host_toks, spec):
         "margins_in_bf16_ulps_where_argmax_differs": [round(float(m), 2) for m in margin_ulp[differ]],
         "max_abs_logit_difference_between_the_two_prefill_paths": dist_max,
         "why": "the GEMM prefill and the token-by-token prefill round the prompt's K/V rows differently (both within the "
-               "reference's own decode-vs-batched noise, profiles/r02_ref_cuda_parity.json); a top-2 margin of ≤ ~2 bf16 "
+               "reference's own decode-vs-batched noise, profiles/ref_cuda_parity.json); a top-2 margin of ≤ ~2 bf16 "
                "ulps then flips one greedy token and the free-running sequences diverge from there",
     }
     # a disagreement on a step whose margin is far above the distance between the two paths would be a bug

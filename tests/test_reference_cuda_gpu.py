@@ -2,7 +2,7 @@
 `make -C oracle cuda` where the reference's sources are) as the parity
 oracle, and the drop-in boundary exercised INSIDE that program (integration/tinytorch_b200_adapter.h).  Skipped only
 when the binary is absent.  Full-size numbers for the four models: tools/ref_cuda_parity.py →
-profiles/r02_ref_cuda_parity.json."""
+profiles/ref_cuda_parity.json."""
 import pytest
 import torch
 
@@ -60,7 +60,7 @@ def test_full_size_against_reference_cuda_and_its_own_noise_floor(built_lib, nam
     kernels) is the measured floor (0 for the shapes where cuBLAS happens to pick the same kernel twice).  Gate:
     |engine − reference| ≤ max(1.75 × that floor, 2 ulp of the top logit) in the mean, ids equal wherever the reference's
     top-2 margin exceeds the observed distance; the near-ties are printed.  Numbers for 24 steps:
-    profiles/r02_ref_cuda_parity.json."""
+    profiles/ref_cuda_parity.json."""
     import sys
     import tempfile
     from pathlib import Path

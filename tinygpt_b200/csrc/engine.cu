@@ -552,7 +552,7 @@ static int engine_build(const b200_model_desc* desc, const b200_weight_table* w,
   e->gen_count = (unsigned long long*)(e->arena + o_cnt);
   e->sample_ws = (void*)(e->arena + o_sample);
 
-  // ---- shared-memory budgets = ring depth per GEMV.  Measured (B200, profiles/r02_ring_depth_sweep.txt): what decides
+  // ---- shared-memory budgets = ring depth per GEMV.  Measured (B200, profiles/ring_depth_sweep.txt): what decides
   // the HBM-bound models is that EVERY kernel keeps ≈ 8 stages (128 KB per SM, 19 MB chip-wide) in flight — enough to
   // cover the HBM latency at full bandwidth.  Splitting 220 KB between consecutive kernels, so that PDL could keep
   // both resident, left down_proj / o_proj with 2–4 stages and they streamed at ≈ 4 TB/s (Mistral-7B 0.60–0.79 of

@@ -11,7 +11,7 @@
 // numbers in profiles/not_kept.md.)  The price: the k-sum of a row is taken in
 // tensor-core order (fp32 accumulation of exact bf16 products, 8 k-slices added in warp order), so a batched step agrees
 // with batch-1 steps to summation-order noise instead of bit for bit — exactly the relation between the reference's own
-// m = 1 and m = B paths (profiles/r02_ref_cuda_parity.json, "reference_cuda_decode_vs_its_own_batched_path").
+// m = 1 and m = B paths (profiles/ref_cuda_parity.json, "reference_cuda_decode_vs_its_own_batched_path").
 //
 // Structure: gemv_stream_kernel's producer, ring and plan geometry, unchanged (one TMA thread, 16 KB stages of
 // [NSEG][8·RPW rows][KB·256 k] bf16).  The 8 consumer warps split every stage along K — warp w takes the KB·32 k-elements
