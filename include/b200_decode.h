@@ -289,7 +289,7 @@ int64_t b200_engine_position(const b200_engine* eng);
 int64_t b200_engine_launches_per_token(const b200_engine* eng);
 /* Which code paths this engine was built with (environment / defaults at create time): bit 0 CUDA graph, bit 1
  * programmatic dependent launch, bit 3 batched GEMM prefill (bit 2 and bits 8-15 belonged to variants that were measured
- * and removed: profiles/not_kept.md). */
+ * and removed). */
 int64_t b200_engine_options(const b200_engine* eng);
 /* Algorithmic HBM bytes one decode step reads on THIS rank at context length ctx (weights once + KV + logits). */
 int64_t b200_engine_bytes_per_token(const b200_engine* eng, int64_t ctx);

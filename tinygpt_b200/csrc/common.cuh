@@ -21,7 +21,7 @@ void set_error(const char* fmt, ...);
 // ------------------------------------------------------------------------------- selectable code paths and their defaults
 // The environment variable overrides the default BOTH ways (the named value), so a measured alternative stays one
 // variable away.  Variants that were measured and lost (flag synchronisation, register-resident small-k GEMV loop,
-// cross-kernel L2 prefetch, whole-token persistent kernel) are not here any more: profiles/not_kept.md.
+// cross-kernel L2 prefetch, whole-token persistent kernel) are not here any more.
 struct Defaults {
   static constexpr bool kPrefillAttnMma = true;   // B200_PREFILL_ATTN   "mma" (tensor cores) | "cuda" (CUDA cores)
   // B200_GEMM "persistent" | "tile" | "wide": chosen per shape when unset (gemm.cu pick_gemm)

@@ -74,8 +74,8 @@ __device__ __forceinline__ uint32_t silu_mul2(uint32_t g0, uint32_t g1, uint32_t
 // accumulator is double-buffered in TMEM (256 columns apart): the epilogue of tile i drains one buffer while the MMA warp
 // fills the other.  Eight epilogue warps, two to a quarter of the rows, turn rows of TMEM lanes into whole 128-byte row pieces through a swizzled
 // 4 KB patch per warp and store 16 bytes per lane along the row (four of them took 13 µs for SiLU products of a 256 × 256 tile, as long as
-// K = 2 048).  Bound by the tensor pipe under the power cap (87 % of the active cycles, at 224 and 192 columns;
-// profiles/prompt_kernels_ncu.md).  The width is what wastes least in the last round of tiles, any
+// K = 2 048).  Bound by the tensor pipe under the power cap (busy 87 % of the active cycles, at 224 and 192 columns).
+// The width is what wastes least in the last round of tiles, any
 // width sums the same bits: 2 048 × 3 072 × 8 192 is 96 tiles of 256 (two rounds of 74 pairs, 83.6 µs) or 128 of 192 (75.0),
 // 2 048 × 12 288 × 2 048 384 (six rounds, 73.1) or 440 of 224 (six, 70.4), 2 048 × 16 400 × 2 048 520 (eight, 95.9) or 592 of 224 (92.7).
 constexpr int kPairBN = 256;

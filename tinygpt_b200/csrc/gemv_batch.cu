@@ -7,8 +7,8 @@
 // passes per step; decode is weight-bound, so B sequences should cost (almost) one.  [B ≤ 8, k] × [k, n] is GEMM-shaped
 // work: on the tensor cores the consumer side costs ~25 warp instructions per 16 KB stage whatever B is, and the step
 // stays bound by the weight stream.  (A first version repeated gemv_stream_kernel's CUDA-core arithmetic per sequence —
-// bit-identical to batch 1, but B × the FMAs per weight vector: a B = 8 step cost 4.1-4.5 × a batch-1 step;
-// numbers in profiles/not_kept.md.)  The price: the k-sum of a row is taken in
+// bit-identical to batch 1, but B × the FMAs per weight vector: a B = 8 step cost 4.1-4.5 × a batch-1
+// step.)  The price: the k-sum of a row is taken in
 // tensor-core order (fp32 accumulation of exact bf16 products, 8 k-slices added in warp order), so a batched step agrees
 // with batch-1 steps to summation-order noise instead of bit for bit — exactly the relation between the reference's own
 // m = 1 and m = B paths (profiles/ref_cuda_parity.json, "reference_cuda_decode_vs_its_own_batched_path").

@@ -129,7 +129,7 @@ __device__ __forceinline__ void cap_scores(float (&s)[8][4], float scale, float 
 }
 
 // Bound by two CTAs of four warps an SM, whose products, softmax and shared loads take turns: 16 heads of 128 over 2 048 rows 64 µs with the tensor pipe 52 % and
-// the issue slots 44 % busy (profiles/prompt_kernels_ncu.md); short prompts by the longest block's chain of tiles.  The launch bound asks for one CTA: two fit
+// the issue slots 44 % busy (an m16n8k16 takes 8 cycles a scheduler); short prompts by the longest block's chain of tiles.  The launch bound asks for one CTA: two fit
 // all the same (239 registers), and the schedule that the compiler chooses without it takes 80 µs (512 rows 18.9 → 14.2, 14 heads of 64
 // over 1 024 rows 21.8 → 19.9).  Heads of 64 keep to the 168 registers with which three fit.  Two row tiles per warp, which halve the reads of
 // keys and values, were slower: 107 µs, and no faster with 32 heads (129 against 123).

@@ -21,7 +21,7 @@
 //
 // Bound by the chain of a block's tiles, S → softmax → P·V in turn, and by how long and short blocks come to lie on the SMs: 16 heads of 128 over 2 048
 // rows keep the tensor pipe 28 % and the issue slots 30 % busy (a tile's products take 640 cycles, those of N = 64 three quarters of what
-// N = 128 takes; profiles/prompt_kernels_ncu.md).  Small calls by what a CTA does once: barriers, TMEM and the first loads, the merge and the stores.  128-key tiles
+// N = 128 takes: 48 and 64 cycles).  Small calls by what a CTA does once: barriers, TMEM and the first loads, the merge and the stores.  128-key tiles
 // (P then shares the only S buffer) and eight softmax warps of 64 keys were no faster: 43 and 40 µs where this form took 38.
 // Masks as bits (two comparisons per key took longer than whole tiles), results stored in whole rows through shared memory
 // (straight from the lanes a store touches 32 rows), the first loads in front of the TMEM allocation, waits whose first look is inline.
