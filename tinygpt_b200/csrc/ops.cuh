@@ -92,8 +92,7 @@ struct TcPrefillAttn {
 };
 bool prefill_attn_tc_ok(const TcPrefillAttn& a, int hd);     // head size, alignment and strides it takes
 bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd, int rows);   // for a prompt of so many rows, against launch_pf's mma.sync kernel
-// rows: the prompt length by which the form is chosen (forms sum in other orders: what must not depend on a call's own rows passes a fixed one)
-int launch_prefill_attn_tc(const TcPrefillAttn& a, int hd, int rows, cudaStream_t st);
+int launch_prefill_attn_tc(const TcPrefillAttn& a, int hd, cudaStream_t st);
 bool prefill_window_ok(int hd);   // head sizes launch_attn_prefill_window takes
 int launch_attn_causal_mma(void* o, const void* q, const void* k, const void* v, int64_t B, int64_t S, int64_t Hq,
                            int64_t Hkv, int64_t hd, cudaStream_t st);

@@ -362,7 +362,7 @@ int launch_pf(const PrefillAttnParams& p, int B, cudaStream_t st, int tc_rows) {
                           p.scale_log2, p.window, p.keep_first, p.sink, p.pdl};
     // "tc" | "mma" forces a side
     if (tc_rows > 0 && prefill_attn_tc_ok(t, HD) && env_choice("B200_ATTN_TC", 't', prefill_attn_tc_wins(t, HD, tc_rows)))
-      return launch_prefill_attn_tc(t, HD, tc_rows, st);
+      return launch_prefill_attn_tc(t, HD, st);
   }
   constexpr int smem_max = (kBM + 4 * kBN) * row_bytes<HD>();
   const int smem = SCORE && p.same ? (kBM + 2 * kBN) * row_bytes<HD>() : smem_max;

@@ -3,31 +3,31 @@
 // fp32, P rounded to bf16, bf16 P·V products summed in fp32), same masks (causal over a cached prefix, sliding window with
 // kept first keys), sink and per-head gate.
 //
-// Shape of the work: 128 query rows of one query head against keys in tiles of 64 in ascending order, by one CTA or by a cluster of two that
-// share the tiles by parity (attn_tc_halves), two CTAs per SM (96 KB of shared memory, 256 TMEM columns each) so that one CTA's softmax
-// runs beside the other's products:
-//   warp 0    TMA producer: the Q block once, then K and V tiles (128-byte swizzle; rows past the sequence are zero-filled)
-//   warp 1    MMA issuer (one thread): S = Q·Kᵀ of the next tile goes out before P·V of this one, so the tensor pipe works
-//             while the softmax warps hold a tile; S is double-buffered in TMEM, O stays in TMEM
-//   warps 2-5 softmax, one row per thread: S from TMEM, row maximum and sum without shuffles, P (bf16) back into the TMEM columns
-//             of S as the A operand of P·V; O is rescaled in TMEM where a row's maximum grew (nearly every tile of 32 rows), behind the
-//             exponentials: by then the product before is over and S's registers are free for two loads of O in flight
-// Late query blocks (most keys) of all heads are scheduled first.  Two CTAs of a cluster end with a maximum, a sum and 128 columns of O per row
-// each: one hands the other half of its columns through distributed shared memory, and each finishes its own half.
+// Shape of the work: blocks of 128 query rows of a head, long ones first, shared out over one CTA per SM that runs through several; a block visits its keys
+// in tiles of 128 in ascending order.  TMEM holds three S and one O of 128 columns:
+//   warps 0-7    softmax, two groups of four warps, which take the tiles by the parity of their place in the cache (so that a row's sums are the same
+//                however its prompt is cut); one row per thread: S from TMEM, row maximum and sum without shuffles, P (bf16) back into the TMEM columns of S
+//                as the A operand of P·V.  Both groups' P go into the same O, so each hands its running maximum on to the other, with the tile's
+//                number, through shared memory
+//   warps 8-11   rescale O where a row's maximum grew, beside the exponentials; at a block's end they normalise and store (TMA), while the
+//                groups are at the next block
+//   warp 12      TMA producer: Q blocks, K and V tiles (128-byte swizzle; rows past the sequence are zero-filled)
+//   warp 13      MMA issuer (one thread): P·V of a tile and right behind it S of the tile three further on, also across blocks
 //
-// A key that a row does not see has P = 0, and 0 · V is 0 only for finite V: tiles that some row of the block sees in part are looked
-// through, and a block that meets an infinity or a NaN there is computed again key by key (see_alone), so that nothing a row
-// does not see reaches it.
+// A key that a row does not see has P = 0, and 0 · V is 0 only for finite V.  So where a result is not finite, V of the tiles that some row of the
+// block sees in part is looked at, and if it holds infinities or NaNs those rows go over the keys that they see, one after another: what a row
+// does not see never reaches it.
 //
-// Bound by the chain of a block's tiles, S → softmax → P·V in turn, and by how long and short blocks come to lie on the SMs: 16 heads of 128 over 2 048
-// rows keep the tensor pipe 28 % and the issue slots 30 % busy (a tile's products take 640 cycles, those of N = 64 three quarters of what
-// N = 128 takes: 48 and 64 cycles).  Small calls by what a CTA does once: barriers, TMEM and the first loads, the merge and the stores.  128-key tiles
-// (P then shares the only S buffer) and eight softmax warps of 64 keys were no faster: 43 and 40 µs where this form took 38.
-// Masks as bits (two comparisons per key took longer than whole tiles), results stored in whole rows through shared memory
-// (straight from the lanes a store touches 32 rows), the first loads in front of the TMEM allocation, waits whose first look is inline.
-// µs, mma.sync / here at first / now, same error against 64 bits: 16 heads of 128 over 2 048 rows 64 / 51 / 34.6, 24 heads
-// 98 / 53 / 41.4, 32 heads 123 / 71 / 52.5; 16 heads over 512 rows 14.2 / 18.2 / 10.6; 14 heads of 64 over 2 048 rows 48 / 41 / 29.2,
-// four sequences of 333 rows 12.1 / - / 9.9.
+// Bound by the chain S → softmax → P·V of three tiles in flight: a group takes some 2 400 cycles a tile (1 024 of them the exponentials' pipe) and 800 until it
+// begins the next one; tensor pipe and exponentials a third busy at 16 heads of 128 over 2 048 rows.  Small calls by what is done once: barriers, TMEM,
+// first loads, code that is not in the caches yet, results (some 5 µs in all; up to 128 keys a kernel of its own, below, takes less).  Slower, at 16 heads of
+// 128 over 2 048 rows, were two O of which each group has one (26 µs where this form takes 21.5: S, whose columns P shares, then waits for P·V), three groups
+// of softmax warps (28), tiles read twice from TMEM in loops (23), the exponentials ahead of the maximum (22), 64-key tiles in two CTAs per SM (36).  A
+// maximum that moves only where weights grow beyond 2^8 needs hardly a rescale (20.5), but the largest weight is then no longer 1, and rounded: 5 % more
+// error against 64 bits, not taken.
+// µs, mma.sync / 64-key tiles in two CTAs per SM / here: 16 heads of 128 over 2 048 rows 63 / 36.2 / 21.5, 24 heads 99 / 42.3 / 32.6, 32 heads
+// 123 / 47.8 / 38.8; 16 heads over 512 rows 15.4 / 9.2 / 9.1, 1 024 rows 33.6 / 16.3 / 13.1; four sequences of 32 heads, 512 rows 43 / 26.2 / 19.9; 14 heads
+// of 64 over 2 048 rows 56 / 30.6 / 18.5, four sequences of 333 rows 11.9 / 9.7 / 7.5.  Errors against 64 bits within 1 % of each other.
 #include "ops.cuh"
 #include "tc.cuh"
 
@@ -38,18 +38,37 @@ namespace b200 {
 
 namespace {
 
-constexpr int kTBM = 128, kTBN = 64, kTThreads = 192;
+constexpr int kTBM = 128, kTBN = 128, kTThreads = 512;
 constexpr unsigned kAttnWaitCode = 0xa7000000u;
+
+// n / d for n below 2³¹ (Granlund and Montgomery 1994)
+struct Div {
+  uint32_t m, s1, s2;
+  Div() = default;
+  explicit Div(uint32_t d) {
+    uint32_t l = 0;
+    while ((1ull << l) < d) ++l;
+    m = (uint32_t)(((1ull << 32) * ((1ull << l) - d)) / d + 1);
+    s1 = l < 1 ? l : 1;
+    s2 = l < 1 ? 0 : l - 1;
+  }
+  __device__ __forceinline__ int operator()(int n) const {
+    const uint32_t t = __umulhi(m, (uint32_t)n);
+    return (int)((t + (((uint32_t)n - t) >> s1)) >> s2);
+  }
+};
 
 struct TcAttn {
   __nv_bfloat16* o;
   const __nv_bfloat16* gate;
   int64_t o_rs, o_bs, q_rs, q_bs;
-  int S, Hq, Hkv, p0;
+  int S, Hq, p0;
   float scale_log2;
   int window, keep_first, sink;
   unsigned* err;
   int pdl;
+  int blocks, heads, last;             // blocks of 128 rows in all; heads of all sequences; the last block of a head
+  Div by_heads, by_hq, by_group;       // by heads, by Hq, by Hq / Hkv
   const __nv_bfloat16 *qp, *kp, *vp;   // see_alone
   int64_t kv_rs, kv_bs;
 };
@@ -57,9 +76,12 @@ struct TcAttn {
 template <int HD>
 struct TcCfg {
   static constexpr int NB = HD / 64;                 // 64-column blocks of a row (one swizzle atom wide)
-  static constexpr int ST = HD == 64 ? 4 : 2;        // K and V stages
-  static constexpr int QB = NB * kTBM * 128, TB = NB * kTBN * 128;
-  static constexpr int smem = QB + 2 * ST * TB + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int KST = HD == 64 ? 4 : 2, VST = HD == 64 ? 4 : 3;   // K and V stages
+  static constexpr int TB = NB * 128 * 128;          // 128 rows of Q, K or V
+  static constexpr int stage = 128 * 128;            // 64 columns of results of 128 rows
+  static constexpr int small = 384 /*barriers*/ + 4 * 1024 /*m_row*/ + 2 * 2 * 1024 /*ml*/;
+  static constexpr int smem_one = 3 * TB + 64 /*barriers*/ + 1024 /*align*/;
+  static constexpr int smem = (1 + KST + VST) * TB + stage + small + 1024 /*align*/;
 };
 
 // weights below 2⁻¹²⁶ of a row's largest count as zero (with subnormals 16 heads over 2 048 rows take 53.9 instead of 51.6 µs)
@@ -93,12 +115,27 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* smem_src, int32_t c0, int32_t c1, int32_t c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }   // this thread's copies have left shared memory
+__device__ __forceinline__ void bulk_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }        // and lie in global memory
 // D[tmem] (+)= A[tmem]·B[smem], B's descriptor by its lower half: the address and, from bit 16 on, the distance of 64-column blocks of an operand
 // whose N runs along the columns (V's [keys][64 columns] rows of 128 bytes, MN-major)
 __device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 b, {%2, %3};\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}" ::"r"(d), "r"(a), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
+      "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -112,471 +149,810 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
       : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// what has been loaded may be read behind this, and not before
+template <int N>
+__device__ __forceinline__ void tmem_loaded(uint32_t (&r)[N]) {
+  tmem_wait_ld();
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
+}
+// waits for some 20 µs at most without taking issue slots from the warps that work
+__device__ __forceinline__ bool mbar_sleep(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(20000u) : "memory");
+  return ok != 0;
+}
 // A wait that gave up says so to the whole CTA and sets `dead`: its role goes on without waiting (what follows neither hangs nor leaves
 // the buffers), and nothing is stored.  The first look is inline and has no loop around it.
-__device__ __noinline__ bool wait_slow(uint64_t* bar, uint32_t parity, unsigned* err, unsigned code, volatile int* gave_up) {
-  if (mbar_wait_limited(bar, parity, err, code)) return false;
-  *gave_up = 1;
-  __threadfence_block();
-  return true;
+__device__ __forceinline__ bool wait_slow(uint64_t* bar, uint32_t parity, unsigned* err, unsigned code, volatile int* gave_up) {
+  const unsigned long long t0 = global_timer_ns();
+  while (!mbar_sleep(bar, parity)) {
+    if (global_timer_ns() - t0 > 2000000000ull) {
+      *reinterpret_cast<volatile unsigned*>(err) = code;
+      *gave_up = 1;
+      __threadfence_system();
+      return true;
+    }
+  }
+  return false;
 }
 __device__ __forceinline__ uint32_t bits_below(int n) { return n >= 32 ? ~0u : n <= 0 ? 0u : (1u << n) - 1; }
 
 // One row, the keys it sees one after another (P rounded to bf16 like above): the way out for a block whose partly visible tiles hold
 // infinities or NaNs in V.  Slow and rare.
 template <int HD>
-__device__ __noinline__ void see_alone(const TcAttn& p, int b, int h, int kvh, int r, float (&ml)[2], int c, float (&acc)[32]) {
+__device__ __forceinline__ void see_alone(const TcAttn& p, int b, int h, int kvh, int r, float (&ml)[2], int c, float (&acc)[8]) {
   const __nv_bfloat16* q = p.qp + (size_t)b * p.q_bs + (size_t)r * p.q_rs + (size_t)h * HD;
   const int rpos = p.p0 + r;
+#pragma unroll 1
   for (int j = 0; j <= rpos; ++j) {
     if (p.window > 0 && rpos - j >= p.window && j >= p.keep_first) continue;
     const size_t row = (size_t)b * p.kv_bs + (size_t)j * p.kv_rs + (size_t)kvh * HD;
     float s = 0.f;
-    for (int d = 0; d < HD; ++d) s = fmaf(bf16_to_f(q[d]), bf16_to_f(p.kp[row + d]), s);
+#pragma unroll 1
+    for (int d = 0; d < HD; d += 8) {
+      float x[8];
+      unpack8(*reinterpret_cast<const uint4*>(q + d), x);
+      s = dot8(*reinterpret_cast<const uint4*>(p.kp + row + d), x, s);
+    }
     if (c < 0) {   // first walk: maximum and sum
       const float top = fmaxf(ml[0], s);
       ml[1] = ml[1] * (ml[0] == -INFINITY ? 0.f : ex2f((ml[0] - top) * p.scale_log2)) + ex2f((s - top) * p.scale_log2);
       ml[0] = top;
     } else {
       const float w = round_bf16(ex2f((s - ml[0]) * p.scale_log2));
-      for (int e = 0; e < 32; ++e) acc[e] = fmaf(w, bf16_to_f(p.vp[row + c + e]), acc[e]);
+      for (int e = 0; e < 8; ++e) acc[e] = fmaf(w, bf16_to_f(p.vp[row + c + e]), acc[e]);
     }
   }
 }
 
-template <int HD, int SPLIT>
-__global__ void __launch_bounds__(kTThreads, 2)
-attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
-               const TcAttn p) {
-  using C = TcCfg<HD>;
-  constexpr int NB = C::NB, ST = C::ST;
-  constexpr uint32_t kIdescS = umma_idesc(kTBM, kTBN), kIdescO = umma_idesc(kTBM, HD, true);
-  constexpr int kCols = 256, kColO = 128;   // S at columns 0 and 64, O from column 128 on
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sQ = smem;                      // [NB][128 rows × 128 bytes]
-  uint8_t* sK = sQ + C::QB;                // [ST][NB][64 keys × 128 bytes]
-  uint8_t* sV = sK + ST * C::TB;
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(sV + ST * C::TB);
-  uint64_t* k_full = q_full + 1;           // [ST]
-  uint64_t* k_empty = k_full + ST;
-  uint64_t* v_full = k_empty + ST;
-  uint64_t* v_empty = v_full + ST;
-  uint64_t* s_full = v_empty + ST;         // [2]
-  uint64_t* p_full = s_full + 2;           // [2], one arrival per softmax warp
-  uint64_t* pv_done = p_full + 2;          // one phase per tile but the last
-  uint64_t* o_full = pv_done + 1;          // the last tile's product, and so all of them
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
-  int* not_finite = reinterpret_cast<int*>(tmem_slot + 1);
-  int* gave_up = not_finite + 1;
-  float4* part = reinterpret_cast<float4*>(sQ);   // [128 rows]: maximum, sum, V is not finite, gave up
-  float4* give = reinterpret_cast<float4*>(sK);   // [HD / 8][128 rows]: the columns that the other CTA finishes
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+__device__ __forceinline__ float2 ld_volatile_f2(const float2* p) {
+  float2 v;
+  asm volatile("ld.volatile.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_u32(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_volatile_f2(float2* p, float2 v) {
+  asm volatile("st.volatile.shared.v2.f32 [%0], {%1, %2};" ::"r"(smem_u32(p)), "f"(v.x), "f"(v.y) : "memory");
+}
+constexpr int kTCtas = 148;   // one per SM; which CTA has a block changes no bit
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int half = SPLIT == 2 ? (int)cluster_rank() : 0;
-  const int h = blockIdx.x / SPLIT, qb = (int)gridDim.y - 1 - (int)blockIdx.y, b = blockIdx.z;
-  const int kvh = h / (p.Hq / p.Hkv);
-  const int q0 = qb * kTBM;
-  const int rows_valid = min(kTBM, p.S - q0);
-  const int first_pos = p.p0 + q0, last_pos = first_pos + rows_valid - 1;
-  const int T = last_pos / kTBN + 1;
-  // tiles to visit: with a window those of the kept first keys, then from the first row's window edge up to the diagonal
-  const int t_lo = p.window > 0 ? max(0, first_pos - p.window + 1) / kTBN : 0;
-  const int n_keep = p.window > 0 ? min(t_lo, (p.keep_first + kTBN - 1) / kTBN) : 0;
-  // this CTA's share of them: all, or the tiles of its parity.  By the tile's place in the cache, so that a row's sums are the same however
-  // its prompt is cut
-  const int own_keep = SPLIT == 2 ? (n_keep + 1 - half) >> 1 : n_keep, own_lo = SPLIT == 2 ? t_lo + ((t_lo ^ half) & 1) : t_lo;
-  const int n_tiles = own_keep + (max(T - own_lo, 0) + SPLIT - 1) / SPLIT;
-  auto tile_of = [&](int it) { return it < own_keep ? half + SPLIT * it : own_lo + SPLIT * (it - own_keep); };
-  bool dead = false;
-  auto wait_for = [&](uint64_t* bar, uint32_t parity, unsigned code) {
-    if (!mbar_try_wait(bar, parity) && !dead) dead = wait_slow(bar, parity, p.err, code, gave_up);
-  };
+// What a block of 128 query rows of a head has to visit: tiles of 128 keys in ascending order
+struct Block {
+  int b, h, kvh, q0, rows_valid, first_pos, last_pos, n_keep, t_lo, n;
+  __device__ __forceinline__ Block(const TcAttn& p, int i) {
+    const int late = p.by_heads(i), hb = i - late * p.heads;
+    b = p.by_hq(hb);
+    h = hb - b * p.Hq;
+    kvh = p.by_group(h);
+    q0 = (p.last - late) * kTBM;   // late blocks (most keys) first
+    rows_valid = min(kTBM, p.S - q0);
+    first_pos = p.p0 + q0;
+    last_pos = first_pos + rows_valid - 1;
+    // with a window the tiles of the kept first keys, then from the first row's window edge up to the diagonal
+    t_lo = p.window > 0 ? max(0, first_pos - p.window + 1) / kTBN : 0;
+    n_keep = p.window > 0 ? min(t_lo, (p.keep_first + kTBN - 1) / kTBN) : 0;
+    n = n_keep + last_pos / kTBN + 1 - t_lo;
+  }
+  // some row does not see some key of the tile
+  __device__ __forceinline__ bool in_part(const TcAttn& p, int kbase) const {
+    return kbase + kTBN - 1 > first_pos || (p.window > 0 && last_pos - kbase >= p.window);
+  }
+  __device__ __forceinline__ int tile(int it) const { return it < n_keep ? it : t_lo + it - n_keep; }   // its place in the cache
+};
 
-  auto load_k = [&](int it, int s) {
-    mbar_arrive_expect_tx(&k_full[s], C::TB);
+// Whether V holds infinities or NaNs in a tile that some row of the block sees in part; one warp
+template <int HD>
+__device__ __forceinline__ bool part_not_finite(const TcAttn& p, const Block& w, int lane) {
+  bool bad = false;
+  for (int it = 0; it < w.n; ++it) {
+    const int kbase = w.tile(it) * kTBN;
+    if (!w.in_part(p, kbase)) continue;
+    const __nv_bfloat16* const v = p.vp + (size_t)w.b * p.kv_bs + (size_t)kbase * p.kv_rs + (size_t)w.kvh * HD;
+    const int rows = min(kTBN, p.p0 + p.S - kbase);
+#pragma unroll 1
+    for (int e = lane; e < rows * (HD / 8); e += 32) {
+      const uint4 x4 = *reinterpret_cast<const uint4*>(v + (size_t)(e / (HD / 8)) * p.kv_rs + e % (HD / 8) * 8);
+      const uint32_t x[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
-    for (int c = 0; c < NB; ++c) tma_load_3d(sK + s * C::TB + c * kTBN * 128, &tk, kvh * HD + c * 64, tile_of(it) * kTBN, b, &k_full[s]);
+      for (int k = 0; k < 4; ++k) bad |= (((x[k] & 0x7f807f80u) + 0x00800080u) & 0x80008000u) != 0;
+    }
+  }
+  return __any_sync(0xffffffffu, bad);
+}
+
+// the weights of 32 keys of a row, rounded to bf16, to TMEM; their sums in fp32
+__device__ __forceinline__ void weights32(const uint32_t (&s)[32], uint64_t scale2, uint64_t neg, uint64_t (&sum)[2], uint32_t at) {
+  uint32_t pk[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const uint64_t z = fma_f2(pack_f2(__uint_as_float(s[2 * e]), __uint_as_float(s[2 * e + 1])), scale2, neg);
+    const float a0 = ex2f(lo_f2(z)), a1 = ex2f(hi_f2(z));
+    sum[e & 1] = add_f2(sum[e & 1], pack_f2(a0, a1));
+    pk[e] = pack2(a0, a1);
+  }
+  tmem_st16(at, pk);
+}
+
+// 32 rows of a block from O in TMEM, this lane's with maximum m and sum l: normalised, through shared memory (64 columns at `mid`, the next 64 `step`
+// bytes further on) into the result.  has_read is called behind the last look at O.
+template <int HD, typename F>
+__device__ __forceinline__ void store_rows(const TcAttn& p, const CUtensorMap* to, const Block& w, uint32_t o_at, int row, float m, float l, uint8_t* mid,
+                                           int step, bool lost, F has_read) {
+  const int lane = row & 31, rr = w.q0 + min(row, w.rows_valid - 1);
+  const float k_scale = p.scale_log2;
+  if (p.sink && m != -INFINITY) l += ex2f(-m * k_scale);
+  const float gate = p.gate != nullptr ? 1.f / (1.f + expf(-bf16_to_f(p.gate[(size_t)w.b * p.q_bs + (size_t)rr * p.q_rs + w.h]))) : 1.f;
+  float inv = (l > 0.f ? 1.f / l : 0.f) * gate;
+  uint32_t odd = 0;   // the sign bits of halves whose exponent is all ones
+#pragma unroll 1
+  for (int c = 0; c < HD; c += 64, mid += step) {
+    if (step == 0) {
+      if (lane == 0) bulk_read();   // the copy before has read
+      __syncwarp();
+    }
+#pragma unroll 1
+    for (int k = 0; k < 64; k += 32) {
+      uint32_t o[32], y[16];
+      tmem_ld32(o_at + c + k, o);
+      tmem_loaded(o);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        y[e] = pack2(__uint_as_float(o[2 * e]) * inv, __uint_as_float(o[2 * e + 1]) * inv);
+        odd |= (y[e] & 0x7f807f80u) + 0x00800080u;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)   // in the tensor map's 128-byte swizzle
+        *reinterpret_cast<uint4*>(mid + lane * 128 + ((k / 8 + e) ^ (lane & 7)) * 16) = make_uint4(y[4 * e], y[4 * e + 1], y[4 * e + 2], y[4 * e + 3]);
+    }
+    if (c + 64 == HD) has_read();
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0 && !lost && row < w.rows_valid) {
+      tma_store_3d(to, mid, w.h * HD + c, w.q0 + row, w.b);   // rows past the sequence are not written
+      bulk_commit();
+    }
+  }
+  // 0 · V is not 0 where V is not finite: then such rows see their keys one after another
+  if (__builtin_expect(__any_sync(0xffffffffu, (odd & 0x80008000u) != 0), 0) && part_not_finite<HD>(p, w, lane) && !lost) {
+    if (lane == 0) bulk_done();
+    __syncwarp();
+    float both[2] = {-INFINITY, 0.f}, x[8];
+    see_alone<HD>(p, w.b, w.h, w.kvh, rr, both, -1, x);
+    l = both[1];
+    if (p.sink && both[0] != -INFINITY) l += ex2f(-both[0] * k_scale);
+    inv = (l > 0.f ? 1.f / l : 0.f) * gate;
+#pragma unroll 1
+    for (int c = 0; c < HD; c += 8) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = 0.f;
+      see_alone<HD>(p, w.b, w.h, w.kvh, rr, both, c, x);
+      if (row < w.rows_valid)
+        *reinterpret_cast<uint4*>(p.o + (size_t)w.b * p.o_bs + (size_t)rr * p.o_rs + (size_t)w.h * HD + c) =
+            make_uint4(pack2(x[0] * inv, x[1] * inv), pack2(x[2] * inv, x[3] * inv), pack2(x[4] * inv, x[5] * inv), pack2(x[6] * inv, x[7] * inv));
+    }
+  }
+}
+
+// The same for 128 keys at most, one tile: nothing is shared out and nothing runs ahead, so four warps do everything one after another, on as many
+// keys as there are (P of those behind is zero, and adding their products changes no bit).
+template <int HD>
+__global__ void __launch_bounds__(128)
+attn_tc_one_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
+                   const __grid_constant__ CUtensorMap to, const __grid_constant__ TcAttn p) {
+  using C = TcCfg<HD>;
+  constexpr int kColO = 128;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* sQ = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* sK = sQ + C::TB;
+  uint8_t* sV = sK + C::TB;
+  uint64_t* qk_full = reinterpret_cast<uint64_t*>(sV + C::TB);
+  uint64_t* v_full = qk_full + 1;
+  uint64_t* s_full = v_full + 1;
+  uint64_t* o_full = s_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
+  int* gave_up = reinterpret_cast<int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = threadIdx.x;
+  bool dead = false;
+  auto wait_for = [&](uint64_t* bar, unsigned code) {
+    if (!mbar_try_wait(bar, 0) && !dead) dead = wait_slow(bar, 0, p.err, code, gave_up);
   };
+  const Block w(p, (int)blockIdx.x);
+  const int keys = p.p0 + p.S, steps = (keys + 15) / 16;
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tq);
     tma_prefetch_desc(&tk);
+    tma_prefetch_desc(&tq);
     tma_prefetch_desc(&tv);
-    mbar_init(q_full, 1);
-    for (int s = 0; s < ST; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], 1);
-      mbar_init(&v_full[s], 1);
-      mbar_init(&v_empty[s], 1);
-    }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&s_full[s], 1);
-      mbar_init(&p_full[s], 4);
-    }
-    mbar_init(pv_done, 1);
-    mbar_init(o_full, 1);
-    *not_finite = 0;
+    tma_prefetch_desc(&to);
+    for (int i = 0; i < 4; ++i) mbar_init(qk_full + i, 1);
     *gave_up = 0;
     fence_mbar_init();
     if (p.pdl) pdl_wait();
-    if (n_tiles > 0) {   // on their way while TMEM is allocated
-      load_k(0, 0);
-      mbar_arrive_expect_tx(q_full, C::QB);
+    mbar_arrive_expect_tx(qk_full, 2 * C::TB);
 #pragma unroll
-      for (int c = 0; c < NB; ++c) tma_load_3d(sQ + c * kTBM * 128, &tq, h * HD + c * 64, q0, b, q_full);
+    for (int c = 0; c < C::NB; ++c) {
+      tma_load_3d(sK + c * kTBN * 128, &tk, w.kvh * HD + c * 64, 0, w.b, qk_full);
+      tma_load_3d(sQ + c * kTBM * 128, &tq, w.h * HD + c * 64, 0, w.b, qk_full);
     }
+    mbar_arrive_expect_tx(v_full, C::TB);
+#pragma unroll
+    for (int c = 0; c < C::NB; ++c) tma_load_3d(sV + c * kTBN * 128, &tv, w.kvh * HD + c * 64, 0, w.b, v_full);
   }
-  if (warp == 2) tmem_alloc<1>(tmem_slot, kCols);
+  if (warp == 1) tmem_alloc<1>(tmem_slot, 256);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  if (p.pdl) pdl_wait();
+  if (p.pdl) {
+    pdl_wait();
+    pdl_trigger();
+  }
+  if (warp == 0 && elect_one()) {
+    const uint32_t q_u = desc_lo(smem_u32(sQ)), k_u = desc_lo(smem_u32(sK)), idesc = umma_idesc(kTBM, steps * 16);
+    wait_for(qk_full, kAttnWaitCode | 17);
+    tc_fence_after();
+#pragma unroll
+    for (int kk = 0; kk < HD / 16; ++kk) {
+      const uint32_t at = ((kk / 4) * 128 * 128 + (kk % 4) * 32) >> 4;
+      umma_lo<1>(tmem, q_u + at, k_u + at, idesc, kk > 0 ? 1u : 0u);
+    }
+    umma_commit(s_full);
+  }
+  __syncwarp();
+  const uint32_t s_at = tmem + ((uint32_t)(warp * 32) << 16);
+  const int rpos = w.first_pos + min(row, w.rows_valid - 1);   // padding rows behave like the last valid row
+  const float k_scale = p.scale_log2;
+  const uint64_t scale2 = pack_f2(k_scale, k_scale);
+  wait_for(s_full, kAttnWaitCode | 18);
+  __syncwarp();
+  tc_fence_after();
+  float m = -INFINITY, l = 0.f;
+  {
+    uint32_t s[4][32];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k * 32 < keys) tmem_ld32(s_at + k * 32, s[k]);
+    tmem_wait_ld();
+    float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k * 32 >= keys) continue;
+      const int k0 = k * 32;
+      const uint32_t seen = bits_below(rpos + 1 - k0) & (p.window > 0 ? ~bits_below(rpos + 1 - p.window - k0) | bits_below(p.keep_first - k0) : ~0u);
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        asm volatile("" : "+r"(s[k][e]));
+        s[k][e] = seen & (1u << e) ? s[k][e] : 0xff800000u;
+      }
+#pragma unroll
+      for (int e = 0; e < 32; e += 2) mx[e / 2 % 4] = max3f(mx[e / 2 % 4], __uint_as_float(s[k][e]), __uint_as_float(s[k][e + 1]));
+    }
+    m = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+    const float ms = m == -INFINITY ? 0.f : m * k_scale;
+    const uint64_t neg = pack_f2(-ms, -ms);
+    uint64_t sum[2] = {0, 0};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k * 32 >= keys) continue;
+      weights32(s[k], scale2, neg, sum, s_at + k * 16);
+    }
+    sum[0] = add_f2(sum[0], sum[1]);
+    l = lo_f2(sum[0]) + hi_f2(sum[0]);
+  }
+  tmem_wait_st();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 0 && elect_one()) {
+    const uint32_t v_u = desc_lo(smem_u32(sV));
+    wait_for(v_full, kAttnWaitCode | 19);
+    tc_fence_after();
+    for (int kk = 0; kk < steps; ++kk)
+      umma_ts(tmem + kColO, tmem + kk * 8, v_u + (kk * 2048 >> 4) + ((kTBN * 128 >> 4) << 16), umma_idesc(kTBM, HD, true), kk > 0 ? 1u : 0u);
+    umma_commit(o_full);
+  }
+  __syncwarp();
+  wait_for(o_full, kAttnWaitCode | 20);
+  __syncwarp();
+  tc_fence_after();
+  const bool lost = __any_sync(0xffffffffu, dead || *reinterpret_cast<volatile int*>(gave_up) != 0);
+  // results on their way out take Q's place: its product is over
+  store_rows<HD>(p, &to, w, s_at + kColO, row, m, l, sQ + warp * (32 * 128), 128 * 128, lost, [&] {});
+  if (lane == 0) bulk_read();
+  if (dead) drain_async();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_free<1>(tmem, 256);
+  }
+}
 
-  float4 mine{};   // of a row: maximum, sum, V is not finite, gave up
-  if (warp == 0) {
-    // ------------------------------------------------------------------------------------------ TMA producer
+template <int HD>
+__global__ void __launch_bounds__(kTThreads, 1)
+attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
+               const __grid_constant__ CUtensorMap to, const __grid_constant__ TcAttn p) {
+  using C = TcCfg<HD>;
+  constexpr int NB = C::NB, KST = C::KST, VST = C::VST;
+  constexpr uint32_t kIdescS = umma_idesc(kTBM, kTBN), kIdescO = umma_idesc(kTBM, HD, true);
+  constexpr int kCols = 512, kColO = 384;   // three S, and P in them, at columns 0, 128 and 256, O behind them
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* sQ = smem;                      // [NB][128 rows × 128 bytes]
+  uint8_t* sK = sQ + C::TB;                // [KST][NB][128 keys × 128 bytes]
+  uint8_t* sV = sK + KST * C::TB;          // [VST]
+  uint8_t* sO = sV + VST * C::TB;          // [4 warps][32 rows × 128 bytes]
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(sO + C::stage);
+  uint64_t* q_empty = q_full + 1;
+  uint64_t* k_full = q_empty + 1;          // [KST]
+  uint64_t* k_empty = k_full + KST;
+  uint64_t* v_full = k_empty + KST;        // [VST]
+  uint64_t* v_empty = v_full + VST;
+  uint64_t* s_full = v_empty + VST;        // [2 groups][3]: a group that has no tile for a while skips no phase of its own barriers
+  uint64_t* p_full = s_full + 6;           // [3], one arrival per warp of the group that has the tile
+  uint64_t* pv_done = p_full + 3;          // [3]: P has been read
+  uint64_t* m_full = pv_done + 3;          // [3], one arrival per warp of the group that has the tile: its maxima are in m_row
+  uint64_t* o_ready = m_full + 3;          // [3], one arrival per correcting warp: O goes by the tile's maxima
+  uint64_t* o_full = o_ready + 3;          // all products of a block are over
+  uint64_t* o_empty = o_full + 1;          // one arrival per storing warp: it has read O
+  uint64_t* ml_full = o_empty + 1;         // [2], one arrival per softmax warp
+  uint64_t* ml_empty = ml_full + 2;        // [2], one arrival per storing warp
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ml_empty + 2);
+  int* gave_up = reinterpret_cast<int*>(tmem_slot + 1);
+  float2* m_row = reinterpret_cast<float2*>(sO + C::stage + 384);   // [4][128]: a row's maximum on its way to the group with the next tile, and the
+                                                                      // tile's number.  Tile c + 4 overwrites what c + 1 has read: its S comes behind P of c + 1.
+  float2* ml = m_row + 4 * kTBM;               // [2][2 groups][128]: a block's maxima and sums
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  bool dead = false;
+  auto wait_for = [&](uint64_t* bar, uint32_t parity, unsigned code) {
+    if (__builtin_expect(!mbar_try_wait(bar, parity), 0) && !dead) dead = wait_slow(bar, parity, p.err, code, gave_up);
+  };
+  auto wait_passed = [&](const float2* at, int tile, float2& v) {   // the row's maximum behind this tile; limited like every wait
+    unsigned long long t0 = 0;
+    for (unsigned spins = 1; __float_as_int(v.y) != tile && !dead; ++spins) {
+      v = ld_volatile_f2(at);
+      if ((spins & 0x3ffu) == 0) {
+        const unsigned long long now = global_timer_ns();
+        if (t0 == 0) t0 = now;
+        if (now - t0 > 2000000000ull) {
+          dead = true;
+          *reinterpret_cast<volatile unsigned*>(p.err) = kAttnWaitCode | 15;
+          *reinterpret_cast<volatile int*>(gave_up) = 1;
+          __threadfence_system();
+        }
+      }
+    }
+    __syncwarp();
+  };
+  // round r's block of this CTA: forwards and backwards in turn, so that who has had a long one gets a short one
+  const int grid = (int)gridDim.x, cta = (int)blockIdx.x;
+  auto block_of = [&](int r) { return r * grid + (r & 1 ? grid - 1 - cta : cta); };
+
+  auto load_q = [&](const Block& w) {
+    mbar_arrive_expect_tx(q_full, C::TB);
+#pragma unroll
+    for (int c = 0; c < NB; ++c) tma_load_3d(sQ + c * kTBM * 128, &tq, w.h * HD + c * 64, w.q0, w.b, q_full);
+  };
+  auto load_k = [&](const Block& w, int key, int s) {
+    mbar_arrive_expect_tx(&k_full[s], C::TB);
+#pragma unroll
+    for (int c = 0; c < NB; ++c) tma_load_3d(sK + s * C::TB + c * kTBN * 128, &tk, w.kvh * HD + c * 64, key, w.b, &k_full[s]);
+  };
+  auto load_v = [&](const Block& w, int key, int s) {
+    mbar_arrive_expect_tx(&v_full[s], C::TB);
+#pragma unroll
+    for (int c = 0; c < NB; ++c) tma_load_3d(sV + s * C::TB + c * kTBN * 128, &tv, w.kvh * HD + c * 64, key, w.b, &v_full[s]);
+  };
+  if (warp == 12) {
     if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 1;
-      for (int it = 0; it < n_tiles; ++it) {
-        if (it > 0) {
-          wait_for(&k_empty[s], ph, kAttnWaitCode | 1);
-          load_k(it, s);
+      tma_prefetch_desc(&tk);
+      tma_prefetch_desc(&tq);
+      tma_prefetch_desc(&tv);
+      tma_prefetch_desc(&to);
+      *gave_up = 0;
+    }
+    const int bars = (int)(ml_empty + 2 - q_full);
+    for (int i = lane; i < bars; i += 32) {
+      const uint64_t* const bar = q_full + i;
+      mbar_init(q_full + i, bar >= p_full && bar < pv_done || bar >= m_full && bar < o_full ? 4 : bar == o_empty || bar >= ml_empty ? 4 : bar >= ml_full ? 8 : 1);
+    }
+    fence_mbar_init();
+    __syncwarp();
+    if (lane == 0) {
+      const Block w(p, cta);
+      if (p.pdl) pdl_wait();
+      load_k(w, w.tile(0) * kTBN, 0);   // on their way while TMEM is allocated
+      load_q(w);
+    }
+  }
+  if (warp == 13) tmem_alloc<1>(tmem_slot, kCols);
+  m_row[threadIdx.x] = make_float2(0.f, __int_as_float(-1));
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  if (p.pdl) {
+    pdl_wait();
+    pdl_trigger();
+  }
+
+  // Registers: 2 × 184 + 88 + 56 are the 4 × 128 that a quarter of the SM has been launched with
+  if (warp >= 12) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp == 12 && lane == 0) {
+      // ---------------------------------------------------------------------------------------- TMA producer
+      int ks = 1, vs = 0;          // the first K tile and the first Q have gone out
+      uint32_t kph = 1, vph = 1;
+      bool first = true;
+      static_assert(KST > 1, "a second K stage");
+      for (int r = 0, i; (i = block_of(r)) < p.blocks; ++r) {
+        const Block w(p, i);
+        if (r > 0) {
+          wait_for(q_empty, (uint32_t)((r - 1) & 1), kAttnWaitCode | 1);
+          load_q(w);
         }
-        wait_for(&v_empty[s], ph, kAttnWaitCode | 2);
-        mbar_arrive_expect_tx(&v_full[s], C::TB);
-#pragma unroll
-        for (int c = 0; c < NB; ++c) tma_load_3d(sV + s * C::TB + c * kTBN * 128, &tv, kvh * HD + c * 64, tile_of(it) * kTBN, b, &v_full[s]);
-        if (++s == ST) {
-          s = 0;
-          ph ^= 1;
+        auto next_k = [&](int it) {
+          if (it >= w.n) return;
+          if (first) {
+            first = false;
+            return;
+          }
+          wait_for(&k_empty[ks], kph, kAttnWaitCode | 2);
+          load_k(w, w.tile(it) * kTBN, ks);
+          if (++ks == KST) {
+            ks = 0;
+            kph ^= 1;
+          }
+        };
+        next_k(0);
+        next_k(1);
+        for (int it = 0; it < w.n; ++it) {
+          next_k(it + 2);
+          wait_for(&v_empty[vs], vph, kAttnWaitCode | 3);
+          load_v(w, w.tile(it) * kTBN, vs);
+          if (++vs == VST) {
+            vs = 0;
+            vph ^= 1;
+          }
         }
       }
       if (dead) drain_async();
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------------------------------- MMA issuer
-    if (n_tiles > 0 && elect_one()) {
+    } else if (warp == 13 && elect_one()) {
+      // ----------------------------------------------------------------------------------------- MMA issuer
+      // Two streams of products that run in the order in which they go out: P·V of a tile as soon as P is there and, right behind it, S of the tile three
+      // further on, those of the next block among them, into the buffer that P has left.  What does not depend on P has been found out by then.
       const uint32_t q_u = desc_lo(smem_u32(sQ)), k_u = desc_lo(smem_u32(sK)), v_u = desc_lo(smem_u32(sV));
-      bool k_ready = false;   // of the tile after the next, looked at before the products of this one go out
-      auto scores = [&](int it) {   // S[it & 1] = Q·Kᵀ of tile it
-        const int s = it % ST;
-        if (!k_ready) wait_for(&k_full[s], (uint32_t)((it / ST) & 1), kAttnWaitCode | 3);
+      int ks = 0, vs = 0, sbuf = 0, pbuf = 0, ahead = 0, sr = 0, s_it = 0, pr = 0, p_it = 0;
+      uint32_t kph = 0, vph = 0, pph = 0;
+      Block sw(p, cta);
+      int p_n = sw.n;
+      bool s_left = true, k_ok = false, v_ok = false;
+      unsigned spins = 0;
+      unsigned long long t0 = 0;
+      for (;;) {
+        if (!k_ok & s_left) k_ok = mbar_test(&k_full[ks], kph) & (s_it > 0 || mbar_test(q_full, (uint32_t)(sr & 1)));
+        if (!v_ok) v_ok = mbar_test(&v_full[vs], vph) & (p_it > 0 || pr == 0 || mbar_test(o_empty, (uint32_t)((pr - 1) & 1)));
+        bool do_p = false;
+        if (ahead > 0) {   // with nothing else to be done the thread sleeps until P is there
+          const bool sleep = v_ok & (!s_left | (k_ok & (ahead == 3)));
+          do_p = sleep ? mbar_sleep(&p_full[pbuf], pph) : mbar_test(&p_full[pbuf], pph);
+          if (do_p) do_p = mbar_try_wait(&o_ready[pbuf], pph) || mbar_sleep(&o_ready[pbuf], pph);
+        }
+        do_p &= v_ok;
+        if (dead) {   // nothing is waited for any more, and nothing leaves the buffers
+          do_p = ahead > 0;
+          k_ok = true;
+        }
+        const bool do_s = s_left & k_ok & (ahead - (int)do_p < 3);
+        if (!do_p & !do_s) {
+          if ((++spins & 0xffu) == 0) {
+            const unsigned long long now = global_timer_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > 2000000000ull && !dead) {
+              dead = true;
+              *reinterpret_cast<volatile unsigned*>(p.err) = kAttnWaitCode | 4;
+              *reinterpret_cast<volatile int*>(gave_up) = 1;
+              __threadfence_system();
+            }
+          }
+          continue;
+        }
+        t0 = 0;
         tc_fence_after();
-        const uint32_t ks = k_u + s * (C::TB >> 4), d = tmem + (uint32_t)((it & 1) * 64);
+        const bool p_last = do_p && p_it + 1 == p_n;
+        if (do_p) {
+          const uint32_t vt = v_u + vs * (C::TB >> 4), more = p_it > 0;
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk)
-          umma_lo<1>(d, q_u + (((kk / 4) * kTBM * 128 + (kk % 4) * 32) >> 4), ks + (((kk / 4) * kTBN * 128 + (kk % 4) * 32) >> 4), kIdescS,
-                     kk > 0 ? 1u : 0u);
-        umma_commit(&k_empty[s]);
-        umma_commit(&s_full[it & 1]);
-      };
-      wait_for(q_full, 0, kAttnWaitCode | 4);
-      scores(0);
-      for (int it = 0; it < n_tiles; ++it) {
-        // the buffer that tile it + 1 overwrites held P of tile it - 1: its product went out before, and products run in order
-        if (it + 1 < n_tiles) scores(it + 1);
-        const int s = it % ST, next = it + 2;
-        wait_for(&v_full[s], (uint32_t)((it / ST) & 1), kAttnWaitCode | 6);
-        wait_for(&p_full[it & 1], (uint32_t)((it >> 1) & 1), kAttnWaitCode | 5);
-        tc_fence_after();
-        k_ready = mbar_test(&k_full[next % ST], (uint32_t)((next / ST) & 1));
-        const uint32_t vs = v_u + s * (C::TB >> 4), ps = tmem + (uint32_t)((it & 1) * 64);
+          for (int kk = 0; kk < kTBN / 16; ++kk)   // 16 keys: 8 columns of P, 2 048 bytes further down V's rows
+            umma_ts(tmem + kColO, tmem + pbuf * 128 + kk * 8, vt + (kk * 2048 >> 4) + ((kTBN * 128 >> 4) << 16), kIdescO, kk > 0 ? 1u : more);
+          umma_commit(&pv_done[pbuf]);   // O may be rescaled while S is on
+          if (p_last) umma_commit(o_full);
+        }
+        if (do_s) {
+          const uint32_t kt = k_u + ks * (C::TB >> 4), d = tmem + sbuf * 128;
 #pragma unroll
-        for (int kk = 0; kk < kTBN / 16; ++kk)   // 16 keys: 8 columns of P, 2 048 bytes further down V's rows
-          umma_ts(tmem + kColO, ps + kk * 8, vs + (kk * 2048 >> 4) + ((kTBN * 128 >> 4) << 16), kIdescO, (it > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&v_empty[s]);
-        umma_commit(it + 1 < n_tiles ? pv_done : o_full);
+          for (int kk = 0; kk < HD / 16; ++kk) {
+            const uint32_t at = ((kk / 4) * 128 * 128 + (kk % 4) * 32) >> 4;
+            umma_lo<1>(d, q_u + at, kt + at, kIdescS, kk > 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[(sw.tile(s_it) & 1) * 3 + sbuf]);
+          umma_commit(&k_empty[ks]);
+          if (++ks == KST) {
+            ks = 0;
+            kph ^= 1;
+          }
+          if (++sbuf == 3) sbuf = 0;
+          ++ahead;
+          k_ok = false;
+          if (++s_it == sw.n) {
+            umma_commit(q_empty);
+            const int i = block_of(++sr);
+            s_it = 0;
+            s_left = i < p.blocks;
+            if (s_left) sw = Block(p, i);
+          }
+        }
+        if (do_p) {
+          umma_commit(&v_empty[vs]);
+          if (++vs == VST) {
+            vs = 0;
+            vph ^= 1;
+          }
+          if (++pbuf == 3) {
+            pbuf = 0;
+            pph ^= 1;
+          }
+          --ahead;
+          ++p_it;
+          v_ok = false;
+          if (p_last) {
+            const int i = block_of(++pr);
+            if (i >= p.blocks) break;
+            p_it = 0;
+            p_n = Block(p, i).n;
+          }
+        }
       }
       if (dead) drain_async();
     }
-  } else {
+  } else if (warp < 8) {
     // ---------------------------------------------------------------------------------------------- softmax
-    const int q = warp & 3, row = q * 32 + lane;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+    const int g = warp >> 2, q = warp & 3, row = q * 32 + lane;
     const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
-    const int rpos = first_pos + min(row, rows_valid - 1);   // padding rows behave like the last valid row
     const float k_scale = p.scale_log2;
     const uint64_t scale2 = pack_f2(k_scale, k_scale);
-    float m = -INFINITY, l = 0.f;
-    for (int it = 0; it < n_tiles; ++it) {
-      wait_for(&s_full[it & 1], (uint32_t)((it >> 1) & 1), kAttnWaitCode | 7);
-      __syncwarp();
-      tc_fence_after();
-      uint32_t s[2][32];
-      const uint32_t sbuf = lane_base + (uint32_t)((it & 1) * 64);
-      tmem_ld32(sbuf, s[0]);
-      tmem_ld32(sbuf + 32, s[1]);
-      tmem_wait_ld();
-      const int kbase = tile_of(it) * kTBN;
-      if (kbase + kTBN - 1 > first_pos || (p.window > 0 && last_pos - kbase >= p.window)) {
-        // the keys this row sees, a bit each (comparing them one by one took longer than a whole tile)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int k0 = kbase + i * 32;
-          const uint32_t seen = bits_below(rpos + 1 - k0) &
-                                (p.window > 0 ? ~bits_below(rpos + 1 - p.window - k0) | bits_below(p.keep_first - k0) : ~0u);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) s[i][j] = seen & (1u << j) ? s[i][j] : 0xff800000u;
-        }
-        const int vs = it % ST;
-        wait_for(&v_full[vs], (uint32_t)((it / ST) & 1), kAttnWaitCode | 10);
-        const uint4* vt = reinterpret_cast<const uint4*>(sV + vs * C::TB);
-        bool bad = false;
-#pragma unroll
-        for (int j = 0; j < C::TB / 16 / 128; ++j) {
-          const uint4 w = vt[j * 128 + row];
-          const uint32_t x[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) bad |= (x[e] & 0x7f80u) == 0x7f80u | (x[e] & 0x7f800000u) == 0x7f800000u;
-        }
-        if (bad) *not_finite = 1;
-        __syncwarp();
-      }
-      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(s[0][j + e]), __uint_as_float(s[1][j + e])));
-      }
-      const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      const bool grow = top > m;
-      const bool rescale = it > 0 && __any_sync(0xffffffffu, grow);
-      const float alpha = grow && it > 0 ? ex2f((m - top) * k_scale) : 1.f;
-      if (grow) m = top;
-      l *= alpha;
-      const float ms = m == -INFINITY ? 0.f : m * k_scale;
-      const uint64_t neg = pack_f2(-ms, -ms);
-      uint64_t sum[2] = {0, 0};
-      uint32_t pk[32];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const uint64_t za = fma_f2(pack_f2(__uint_as_float(s[0][2 * j]), __uint_as_float(s[0][2 * j + 1])), scale2, neg);
-        const uint64_t zb = fma_f2(pack_f2(__uint_as_float(s[1][2 * j]), __uint_as_float(s[1][2 * j + 1])), scale2, neg);
-        const float a0 = ex2f(lo_f2(za)), a1 = ex2f(hi_f2(za)), b0 = ex2f(lo_f2(zb)), b1 = ex2f(hi_f2(zb));
-        sum[0] = add_f2(sum[0], pack_f2(a0, a1));
-        sum[1] = add_f2(sum[1], pack_f2(b0, b1));
-        pk[j] = pack2(a0, a1);
-        pk[16 + j] = pack2(b0, b1);
-      }
-      sum[0] = add_f2(sum[0], sum[1]);
-      l += lo_f2(sum[0]) + hi_f2(sum[0]);
-      tmem_st32(sbuf, pk);
-      if (rescale) {
-        wait_for(pv_done, (uint32_t)((it - 1) & 1), kAttnWaitCode | 8);
+    int c = -1, buf = 2;   // the tile's number, its S buffer
+    uint32_t s_ph = 0;
+    for (int r = 0, i; (i = block_of(r)) < p.blocks; ++r) {
+      const Block w(p, i);
+      const int rpos = w.first_pos + min(row, w.rows_valid - 1);   // padding rows behave like the last valid row
+      float held = -INFINITY;         // the maximum of the tiles before, where this group has had the last of them
+      float m = -INFINITY, l = 0.f;   // of this group's tiles: the maximum that the weights were last taken against, their sum
+      for (int it = 0, prev = -1; it < w.n; ++it) {
+        const int tile = w.tile(it), mine = tile & 1;
+        ++c;
+        if (++buf == 3) buf = 0;
+        const bool from_other = it > 0 && prev != g;
+        prev = mine;
+        if (mine != g) continue;
+        const int kbase = tile * kTBN;
+        const uint32_t s_at = lane_base + buf * 128;
+        const bool part = w.in_part(p, kbase);
+        wait_for(&s_full[g * 3 + buf], s_ph >> buf & 1, kAttnWaitCode | 10);
+        s_ph ^= 1u << buf;
         __syncwarp();
         tc_fence_after();
-        const uint64_t alpha2 = pack_f2(alpha, alpha);
-#pragma unroll 1
-        for (int c = 0; c < HD; c += 64) {
-          uint32_t o[2][32];
-          tmem_ld32(lane_base + kColO + c, o[0]);
-          tmem_ld32(lane_base + kColO + c + 32, o[1]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              const uint64_t y = mul_f2(pack_f2(__uint_as_float(o[i][j]), __uint_as_float(o[i][j + 1])), alpha2);
-              o[i][j] = (uint32_t)y;
-              o[i][j + 1] = (uint32_t)(y >> 32);
-            }
-          tmem_st32(lane_base + kColO + c, o[0]);
-          tmem_st32(lane_base + kColO + c + 32, o[1]);
+        const float2* const from = &m_row[((c - 1) & 3) * kTBM + row];
+        float2 passed = ld_volatile_f2(from);
+        uint32_t s[4][32];
+        tmem_ld32(s_at, s[0]);
+        tmem_ld32(s_at + 32, s[1]);
+        // the maximum of the tiles before, from the group that had the last of them
+        if (from_other) {
+          if (__builtin_expect(__any_sync(0xffffffffu, __float_as_int(passed.y) != c - 1), 0)) wait_passed(from, c - 1, passed);
+          held = passed.x;
         }
+        tmem_loaded(s[0]);
+        tmem_loaded(s[1]);
+        tmem_ld32(s_at + 64, s[2]);
+        tmem_ld32(s_at + 96, s[3]);
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        auto look = [&](int k) {
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) mx[e / 2 % 4] = max3f(mx[e / 2 % 4], __uint_as_float(s[k][e]), __uint_as_float(s[k][e + 1]));
+        };
+        if (__builtin_expect(part, 0)) {   // the keys this row sees, a bit each (comparing them one by one took longer than a whole tile)
+          tmem_loaded(s[2]);
+          tmem_loaded(s[3]);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int k0 = kbase + k * 32;
+            const uint32_t seen = bits_below(rpos + 1 - k0) &
+                                  (p.window > 0 ? ~bits_below(rpos + 1 - p.window - k0) | bits_below(p.keep_first - k0) : ~0u);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) s[k][e] = seen & (1u << e) ? s[k][e] : 0xff800000u;
+          }
+          asm volatile("" ::: "memory");   // a branch, and not two selections per key of every tile
+        }
+        look(0);
+        look(1);
+        tmem_loaded(s[2]);
+        tmem_loaded(s[3]);
+        look(2);
+        look(3);
+        const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        const float next = fmaxf(held, top);
+        st_volatile_f2(&m_row[(c & 3) * kTBM + row], make_float2(next, __int_as_float(c)));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&m_full[buf]);
+        held = next;
+        const float ms = next == -INFINITY ? 0.f : next * k_scale;
+        const uint64_t neg = pack_f2(-ms, -ms);
+        uint64_t sum[2] = {0, 0};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) weights32(s[k], scale2, neg, sum, s_at + k * 16);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[buf]);
+        if (top != -INFINITY) {   // a tile of which the row sees nothing leaves its sums as they are, however its prompt is cut
+          l *= m == -INFINITY ? 1.f : ex2f((m - held) * k_scale);
+          m = held;
+        }
+        sum[0] = add_f2(sum[0], sum[1]);
+        l += lo_f2(sum[0]) + hi_f2(sum[0]);
       }
-      tmem_wait_st();
-      tc_fence_before();
+      wait_for(&ml_empty[r & 1], (uint32_t)(((r >> 1) & 1) ^ 1), kAttnWaitCode | 12);
+      ml[((r & 1) * 2 + g) * kTBM + row] = make_float2(m, l);
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[it & 1]);
+      if (lane == 0) mbar_arrive(&ml_full[r & 1]);
     }
-    // ---- the end has a barrier of its own: a parity tells a phase from its neighbours only, and here the products of the last two tiles may
-    // both be running (inside the loop S of tile it says that the product of tile it - 2 is over).
-    if (n_tiles > 0) wait_for(o_full, 0, kAttnWaitCode | 9);
-    __syncwarp();
-    tc_fence_after();
-    named_bar_sync(1, 128);   // every load and product of this CTA is over
-    mine = make_float4(m, l, *not_finite != 0 ? 1.f : 0.f, dead || *gave_up != 0 ? 1.f : 0.f);
-    if constexpr (SPLIT == 2) {   // the other CTA's columns, the maxima and the sums go where Q and K were
-      part[row] = mine;
-      if (n_tiles > 0) {
-#pragma unroll 1
-        for (int c = 0; c < HD / 2; c += 32) {
-          uint32_t o[32];
-          tmem_ld32(lane_base + kColO + (half ^ 1) * (HD / 2) + c, o);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            give[(c / 4 + j) * kTBM + row] = make_float4(__uint_as_float(o[4 * j]), __uint_as_float(o[4 * j + 1]), __uint_as_float(o[4 * j + 2]),
-                                                         __uint_as_float(o[4 * j + 3]));
-        }
-      }
-    }
-  }
-  // The next launch may come in only now: started with this one, its blocks, the longest first, would take the places that free up early, two long
-  // ones to an SM (16 heads of 128 over 2 048 rows, calls behind each other: 42.2 µs)
-  if (p.pdl) pdl_trigger();
-  __syncwarp();
-  if constexpr (SPLIT == 2) cluster_sync_all();   // both halves have written
-  if (warp >= 2) {
-    // ---- merge, normalise and store this CTA's columns
-    constexpr int W = HD / SPLIT, CH = W / 8;   // columns; 16-byte pieces of a row of results
+  } else {
+    // ----------------------------------------------------------------------------- O: rescaled, in the end normalised and stored
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
     const int q = warp & 3, row = q * 32 + lane;
-    const int r = q0 + min(row, rows_valid - 1);
-    const uint32_t o_at = tmem + ((uint32_t)(q * 32) << 16) + kColO + half * W;
+    const uint32_t o_at = tmem + ((uint32_t)(q * 32) << 16) + kColO;
     const float k_scale = p.scale_log2;
-    float4 other = make_float4(-INFINITY, 0.f, 0.f, 0.f), y[SPLIT == 2 ? W / 4 : 1];
-    if constexpr (SPLIT == 2) {
-      const uint32_t take = mapa_u32(smem_u32(&give[row]), (uint32_t)(half ^ 1));
-      other = ld_cluster_f4(mapa_u32(smem_u32(&part[row]), (uint32_t)(half ^ 1)));
-#pragma unroll
-      for (int j = 0; j < W / 4; ++j) y[j] = ld_cluster_f4(take + j * kTBM * 16);
-      cluster_arrive();   // the other half may leave; its wait lies behind the store
-    }
-    const bool alone = __any_sync(0xffffffffu, mine.z + other.z != 0.f);
-    float m = fmaxf(mine.x, other.x);
-    // a half whose tiles the row does not see has no maximum and a sum of 0, or of NaN where its scores were
-    const float fm = SPLIT == 1 ? 1.f : mine.x == -INFINITY ? mine.y : ex2f((mine.x - m) * k_scale);
-    const float fo = SPLIT == 1 ? 0.f : other.x == -INFINITY ? other.y : ex2f((other.x - m) * k_scale);
-    float l = SPLIT == 1 ? mine.y : mine.y * fm + other.y * fo;
-    if (__all_sync(0xffffffffu, mine.w + other.w == 0.f)) {
-      if (alone) {
-        float ml[2] = {-INFINITY, 0.f}, none[32];
-        see_alone<HD>(p, b, h, kvh, r, ml, -1, none);
-        m = ml[0];
-        l = ml[1];
-      }
-      if (p.sink && m != -INFINITY) l += ex2f(-m * k_scale);
-      float inv = l > 0.f ? 1.f / l : 0.f;
-      if (p.gate != nullptr && row < rows_valid)
-        inv *= 1.f / (1.f + expf(-bf16_to_f(p.gate[(size_t)b * p.q_bs + (size_t)(q0 + row) * p.q_rs + h])));
-      // through shared memory (where V was), so that a store covers whole rows: straight from the lanes it touches 32 of them
-      uint8_t* const mid = sV + q * (32 * W * 2);
-      auto place = [&](int rw, int c) { return mid + rw * (W * 2) + (c ^ ((CH >= 8 ? rw : rw >> 1) & (CH >= 8 ? 7 : 3))) * 16; };
-      const uint32_t km = fm != 0.f ? ~0u : 0u, ko = fo != 0.f ? ~0u : 0u;   // what a half of weight 0 holds is not looked at
-      const float wm = fm * inv, wo = fo * inv;
-      auto mix = [&](uint32_t a, float b) {
-        if constexpr (SPLIT == 1) return __uint_as_float(a) * inv;
-        return __uint_as_float(a & km) * wm + __uint_as_float(__float_as_uint(b) & ko) * wo;
-      };
-#pragma unroll
-      for (int c = 0; c < W; c += 32) {
-        uint32_t o[32];
-        tmem_ld32(o_at + c, o);
-        tmem_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 ya = y[SPLIT == 2 ? c / 4 + 2 * j : 0], yb = y[SPLIT == 2 ? c / 4 + 2 * j + 1 : 0];
-          uint4 v;
-          v.x = pack2(mix(o[8 * j], ya.x), mix(o[8 * j + 1], ya.y));
-          v.y = pack2(mix(o[8 * j + 2], ya.z), mix(o[8 * j + 3], ya.w));
-          v.z = pack2(mix(o[8 * j + 4], yb.x), mix(o[8 * j + 5], yb.y));
-          v.w = pack2(mix(o[8 * j + 6], yb.z), mix(o[8 * j + 7], yb.w));
-          *reinterpret_cast<uint4*>(place(lane, c / 8 + j)) = v;
+    int c = -1, buf = 2;   // the tile's number, its S buffer
+    uint32_t ph = 1;
+    for (int r = 0, i; (i = block_of(r)) < p.blocks; ++r) {
+      const Block w(p, i);
+      float was = -INFINITY;
+      for (int it = 0; it < w.n; ++it) {
+        ++c;
+        const int before = buf;
+        const uint32_t before_ph = ph;
+        if (++buf == 3) {
+          buf = 0;
+          ph ^= 1;
         }
-      }
-      if (alone) {
+        wait_for(&m_full[buf], ph, kAttnWaitCode | 11);
+        __syncwarp();
+        const float now = ld_volatile_f2(&m_row[(c & 3) * kTBM + row]).x;
+        if (it > 0 && __any_sync(0xffffffffu, now != was)) {
+          const float alpha = now != was ? ex2f((was - now) * k_scale) : 1.f;
+          const uint64_t alpha2 = pack_f2(alpha, alpha);
+          wait_for(&pv_done[before], before_ph, kAttnWaitCode | 21);
+          __syncwarp();
+          tc_fence_after();
 #pragma unroll 1
-        for (int c = 0; c < W; c += 32) {
-          float ml[2] = {m, l}, x[32];
-          for (int e = 0; e < 32; ++e) x[e] = 0.f;
-          see_alone<HD>(p, b, h, kvh, r, ml, half * W + c, x);
-          for (int e = 0; e < 32; ++e) reinterpret_cast<__nv_bfloat16*>(place(lane, (c + e) / 8))[e & 7] = f_to_bf16(x[e] * inv);
-        }
-      }
-      __syncwarp();
-      __nv_bfloat16* const dst = p.o + (size_t)b * p.o_bs + (size_t)h * HD + half * W + (lane % CH) * 8;
+          for (int k = 0; k < HD; k += 64) {
+            uint32_t o[2][32];
+            tmem_ld32(o_at + k, o[0]);
+            tmem_ld32(o_at + k + 32, o[1]);
 #pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int rw = i * (32 / CH) + lane / CH;
-        if (q * 32 + rw < rows_valid)
-          *reinterpret_cast<uint4*>(dst + (size_t)(q0 + q * 32 + rw) * p.o_rs) = *reinterpret_cast<const uint4*>(place(rw, lane % CH));
+            for (int i = 0; i < 2; ++i) {
+              tmem_loaded(o[i]);
+#pragma unroll
+              for (int e = 0; e < 32; e += 2) {
+                const uint64_t y = mul_f2(pack_f2(__uint_as_float(o[i][e]), __uint_as_float(o[i][e + 1])), alpha2);
+                o[i][e] = (uint32_t)y;
+                o[i][e + 1] = (uint32_t)(y >> 32);
+              }
+              tmem_st32(o_at + k + i * 32, o[i]);
+            }
+          }
+          tmem_wait_st();
+          tc_fence_before();
+        }
+        was = now;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&o_ready[buf]);
       }
+      wait_for(&ml_full[r & 1], (uint32_t)((r >> 1) & 1), kAttnWaitCode | 13);
+      __syncwarp();
+      float2 part[2];
+#pragma unroll
+      for (int g = 0; g < 2; ++g) part[g] = ml[((r & 1) * 2 + g) * kTBM + row];
+      float m = fmaxf(part[0].x, part[1].x), l = 0.f;
+#pragma unroll
+      for (int g = 0; g < 2; ++g)   // a group whose tiles the row does not see has no maximum and a sum of 0, or of NaN where its scores were
+        l = __fadd_rn(l, part[g].x == -INFINITY ? part[g].y : __fmul_rn(part[g].y, ex2f((part[g].x - m) * k_scale)));
+      wait_for(o_full, (uint32_t)(r & 1), kAttnWaitCode | 14);
+      __syncwarp();
+      tc_fence_after();
+      const bool lost = __any_sync(0xffffffffu, dead || *reinterpret_cast<volatile int*>(gave_up) != 0);
+      store_rows<HD>(p, &to, w, o_at, row, m, l, sO + q * (32 * 128), 0, lost, [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(o_empty);
+      });
+      if (lane == 0) mbar_arrive(&ml_empty[r & 1]);
     }
-    tc_fence_before();
-    __syncwarp();
-  } else if constexpr (SPLIT == 2) {
-    cluster_arrive();
+    if (lane == 0) bulk_read();
   }
-  if constexpr (SPLIT == 2) cluster_wait();   // neither half leaves while the other still reads
-  __syncthreads();                            // nor frees its TMEM before its own warps have read
-  if (warp == 2) {
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 13) {
     tc_fence_after();
     tmem_free<1>(tmem, kCols);
   }
 }
 
-template <int HD, int SPLIT>
+template <int HD>
 int launch_tc(const TcPrefillAttn& a, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(attn_tc_kernel<HD, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::smem);
+    attr_err = cudaFuncSetAttribute(attn_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::smem);
+    if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(attn_tc_one_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::smem_one);
   });
   B200_CUDA(attr_err);
   TcAttn p{};
   int rc;
   if ((rc = wait_word(&p.err)) != B200_OK) return rc;
   p.o = a.o; p.gate = a.gate; p.o_rs = a.o_rs; p.o_bs = a.o_bs; p.q_rs = a.q_rs; p.q_bs = a.q_bs;
-  p.S = a.S; p.Hq = a.Hq; p.Hkv = a.Hkv; p.p0 = a.p0;
+  p.S = a.S; p.Hq = a.Hq; p.p0 = a.p0;
   p.scale_log2 = a.scale_log2; p.window = a.window; p.keep_first = a.keep_first; p.sink = a.sink;
   p.qp = a.q; p.kp = a.k; p.vp = a.v; p.kv_rs = a.kv_rs; p.kv_bs = a.kv_bs;
+  p.heads = a.B * a.Hq;
+  p.last = (a.S - 1) / kTBM;
+  p.blocks = p.heads * (p.last + 1);
+  p.by_heads = Div((uint32_t)p.heads);
+  p.by_hq = Div((uint32_t)a.Hq);
+  p.by_group = Div((uint32_t)(a.Hq / a.Hkv));
+  p.pdl = a.pdl;
   const int64_t keys = (int64_t)a.p0 + a.S;
-  CUtensorMap tq, tk, tv;
+  CUtensorMap tq, tk, tv, to;
   if ((rc = make_tmap_sw128(&tq, 3, a.q, a.B, a.S, (int64_t)a.Hq * HD, a.q_bs, a.q_rs, kTBM)) != B200_OK) return rc;
   if ((rc = make_tmap_sw128(&tk, 3, a.k, a.B, keys, (int64_t)a.Hkv * HD, a.kv_bs, a.kv_rs, kTBN)) != B200_OK) return rc;
   if ((rc = make_tmap_sw128(&tv, 3, a.v, a.B, keys, (int64_t)a.Hkv * HD, a.kv_bs, a.kv_rs, kTBN)) != B200_OK) return rc;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)a.Hq * SPLIT, (unsigned)((a.S + kTBM - 1) / kTBM), (unsigned)a.B);
-  cfg.blockDim = dim3(kTThreads);
-  cfg.dynamicSmemBytes = TcCfg<HD>::smem;
-  cfg.stream = st;
-  // Behind another launch's end the blocks find some SMs still busy and the longest ones pair up on the others: where two CTAs an SM hold the whole
-  // grid and the chains are long, that costs more than the launch (16 heads of 128 over 2 048 rows 40.3 against 37.9 µs; four sequences of 14
-  // heads of 64 over 333 rows, six tiles, 10.0 against 12.1; 32 heads of 128 over 2 048 rows, two rounds, 48.2 against 54).
-  const int64_t blocks = (int64_t)a.B * a.Hq * ((a.S + kTBM - 1) / kTBM);
-  p.pdl = a.pdl && (SPLIT == 2 || blocks <= 148 || blocks > 296 || keys < 16 * kTBN);
-  cudaLaunchAttribute attr[2] = {};
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = p.pdl;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = 2;
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = SPLIT == 2 ? 2 : 1;
-  g_launches.fetch_add(1);
-  B200_CUDA(cudaLaunchKernelEx(&cfg, attn_tc_kernel<HD, SPLIT>, tq, tk, tv, p));
+  if ((rc = make_tmap_sw128(&to, 3, a.o, a.B, a.S, (int64_t)a.Hq * HD, a.o_bs, a.o_rs, 32)) != B200_OK) return rc;
+  if (keys <= kTBN) {
+    B200_CUDA(launch_pdl(attn_tc_one_kernel<HD>, dim3((unsigned)p.blocks), dim3(128), (size_t)TcCfg<HD>::smem_one, st, p.pdl != 0, tq, tk, tv, to, p));
+    return B200_OK;
+  }
+  B200_CUDA(launch_pdl(attn_tc_kernel<HD>, dim3((unsigned)std::min(p.blocks, kTCtas)), dim3(kTThreads), (size_t)TcCfg<HD>::smem, st, p.pdl != 0, tq, tk, tv, to, p));
   return B200_OK;
 }
 
 }  // namespace
 
 bool prefill_attn_tc_ok(const TcPrefillAttn& a, int hd) {
-  return (hd == 64 || hd == 128) && (a.S + kTBM - 1) / kTBM < 65536 && a.B < 65536 && aligned16(a.o, a.q, a.k, a.v) && a.q_rs % 8 == 0 &&
+  return (hd == 64 || hd == 128) && (int64_t)a.B * a.Hq * ((a.S + kTBM - 1) / kTBM) < (1ll << 31) && aligned16(a.o, a.q, a.k, a.v) && a.q_rs % 8 == 0 &&
          a.q_bs % 8 == 0 && a.kv_rs % 8 == 0 && a.kv_bs % 8 == 0 && a.o_rs % 8 == 0 && a.o_bs % 8 == 0;
 }
-// Whether this kernel beats the mma.sync one: where the longest block walks enough tiles of 64 keys, or a few of them in more blocks than that one
-// runs at once.  µs here / there: 16 heads of 128, one sequence 192 rows (three tiles) 8.5 / 7.3, 256 rows 8.5 / 8.6, 320 rows (five)
-// 9.3 / 10.0, two sequences 11.9 / 11.2, four 12.9 / 14.2; four sequences of 32 heads 128 rows (256 blocks of 64) 8.1 / 8.2, 160 rows
-// (384) 10.0 / 12.1, of 24 heads 160 rows (288) 9.9 / 9.8, 256 rows (384) 12.3 / 15.5; 14 heads of 64, one, two and four sequences: 320 rows (five)
-// 7.4 / 7.1, 8.9 / 7.3, 9.8 / 9.5, 333 rows (six) 7.4 / 7.8, 8.9 / 9.0, 10.1 / 12.1.
+// Whether this kernel beats the mma.sync one: where a block of 64 rows, that one's, walks enough tiles of 64 keys, or fewer in more blocks than that one
+// runs at once.  µs here / there: 16 heads of 128, one sequence 128 rows (two tiles) 5.3 / 5.5, 160 rows 6.3 / 6.6, 256 rows 6.8 / 8.2; 24 heads, two
+// sequences of 128 rows (96 blocks) 5.4 / 6.8; 14 heads of 64, one, two and four sequences: 160 rows (three) 5.4 / 4.6, 5.4 / 5.1, 6.0 / 6.2 (168 blocks),
+// 192 rows 5.4 / 4.9, 5.5 / 5.4, 6.0 / 6.9, 256 rows 5.6 / 5.8, 5.6 / 7.3, 6.2 / 8.8; 32 heads of 64, four sequences: 128 rows (256 blocks) 5.1 / 6.0, 160 rows
+// (384) 7.7 / 7.4.
 bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd, int rows) {
   const int last = (rows - 1) / 64 * 64;   // first row of the last block
   const int edge = a.window > 0 ? std::max(0, last - a.window + 1) / 64 : 0;
   const int tiles = last / 64 + 1 - edge + (a.window > 0 ? std::min(edge, (a.keep_first + 63) / 64) : 0);
-  return tiles >= (hd == 64 ? 6 : 5) || (hd == 128 && tiles >= 3 && (int64_t)a.B * a.Hq * (last / 64 + 1) > 296);
+  const int64_t blocks = (int64_t)a.B * a.Hq * (last / 64 + 1);
+  return hd == 128 ? tiles >= 3 || (tiles == 2 && blocks > 74) : tiles >= 4 || (tiles >= 2 && blocks > 148 && (tiles == 2 || blocks <= 296));
 }
-// Two CTAs per 128 rows of a head while all of them still run at once (two to an SM; a constant, since the two forms sum in other orders): the longest chain of tiles is half as long.  Beyond that the
-// second CTA's start and end cost more than the chain.  µs, one / two: 16 heads of 128 512 rows 12.9 / 10.6, 1 024 rows (128 blocks)
-// 20.5 / 15.7, 1 536 rows (192) 27.2 / 27.0, 2 048 rows 34.6 / 35.5; 32 heads 512 rows (128) 13.4 / 12.7, 768 rows (192) 17.7 / 22.0; a single
-// tile or two of them per block 5.7 / 7.4.
-static bool attn_tc_halves(const TcPrefillAttn& a, int rows) {
-  return rows > kTBM && (int64_t)a.B * a.Hq * ((rows + kTBM - 1) / kTBM) <= 148;
-}
-int launch_prefill_attn_tc(const TcPrefillAttn& a, int hd, int rows, cudaStream_t st) {
-  const bool two = attn_tc_halves(a, rows);
-  if (hd == 64) return two ? launch_tc<64, 2>(a, st) : launch_tc<64, 1>(a, st);
-  return two ? launch_tc<128, 2>(a, st) : launch_tc<128, 1>(a, st);
+int launch_prefill_attn_tc(const TcPrefillAttn& a, int hd, cudaStream_t st) {
+  return hd == 64 ? launch_tc<64>(a, st) : launch_tc<128>(a, st);
 }
 
 }  // namespace b200
