@@ -342,7 +342,8 @@ int launch_scan_cols(const LinScan& p, cudaStream_t st) {
 // columns (lane g holds rows 4g … 4g + 3 of every 4·LN): four shuffles to sum, and an operand that is read serves two columns —
 // shared loads and shuffles queue in one pipe, so one column per lane costs more (201 against 176 ns a token) although its chain
 // is shorter.  The decay and write of the old column and the output of the token before run beside the shuffles, the next token's
-// operands are asked for behind the last one, and the outputs of four tokens are summed together.  Keys past 256 take 32
+// operands are asked for behind the last one (its key ahead of them: 390 µs where this took 377), and the outputs of four tokens are summed together,
+// beside the shuffles of the next four: on their own they cost 18 to 20 ns a token.  Keys past 256 take 32
 // lanes, 32 and less take 8: at most 16 rows a lane is what the registers hold.
 // A CTA has four such warps, one per scheduler, and a fifth that keeps kRemBuf chunks in flight: staging from the walking warps
 // costs them 60 ns a token, and bulk copies of a row were no faster than cp.async.  The ring of keys past 64 with a decay per channel
@@ -350,7 +351,9 @@ int launch_scan_cols(const LinScan& p, cudaStream_t st) {
 // result of a sequence does not depend on what else is in the step; the order of the sums inside a column is fixed by dk alone.  fp32 throughout.
 // 2 048 tokens, 16 heads, per-channel decay, against one warp per two columns with chunks staged through registers:
 // 128 × 128 1 091 → 374 µs (183 ns a token), 64 × 64 742 → 312 µs, 126 × 128 (copies of 4 bytes) 1 117 → 406 µs;
-// 64 sequences of one token 130 → 120 µs.
+// 64 sequences of one token 130 → 120 µs; with outputs beside the next tokens 128 × 128 377 → 339 µs (166 ns a token), 64 × 64 316 → 275 µs,
+// 32 × 64 282 → 256 µs, one decay per head 128 × 128 369 → 329 µs.  What is left is the chain of a token, 150 cycles of latencies and the
+// instructions beside it that wait for one another in order: 32 lanes a column with half of the rows each take 173 ns, four columns a lane 234.
 constexpr int kRemBuf = 3, kRemThreads = 4 * 32 + 32;   // four warps that walk, one that stages
 template <int LN, int RPL, int C, bool SCALAR>
 struct ScanRem {
@@ -477,6 +480,65 @@ __global__ void __launch_bounds__(kRemThreads, (ScanRem<LN, RPL, C, SCALAR>::CTA
       const bool in = !fresh && j + c < dv;
       S[c][i] = pair2(in && d < dk ? st[(int64_t)d * dv + j + c] : 0.f, in && d + 1 < dk ? st[(int64_t)(d + 1) * dv + j + c] : 0.f);
     }
+  auto sum_rows = [&](const uint64_t(&w)[NP], const uint64_t(&y)[NP]) {   // this lane's rows of w · y, in two chains
+    uint64_t a0 = mul2(w[0], y[0]), a1 = mul2(w[1], y[1]);
+#pragma unroll
+    for (int i = 2; i < NP; i += 2) {
+      a0 = fma2(w[i], y[i], a0);
+      a1 = fma2(w[i + 1], y[i + 1], a1);
+    }
+    const float2 e = split2(a0), f = split2(a1);
+    return (e.x + e.y) + (f.x + f.y);
+  };
+  // Outputs of the last four tokens on their way: the last one's rows are summed, and the lanes' sums meet, beside the next four tokens' shuffles, where a
+  // lane has registers for that (not with 16 rows: 8 heads of 256 × 128 over 1 024 tokens 287 for 280 µs, 4 heads of 512 × 128 369 for 340).
+  // Tokens and columns change hands while they are summed: lane g ends with value g / (LN / (4·C)).
+  constexpr bool kBeside = RPL <= 8;
+  constexpr int kLevels = LN == 32 ? 5 : LN == 16 ? 4 : 3;
+  uint64_t r_old[NP];
+  float out[4 * C];
+  int out_row = -1;   // of the first of them; none on their way
+  auto meet = [&](auto level, float(&o)[4 * C]) {
+    constexpr int m = LN >> (decltype(level)::value + 1), w = 4 * C >> (decltype(level)::value + 1);
+    if constexpr (w > 0) {
+      const bool hi = gl & m;
+#pragma unroll
+      for (int i = 0; i < w; ++i) o[i] = (hi ? o[w + i] : o[i]) + shfl_xor_ordered(hi ? o[i] : o[w + i], m);
+    } else {
+      o[0] += shfl_xor_ordered(o[0], m);
+    }
+  };
+  auto put = [&] {
+    constexpr int each = LN / (4 * C);
+    const int c = j + gl / each % C;
+    if (out_row >= 0 && gl % each == 0 && c < dv) p.o[(int64_t)(out_row + gl / each / C) * p.ld_o + (int64_t)hd * dv + c] = out[0];
+  };
+  auto beside = [&](auto token) {   // what is done for them beside token 0, 1, 2 and 3
+    constexpr int u = decltype(token)::value;
+    if constexpr (u == 0) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) out[3 * C + c] = sum_rows(r_old, S[c]);
+    } else {
+      meet(std::integral_constant<int, u - 1>{}, out);
+    }
+    if constexpr (u == 3) {
+      if constexpr (kLevels > 3) meet(std::integral_constant<int, 3>{}, out);
+      if constexpr (kLevels > 4) meet(std::integral_constant<int, 4>{}, out);
+      put();
+    }
+  };
+  auto flush = [&] {
+    if (out_row < 0) return;
+    beside(std::integral_constant<int, 0>{});
+    beside(std::integral_constant<int, 1>{});
+    beside(std::integral_constant<int, 2>{});
+    beside(std::integral_constant<int, 3>{});
+    out_row = -1;
+  };
+#pragma unroll
+  for (int i = 0; i < NP; ++i) r_old[i] = 0;
+#pragma unroll
+  for (int i = 0; i < 4 * C; ++i) out[i] = 0.f;
   for (int c0 = 0; c0 < cnt; c0 += CH) {
     const int n = min(CH, cnt - c0);
     __syncthreads();
@@ -496,52 +558,24 @@ __global__ void __launch_bounds__(kRemThreads, (ScanRem<LN, RPL, C, SCALAR>::CTA
       load(pp, 2);
       load(r, 3);
     };
-    auto sum_rows = [&](const uint64_t(&w)[NP], const uint64_t(&y)[NP]) {   // this lane's rows of w · y, in two chains
-      uint64_t a0 = mul2(w[0], y[0]), a1 = mul2(w[1], y[1]);
-#pragma unroll
-      for (int i = 2; i < NP; i += 2) {
-        a0 = fma2(w[i], y[i], a0);
-        a1 = fma2(w[i + 1], y[i + 1], a1);
-      }
-      const float2 e = split2(a0), f = split2(a1);
-      return (e.x + e.y) + (f.x + f.y);
-    };
     operands();
-    auto walk = [&](int t, auto group) {   // `group` tokens from t on
-      constexpr int U = decltype(group)::value;
-      float vj[C][U], dc[U], out[U * C];
-      if constexpr (U == 4) {
-        const float4 e = scaled ? *reinterpret_cast<const float4*>(vs + t) : make_float4(1.f, 1.f, 1.f, 1.f);
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          const float4 a = *reinterpret_cast<const float4*>(v + c * CH + t);
-          vj[c][0] = a.x * e.x, vj[c][1] = a.y * e.y, vj[c][2] = a.z * e.z, vj[c][3] = a.w * e.w;
-        }
-        if constexpr (SCALAR) {
-          const float4 g = *reinterpret_cast<const float4*>(sd + t);
-          dc[0] = g.x, dc[1] = g.y, dc[2] = g.z, dc[3] = g.w;
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < C; ++c) vj[c][0] = scaled ? v[c * CH + t] * vs[t] : v[c * CH + t];
-        if constexpr (SCALAR) dc[0] = sd[t];
-      }
-      uint64_t r_old[NP];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
+    if constexpr (kBeside) {
+      // one token: its dot, the sum over the lanes with `between` behind the first shuffles, the new column; then the next one's operands
+      auto step = [&](int t, const float(&vj)[C], float dc, auto between) {
         float rem[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) rem[c] = sum_rows(q, S[c]);
 #pragma unroll
-        for (int m = LN / 2; m > 0; m >>= 1)
+        for (int m = LN / 2; m > 0; m >>= 1) {
 #pragma unroll
           for (int c = 0; c < C; ++c) rem[c] += shfl_xor_ordered(rem[c], m);
+          if (m == LN / 2) between();
+        }
         uint64_t kept[C][NP];
-        const uint64_t d2 = SCALAR ? pair2(dc[u], dc[u]) : 0;
+        const uint64_t d2 = SCALAR ? pair2(dc, dc) : 0;
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-          if (u > 0) out[(u > 0 ? u - 1 : 0) * C + c] = sum_rows(r_old, S[c]);
-          const uint64_t v2 = pair2(vj[c][u], vj[c][u]);
+          const uint64_t v2 = pair2(vj[c], vj[c]);
 #pragma unroll
           for (int i = 0; i < NP; ++i) kept[c][i] = fma2(b[i], v2, mul2(SCALAR ? d2 : d[i], S[c][i]));
         }
@@ -553,28 +587,137 @@ __global__ void __launch_bounds__(kRemThreads, (ScanRem<LN, RPL, C, SCALAR>::CTA
         }
 #pragma unroll
         for (int i = 0; i < NP; ++i) r_old[i] = r[i];
-        at += t + u + 1 < n ? NV * DK * 4 : 0;
+        at += t + 1 < n ? NV * DK * 4 : 0;
         operands();
+      };
+      auto walk4 = [&](int t) {
+        float vj[4][C], dc[4];
+        const float4 e = scaled ? *reinterpret_cast<const float4*>(vs + t) : make_float4(1.f, 1.f, 1.f, 1.f);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const float4 a = *reinterpret_cast<const float4*>(v + c * CH + t);
+          vj[0][c] = a.x * e.x, vj[1][c] = a.y * e.y, vj[2][c] = a.z * e.z, vj[3][c] = a.w * e.w;
+        }
+        if constexpr (SCALAR) {
+          const float4 g = *reinterpret_cast<const float4*>(sd + t);
+          dc[0] = g.x, dc[1] = g.y, dc[2] = g.z, dc[3] = g.w;
+        }
+        float fresh[4 * C];
+        auto token = [&](auto u) {
+          constexpr int U = decltype(u)::value;
+          step(t + U, vj[U], SCALAR ? dc[U] : 0.f, [&] {
+            if constexpr (U > 0) {
+#pragma unroll
+              for (int c = 0; c < C; ++c) fresh[(U - 1) * C + c] = sum_rows(r_old, S[c]);
+            }
+            beside(u);
+          });
+        };
+        token(std::integral_constant<int, 0>{});
+        token(std::integral_constant<int, 1>{});
+        token(std::integral_constant<int, 2>{});
+        token(std::integral_constant<int, 3>{});
+#pragma unroll
+        for (int i = 0; i < 3 * C; ++i) out[i] = fresh[i];
+        out_row = r0 + c0 + t;
+      };
+      auto walk1 = [&](int t) {
+        float vj[C], o[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) vj[c] = scaled ? v[c * CH + t] * vs[t] : v[c * CH + t];
+        step(t, vj, SCALAR ? sd[t] : 0.f, [] {});
+#pragma unroll
+        for (int c = 0; c < C; ++c) o[c] = sum_rows(r_old, S[c]);
+        int m = LN / 2;
+#pragma unroll
+        for (int w = C / 2; w > 0; w >>= 1, m >>= 1) {
+          const bool hi = gl & m;
+#pragma unroll
+          for (int i = 0; i < w; ++i) o[i] = (hi ? o[w + i] : o[i]) + shfl_xor_ordered(hi ? o[i] : o[w + i], m);
+        }
+#pragma unroll
+        for (; m > 0; m >>= 1) o[0] += shfl_xor_ordered(o[0], m);
+        constexpr int each = LN / C;
+        const int c = j + gl / each;
+        if (gl % each == 0 && c < dv) p.o[(int64_t)(r0 + c0 + t) * p.ld_o + (int64_t)hd * dv + c] = o[0];
+      };
+      int t = 0;
+      for (; t + 4 <= n; t += 4) walk4(t);
+      if (t < n) {
+        flush();
+        for (; t < n; ++t) walk1(t);
       }
+    } else {   // as they come, four tokens at a time
+      auto walk = [&](int t, auto group) {   // `group` tokens from t on
+        constexpr int U = decltype(group)::value;
+        float vj[C][U], dc[U], out[U * C];
+        if constexpr (U == 4) {
+          const float4 e = scaled ? *reinterpret_cast<const float4*>(vs + t) : make_float4(1.f, 1.f, 1.f, 1.f);
 #pragma unroll
-      for (int c = 0; c < C; ++c) out[(U - 1) * C + c] = sum_rows(r_old, S[c]);
-      int m = LN / 2;   // tokens and columns change hands while they are summed: lane g ends with value g / (LN / (U·C))
+          for (int c = 0; c < C; ++c) {
+            const float4 a = *reinterpret_cast<const float4*>(v + c * CH + t);
+            vj[c][0] = a.x * e.x, vj[c][1] = a.y * e.y, vj[c][2] = a.z * e.z, vj[c][3] = a.w * e.w;
+          }
+          if constexpr (SCALAR) {
+            const float4 g = *reinterpret_cast<const float4*>(sd + t);
+            dc[0] = g.x, dc[1] = g.y, dc[2] = g.z, dc[3] = g.w;
+          }
+        } else {
 #pragma unroll
-      for (int w = U * C / 2; w > 0; w >>= 1, m >>= 1) {
-        const bool hi = gl & m;
+          for (int c = 0; c < C; ++c) vj[c][0] = scaled ? v[c * CH + t] * vs[t] : v[c * CH + t];
+          if constexpr (SCALAR) dc[0] = sd[t];
+        }
+        uint64_t r_old[NP];
 #pragma unroll
-        for (int i = 0; i < w; ++i) out[i] = (hi ? out[w + i] : out[i]) + shfl_xor_ordered(hi ? out[i] : out[w + i], m);
-      }
+        for (int u = 0; u < U; ++u) {
+          float rem[C];
 #pragma unroll
-      for (; m > 0; m >>= 1) out[0] += shfl_xor_ordered(out[0], m);
-      constexpr int each = LN / (U * C);
-      const int u = gl / each / C, c = j + gl / each % C;
-      if (gl % each == 0 && c < dv) p.o[(int64_t)(r0 + c0 + t + u) * p.ld_o + (int64_t)hd * dv + c] = out[0];
-    };
-    int t = 0;
-    for (; t + 4 <= n; t += 4) walk(t, std::integral_constant<int, 4>{});
-    for (; t < n; ++t) walk(t, std::integral_constant<int, 1>{});
+          for (int c = 0; c < C; ++c) rem[c] = sum_rows(q, S[c]);
+#pragma unroll
+          for (int m = LN / 2; m > 0; m >>= 1)
+#pragma unroll
+            for (int c = 0; c < C; ++c) rem[c] += shfl_xor_ordered(rem[c], m);
+          uint64_t kept[C][NP];
+          const uint64_t d2 = SCALAR ? pair2(dc[u], dc[u]) : 0;
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            if (u > 0) out[(u > 0 ? u - 1 : 0) * C + c] = sum_rows(r_old, S[c]);
+            const uint64_t v2 = pair2(vj[c][u], vj[c][u]);
+#pragma unroll
+            for (int i = 0; i < NP; ++i) kept[c][i] = fma2(b[i], v2, mul2(SCALAR ? d2 : d[i], S[c][i]));
+          }
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            const uint64_t nr = pair2(-rem[c], -rem[c]);
+#pragma unroll
+            for (int i = 0; i < NP; ++i) S[c][i] = fma2(pp[i], nr, kept[c][i]);
+          }
+#pragma unroll
+          for (int i = 0; i < NP; ++i) r_old[i] = r[i];
+          at += t + u + 1 < n ? NV * DK * 4 : 0;
+          operands();
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) out[(U - 1) * C + c] = sum_rows(r_old, S[c]);
+        int m = LN / 2;   // tokens and columns change hands while they are summed: lane g ends with value g / (LN / (U·C))
+#pragma unroll
+        for (int w = U * C / 2; w > 0; w >>= 1, m >>= 1) {
+          const bool hi = gl & m;
+#pragma unroll
+          for (int i = 0; i < w; ++i) out[i] = (hi ? out[w + i] : out[i]) + shfl_xor_ordered(hi ? out[i] : out[w + i], m);
+        }
+#pragma unroll
+        for (; m > 0; m >>= 1) out[0] += shfl_xor_ordered(out[0], m);
+        constexpr int each = LN / (U * C);
+        const int u = gl / each / C, c = j + gl / each % C;
+        if (gl % each == 0 && c < dv) p.o[(int64_t)(r0 + c0 + t + u) * p.ld_o + (int64_t)hd * dv + c] = out[0];
+      };
+      int t = 0;
+      for (; t + 4 <= n; t += 4) walk(t, std::integral_constant<int, 4>{});
+      for (; t < n; ++t) walk(t, std::integral_constant<int, 1>{});
+    }
   }
+  if constexpr (kBeside) flush();
 #pragma unroll
   for (int c = 0; c < C; ++c)
 #pragma unroll
