@@ -24,7 +24,7 @@ void set_error(const char* fmt, ...);
 // cross-kernel L2 prefetch, whole-token persistent kernel) are not here any more.
 struct Defaults {
   static constexpr bool kPrefillAttnMma = true;   // B200_PREFILL_ATTN   "mma" (tensor cores) | "cuda" (CUDA cores)
-  // B200_GEMM "persistent" | "tile" | "wide": chosen per shape when unset (gemm.cu pick_gemm)
+  // B200_GEMM "persistent" | "tile" | "wide" | "half" | "narrow": chosen per shape when unset (gemm.cu pick_gemm)
 };
 bool env_flag(const char* name, bool dflt);                       // unset → dflt; else first character == '1'
 bool env_choice(const char* name, char yes_initial, bool dflt);   // unset → dflt; else first character == yes_initial

@@ -339,37 +339,41 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 //               a residual's row is on its way while the products run.  As a cluster of one, through shared memory, a tile took 1.5 to 3 µs longer
 //               (µs: 37 × 2 048 × 2 048 15.1, now 13.5; 1 024 × 10 944 × 2 048 83, now 71).
 //   kWide       the same with 256 columns: half the tiles, for row counts at which pairs of 256 rows leave a second round to a few of them
+//   kHalf, kNarrow   the same with 64 and 32 columns: short prompts of a narrow model, whose 128-column tiles would leave all of W to a few SMs
 //   kSplit      a cluster per 128 × 128 tile, for operators whose whole-K tiles would leave most SMs idle while the few busy ones stream
 //               all of W: `splits` CTAs take neighbouring ranges of K, leave their fp32 partial tiles in their own shared memory
 //               (the drained operand ring), and after one cluster barrier each sums its share of the rows over all partials
 //               through distributed shared memory, in rank order, and stores it.  No workspace, no second launch, no atomics.
 //   kSplitPair  the same with 256 × 256 tiles on CTA pairs; one split is a pair's plain tile.
-enum GemmForm : int { kWhole = 0, kSplit = 1, kSplitPair = 2, kWide = 3 };
-// The ring holds as many stages as 192 KB take: six of 128 rows of A, ten of 16 rows and fewer.
+enum GemmForm : int { kWhole = 0, kSplit = 1, kSplitPair = 2, kWide = 3, kHalf = 4, kNarrow = 5 };
+constexpr int form_columns(int form) { return form == kSplitPair || form == kWide ? 256 : form == kHalf ? 64 : form == kNarrow ? 32 : 128; }
+
+// The ring holds as many stages as 192 KB take: six of 128 rows of A, ten of 16 rows and fewer; up to fourteen of the narrow forms.
 constexpr int kSplitRing = 192 * 1024;
-constexpr int kSplitStagesMax = 10;
+constexpr int kSplitStagesMax = 14;
 constexpr int kSplitSmem = kSplitRing + 1024 /*align*/ + 256 /*barriers*/;
 static_assert(128 * (256 + 4) * 4 <= kSplitRing, "a partial tile fits in the drained ring");
 __host__ __device__ constexpr int split_stages(int box_rows, int b_bytes) {   // the MMA reads 128 rows (16 KB) from the last stage's A on
-  return (kSplitRing - kTileBytes + box_rows * kBK * 2) / (box_rows * kBK * 2 + b_bytes) < kSplitStagesMax
-             ? (kSplitRing - kTileBytes + box_rows * kBK * 2) / (box_rows * kBK * 2 + b_bytes) : kSplitStagesMax;
+  const int fit = (kSplitRing - kTileBytes + box_rows * kBK * 2) / (box_rows * kBK * 2 + b_bytes), most = b_bytes < kTileBytes ? kSplitStagesMax : 10;
+  return fit < most ? fit : most;
 }
 constexpr bool split_ring_holds(int b_bytes) {
   for (int r = 8; r <= 128; r += 8)
     if (split_stages(r, b_bytes) * b_bytes + (split_stages(r, b_bytes) - 1) * r * kBK * 2 + kTileBytes > kSplitRing) return false;
   return true;
 }
-static_assert(split_ring_holds(kTileBytes) && split_ring_holds(2 * kTileBytes), "what the MMA reads stays inside the ring");
+static_assert(split_ring_holds(kTileBytes / 4) && split_ring_holds(kTileBytes / 2) && split_ring_holds(kTileBytes) && split_ring_holds(2 * kTileBytes), "what the MMA reads stays inside the ring");
 
 template <typename OT, int EPI, int FORM>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmArgs<OT> p,
                   const int splits, const int box_rows) {
-  constexpr bool PAIR = FORM == kSplitPair, STRAIGHT = FORM == kWhole || FORM == kWide;
-  constexpr int BN = PAIR || FORM == kWide ? 256 : 128, BMT = PAIR ? 256 : 128, LD = BN + 4, GROUP = PAIR ? 2 : 1;
+  constexpr bool PAIR = FORM == kSplitPair, STRAIGHT = FORM != kSplit && FORM != kSplitPair;
+  constexpr int BN = form_columns(FORM), BMT = PAIR ? 256 : 128, LD = BN + 4, GROUP = PAIR ? 2 : 1;
   constexpr int B_BYTES = BN / GROUP * kBK * 2;   // of a k-block, per CTA
   constexpr int OUT = EPI == GEPI_SILU ? BN / 2 : BN;
   constexpr uint32_t kIdesc = umma_idesc(BMT, BN);
+  static_assert(BN >= 128 || EPI != GEPI_SILU, "an epilogue thread reads 32 gate and 32 up columns");
   static_assert(STRAIGHT || (sizeof(OT) == 2 && (EPI == GEPI_STORE || EPI == GEPI_BIAS)), "what operators ask for");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -710,7 +714,7 @@ int launch_split(const GemmArgs<OT>& args, const void* A, const void* B, int64_t
   GemmArgs<OT> p = args;
   int rc;
   if ((rc = split_setup<OT, EPI, FORM>()) != B200_OK || (rc = wait_word(&p.err)) != B200_OK) return rc;
-  constexpr int W = FORM == kSplitPair ? 2 : 1, BN = FORM == kSplitPair || FORM == kWide ? 256 : 128, OUT = BN / (EPI == GEPI_SILU ? 2 : 1);
+  constexpr int W = FORM == kSplitPair ? 2 : 1, BN = form_columns(FORM), OUT = BN / (EPI == GEPI_SILU ? 2 : 1);
   const int box_rows = (int)std::min<int64_t>(128, ((int64_t)p.M + 7) / 8 * 8);
   CUtensorMap ta, tb;
   if ((rc = make_tmap(&ta, A, p.M, p.K, box_rows)) != B200_OK) return rc;
@@ -729,12 +733,15 @@ constexpr int kSplitMinKb = 8;   // k-blocks that a split takes at least: shorte
 // every SM runs several tiles (power, L2); the rest is launch, pipeline fill and epilogue.  Measured, µs, M × N × K, one-CTA tiles / wide ones /
 // pairs / splits: 40 × 2 048 × 6 144 23.2 / 34.0 / 26.9 / 11.0; 128 × 16 384 × 3 072 22.3 / 27.3 / 24.7; 300 × 12 288 × 2 048, where 96 tiles are
 // two rounds of pairs and 288 two of single CTAs, but 144 wide ones a single round, 26.2 / 22.1 / 23.6; 2 048 × 2 048 × 2 048 21.6 / 16.2 / 17.0;
-// 2 048 × 12 288 × 2 048 123 / 108 / 71.  B200_GEMM = "persistent" (with a width: "persistent192") | "tile" | "wide" forces the
-// persistent pairs or one whole-K tile of 128 or 256 columns per CTA.  The products of a prompt pass (no split) find their weights in HBM and their epilogue
+// 2 048 × 12 288 × 2 048 123 / 108 / 71.  Narrower tiles are as many k-blocks long, and a k-block of theirs takes hardly less (0.2 µs, what the issuing
+// thread needs), but their results leave sooner and weights come through more SMs: 128 / 64 / 32 columns, 60 × 896 × 896 6.7 / 6.2 / 6.1, 128 × 896 × 896
+// 8.0 / 6.8 / 6.3, 300 × 1 152 × 896 7.9 / 6.8 / 6.2, 300 × 896 × 4 864 20.3 / 19.0 / 18.3, 128 × 4 096 × 4 096 18.4 / 17.4 / 17.2, 512 × 2 048 × 2 048 10.9 /
+// 10.3 / 18.2 (two rounds).  B200_GEMM = "persistent" (with a width: "persistent192") | "tile" | "wide" | "half" | "narrow" forces the
+// persistent pairs or one whole-K tile of 128, 256, 64 or 32 columns per CTA (SiLU pairs have none of the last two).  The products of a prompt pass (no split) find their weights in HBM and their epilogue
 // is not hidden when a pair has one tile: 5 µs on top of the fit, so pairs start later there (ms a prompt, tiles / pairs / the choice: 24 layers,
 // 896 wide, 60 rows 1.76 / 2.31 / 1.75, 300 rows 2.15 / 2.67 / 2.05; 28 layers, 2 048 wide, 500 rows 3.68 / 4.03 / 3.59, 1 000 rows 5.62 / 4.84 / 4.56).
 struct GemmPick {
-  int kind;     // 0: a CTA per tile (and split); 1: a pair per tile (and split); 2: persistent pairs; 3: a CTA per wide tile
+  int kind;     // 0: a CTA per tile (and split); 1: a pair per tile (and split); 2: persistent pairs; 3, 4, 5: a CTA per tile of 256, 64, 32 columns
   int splits;
   int bn;       // kind 2: columns of a tile
 };
@@ -758,8 +765,10 @@ void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
   const double f32_us = sizeof(OT) == 4 ? 2.5 : 0.0;   // 128 columns of fp32 results, a row per thread (2 049 × 2 048 × 2 048 logits: wide 24.9, pairs 22.1)
   const char* env = std::getenv("B200_GEMM");   // looked up once: routed experts' products wait for the host
   const char forced = env != nullptr ? env[0] : 0;
+  const bool slim = fits && EPI != GEPI_SILU && (forced == 'h' || forced == 'n');
   const bool tile = fits && forced == 't', wide = fits && forced == 'w', any_split = fits && !wide && forced != 'p';
   if (wide) consider(3, 1, 0.0);
+  if (slim) consider(forced == 'h' ? 4 : 5, 1, -1.0);
   if (!tile) {
     int only = forced == 'p' ? std::atoi(env + std::strcspn(env, "0123456789")) : 0;   // "persistent224": that width
     if (only != kPairBN && only != 224 && only != 192) only = 0;                       // one that is not built: any
@@ -776,6 +785,11 @@ void pick_gemm(int64_t M, int64_t N, int64_t K, GemmPick* out) {
     const int64_t t = up(M, 128) * up(N, 256 / D);
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
     consider(3, 1, (double)up(t, 2 * pairs) * (4.0 + 2.2 * rows + (t >= 100 ? 0.42 : 0.33) * (double)kb + (EPI == GEPI_SILU ? 2.0 : f32_us * 2)));
+  }
+  if (any_split && !tile && EPI != GEPI_SILU) {
+    const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
+    consider(4, 1, (double)up(up(M, 128) * up(N, 64), 2 * pairs) * (3.3 + 0.7 * rows + 0.2 * (double)kb + f32_us / 2));
+    consider(5, 1, (double)up(up(M, 128) * up(N, 32), 2 * pairs) * (3.25 + 0.25 * rows + 0.2 * (double)kb + f32_us / 4));
   }
   if (any_split) {
     const double rows = (double)std::min<int64_t>(M, 128) / 128.0;
@@ -804,6 +818,10 @@ int launch_gemm(const GemmArgs<OT>& args, const void* A, const void* B, int64_t 
   GemmPick g{};
   pick_gemm<OT, EPI, SPLIT>(p.M, p.N, p.K, &g);
   if (g.kind == 3) return launch_split<OT, EPI, kWide>(p, A, B, rows_b, 1, st);
+  if constexpr (EPI != GEPI_SILU) {
+    if (g.kind == 4) return launch_split<OT, EPI, kHalf>(p, A, B, rows_b, 1, st);
+    if (g.kind == 5) return launch_split<OT, EPI, kNarrow>(p, A, B, rows_b, 1, st);
+  }
   if (g.kind == 0 && g.splits == 1) return launch_split<OT, EPI, kWhole>(p, A, B, rows_b, 1, st);
   if constexpr (SPLIT) {
     if (g.kind == 0) return launch_split<OT, EPI, kSplit>(p, A, B, rows_b, g.splits, st);
