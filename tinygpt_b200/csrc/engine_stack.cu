@@ -98,8 +98,8 @@ struct StackEngine {
   int32_t *m_tok = nullptr, *m_slot = nullptr, *m_pos = nullptr, *m_want = nullptr, *m_upd = nullptr;
   int n_in_max = 0, k_out_max = 0;
   // bf16 engines: the big products leave the general kernel where their shapes allow — the weight-streaming GEMV
-  // (gemv.cu / gemv_batch.cu) for steps of up to kMaxBatch rows, the tcgen05 GEMM (gemm.cu) for steps of kGemmRows and
-  // more rows; B200_STACK_PLAIN=1 keeps everything on the general kernels
+  // (gemv.cu / gemv_batch.cu) for steps of up to kMaxBatch rows, the tcgen05 GEMM (gemm.cu) for steps of kProductRows or
+  // kGemmRows and more rows; B200_STACK_PLAIN=1 keeps everything on the general kernels
   bool fast = false;
   // the GEMV kernels wait for their producer themselves (griddepcontrol.wait) after they have filled their weight ring,
   // so they may be launched ahead of the end of whatever kernel precedes them; B200_NO_PDL=1 turns that off
@@ -177,7 +177,10 @@ struct StackEngine {
 constexpr int64_t kPoolScoreFloats = 32ll << 20;   // score workspace of prompts on the general kernels (rows go in portions)
 constexpr int kPoolSplitCtas = 4 * 148;            // split launches aim at this many CTAs
 static inline int up8i(int n) { return (n + 7) / 8 * 8; }
-constexpr int kGemmRows = 32;
+// Steps of a decode batch's rows stream W through GEMVs.  From kProductRows on a product whose sums are rounded alike goes to the tcgen05 GEMM (a layer
+// of width 2 048, 24 rows: in- and out-product 375 and 1 330 µs on the general kernel, 13 and 25 there); from kGemmRows on those, too, whose raw sums are
+// rounded to bf16 on the way there and stay fp32 in the general kernel.
+constexpr int kProductRows = kMaxBatch + 1, kGemmRows = 32;
 
 namespace {
 
@@ -343,6 +346,10 @@ static int stack_workspace(StackEngine* s, int tok, int rows) {
 }
 
 static inline bool gemm_shape_ok(int64_t N, int64_t K) { return N % 8 == 0 && K % 8 == 0 && K >= 64; }
+// a product of so many rows with a matrix [N, K] on the tcgen05 GEMM (a matrix off the 16-byte boundary: the general kernel, up to kGemmRows)
+static inline bool product_ok(const StackEngine* s, int rows, int64_t N, int64_t K, const void* w) {
+  return s->fast && rows >= kProductRows && gemm_shape_ok(N, K) && (rows >= kGemmRows || aligned16(w));
+}
 
 // proj = rmsnorm(x)·(offset + w) · w_inᵀ + b_in
 static int stack_product_in(StackEngine* s, int li, const float* x, int n_tok, cudaStream_t st) {
@@ -363,7 +370,7 @@ static int stack_product_in(StackEngine* s, int li, const float* x, int n_tok, c
   }
   if ((rc = launch_stack_rmsnorm(s->h, x, L.norm, nullptr, n_tok, W, d.norm_eps, d.norm_offset, s->dtype, st)) != B200_OK)
     return rc;
-  if (s->fast && n_tok >= kGemmRows && gemm_shape_ok(L.n_in, W)) {
+  if (product_ok(s, n_tok, L.n_in, W, L.w_in)) {
     return launch_gemm_bf16_bias(s->proj, s->h, L.w_in, L.b_in, n_tok, L.n_in, W, st);
   }
   StackGemm g;
@@ -386,7 +393,7 @@ static int stack_product_out(StackEngine* s, int li, float* x, int n_tok, cudaSt
     if ((rc = gemv_plan_set_batch(&pl, n_tok)) != B200_OK) return rc;
     return gemv_launch(pl, st, s->pdl);
   }
-  if (s->fast && n_tok >= kGemmRows && gemm_shape_ok(W, L.k_out))
+  if (product_ok(s, n_tok, W, L.k_out, L.w_out))
     return launch_gemm_bf16_accum(x, s->mid, L.w_out, s->d.residual_mult, n_tok, W, L.k_out, st);
   StackGemm g;
   g.a = s->mid; g.lda = L.k_out; g.k1 = L.k_out;
@@ -400,7 +407,7 @@ static int stack_product_mix(StackEngine* s, const float* cur, float* other, int
   const int W = s->d.width;
   int rc;
   const bool gemv = s->fast && n_tok <= kMaxBatch && s->ok_mix;
-  const bool gemm = s->fast && n_tok >= kGemmRows && gemm_shape_ok(W, 2 * W);
+  const bool gemm = product_ok(s, n_tok, W, 2 * W, s->d.mix_in);
   if (gemv || gemm) {
     if ((rc = launch_stack_cat_cast(s->cat, cur, s->x0, gemv ? other : nullptr, n_tok, W, st)) != B200_OK) return rc;
     if (gemv) {
@@ -554,6 +561,10 @@ static int stack_side(StackEngine* s, int li, float* cur, int n_tok, cudaStream_
   g.epi = SEPI_ACT_TABLE; g.c = s->sg; g.ldc = sd;
   g.table = d.side_table; g.tok = s->m_tok; g.table_ld = d.side_stride; g.table_col = L.side_col;
   if ((rc = launch_stack_gemm(g, s->dtype, st)) != B200_OK) return rc;
+  if (product_ok(s, n_tok, W, sd, L.side_proj)) {
+    if ((rc = launch_gemm_bf16_f32(s->y, s->sg, L.side_proj, nullptr, n_tok, W, sd, st)) != B200_OK) return rc;
+    return launch_stack_rms_add(cur, s->y, L.side_norm, n_tok, W, d.norm_eps, d.residual_mult, st);
+  }
   StackGemm p;
   p.a = s->sg; p.lda = sd; p.k1 = sd;
   p.w = L.side_proj; p.M = n_tok; p.N = W; p.K = sd;
@@ -565,8 +576,8 @@ static int stack_side(StackEngine* s, int li, float* cur, int n_tok, cudaStream_
 
 // ---------------------------------------------------------------------------------------------------- sandwich blocks
 // C = A·Wᵀ + bias for dense T-typed rows A [M, K]: out_t (T [M, N]) and / or out_f (fp32 [M, N]).  bf16 engines stream W
-// once for steps of up to kMaxBatch rows (GEMV; both outputs from the same fp32 sums), use the tcgen05 GEMM from kGemmRows
-// rows on (bias in its epilogue; fp32 alone is handed out unrounded, beside T it is the widened T), and the general kernel
+// once for steps of up to kMaxBatch rows (GEMV; both outputs from the same fp32 sums), use the tcgen05 GEMM from kProductRows
+// rows on (bias in its epilogue; fp32 alone is handed out unrounded, beside T it is the widened T from kGemmRows rows on), and the general kernel
 // otherwise.
 static int stack_lin(StackEngine* s, const void* A, const void* Wt, const float* bias, int M, int N, int K, const GemvPlan* plan,
                      void* out_t, float* out_f, cudaStream_t st) {
@@ -580,9 +591,10 @@ static int stack_lin(StackEngine* s, const void* A, const void* Wt, const float*
     if ((rc = gemv_plan_set_batch(&pl, M)) != B200_OK) return rc;
     return gemv_launch(pl, st, s->pdl);
   }
-  if (s->fast && M >= kGemmRows && gemm_shape_ok(N, K)) {
+  if (product_ok(s, M, N, K, Wt)) {
     if (out_t == nullptr) return launch_gemm_bf16_f32(out_f, A, Wt, bias, M, N, K, st);
     if ((rc = launch_gemm_bf16_bias(out_t, A, Wt, bias, M, N, K, st)) != B200_OK) return rc;
+    if (out_f && M < kGemmRows) return launch_gemm_bf16_f32(out_f, A, Wt, bias, M, N, K, st);
     return out_f ? launch_stack_widen(out_f, (const __nv_bfloat16*)out_t, (int64_t)M * N, st) : B200_OK;
   }
   StackGemm g;
@@ -1038,7 +1050,7 @@ static int stack_wkv(StackEngine* s, const b200_stack_layer& L, float* state, vo
     w2.M = n_tok; w2.N = hd; w2.K = rk;
     if ((rc = launch_small_gemv(w2, dt, st)) != B200_OK) return rc;
   } else {
-    if (s->fast && n_tok >= kGemmRows && gemm_shape_ok(hd, W)) {
+    if (product_ok(s, n_tok, hd, W, q.w_rkvg)) {
       for (int z = 0; z < 4; ++z)
         if ((rc = launch_gemm_bf16((uint8_t*)s->p4 + (size_t)z * n_tok * hd * 2, mix + (size_t)z * n_tok * W * 2,
                                    (const uint8_t*)q.w_rkvg + (size_t)z * hd * W * 2, n_tok, hd, W, st)) != B200_OK)
