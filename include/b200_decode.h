@@ -145,8 +145,8 @@ int b200_gemv_fused_bf16(void* y, const void* x, const void* W, int64_t n, int64
 /* Decode attention of one layer for one new token (B = 1, Sq = 1), one launch:
  *   q|k|v = qkv  →  [q_norm/k_norm per head]  →  RoPE(q), RoPE(k) at position *pos  →  K/V row *pos written in place
  *   into kcache/vcache [max_ctx, Hkv, hd]  →  split-KV softmax(q kᵀ/√hd) v over rows 0…*pos  →  out [Hq*hd].
- * Caches of up to eight splits of 256 (hd 64) / 128 (hd 128) keys: one CTA per (head group, split); larger ones: a cluster of
- * eight CTAs per head group shares the keys that exist.
+ * A cluster of up to sixteen CTAs per head group shares the keys that exist.  Where `out` lies off the 8-byte boundary and the caches have up to eight
+ * splits of 256 (hd 64) / 128 (hd 128) keys: one CTA per (head group, split), and the workspace is used.
  * *pos must have been written before the kernel that produced `qkv` was launched (the kernel reads it, and the cached
  * rows below it, ahead of its programmatic-dependency wait).
  * pos == NULL: plain attention over `fixed_len` cached rows, nothing appended; with a rope_table q is rotated as the token at position

@@ -155,8 +155,7 @@ PyObject* gemv_fused(PyObject*, PyObject* const* a, Py_ssize_t n_args) {   // x,
   END_HANDLE_TH_ERRORS
 }
 
-// qkv, kcache, vcache, q_heads, kv_heads, head_dim, pos or None, fixed_len, rope table or None, q_norm or None, k_norm or None, eps: caches whose
-// attention takes no workspace.  Shorter ones take tickets that are zeroed first, a torch kernel of its own that ops.py launches.
+// qkv, kcache, vcache, q_heads, kv_heads, head_dim, pos or None, fixed_len, rope table or None, q_norm or None, k_norm or None, eps
 PyObject* attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
   const at::Tensor *qkv, *kc, *vc, *pos, *rope, *qn, *kn;
@@ -169,12 +168,14 @@ PyObject* attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     PyErr_Clear();
     Py_RETURN_NONE;
   }
-  const int64_t ctx = kc->size(0), tickets = (4 * Hq + 15) / 16 * 16;
-  if (Hq < 1 || Hq > (1 << 20) || hd < 1 || hd > 1024 || abi.attn_decode_workspace_bytes(Hq, Hkv, hd, ctx) != tickets) Py_RETURN_NONE;
+  const int64_t ctx = kc->size(0);
+  if (Hq < 1 || Hq > (1 << 20) || hd < 1 || hd > 1024) Py_RETURN_NONE;
+  if (abi.attn_decode_workspace_bytes(Hq, Hkv, hd, ctx) < 0) Py_RETURN_NONE;
   const float eps = (float)PyFloat_AS_DOUBLE(a[11]);
-  return run(*qkv, {Hq * hd}, [&](void* y, void* st) {   // no tickets are taken and no partials written: any address will do
+  return run(*qkv, {Hq * hd}, [&](void* y, void* st) {
+    // a result from the allocator lies as the cluster kernel wants it, which takes no workspace: any address will do
     return abi.attn_decode_bf16(y, qkv->data_ptr(), ptr(qn), ptr(kn), eps, (const float*)ptr(rope), (const int32_t*)ptr(pos), len, kc->data_ptr(),
-                                 vc->data_ptr(), Hq, Hkv, hd, ctx, y, st);
+                                vc->data_ptr(), Hq, Hkv, hd, ctx, y, st);
   });
   END_HANDLE_TH_ERRORS
 }
