@@ -19,7 +19,7 @@
 // does not see never reaches it.
 //
 // Bound by the chain S → softmax → P·V of three tiles in flight: a group takes some 2 400 cycles a tile (1 024 of them the exponentials' pipe) and 800 until it
-// begins the next one; tensor pipe and exponentials a third busy at 16 heads of 128 over 2 048 rows.  Small calls by what is done once: barriers, TMEM,
+// begins the next one; tensor pipe and exponentials 40 % of the active cycles at 16 heads of 128 over 2 048 rows.  Small calls by what is done once: barriers, TMEM,
 // first loads, code that is not in the caches yet, results (some 5 µs in all; up to 128 keys a kernel of its own, below, takes less).  Slower, at 16 heads of
 // 128 over 2 048 rows, were two O of which each group has one (26 µs where this form takes 21.5: S, whose columns P shares, then waits for P·V), three groups
 // of softmax warps (28), tiles read twice from TMEM in loops (23), the exponentials ahead of the maximum (22), 64-key tiles in two CTAs per SM (36).  A
