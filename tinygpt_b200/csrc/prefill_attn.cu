@@ -411,8 +411,8 @@ int launch_attn_prefill_mma(void* o, const void* qkv, const void* kcache, const 
 // softcap > 0: capped scores; slopes [Hq]: a distance bias per head; vcache == kcache: the values are the keys.  The kernel is chosen by
 // `ctx`, the positions that the caches are made for, as if a prompt filled them (up to 2 048 rows, the range of the fits): a choice by
 // S and p0 would give a row other bits when its prompt is cut in another way.  Long caches take tcgen05, at any length of their prompts (8
-// layers of 2 048, 16 / 8 heads of 128, caches for 4 096, µs, mma.sync / tcgen05: 64 rows 549 / 542, 512 rows 762 / 734, 1 024 rows
-// 1 083 / 987, 2 048 rows 1 885 / 1 717).
+// layers of 2 048, 16 / 8 heads of 128, caches for 4 096, µs, mma.sync / tcgen05: 64 rows 509 / 503, 512 rows 727 / 682, 1 024 rows
+// 1 090 / 973, 2 048 rows 2 070 / 1 727).
 bool prefill_window_ok(int hd) { return hd == 64 || hd == 96 || hd == 128; }
 int launch_attn_prefill_window(void* o, int64_t o_rs, const void* q, const void* gate_or_null, int64_t q_rs,
                                const void* kcache, const void* vcache, int S, int Hq, int Hkv, int hd, int p0, float scale,
