@@ -15,8 +15,8 @@
 //   warp 13      MMA issuer (one thread): P·V of a tile and right behind it S of the tile three further on, also across blocks
 //
 // A key that a row does not see has P = 0, and 0 · V is 0 only for finite V.  So where a result is not finite, V of the tiles that some row of the
-// block sees in part is looked at, and if it holds infinities or NaNs those rows go over the keys that they see, one after another: what a row
-// does not see never reaches it.
+// block sees in part is looked at, and if it holds infinities or NaNs those rows go over the keys that they see, one after another, behind the CTA's last
+// block: what a row does not see never reaches it.
 //
 // Bound by the chain S → softmax → P·V of three tiles in flight: a group takes some 2 400 cycles a tile (1 024 of them the exponentials' pipe) and 800 until it
 // begins the next one; tensor pipe and exponentials 40 % of the active cycles at 16 heads of 128 over 2 048 rows.  Small calls by what is done once: barriers, TMEM,
@@ -179,34 +179,6 @@ __device__ __forceinline__ bool wait_slow(uint64_t* bar, uint32_t parity, unsign
 }
 __device__ __forceinline__ uint32_t bits_below(int n) { return n >= 32 ? ~0u : n <= 0 ? 0u : (1u << n) - 1; }
 
-// One row, the keys it sees one after another (P rounded to bf16 like above): the way out for a block whose partly visible tiles hold
-// infinities or NaNs in V.  Slow and rare.
-template <int HD>
-__device__ __forceinline__ void see_alone(const TcAttn& p, int b, int h, int kvh, int r, float (&ml)[2], int c, float (&acc)[8]) {
-  const __nv_bfloat16* q = p.qp + (size_t)b * p.q_bs + (size_t)r * p.q_rs + (size_t)h * HD;
-  const int rpos = p.p0 + r;
-#pragma unroll 1
-  for (int j = 0; j <= rpos; ++j) {
-    if (p.window > 0 && rpos - j >= p.window && j >= p.keep_first) continue;
-    const size_t row = (size_t)b * p.kv_bs + (size_t)j * p.kv_rs + (size_t)kvh * HD;
-    float s = 0.f;
-#pragma unroll 1
-    for (int d = 0; d < HD; d += 8) {
-      float x[8];
-      unpack8(*reinterpret_cast<const uint4*>(q + d), x);
-      s = dot8(*reinterpret_cast<const uint4*>(p.kp + row + d), x, s);
-    }
-    if (c < 0) {   // first walk: maximum and sum
-      const float top = fmaxf(ml[0], s);
-      ml[1] = ml[1] * (ml[0] == -INFINITY ? 0.f : ex2f((ml[0] - top) * p.scale_log2)) + ex2f((s - top) * p.scale_log2);
-      ml[0] = top;
-    } else {
-      const float w = round_bf16(ex2f((s - ml[0]) * p.scale_log2));
-      for (int e = 0; e < 8; ++e) acc[e] = fmaf(w, bf16_to_f(p.vp[row + c + e]), acc[e]);
-    }
-  }
-}
-
 __device__ __forceinline__ float max3f(float a, float b, float c) {
   float y;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
@@ -266,6 +238,84 @@ __device__ __forceinline__ bool part_not_finite(const TcAttn& p, const Block& w,
   return __any_sync(0xffffffffu, bad);
 }
 
+// The way out for such a block: this warp's 32 rows, each over the keys that it sees and no others (weights rounded to bf16 like above).  A row's scores go to
+// the lanes, 32 keys at a time, once for its maximum and sum and once for its weights; its columns to the lanes, key after key.  Slow and rare: 32 rows
+// over 300 000 keys take 1.7 s (heads of 64: 0.86 s), bound by the latency of loads.
+template <int HD>
+__device__ __forceinline__ void see_alone(const TcAttn& p, const Block& w, int quarter, int lane) {
+  constexpr int E = HD / 32;   // columns of a lane
+  const int end = min(w.rows_valid, quarter * 32 + 32);
+#pragma unroll 1
+  for (int row = quarter * 32; row < end; ++row) {
+    const int r = w.q0 + row, rpos = p.p0 + r;
+    const __nv_bfloat16* const q = p.qp + (size_t)w.b * p.q_bs + (size_t)r * p.q_rs + (size_t)w.h * HD;
+    const size_t kv = (size_t)w.b * p.kv_bs + (size_t)w.kvh * HD;
+    auto score = [&](int j, float& s) {   // whether the row sees key j; its score
+      if (j > rpos || (p.window > 0 && rpos - j >= p.window && j >= p.keep_first)) return false;
+      const __nv_bfloat16* const k = p.kp + kv + (size_t)j * p.kv_rs;
+      s = 0.f;
+#pragma unroll 4
+      for (int d = 0; d < HD; d += 8) {
+        float x[8];
+        unpack8(*reinterpret_cast<const uint4*>(q + d), x);
+        s = dot8(*reinterpret_cast<const uint4*>(k + d), x, s);
+      }
+      return true;
+    };
+    // the keys behind the kept ones and in front of the window are passed over, 32 at a time
+    const int edge = p.window > 0 ? max(0, rpos - p.window + 1) & ~31 : 0;
+    auto next = [&](int j0) { return j0 + 32 >= p.keep_first && j0 + 32 < edge ? edge : j0 + 32; };
+    const int from = p.keep_first > 0 ? 0 : edge;
+    float m = -INFINITY, l = 0.f;
+#pragma unroll 1
+    for (int j0 = from; j0 <= rpos; j0 = next(j0)) {
+      float s;
+      if (!score(j0 + lane, s)) continue;
+      const float top = fmaxf(m, s), ms = top == -INFINITY ? 0.f : top * p.scale_log2;
+      l = l * (m == -INFINITY ? 1.f : ex2f((m - top) * p.scale_log2)) + ex2f(fmaf(s, p.scale_log2, -ms));
+      m = top;
+    }
+    const float mine = m;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    l *= mine == -INFINITY ? 1.f : ex2f((mine - m) * p.scale_log2);
+    l = warp_sum(l);
+    const float ms = m == -INFINITY ? 0.f : m * p.scale_log2;
+    float acc[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) acc[e] = 0.f;
+#pragma unroll 1
+    for (int j0 = from; j0 <= rpos; j0 = next(j0)) {
+      float s = 0.f;
+      const bool sees = score(j0 + lane, s);
+      const float weight = round_bf16(ex2f(fmaf(s, p.scale_log2, -ms)));
+      const unsigned seen = __ballot_sync(0xffffffffu, sees);
+      const __nv_bfloat16* const v = p.vp + kv + (size_t)j0 * p.kv_rs + lane * E;
+      auto add = [&](int j) {
+        const float x = __shfl_sync(0xffffffffu, weight, j);
+        uint32_t y[E / 2];
+        if constexpr (E == 4) *reinterpret_cast<uint2*>(y) = *reinterpret_cast<const uint2*>(v + (size_t)j * p.kv_rs);
+        else y[0] = *reinterpret_cast<const uint32_t*>(v + (size_t)j * p.kv_rs);
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[e] = fmaf(x, __uint_as_float(e & 1 ? y[e / 2] & 0xffff0000u : y[e / 2] << 16), acc[e]);
+      };
+      if (seen == 0xffffffffu) {   // sixteen loads in flight
+#pragma unroll 16
+        for (int j = 0; j < 32; ++j) add(j);
+      } else {
+#pragma unroll 1
+        for (unsigned left = seen; left != 0; left &= left - 1) add(__ffs(left) - 1);
+      }
+    }
+    if (p.sink && m != -INFINITY) l += ex2f(-m * p.scale_log2);
+    const float gate = p.gate != nullptr ? 1.f / (1.f + expf(-bf16_to_f(p.gate[(size_t)w.b * p.q_bs + (size_t)r * p.q_rs + w.h]))) : 1.f;
+    const float inv = (l > 0.f ? 1.f / l : 0.f) * gate;
+    __nv_bfloat16* const o = p.o + (size_t)w.b * p.o_bs + (size_t)r * p.o_rs + (size_t)w.h * HD + lane * E;
+#pragma unroll
+    for (int e = 0; e < E; e += 2) *reinterpret_cast<uint32_t*>(o + e) = pack2(acc[e] * inv, acc[e + 1] * inv);
+  }
+}
+
 // the weights of 32 keys of a row, rounded to bf16, to TMEM; their sums in fp32
 __device__ __forceinline__ void weights32(const uint32_t (&s)[32], uint64_t scale2, uint64_t neg, uint64_t (&sum)[2], uint32_t at) {
   uint32_t pk[16];
@@ -280,15 +330,16 @@ __device__ __forceinline__ void weights32(const uint32_t (&s)[32], uint64_t scal
 }
 
 // 32 rows of a block from O in TMEM, this lane's with maximum m and sum l: normalised, through shared memory (64 columns at `mid`, the next 64 `step`
-// bytes further on) into the result.  has_read is called behind the last look at O.
+// bytes further on) into the result.  has_read is called behind the last look at O.  Whether some result is not finite, which is what 0 · V may have left
+// where V is not.
 template <int HD, typename F>
-__device__ __forceinline__ void store_rows(const TcAttn& p, const CUtensorMap* to, const Block& w, uint32_t o_at, int row, float m, float l, uint8_t* mid,
+__device__ __forceinline__ bool store_rows(const TcAttn& p, const CUtensorMap* to, const Block& w, uint32_t o_at, int row, float m, float l, uint8_t* mid,
                                            int step, bool lost, F has_read) {
   const int lane = row & 31, rr = w.q0 + min(row, w.rows_valid - 1);
   const float k_scale = p.scale_log2;
   if (p.sink && m != -INFINITY) l += ex2f(-m * k_scale);
   const float gate = p.gate != nullptr ? 1.f / (1.f + expf(-bf16_to_f(p.gate[(size_t)w.b * p.q_bs + (size_t)rr * p.q_rs + w.h]))) : 1.f;
-  float inv = (l > 0.f ? 1.f / l : 0.f) * gate;
+  const float inv = (l > 0.f ? 1.f / l : 0.f) * gate;
   uint32_t odd = 0;   // the sign bits of halves whose exponent is all ones
 #pragma unroll 1
   for (int c = 0; c < HD; c += 64, mid += step) {
@@ -318,25 +369,7 @@ __device__ __forceinline__ void store_rows(const TcAttn& p, const CUtensorMap* t
       bulk_commit();
     }
   }
-  // 0 · V is not 0 where V is not finite: then such rows see their keys one after another
-  if (__builtin_expect(__any_sync(0xffffffffu, (odd & 0x80008000u) != 0), 0) && part_not_finite<HD>(p, w, lane) && !lost) {
-    if (lane == 0) bulk_done();
-    __syncwarp();
-    float both[2] = {-INFINITY, 0.f}, x[8];
-    see_alone<HD>(p, w.b, w.h, w.kvh, rr, both, -1, x);
-    l = both[1];
-    if (p.sink && both[0] != -INFINITY) l += ex2f(-both[0] * k_scale);
-    inv = (l > 0.f ? 1.f / l : 0.f) * gate;
-#pragma unroll 1
-    for (int c = 0; c < HD; c += 8) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) x[e] = 0.f;
-      see_alone<HD>(p, w.b, w.h, w.kvh, rr, both, c, x);
-      if (row < w.rows_valid)
-        *reinterpret_cast<uint4*>(p.o + (size_t)w.b * p.o_bs + (size_t)rr * p.o_rs + (size_t)w.h * HD + c) =
-            make_uint4(pack2(x[0] * inv, x[1] * inv), pack2(x[2] * inv, x[3] * inv), pack2(x[4] * inv, x[5] * inv), pack2(x[6] * inv, x[7] * inv));
-    }
-  }
+  return __any_sync(0xffffffffu, (odd & 0x80008000u) != 0);
 }
 
 // The same for 128 keys at most, one tile: nothing is shared out and nothing runs ahead, so four warps do everything one after another, on as many
@@ -462,7 +495,12 @@ attn_tc_one_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   tc_fence_after();
   const bool lost = __any_sync(0xffffffffu, dead || *reinterpret_cast<volatile int*>(gave_up) != 0);
   // results on their way out take Q's place: its product is over
-  store_rows<HD>(p, &to, w, s_at + kColO, row, m, l, sQ + warp * (32 * 128), 128 * 128, lost, [&] {});
+  const bool odd = store_rows<HD>(p, &to, w, s_at + kColO, row, m, l, sQ + warp * (32 * 128), 128 * 128, lost, [&] {});
+  if (__builtin_expect(odd, 0) && !lost && part_not_finite<HD>(p, w, lane)) {
+    if (lane == 0) bulk_done();   // the stores that these rows write over
+    __syncwarp();
+    see_alone<HD>(p, w, warp, lane);
+  }
   if (lane == 0) bulk_read();
   if (dead) drain_async();
   tc_fence_before();
@@ -822,6 +860,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
     const float k_scale = p.scale_log2;
     int c = -1, buf = 2;   // the tile's number, its S buffer
     uint32_t ph = 1;
+    bool odd = false, any_lost = false;   // of the blocks so far
     for (int r = 0, i; (i = block_of(r)) < p.blocks; ++r) {
       const Block w(p, i);
       float was = -INFINITY;
@@ -879,12 +918,24 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
       __syncwarp();
       tc_fence_after();
       const bool lost = __any_sync(0xffffffffu, dead || *reinterpret_cast<volatile int*>(gave_up) != 0);
-      store_rows<HD>(p, &to, w, o_at, row, m, l, sO + q * (32 * 128), 0, lost, [&] {
+      any_lost |= lost;
+      odd |= store_rows<HD>(p, &to, w, o_at, row, m, l, sO + q * (32 * 128), 0, lost, [&] {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(o_empty);
       });
       if (lane == 0) mbar_arrive(&ml_empty[r & 1]);
+    }
+    // Rows that go over their keys one after another do so here, where nobody waits for this warp any more: over a long cache they take longer than
+    // a wait lasts.  A block whose results are all finite has no such V in the tiles that are looked at, so which ones were not need not be kept.
+    if (__builtin_expect(odd, 0) && !any_lost) {
+      if (lane == 0) bulk_done();   // the stores that these rows write over
+      __syncwarp();
+#pragma unroll 1
+      for (int r = 0, i; (i = block_of(r)) < p.blocks; ++r) {
+        const Block w(p, i);
+        if (part_not_finite<HD>(p, w, lane)) see_alone<HD>(p, w, q, lane);
+      }
     }
     if (lane == 0) bulk_read();
   }
