@@ -184,13 +184,15 @@ __device__ __forceinline__ float max3f(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
   return y;
 }
-__device__ __forceinline__ float2 ld_volatile_f2(const float2* p) {
+// A row's maximum and the number of the tile that it is from (as a float's bits), which says whether it is there: one access of 64 bits, so that no reader sees
+// a new number beside an old maximum (a vector access may be carried out element by element).
+__device__ __forceinline__ float2 ld_max(const float2* p) {
   float2 v;
-  asm volatile("ld.volatile.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_u32(p)) : "memory");
+  asm volatile("{\n\t.reg .b64 t;\n\tld.volatile.shared.b64 t, [%2];\n\tmov.b64 {%0, %1}, t;\n\t}" : "=f"(v.x), "=f"(v.y) : "r"(smem_u32(p)) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_volatile_f2(float2* p, float2 v) {
-  asm volatile("st.volatile.shared.v2.f32 [%0], {%1, %2};" ::"r"(smem_u32(p)), "f"(v.x), "f"(v.y) : "memory");
+__device__ __forceinline__ void st_max(float2* p, float2 v) {
+  asm volatile("{\n\t.reg .b64 t;\n\tmov.b64 t, {%1, %2};\n\tst.volatile.shared.b64 [%0], t;\n\t}" ::"r"(smem_u32(p)), "f"(v.x), "f"(v.y) : "memory");
 }
 constexpr int kTCtas = 148;   // one per SM; which CTA has a block changes no bit
 
@@ -554,7 +556,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
   auto wait_passed = [&](const float2* at, int tile, float2& v) {   // the row's maximum behind this tile; limited like every wait
     unsigned long long t0 = 0;
     for (unsigned spins = 1; __float_as_int(v.y) != tile && !dead; ++spins) {
-      v = ld_volatile_f2(at);
+      v = ld_max(at);
       if ((spins & 0x3ffu) == 0) {
         const unsigned long long now = global_timer_ns();
         if (t0 == 0) t0 = now;
@@ -788,7 +790,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
         __syncwarp();
         tc_fence_after();
         const float2* const from = &m_row[((c - 1) & 3) * kTBM + row];
-        float2 passed = ld_volatile_f2(from);
+        float2 passed = ld_max(from);
         uint32_t s[4][32];
         tmem_ld32(s_at, s[0]);
         tmem_ld32(s_at + 32, s[1]);
@@ -827,7 +829,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
         look(3);
         const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
         const float next = fmaxf(held, top);
-        st_volatile_f2(&m_row[(c & 3) * kTBM + row], make_float2(next, __int_as_float(c)));
+        st_max(&m_row[(c & 3) * kTBM + row], make_float2(next, __int_as_float(c)));
         __syncwarp();
         if (lane == 0) mbar_arrive(&m_full[buf]);
         held = next;
@@ -860,7 +862,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
     const float k_scale = p.scale_log2;
     int c = -1, buf = 2;   // the tile's number, its S buffer
     uint32_t ph = 1;
-    bool odd = false, any_lost = false;   // of the blocks so far
+    bool odd = false;   // in the blocks so far
     for (int r = 0, i; (i = block_of(r)) < p.blocks; ++r) {
       const Block w(p, i);
       float was = -INFINITY;
@@ -874,7 +876,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
         }
         wait_for(&m_full[buf], ph, kAttnWaitCode | 11);
         __syncwarp();
-        const float now = ld_volatile_f2(&m_row[(c & 3) * kTBM + row]).x;
+        const float now = ld_max(&m_row[(c & 3) * kTBM + row]).x;
         if (it > 0 && __any_sync(0xffffffffu, now != was)) {
           const float alpha = now != was ? ex2f((was - now) * k_scale) : 1.f;
           const uint64_t alpha2 = pack_f2(alpha, alpha);
@@ -918,7 +920,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
       __syncwarp();
       tc_fence_after();
       const bool lost = __any_sync(0xffffffffu, dead || *reinterpret_cast<volatile int*>(gave_up) != 0);
-      any_lost |= lost;
       odd |= store_rows<HD>(p, &to, w, o_at, row, m, l, sO + q * (32 * 128), 0, lost, [&] {
         tc_fence_before();
         __syncwarp();
@@ -928,7 +929,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
     }
     // Rows that go over their keys one after another do so here, where nobody waits for this warp any more: over a long cache they take longer than
     // a wait lasts.  A block whose results are all finite has no such V in the tiles that are looked at, so which ones were not need not be kept.
-    if (__builtin_expect(odd, 0) && !any_lost) {
+    if (__builtin_expect(odd, 0) && !__any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(gave_up) != 0)) {
       if (lane == 0) bulk_done();   // the stores that these rows write over
       __syncwarp();
 #pragma unroll 1
