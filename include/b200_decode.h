@@ -145,13 +145,12 @@ int b200_gemv_fused_bf16(void* y, const void* x, const void* W, int64_t n, int64
 /* Decode attention of one layer for one new token (B = 1, Sq = 1), one launch:
  *   q|k|v = qkv  →  [q_norm/k_norm per head]  →  RoPE(q), RoPE(k) at position *pos  →  K/V row *pos written in place
  *   into kcache/vcache [max_ctx, Hkv, hd]  →  split-KV softmax(q kᵀ/√hd) v over rows 0…*pos  →  out [Hq*hd].
- * A cluster of up to sixteen CTAs per head group shares the keys that exist.  Where `out` lies off the 8-byte boundary and the caches have up to eight
- * splits of 256 (hd 64) / 128 (hd 128) keys: one CTA per (head group, split), and the workspace is used.
+ * A cluster of up to sixteen CTAs per head group shares the keys that exist.
  * *pos must have been written before the kernel that produced `qkv` was launched (the kernel reads it, and the cached
  * rows below it, ahead of its programmatic-dependency wait).
  * pos == NULL: plain attention over `fixed_len` cached rows, nothing appended; with a rope_table q is rotated as the token at position
  * fixed_len - 1, without one it is taken as it is.
- * workspace: b200_attn_decode_workspace_bytes() bytes, ZERO-INITIALISED once by the caller (tickets self-reset).
+ * workspace: any address but NULL; nothing is read or written there (callers that bring b200_attn_decode_workspace_bytes() zeroed bytes may go on).
  * [ref: src/layer/Attention.h:71-112,156-163; src/engine/CacheManager.h:24-42; TFA/mma/kernel.cuh:18-203] */
 int64_t b200_attn_decode_workspace_bytes(int64_t Hq, int64_t Hkv, int64_t hd, int64_t max_ctx);
 int b200_attn_decode_bf16(void* out, const void* qkv, const void* q_norm_or_null, const void* k_norm_or_null,

@@ -1,6 +1,6 @@
 """attn_decode over caches of any length on the cluster kernel (csrc/attn.cu), as a native call (csrc/torch_ops.cpp) and from Python (a strided view of the
 rows goes that way): the same bits, call after call, on the edges of the key ranges, on another stream and captured; against 64 bits within
-two bf16 roundings of the largest value; and into a result off the 8-byte boundary, which the other kernel writes."""
+two bf16 roundings of the largest value; and into a result at any address of a bf16, with the same bits and whatever lies in the workspace."""
 import pytest
 import torch
 
@@ -45,7 +45,7 @@ def test_result_off_the_boundary(built_lib):
     from tinygpt_b200._lib import lib
     qkv, k, v = _inputs(4, 2, 64, 600)
     want = _call(qkv, k, v, 4, 2, 64, 555)[0]
-    ws = torch.zeros(lib().b200_attn_decode_workspace_bytes(4, 2, 64, 600), dtype=torch.uint8, device="cuda")
+    ws = torch.full((lib().b200_attn_decode_workspace_bytes(4, 2, 64, 600),), 0xa5, dtype=torch.uint8, device="cuda")
     buf, pos = torch.zeros(4 * 64 + 4, dtype=torch.bfloat16, device="cuda"), torch.tensor([555], dtype=torch.int32, device="cuda")
     for off in (1, 2, 4):
         out = buf[off:off + 256]
@@ -53,7 +53,7 @@ def test_result_off_the_boundary(built_lib):
                                          ws.data_ptr(), torch.cuda.current_stream().cuda_stream)
         assert rc == 0
         torch.cuda.synchronize()
-        assert float((out.double() - want.double()).abs().max()) <= 2.0 ** -7 * float(v.double().abs().max())
+        assert torch.equal(out, want) and bool((ws == 0xa5).all())
 
 
 def test_captured(built_lib):

@@ -130,8 +130,6 @@ int b200_attn_decode_bf16(void* out, const void* qkv, const void* q_norm, const 
   a.kcache = (__nv_bfloat16*)kcache;
   a.vcache = (__nv_bfloat16*)vcache;
   a.out = (__nv_bfloat16*)out;
-  a.tickets = (unsigned int*)workspace;
-  a.ws = (float*)((uint8_t*)workspace + ((Hq * 4 + 15) / 16) * 16);
   a.Hq = (int)Hq;
   a.Hkv = (int)Hkv;
   a.nsplit = attn_decode_nsplit((int)hd, (int)max_ctx);

@@ -92,7 +92,6 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_reg_kernel(const Att
   const bool kv_leader = (h0 % group) == 0;
   if (p.trace != nullptr && hg == 0 && split == 0 && blockIdx.z == 0 && tid == 0) p.trace[0] = global_timer_ns();
   pdl_trigger();
-  if (p.late) pdl_wait();
   const bool append = (p.pos != nullptr);
   const int pos = append ? *p.pos : p.fixed_len - 1;   // stable since before the producer kernel started (engine.cu)
   const int L = pos + 1;
@@ -812,8 +811,8 @@ int launch_attn_decode(const AttnDecodeParams& p, int hd, cudaStream_t st, bool 
   const unsigned nb = (unsigned)std::max(1, p.batch);
   // The operator takes the cluster kernel at any length: no tickets to be zeroed by a launch of their own, which cost it more than its attention (µs a call,
   // 16 / 8 heads of 128, caches for 256 / 1 024: 19.8 / 19.8, with a native call 12.1 / 17.4, here 5.4 / 5.5).  The engines' steps stay with the
-  // other kernel up to kLongSplits, whose bits theirs are.  Results go out 8 bytes at a time.
-  if (p.nsplit > kLongSplits || (p.late && (reinterpret_cast<uintptr_t>(p.out) & 7) == 0)) {
+  // other kernel up to kLongSplits, whose bits theirs are.
+  if (p.nsplit > kLongSplits || p.late) {
     AttnRow a{p, 0, p.cache_bstride, 1, 1, 0};
     return launch_row(a, hd, p.max_ctx, (int)nb, true, st, pdl);
   }

@@ -173,7 +173,7 @@ PyObject* attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   if (abi.attn_decode_workspace_bytes(Hq, Hkv, hd, ctx) < 0) Py_RETURN_NONE;
   const float eps = (float)PyFloat_AS_DOUBLE(a[11]);
   return run(*qkv, {Hq * hd}, [&](void* y, void* st) {
-    // a result from the allocator lies as the cluster kernel wants it, which takes no workspace: any address will do
+    // no workspace is taken: any address will do
     return abi.attn_decode_bf16(y, qkv->data_ptr(), ptr(qn), ptr(kn), eps, (const float*)ptr(rope), (const int32_t*)ptr(pos), len, kc->data_ptr(),
                                 vc->data_ptr(), Hq, Hkv, hd, ctx, y, st);
   });

@@ -235,15 +235,10 @@ def attn_decode(qkv, kcache, vcache, *, q_heads, kv_heads, head_dim, pos=None, f
         check(out, "b200_attn_decode_bf16")
     qkv, kcache, vcache = _chk(qkv, "attn_decode.qkv"), _chk(kcache, "attn_decode.kcache"), _chk(vcache, "attn_decode.vcache")
     max_ctx = kcache.shape[0]
-    n, tickets = lib().b200_attn_decode_workspace_bytes(q_heads, kv_heads, head_dim, max_ctx), (4 * q_heads + 15) // 16 * 16
-    # tickets first, then partials that are written before they are read; long contexts have no partials and take no tickets
-    ws = torch.empty(max(n, tickets), dtype=torch.uint8, device=qkv.device)
-    if n > tickets:
-        ws[:tickets].zero_()
     out = torch.empty(q_heads * head_dim, dtype=torch.bfloat16, device=qkv.device)
     check(lib().b200_attn_decode_bf16(out.data_ptr(), qkv.data_ptr(), _ptr(q_norm), _ptr(k_norm), float(eps),
                                       _ptr(rope_table), _ptr(pos), int(fixed_len), kcache.data_ptr(),
-                                      vcache.data_ptr(), q_heads, kv_heads, head_dim, max_ctx, ws.data_ptr(),
+                                      vcache.data_ptr(), q_heads, kv_heads, head_dim, max_ctx, out.data_ptr(),   # no workspace
                                       _stream()), "b200_attn_decode_bf16")
     return out
 
