@@ -146,6 +146,7 @@ int b200_gemv_fused_bf16(void* y, const void* x, const void* W, int64_t n, int64
  *   q|k|v = qkv  →  [q_norm/k_norm per head]  →  RoPE(q), RoPE(k) at position *pos  →  K/V row *pos written in place
  *   into kcache/vcache [max_ctx, Hkv, hd]  →  split-KV softmax(q kᵀ/√hd) v over rows 0…*pos  →  out [Hq*hd].
  * A cluster of up to sixteen CTAs per head group shares the keys that exist.
+ * A *pos outside the caches leaves them as they are, and `out` is zero.
  * *pos must have been written before the kernel that produced `qkv` was launched (the kernel reads it, and the cached
  * rows below it, ahead of its programmatic-dependency wait).
  * pos == NULL: plain attention over `fixed_len` cached rows, nothing appended; with a rope_table q is rotated as the token at position

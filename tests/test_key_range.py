@@ -1,5 +1,5 @@
 """How attn_row_kernel's CTAs share a row's keys (csrc/key_range.cuh, compiled for the host): the ranges follow each other without a gap, cached keys and the new
-one are in one of them each, and one range alone owns the new row, also where the last ranges are empty."""
+one are in one of them each, and one range alone owns the new row, also where the last ranges are empty; with -1 cached keys, a position outside the cache, all are."""
 import subprocess
 
 from tinygpt_b200 import build
@@ -8,6 +8,11 @@ MAIN = """
 #include <cstdio>
 #include "key_range.cuh"
 int main() {
+  for (int log = 0; log <= 4; ++log)
+    for (int r = 0; r < 1 << log; ++r) {
+      const b200::KeyRange k = b200::key_range(-1, true, r, log);
+      if (k.first != 0 || k.n != 0 || k.n_cached > 0 || k.owns_new) return printf("range %d of %d without keys: %d of them\n", r, 1 << log, k.n), 1;
+    }
   for (int log = 0; log <= 4; ++log)
     for (int append = 0; append < 2; ++append)
       for (int cached = 0; cached <= 5000; cached += cached < 700 ? 1 : 37) {

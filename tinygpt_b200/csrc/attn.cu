@@ -356,7 +356,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_row_kernel(const AttnRow
   if (!DECODE || p.late) pdl_wait();
   cluster_arrive_relaxed();                // this CTA runs: the others may write to it once they have waited for that
   const bool append = DECODE && p.pos != nullptr;
-  const int pos = append ? *p.pos : p.fixed_len - 1;   // where q is rotated; stable since before the producer kernel started
+  int pos = append ? *p.pos : p.fixed_len - 1;   // where q is rotated; stable since before the producer kernel started
+  if (append && (unsigned)pos >= (unsigned)p.max_ctx) pos = -1;   // outside the caches: no keys, and none of the ranges has the new one
   const int cached = append ? pos : DECODE ? p.fixed_len : a.nkeys;   // rows that are in the cache already
   const KeyRange keys = key_range(cached, append, rank, a.log_splits);
   const int k0 = keys.first, n = keys.n, n_cached = keys.n_cached;   // this CTA's keys
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_row_kernel(const AttnRow
   if constexpr (DECODE) {
     float rc[EPL / 2], rs[EPL / 2];
     if (p.rope != nullptr) {
-      const float* row = p.rope + (size_t)pos * HD * 2;
+      const float* row = p.rope + (size_t)max(pos, 0) * HD * 2;
 #pragma unroll
       for (int j = 0; j < EPL / 2; ++j) {
         rc[j] = row[(lane + 32 * j) * 2];
