@@ -11,7 +11,7 @@ int main() {
   for (int log = 0; log <= 4; ++log)
     for (int r = 0; r < 1 << log; ++r) {
       const b200::KeyRange k = b200::key_range(-1, true, r, log);
-      if (k.first != 0 || k.n != 0 || k.n_cached > 0 || k.owns_new) return printf("range %d of %d without keys: %d of them\n", r, 1 << log, k.n), 1;
+      if (k.first != 0 || k.n != 0 || k.n_cached > 0 || k.owns_new) return printf("range %d of %d without keys: %d of them\\n", r, 1 << log, k.n), 1;
     }
   for (int log = 0; log <= 4; ++log)
     for (int append = 0; append < 2; ++append)
