@@ -19,7 +19,6 @@
 #include "tc.cuh"
 
 #include <algorithm>
-#include <mutex>
 
 namespace b200 {
 
@@ -731,13 +730,11 @@ int attn_decode_nsplit(int hd, int max_ctx) {
 
 template <int HD, int GM, bool DECODE>
 static int launch_row_t(const AttnRow& a, int splits, int B, cudaStream_t st, bool pdl) {
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(attn_row_kernel<HD, GM, DECODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, KeyRing<HD>::smem);
-    if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(attn_row_kernel<HD, GM, DECODE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  });
-  B200_CUDA(attr_err);
+  static PerDevice attrs;
+  B200_CUDA(attrs([] {
+    const cudaError_t e = cudaFuncSetAttribute(attn_row_kernel<HD, GM, DECODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, KeyRing<HD>::smem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(attn_row_kernel<HD, GM, DECODE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  }));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)splits, (unsigned)(a.d.Hq / a.G), (unsigned)B);
   cfg.blockDim = dim3(kAttnThreads);

@@ -12,6 +12,7 @@
 #include <cstdio>
 
 #include "../../include/b200_decode.h"
+#include "per_device.cuh"
 
 namespace b200 {
 
@@ -47,6 +48,22 @@ extern std::atomic<int64_t> g_launches;
       return B200_ERR_CUDA;                                                                             \
     }                                                                                                   \
   } while (0)
+
+// `set`, which sets kernels' attributes, once on each device that is current here
+class PerDevice {
+ public:
+  template <typename F>
+  cudaError_t operator()(F set) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = once_(device, set);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+  }
+
+ private:
+  OncePerDevice<cudaError_t> once_;
+};
 
 // Kernel launch through cudaLaunchKernelEx with the programmatic-dependent-launch attribute (PDL): the kernel may
 // start while its predecessor on the stream is still running and must call pdl_wait() before touching anything the

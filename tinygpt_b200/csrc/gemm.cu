@@ -27,7 +27,6 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 
 namespace b200 {
 
@@ -647,10 +646,8 @@ int sm_pairs() {
 
 template <typename OT, int EPI>
 int launch_pair(const GemmArgs<OT>& args, const void* A, const void* B, int64_t rows_b, int bn, cudaStream_t st) {
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] { attr_err = cudaFuncSetAttribute(gemm_pair_kernel<OT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem); });
-  B200_CUDA(attr_err);
+  static PerDevice attrs;
+  B200_CUDA(attrs([] { return cudaFuncSetAttribute(gemm_pair_kernel<OT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem); }));
   GemmArgs<OT> p = args;
   int rc;
   if ((rc = wait_word(&p.err)) != B200_OK) return rc;
@@ -667,10 +664,8 @@ int launch_pair(const GemmArgs<OT>& args, const void* A, const void* B, int64_t 
 
 template <typename OT, int EPI, int FORM>
 int split_setup() {
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] { attr_err = cudaFuncSetAttribute(gemm_split_kernel<OT, EPI, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem); });
-  B200_CUDA(attr_err);
+  static PerDevice attrs;
+  B200_CUDA(attrs([] { return cudaFuncSetAttribute(gemm_split_kernel<OT, EPI, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem); }));
   return B200_OK;
 }
 

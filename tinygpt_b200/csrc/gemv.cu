@@ -25,7 +25,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
-#include <mutex>
 
 namespace b200 {
 
@@ -458,9 +457,8 @@ KernelFn pick(int rpw, int nseg, int pro, int epi) {
 }  // namespace
 
 int gemv_setup_attributes() {
-  static std::once_flag once;
-  static int rc = B200_OK;
-  std::call_once(once, [] {
+  static PerDevice attrs;
+  B200_CUDA(attrs([] {
     const int rpws[3] = {1, 2, 4};
     for (int rpw : rpws)
       for (int nseg = 1; nseg <= 2; ++nseg)
@@ -474,15 +472,11 @@ int gemv_setup_attributes() {
             if (e == cudaSuccess)
               e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        cudaSharedmemCarveoutMaxShared);
-            if (e != cudaSuccess) {
-              set_error("cudaFuncSetAttribute(gemv smem) failed: %s", cudaGetErrorString(e));
-              rc = B200_ERR_CUDA;
-              (void)cudaGetLastError();
-              return;
-            }
+            if (e != cudaSuccess) return e;
           }
-  });
-  return rc;
+    return cudaSuccess;
+  }));
+  return B200_OK;
 }
 
 namespace {

@@ -112,6 +112,6 @@ int gemv_plan_set_batch(GemvPlan* plan, int B);
 int gemv_batch_launch(const GemvPlan& plan, cudaStream_t stream, bool pdl);   // gemv_batch.cu
 int gemv_batch_setup_attributes();
 int gemv_batch_fixed_smem(const GemvPlan& plan, int nb);   // shared memory beside the ring for nb sequences
-int gemv_setup_attributes();  // cudaFuncSetAttribute(max dynamic smem) for every instantiation, once per process
+int gemv_setup_attributes();  // cudaFuncSetAttribute(max dynamic smem) for every instantiation, once per device
 
 }  // namespace b200

@@ -27,7 +27,6 @@
 // ≤ 23 bytes/clk/SM of HBM feed is far from the shared-memory limit.
 #include "gemv.cuh"
 
-#include <mutex>
 
 namespace b200 {
 
@@ -419,9 +418,8 @@ int gemv_batch_fixed_smem(const GemvPlan& plan, int nb) {
 }
 
 int gemv_batch_setup_attributes() {
-  static std::once_flag once;
-  static int rc = B200_OK;
-  std::call_once(once, [] {
+  static PerDevice attrs;
+  B200_CUDA(attrs([] {
     const int rpws[3] = {1, 2, 4};
     for (int rpw : rpws)
       for (int nseg = 1; nseg <= 2; ++nseg)
@@ -432,15 +430,11 @@ int gemv_batch_setup_attributes() {
             cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvMaxSmem + 4096);
             if (e == cudaSuccess)
               e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-            if (e != cudaSuccess) {
-              set_error("cudaFuncSetAttribute(batched gemv smem) failed: %s", cudaGetErrorString(e));
-              rc = B200_ERR_CUDA;
-              (void)cudaGetLastError();
-              return;
-            }
+            if (e != cudaSuccess) return e;
           }
-  });
-  return rc;
+    return cudaSuccess;
+  }));
+  return B200_OK;
 }
 
 int gemv_batch_launch(const GemvPlan& plan, cudaStream_t stream, bool pdl) {

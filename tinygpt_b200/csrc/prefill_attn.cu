@@ -18,7 +18,6 @@
 #include "ops.cuh"
 
 #include <cstdlib>
-#include <mutex>
 
 namespace b200 {
 
@@ -366,12 +365,8 @@ int launch_pf(const PrefillAttnParams& p, int B, cudaStream_t st, int tc_rows) {
   }
   constexpr int smem_max = (kBM + 4 * kBN) * row_bytes<HD>();
   const int smem = SCORE && p.same ? (kBM + 2 * kBN) * row_bytes<HD>() : smem_max;
-  static std::once_flag once;   // one per instantiation; the reference's server has a worker thread next to main
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(attn_prefill_mma_kernel<HD, SCORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
-  });
-  B200_CUDA(attr_err);
+  static PerDevice attrs;   // one per instantiation; the reference's server has a worker thread next to main
+  B200_CUDA(attrs([] { return cudaFuncSetAttribute(attn_prefill_mma_kernel<HD, SCORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max); }));
   dim3 grid((unsigned)((p.S + kBM - 1) / kBM) * (unsigned)p.Hq, (unsigned)B);
   B200_CUDA(launch_pdl(attn_prefill_mma_kernel<HD, SCORE>, grid, dim3(kPfThreads), (size_t)smem, st, p.pdl != 0, p));
   return B200_OK;

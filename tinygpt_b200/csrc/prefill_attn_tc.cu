@@ -32,7 +32,6 @@
 #include "tc.cuh"
 
 #include <algorithm>
-#include <mutex>
 
 namespace b200 {
 
@@ -950,13 +949,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
 
 template <int HD>
 int launch_tc(const TcPrefillAttn& a, cudaStream_t st) {
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(attn_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::smem);
-    if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(attn_tc_one_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::smem_one);
-  });
-  B200_CUDA(attr_err);
+  static PerDevice attrs;
+  B200_CUDA(attrs([] {
+    const cudaError_t e = cudaFuncSetAttribute(attn_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::smem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(attn_tc_one_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<HD>::smem_one);
+  }));
   TcAttn p{};
   int rc;
   if ((rc = wait_word(&p.err)) != B200_OK) return rc;

@@ -361,11 +361,9 @@ int launch_hyper_step(const HyperStep& p, int dtype, cudaStream_t st) {
   const int threads = p.n_tok <= 148 && items > 256 ? 512 : 256;
 #define B200_HS(T, S, V, CT)                                                                                            \
   do {                                                                                                              \
-    static bool attr_done = false;                                                                                  \
-    if (smem > 40 * 1024 && !attr_done) {                                                                           \
-      B200_CUDA(cudaFuncSetAttribute(hyper_step_kernel<T, S, V, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); \
-      attr_done = true;                                                                                             \
-    }                                                                                                               \
+    static PerDevice attrs;                                                                                         \
+    if (smem > 40 * 1024)                                                                                           \
+      B200_CUDA(attrs([] { return cudaFuncSetAttribute(hyper_step_kernel<T, S, V, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); })); \
     B200_CUDA(launch_pdl(hyper_step_kernel<T, S, V, CT>, dim3(p.n_tok), dim3(threads), smem, st, stack_pdl(), p));       \
   } while (0)
 #define B200_HS_S(T, V, CT)                        \

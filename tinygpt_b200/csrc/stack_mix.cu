@@ -1221,12 +1221,11 @@ int run_latent_attention(const LatentRun& p0, int dtype, cudaStream_t st) {
   const size_t split_smem = (size_t)(H + 32) * kd * 4;
   if (small && p.split_ws != nullptr && p.nsplit >= 1 && H <= 8 * kLatHeadsPerWarp && kd <= 32 * kLatKeyRegs && r <= 32 * kLatVR &&
       split_smem <= 200 * 1024) {
-    static bool attr_done = false;
-    if (!attr_done) {
-      B200_CUDA(cudaFuncSetAttribute(latent_attn_split_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      B200_CUDA(cudaFuncSetAttribute(latent_attn_split_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr_done = true;
-    }
+    static PerDevice attrs;
+    B200_CUDA(attrs([] {
+      cudaError_t e = cudaFuncSetAttribute(latent_attn_split_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      return e != cudaSuccess ? e : cudaFuncSetAttribute(latent_attn_split_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    }));
     const dim3 grid(p.n_tok, p.nsplit);
     LatentRun q = p;
     const size_t al = dtype == B200_F32 ? 32 : 16;

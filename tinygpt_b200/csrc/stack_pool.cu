@@ -633,16 +633,15 @@ int launch_pool_attention(const PoolAttn& p, int dtype, cudaStream_t st) {
                  "pool attention: bad workspace");
   const size_t sm_q = (size_t)H * dk * 4, sm_v = (size_t)(2 * H + 2 * H * (kPoolTile + 1) + H * dv) * 4;
   B200_CHECK_ARG(sm_q <= 200 * 1024 && sm_v <= 200 * 1024, "pool attention: heads · head size exceeds one CTA's shared memory");
-  static bool attr_done = false;
-  if (!attr_done) {
-    B200_CUDA(cudaFuncSetAttribute(pool_scores_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    B200_CUDA(cudaFuncSetAttribute(pool_scores_kernel<__nv_bfloat16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    B200_CUDA(cudaFuncSetAttribute(pool_scores_kernel<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    B200_CUDA(cudaFuncSetAttribute(pool_values_kernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    B200_CUDA(cudaFuncSetAttribute(pool_values_kernel<__nv_bfloat16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    B200_CUDA(cudaFuncSetAttribute(pool_values_kernel<__nv_bfloat16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr_done = true;
-  }
+  static PerDevice attrs;
+  B200_CUDA(attrs([] {
+    cudaError_t e = cudaFuncSetAttribute(pool_scores_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(pool_scores_kernel<__nv_bfloat16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(pool_scores_kernel<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(pool_values_kernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(pool_values_kernel<__nv_bfloat16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(pool_values_kernel<__nv_bfloat16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  }));
   const dim3 grid(p.n_tok, p.nsplit);
   const bool kvec = dtype == B200_BF16 && dk % 8 == 0 && p.k_slot_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(p.kcache) & 15) == 0;
   const bool vvec = dtype == B200_BF16 && dv % 2 == 0 && p.v_slot_stride % 2 == 0 && (reinterpret_cast<uintptr_t>(p.vcache) & 3) == 0;

@@ -510,11 +510,8 @@ template <int KS>
 int launch_stats(const PoolMma& m, int n_seg, int max_count, cudaStream_t st) {
   constexpr int smem = 3 * 64 * (KS * 32 + 16);
   if (smem > 48 * 1024) {
-    static bool attr_done = false;
-    if (!attr_done) {
-      B200_CUDA(cudaFuncSetAttribute(pool_stats_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      attr_done = true;
-    }
+    static PerDevice attrs;
+    B200_CUDA(attrs([] { return cudaFuncSetAttribute(pool_stats_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); }));
   }
   const dim3 grid((max_count + kStM - 1) / kStM, m.p.a.heads, n_seg);
   B200_CUDA(launch_pdl(pool_stats_kernel<KS>, grid, dim3(128), (size_t)smem, st, false, m));
@@ -525,11 +522,8 @@ template <int HPW, int KS>
 int launch_mix(PoolMma m, int n_seg, int max_count, cudaStream_t st) {
   using SH = MixShape<HPW>;
   const b200_attn_desc& a = m.p.a;
-  static bool attr_done = false;
-  if (!attr_done) {
-    B200_CUDA(cudaFuncSetAttribute(pool_mix_kernel<HPW, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    attr_done = true;
-  }
+  static PerDevice attrs;
+  B200_CUDA(attrs([] { return cudaFuncSetAttribute(pool_mix_kernel<HPW, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); }));
   const int splits = (a.vdim + SH::NT * 8 - 1) / (SH::NT * 8);
   m.vcols = ((a.vdim + splits - 1) / splits + 15) / 16 * 16;
   m.kstages = mix_smem(a.heads, a.kv_heads, a.dim, m.vcols, 2, SH::WBYTES, SH::XBYTES) <= 227 * 1024 ? 2 : 1;

@@ -322,8 +322,8 @@ __global__ void __launch_bounds__(NT, RS <= 8 ? 512 / NT : 2) lin_scan_cols_kern
 template <int RS, int NT, int MODE, bool SCALAR>
 int launch_scan_cols(const LinScan& p, cudaStream_t st) {
   constexpr int smem = ScanCols<RS, NT, SCALAR>::smem;
-  static cudaError_t attr = cudaFuncSetAttribute(lin_scan_cols_kernel<RS, NT, MODE, SCALAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  B200_CUDA(attr);
+  static PerDevice attrs;
+  B200_CUDA(attrs([] { return cudaFuncSetAttribute(lin_scan_cols_kernel<RS, NT, MODE, SCALAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); }));
   auto al = [](const float* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   const bool wide = p.dk % 4 == 0 && p.ld % 4 == 0 && al(p.b) && al(p.r) && (SCALAR || al(p.d));
   const dim3 grid(p.n_seg, p.heads, (p.dv + kScanCols - 1) / kScanCols);
@@ -731,8 +731,8 @@ __global__ void __launch_bounds__(kRemThreads, (ScanRem<LN, RPL, C, SCALAR>::CTA
 template <int LN, int RPL, int C, bool SCALAR>
 int launch_scan_rem(const LinScan& p, cudaStream_t st) {
   using F = ScanRem<LN, RPL, C, SCALAR>;
-  static cudaError_t attr = cudaFuncSetAttribute(lin_scan_rem_kernel<LN, RPL, C, SCALAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem);
-  B200_CUDA(attr);
+  static PerDevice attrs;
+  B200_CUDA(attrs([] { return cudaFuncSetAttribute(lin_scan_rem_kernel<LN, RPL, C, SCALAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::smem); }));
   const bool wide = p.dk % 4 == 0 && p.ld % 4 == 0 && aligned16(p.b, p.r, p.p, p.q) && (SCALAR || aligned16(p.d));
   const dim3 grid(p.n_seg, p.heads, (p.dv + F::COLS - 1) / F::COLS);
   B200_CUDA(launch_pdl(lin_scan_rem_kernel<LN, RPL, C, SCALAR>, grid, dim3(kRemThreads), F::smem, st, stack_pdl(), p, wide));
@@ -1571,12 +1571,11 @@ int run_gdelta(const GatedDeltaRun& p, int dtype, cudaStream_t st) {
   const size_t smem = (size_t)(2 * dk + (H / G) * dv) * 4;
   B200_CHECK_ARG(smem <= 200 * 1024, "gated delta rule: the channels of one query / key head and its value heads exceed one CTA's shared memory");
   if (smem > 48 * 1024) {
-    static bool attr_done = false;
-    if (!attr_done) {
-      B200_CUDA(cudaFuncSetAttribute(gdelta_prep_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      B200_CUDA(cudaFuncSetAttribute(gdelta_prep_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      attr_done = true;
-    }
+    static PerDevice attrs;
+    B200_CUDA(attrs([] {
+      cudaError_t e = cudaFuncSetAttribute(gdelta_prep_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      return e != cudaSuccess ? e : cudaFuncSetAttribute(gdelta_prep_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    }));
   }
   const dim3 pg(p.scan.n_tok, G);
   if (dtype == B200_F32) B200_CUDA(launch_pdl(gdelta_prep_kernel<float>, pg, dim3(256), smem, st, stack_pdl(), p));
