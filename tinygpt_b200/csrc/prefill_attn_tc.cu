@@ -989,16 +989,29 @@ bool prefill_attn_tc_ok(const TcPrefillAttn& a, int hd) {
          a.q_bs % 8 == 0 && a.kv_rs % 8 == 0 && a.kv_bs % 8 == 0 && a.o_rs % 8 == 0 && a.o_bs % 8 == 0;
 }
 // Whether this kernel beats the mma.sync one: where a block of 64 rows, that one's, walks enough tiles of 64 keys, or fewer in more blocks than that one
-// runs at once.  µs here / there: 16 heads of 128, one sequence 128 rows (two tiles) 5.3 / 5.5, 160 rows 6.3 / 6.6, 256 rows 6.8 / 8.2; 24 heads, two
-// sequences of 128 rows (96 blocks) 5.4 / 6.8; 14 heads of 64, one, two and four sequences: 160 rows (three) 5.4 / 4.6, 5.4 / 5.1, 6.0 / 6.2 (168 blocks),
-// 192 rows 5.4 / 4.9, 5.5 / 5.4, 6.0 / 6.9, 256 rows 5.6 / 5.8, 5.6 / 7.3, 6.2 / 8.8; 32 heads of 64, four sequences: 128 rows (256 blocks) 5.1 / 6.0, 160 rows
-// (384) 7.7 / 7.4.
+// runs at once.  µs here / there, calls back to back:
+//   heads of 128  one sequence of 16: 64 rows 4.9 / 4.0, 100 rows (two tiles, 32 blocks) 5.1 / 5.1, 128 rows 5.2 / 5.4, 160 rows 6.3 / 6.4, 192 rows 6.4 / 6.8, 256 rows
+//                 6.7 / 8.1; two of 32, 100 rows (128 blocks) 5.2 / 6.9
+//   heads of 64   14 heads, one, two, four and eight sequences: 160 rows (three tiles) 5.3 / 4.6, 5.4 / 5.1, 6.0 / 6.5 (168 blocks), 7.6 / 7.3 (336 blocks), 192 rows
+//                 5.4 / 4.9, 5.5 / 5.3, 6.1 / 6.9, 7.7 / 7.9, 200 rows (four) 5.4 / 5.3, 5.6 / 6.7, 6.1 / 8.3, 7.7 / 8.7; 32 heads, four sequences: 128 rows (256
+//                 blocks) 4.9 / 6.0, 160 rows (384) 7.7 / 7.3, 192 rows 7.8 / 7.7
+// In a captured graph, where nothing overlaps, short prompts lose up to 0.6 µs here (14 heads of 64 over 200 rows 6.0 / 5.4, 16 of 128 over 160 6.8 / 6.6): a call has the same bits
+// either way, so the rule does not ask.
+// With a window, heads of 64 stay with the other kernel where a block there walks as few tiles, of half as many keys, or where its blocks just fill the SMs and those here
+// begin a second round (µs a layer of such heads, here / there: window of 64, 24 heads over 1 024 rows 42.8 / 40.0, 14 over 2 048 43.7 / 42.7, 8 over 2 048 35.0 /
+// 33.9; of 64 behind 4 kept keys 14 over 2 048 46.7 / 42.9; of 100 behind 4, 384 blocks 44.0 / 44.2, 448 blocks 46.5 / 45.0,
+// 512 blocks 47.1 / 50.1; of 130 behind 64, 384 blocks 44.0 / 46.1, 448 blocks 49.0 / 46.7).  From six tiles on there is hardly a
+// loss: a window of 256, 448 blocks 49.5 / 49.1, 384 blocks 43.8 / 48.2.  Heads of 128, window of 16: 512 blocks 52.5 / 56.7, 128 blocks 33.5 / 34.5 and 39.9 / 38.9.
 bool prefill_attn_tc_wins(const TcPrefillAttn& a, int hd, int rows) {
-  const int last = (rows - 1) / 64 * 64;   // first row of the last block
-  const int edge = a.window > 0 ? std::max(0, last - a.window + 1) / 64 : 0;
-  const int tiles = last / 64 + 1 - edge + (a.window > 0 ? std::min(edge, (a.keep_first + 63) / 64) : 0);
-  const int64_t blocks = (int64_t)a.B * a.Hq * (last / 64 + 1);
-  return hd == 128 ? tiles >= 3 || (tiles == 2 && blocks > 74) : tiles >= 4 || (tiles >= 2 && blocks > 148 && (tiles == 2 || blocks <= 296));
+  auto tiles_of = [&](int n) {   // of the last block of n rows, n keys each
+    const int last = (rows - 1) / n * n, edge = a.window > 0 ? std::max(0, last - a.window + 1) / n : 0;
+    return last / n + 1 - edge + (a.window > 0 ? std::min(edge, (a.keep_first + n - 1) / n) : 0);
+  };
+  const int tiles = tiles_of(64);
+  const int64_t blocks = (int64_t)a.B * a.Hq * ((rows - 1) / 64 + 1);
+  if (hd == 128) return tiles >= 3 || (tiles == 2 && blocks > 74);
+  const bool enough = tiles >= 4 || (tiles >= 2 && blocks > 148 && (tiles == 2 || blocks <= 296));
+  return enough && (a.window == 0 || tiles >= 6 || (tiles > tiles_of(128) && (blocks <= 384 || blocks > 448)));
 }
 int launch_prefill_attn_tc(const TcPrefillAttn& a, int hd, cudaStream_t st) {
   return hd == 64 ? launch_tc<64>(a, st) : launch_tc<128>(a, st);
