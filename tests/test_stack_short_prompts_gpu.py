@@ -1,6 +1,6 @@
 """Layer-stack prompts of 9 to 31 rows, whose products run on the tcgen05 GEMM like those of longer ones: portions of such lengths give the bits of the whole
-prompt (attention takes one kernel from 16 rows on), and results agree with the general kernels' to the bf16 roundings of a few layers; a
-matrix off the 16-byte boundary stays with the general kernel."""
+prompt (attention takes one kernel from 16 rows on), and results agree with the general kernels' to the bf16 roundings of a few layers; matrices
+off the 16-byte boundary stay with the general kernel, those of the side input in a narrow model at any length."""
 import pytest
 import torch
 
@@ -41,3 +41,36 @@ def test_against_the_general_kernels(built_lib, monkeypatch, rows):
         out.append(eng.forward(_ids(rows), True).double())
         eng.close()
     assert float((out[0] - out[1]).norm() / out[1].norm()) < 1e-2
+
+
+def _off_boundary(w, name):
+    t = w[name]
+    room = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+    return {**w, name: room[1:1 + t.numel()].copy_(t.view(-1)).view(t.shape)}
+
+
+@pytest.mark.parametrize("name", ["l0.w_in", "l1.w_out"])
+@pytest.mark.parametrize("rows", [9, 16, 31])
+def test_matrix_off_the_boundary(built_lib, name, rows):
+    w = stack_bench.device_stack_weights(_spec(), torch.device(DEV), 5)
+    out = []
+    for weights in (w, _off_boundary(w, name)):
+        eng = engine.DecodeEngine(_spec(), weights)
+        out.append(eng.forward(_ids(rows), True).double())
+        eng.close()
+    assert float((out[0] - out[1]).norm() / out[0].norm()) < 1e-2
+
+
+@pytest.mark.parametrize("rows", [4, 9, 31, 32, 40])
+def test_side_input_of_a_narrow_model_off_the_boundary(built_lib, rows):
+    """Width 32: the side input's first product has too few columns for the GEMM, its second one has enough."""
+    attn = models.AttnSpec(2, 2, 16, 16, 0.25, 0, 0)
+    spec = models.StackSpec(name="s", architecture="Kozusun", width=32, vocab=500, layers=(models.StackLayerSpec(attn, 64),) * 2, embed_scale=4.0,
+                            residual_mult=0.5, norm_eps=1e-5, norm_offset=1.0, max_ctx=64, max_slots=1, side_dim=64)
+    w = stack_bench.device_stack_weights(spec, torch.device(DEV), 6)
+    out = []
+    for weights in (w, _off_boundary(w, "l0.side_proj")):
+        eng = engine.DecodeEngine(spec, weights)
+        out.append(eng.forward(_ids(rows), True).double())
+        eng.close()
+    assert float((out[0] - out[1]).norm() / out[0].norm()) < 1e-2

@@ -561,7 +561,7 @@ static int stack_side(StackEngine* s, int li, float* cur, int n_tok, cudaStream_
   g.epi = SEPI_ACT_TABLE; g.c = s->sg; g.ldc = sd;
   g.table = d.side_table; g.tok = s->m_tok; g.table_ld = d.side_stride; g.table_col = L.side_col;
   if ((rc = launch_stack_gemm(g, s->dtype, st)) != B200_OK) return rc;
-  if (product_ok(s, n_tok, W, sd, L.side_proj)) {
+  if (product_ok(s, n_tok, W, sd, L.side_proj) && aligned16(L.side_proj)) {   // here longer steps have the general kernel, too
     if ((rc = launch_gemm_bf16_f32(s->y, s->sg, L.side_proj, nullptr, n_tok, W, sd, st)) != B200_OK) return rc;
     return launch_stack_rms_add(cur, s->y, L.side_norm, n_tok, W, d.norm_eps, d.residual_mult, st);
   }
