@@ -1,6 +1,6 @@
-"""The two forms of the tcgen05 prompt attention — a CTA per 128 rows of a head, and a cluster of two that share the key tiles — against fp64 at
-the edges of their tiles.  Up to 148 blocks of 128 rows take two CTAs, more take one; P and the result are bf16 (2-norm error below 2⁻⁸
-of the result's, each element within 2⁻⁷ of the largest |V|)."""
+"""The two kernels of the tcgen05 prompt attention — one for up to 128 keys, a CTA per block of 128 rows, and one whose CTAs, one per SM, run through blocks with
+tiles of 128 keys that two groups of warps take in turn — against fp64 at the edges of their tiles, with as many blocks as CTAs and a few more; P and
+the result are bf16 (2-norm error below 2⁻⁸ of the result's, each element within 2⁻⁷ of the largest |V|)."""
 import pytest
 import torch
 
@@ -10,7 +10,7 @@ from tinygpt_b200 import engine, models, ops, stack_bench
 pytestmark = pytest.mark.gpu
 
 
-# sequences · heads · ceil(rows / 128): up to 148 take two CTAs per block, more take one; one tile of 64 keys, an odd and an even number of them
+# sequences · heads · ceil(rows / 128) blocks: some 148, one for each CTA, and a second for two of them; one to five tiles of 128 keys, the last one full or not
 @pytest.mark.parametrize("B,S,Hq,Hkv", [(1, 1, 150, 10), (1, 64, 160, 8), (3, 65, 64, 8), (1, 129, 74, 37), (1, 129, 75, 25), (2, 192, 40, 8), (1, 200, 80, 16),
                                         (1, 385, 37, 1), (1, 385, 38, 19), (1, 577, 32, 4)])
 @pytest.mark.parametrize("D", [64, 128])
@@ -39,12 +39,17 @@ def test_what_a_row_does_not_see(built_lib, monkeypatch, D, heads):
 
 @pytest.mark.parametrize("D", [64, 128])
 def test_keys_without_a_number(built_lib, monkeypatch, D):
-    """Scores that are all NaN in the tiles of one parity and finite in the others': the row is NaN, not what the other half holds."""
+    """Scores that are NaN in part of a tile, and in the whole of a tile, which is all that one of the two groups has for the rows of one block (it has no maximum, and a
+    sum that is NaN): a row that sees one is NaN, not what the other group holds, and no other row is."""
     monkeypatch.setenv("B200_ATTN_TC", "tc")
-    q, k, v = randn(1, 200, 2, D, seed=7), randn(1, 200, 2, D, seed=8), randn(1, 200, 2, D, seed=9)
-    k[0, 64:128] = float("nan")
-    got = ops.flash_attention(q, k, v, True).float()
-    assert bool(torch.isfinite(got[0, :64]).all()) and bool(got[0, 64:].isnan().all())
+    for S, a, b in ((200, 64, 128), (400, 0, 128), (400, 128, 256), (500, 256, 384), (700, 128, 256)):
+        q, k, v = randn(1, S, 2, D, seed=7), randn(1, S, 2, D, seed=8), randn(1, S, 2, D, seed=9)
+        want = attend(q, k, v)
+        k[0, a:b] = float("nan")
+        got = ops.flash_attention(q, k, v, True)
+        if a > 0:
+            close(got[:, :a], want[:, :a], float(v.float().abs().max()))
+        assert bool(got[0, a:].isnan().all())
 
 
 @pytest.mark.parametrize("heads,window,keep", [(16, 0, 0), (16, 130, 5), (16, 65, 64), (6, 300, 70), (6, 1, 0)])

@@ -1,4 +1,4 @@
-"""Prefill attention on tcgen05 (csrc/prefill_attn_tc.cu) against fp64 softmax attention at the edges of its tiles: row counts around 64 and 128,
+"""Prompt attention on tcgen05 (csrc/prefill_attn_tc.cu) against fp64 softmax attention at the edges of its tiles: row counts around 64 and 128,
 both head sizes, grouped heads, batches, cached prefixes, windows with kept first keys, and infinities in keys and values that a row does
 not see.  P and the result are bf16: 2-norm error below 2⁻⁸ of the result's, each element within 2⁻⁷ of the largest |V|."""
 import pytest
@@ -40,11 +40,11 @@ def test_causal(built_lib, monkeypatch, B, S, Hq, Hkv, D):
     assert torch.equal(got, ops.flash_attention(q, k, v, True))
 
 
-@pytest.mark.parametrize("S", [65, 129, 150, 192, 321, 449])
+@pytest.mark.parametrize("S", [65, 129, 150, 192, 256, 321, 449])
 @pytest.mark.parametrize("D", [64, 128])
 def test_last_tile_sees_part_of_the_block(built_lib, monkeypatch, S, D):
-    """The result is read after the products of the last two key tiles, also where no softmax warp has waited for either: S % 128 in 1 … 64 (the
-    tile before the last is visible as a whole), maxima in the first tile (no rescale), two blocks beside each other on every SM."""
+    """The result is read after the products of a block's last tiles, also where no warp has waited for them to rescale: maxima in the first tile; last tiles of one key, of
+    half of them and of all; up to eleven blocks to a CTA, the next of which is under way while one is stored."""
     monkeypatch.setenv("B200_ATTN_TC", "tc")
     q, k, v = randn(4, S, 96, D, seed=11), randn(4, S, 96, D, seed=12), randn(4, S, 96, D, seed=13)
     q, k[:, 0] = q.abs(), 6.0 * D ** -0.5   # key 0: a score of about five, the others' stay below four
