@@ -240,8 +240,8 @@ __device__ __forceinline__ bool part_not_finite(const TcAttn& p, const Block& w,
 }
 
 // The way out for such a block: this warp's 32 rows, each over the keys that it sees and no others (weights rounded to bf16 like above).  A row's scores go to
-// the lanes, 32 keys at a time, once for its maximum and sum and once for its weights; its columns to the lanes, key after key.  Slow and rare: 32 rows
-// over 300 000 keys take 1.7 s (heads of 64: 0.86 s), bound by the latency of loads.
+// the lanes, 32 keys at a time, its columns to the lanes, key after key.  Slow and rare: 32 rows over 300 000 keys take 1.6 s (heads of 64: 0.92 s), bound by the
+// latency of loads; kept small, since a call also pays for code that it only jumps over.
 template <int HD>
 __device__ __forceinline__ void see_alone(const TcAttn& p, const Block& w, int quarter, int lane) {
   constexpr int E = HD / 32;   // columns of a lane
@@ -255,7 +255,7 @@ __device__ __forceinline__ void see_alone(const TcAttn& p, const Block& w, int q
       if (j > rpos || (p.window > 0 && rpos - j >= p.window && j >= p.keep_first)) return false;
       const __nv_bfloat16* const k = p.kp + kv + (size_t)j * p.kv_rs;
       s = 0.f;
-#pragma unroll 4
+#pragma unroll 2
       for (int d = 0; d < HD; d += 8) {
         float x[8];
         unpack8(*reinterpret_cast<const uint4*>(q + d), x);
@@ -264,50 +264,46 @@ __device__ __forceinline__ void see_alone(const TcAttn& p, const Block& w, int q
       return true;
     };
     // the keys behind the kept ones and in front of the window are passed over, 32 at a time
-    const int edge = p.window > 0 ? max(0, rpos - p.window + 1) & ~31 : 0;
-    auto next = [&](int j0) { return j0 + 32 >= p.keep_first && j0 + 32 < edge ? edge : j0 + 32; };
-    const int from = p.keep_first > 0 ? 0 : edge;
-    float m = -INFINITY, l = 0.f;
-#pragma unroll 1
-    for (int j0 = from; j0 <= rpos; j0 = next(j0)) {
-      float s;
-      if (!score(j0 + lane, s)) continue;
-      const float top = fmaxf(m, s), ms = top == -INFINITY ? 0.f : top * p.scale_log2;
-      l = l * (m == -INFINITY ? 1.f : ex2f((m - top) * p.scale_log2)) + ex2f(fmaf(s, p.scale_log2, -ms));
-      m = top;
-    }
-    const float mine = m;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    l *= mine == -INFINITY ? 1.f : ex2f((mine - m) * p.scale_log2);
-    l = warp_sum(l);
-    const float ms = m == -INFINITY ? 0.f : m * p.scale_log2;
-    float acc[E];
+    const int edge = p.window > 0 ? max(0, rpos - p.window + 1) & ~31 : 0, from = p.keep_first > 0 ? 0 : edge;
+    float m = -INFINITY, l = 0.f, acc[E];   // the maximum so far; of this lane's keys; of its columns
 #pragma unroll
     for (int e = 0; e < E; ++e) acc[e] = 0.f;
 #pragma unroll 1
-    for (int j0 = from; j0 <= rpos; j0 = next(j0)) {
-      float s = 0.f;
+    for (int j0 = from; j0 <= rpos; j0 = j0 + 32 >= p.keep_first && j0 + 32 < edge ? edge : j0 + 32) {
+      float s = -INFINITY;
       const bool sees = score(j0 + lane, s);
-      const float weight = round_bf16(ex2f(fmaf(s, p.scale_log2, -ms)));
+      float top = fmaxf(m, s);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      if (top != m) {
+        const float f = m == -INFINITY ? 1.f : ex2f((m - top) * p.scale_log2);
+        l *= f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[e] *= f;
+        m = top;
+      }
+      const float weight = sees ? ex2f(fmaf(s, p.scale_log2, m == -INFINITY ? 0.f : -m * p.scale_log2)) : 0.f;
+      l += weight;
+      const float rounded = round_bf16(weight);
       const unsigned seen = __ballot_sync(0xffffffffu, sees);
       const __nv_bfloat16* const v = p.vp + kv + (size_t)j0 * p.kv_rs + lane * E;
       auto add = [&](int j) {
-        const float x = __shfl_sync(0xffffffffu, weight, j);
+        const float x = __shfl_sync(0xffffffffu, rounded, j);
         uint32_t y[E / 2];
         if constexpr (E == 4) *reinterpret_cast<uint2*>(y) = *reinterpret_cast<const uint2*>(v + (size_t)j * p.kv_rs);
         else y[0] = *reinterpret_cast<const uint32_t*>(v + (size_t)j * p.kv_rs);
 #pragma unroll
         for (int e = 0; e < E; ++e) acc[e] = fmaf(x, __uint_as_float(e & 1 ? y[e / 2] & 0xffff0000u : y[e / 2] << 16), acc[e]);
       };
-      if (seen == 0xffffffffu) {   // sixteen loads in flight
-#pragma unroll 16
+      if (seen == 0xffffffffu) {
+#pragma unroll 8
         for (int j = 0; j < 32; ++j) add(j);
       } else {
 #pragma unroll 1
         for (unsigned left = seen; left != 0; left &= left - 1) add(__ffs(left) - 1);
       }
     }
+    l = warp_sum(l);
     if (p.sink && m != -INFINITY) l += ex2f(-m * p.scale_log2);
     const float gate = p.gate != nullptr ? 1.f / (1.f + expf(-bf16_to_f(p.gate[(size_t)w.b * p.q_bs + (size_t)r * p.q_rs + w.h]))) : 1.f;
     const float inv = (l > 0.f ? 1.f / l : 0.f) * gate;
